@@ -38,7 +38,10 @@ template <class R>
 struct Bulk {
     R *Fcons, *Fmx, *Fmy, *Fmz;   // slow right-hand sides
     R *avx, *avy, *avz;           // average momenta of the substeps
-    R* lag[2];                    // lagged d(rho theta), ping-pong
+    R* lag[2];                    // lagged d(rho theta) (flat: the extrapolated one), ping-pong
+    SubCoef<R> sc{};              // flat substeps: the stage's coefficients,
+    R *du[2], *dv[2], *dw[2];     // the momentum increments, ping-pong,
+    double *dr, *drt;             // and the deviations of rho and rho theta
     StageAux<R> aux[2];           // stage primitives, Exner, p'
     R* mut;                       // eddy viscosity
     R *t11, *t22, *t33, *t12, *t13, *t23;
@@ -48,11 +51,6 @@ struct Bulk {
     TkeBuf<R> tke{nullptr, nullptr, nullptr, nullptr}; // Deardorff closure arrays
     TerBuf<R> ter{};                                    // static terrain scratch
 };
-
-// Threads per block of the vertical acoustic kernel (columns x level groups).
-#ifndef ERFB_VERT_THREADS
-#define ERFB_VERT_THREADS 1024
-#endif
 
 struct erf_b200_ctx {
     erf_b200_config cfg;
@@ -68,6 +66,9 @@ struct erf_b200_ctx {
     int device = 0;
     size_t bytes = 0;
     std::vector<void*> allocs;
+    struct Want { void** p; size_t bytes; };
+    std::vector<Want> wants;   // arrays asked for while erf_b200_create collects them
+    bool collect = false;
 
     StateBuf S[4];            // [0],[1] alternate old/new, [2] second stage buffer, [3] fast sum
     double* vel[2][3];        // alternating old/new face velocities (FP64 prognostic)
@@ -82,9 +83,10 @@ struct erf_b200_ctx {
     int closure_grid = 1;
     double* feat_theta = nullptr;        // feature extraction scratch
     float* feat_out = nullptr;
-    int tile_tx = 32, vert_warps = 32, coef_warps = 8;
+    int tile_tx = 32, coef_warps = 8;   // k_fast_coef: columns and warps per block
     TiledKz tkz{1, 1, 1};
-    size_t vert_smem = 0, coef_smem = 0;
+    size_t coef_smem = 0;
+    SubShape sub;                       // flat substeps
     double *r0, *p0, *pi0, *th0;   // nz+2 values, or (nz+2) planes with terrain
     double *znd = nullptr, *detJ = nullptr, *zcc = nullptr;   // static terrain
     double* met = nullptr;                                    // its metric tables
@@ -130,8 +132,16 @@ int cuda_fail(cudaError_t e) {
         if (e_ != cudaSuccess) return cuda_fail(e_); \
     } while (0)
 
+// A zeroed device array of the context.  While erf_b200_create collects
+// (c->collect) the request is noted and commit_allocs makes one allocation of
+// all of them: an array at a time costs about 0.3 ms each.
 template <class T>
 int dalloc(erf_b200_ctx* c, T** p, size_t n) {
+    if (c->collect) {
+        *p = nullptr;
+        c->wants.push_back({reinterpret_cast<void**>(p), n * sizeof(T)});
+        return ERF_B200_OK;
+    }
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, n * sizeof(T));
     if (e != cudaSuccess) return cuda_fail(e);
@@ -139,6 +149,25 @@ int dalloc(erf_b200_ctx* c, T** p, size_t n) {
     c->allocs.push_back(q);
     c->bytes += n * sizeof(T);
     *p = (T*)q;
+    return ERF_B200_OK;
+}
+int commit_allocs(erf_b200_ctx* c) {
+    c->collect = false;
+    const auto padded = [](size_t n) { return (n + 511) / 512 * 512; };   // cudaMalloc's own alignment and more
+    size_t total = 0;
+    for (const auto& w : c->wants) total += padded(w.bytes);
+    void* q = nullptr;
+    cudaError_t e = cudaMalloc(&q, total);
+    if (e != cudaSuccess) return cuda_fail(e);
+    c->allocs.push_back(q);
+    cudaMemsetAsync(q, 0, total, c->stream);
+    char* at = static_cast<char*>(q);
+    for (const auto& w : c->wants) {
+        *w.p = at;
+        at += padded(w.bytes);
+        c->bytes += w.bytes;
+    }
+    c->wants.clear();
     return ERF_B200_OK;
 }
 
@@ -548,6 +577,25 @@ void enqueue_step_mt(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
     launch_mt_advance_time(st, c->mt.time, dt);
 }
 
+// Arguments of a flat substep: deviations read from one set of buffers and
+// written to the other (`flip` swaps them).
+template <class R>
+SubArgs<R> sub_args(const Geo& g, Bulk<R>& B, StateBuf old, StateBuf st, StateBuf sum, StageAux<R> A, double dtau,
+                    double facinv, int flip) {
+    SubArgs<R> a{};
+    a.dtau = dtau; a.facinv = facinv; a.b1 = 0.5 * (1.0 - 0.1); a.b2 = 0.5 * (1.0 + 0.1);
+    a.old = old; a.st = st; a.sum = sum;
+    a.th = A.prim;
+    a.Fr = B.Fcons; a.Ft = B.Fcons + g.ncell; a.Fmx = B.Fmx; a.Fmy = B.Fmy; a.Fmz = B.Fmz;
+    a.fx = B.sc.fx; a.fy = B.sc.fy; a.cE = B.sc.E; a.cG = B.sc.G; a.cI = B.sc.I; a.cP = B.sc.P; a.cQ = B.sc.Q;
+    a.ui = B.du[1 - flip]; a.vi = B.dv[1 - flip]; a.wi = B.dw[1 - flip]; a.ei = B.lag[1 - flip];
+    a.uo = B.du[flip]; a.vo = B.dv[flip]; a.wo = B.dw[flip]; a.eo = B.lag[flip];
+    a.dr = B.dr; a.drt = B.drt;
+    a.avx = B.avx; a.avy = B.avy; a.avz = B.avz;
+    a.grad = 1;
+    return a;
+}
+
 // Enqueue one full step with parity p (state slot p is the old state).
 template <class R>
 void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
@@ -572,13 +620,9 @@ void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
     StateBuf outs[3] = {N0, N1, N0};
     if (P.moist) { outs[0] = N1; outs[1] = N0; outs[2] = N1; }
     StateBuf stage[3] = {OLD, outs[0], outs[1]};
-    dim3 tb(c->tile_tx, c->vert_warps, 1), tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1);
-    dim3 tcb(c->tile_tx, c->coef_warps, 1);
     const bool fork = T == nullptr && c->side;   // per-kernel timing keeps one stream
     int a = 0;
-    int lp = (p * c->lag_parity_per_step) & 1;
-    const double beta_s = 0.1;
-    const double beta_1 = 0.5 * (1.0 - beta_s), beta_2 = 0.5 * (1.0 + beta_s);
+    const double beta_2 = 0.5 * (1.0 + 0.1);
     const bool nosub = no_substepping(c->cfg);
     for (int nrk = 0; nrk < 3; ++nrk) {
         StateBuf Sst = stage[nrk], Snew = outs[nrk];
@@ -595,8 +639,7 @@ void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
                 launch_plane_avg<R>(P, c->side, Sst.cons, Acur.prim, c->pavg);
                 cudaEventRecord(c->ev_pavg, c->side);
             }
-            if (!nosub)
-                launch_fast_coef<R>(P, c->side, tg, tcb, c->coef_smem, D, Sst, Acur, B.cA, B.cInvB, B.cCB, B.cP, B.cQ);
+            if (!nosub) launch_sub_coef<R>(P, c->side, c->sub, D, Sst, Acur, B.sc);
             cudaEventRecord(c->ev_coef, c->side);
         }
         if (P.les == ERF_LES_MLP) {
@@ -608,8 +651,9 @@ void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
             TIMED(1, launch_tau<R>(P, st, Sst.cons, Vnew[0], Vnew[1], Vnew[2], B.mut, B.t11, B.t22, B.t33, B.t12,
                                    B.t13, B.t23));
         }
-        TIMED(2, launch_slow_cell<R>(P, c->tkz, st, Sst, Acur, B.mut, B.hx, B.hy, B.hz, B.tke, B.Fcons, B.avx,
-                                     B.avy, B.avz));
+        // (the first substep starts the average momenta itself)
+        TIMED(2, launch_slow_cell<R>(P, c->tkz, st, Sst, Acur, B.mut, B.hx, B.hy, B.hz, B.tke, B.Fcons,
+                                     nosub ? B.avx : nullptr, B.avy, B.avz));
         if (plane && !fork) TIMED(3, launch_plane_avg<R>(P, st, Sst.cons, Acur.prim, c->pavg));
         if (plane && fork) cudaStreamWaitEvent(st, c->ev_pavg, 0);
         TIMED(4, launch_slow_mom<R>(P, c->tkz, st, Sst, Acur, Vnew[0], Vnew[1], Vnew[2], B.t11, B.t22, B.t33, B.t12,
@@ -619,16 +663,11 @@ void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
         if (nosub)
             TIMED(10, launch_no_substep<R>(P, st, slow_dt, OLD, B.Fcons, B.Fmx, B.Fmy, B.Fmz, SUM));
         else if (!fork)
-            TIMED(9, launch_fast_coef<R>(P, st, tg, tcb, c->coef_smem, D, Sst, Acur, B.cA, B.cInvB, B.cCB, B.cP, B.cQ));
+            TIMED(9, launch_sub_coef<R>(P, st, c->sub, D, Sst, Acur, B.sc));
         for (int ks = 0; ks < (nosub ? 0 : nsub); ++ks) {
-            StateBuf Sprev = (ks == 0) ? OLD : SUM;
-            int prt = ks > 0;
-            TIMED(5, launch_fast_h<R>(P, st, ks, nrk, dtau, facinv, Sprev, prt, Sst, Acur, B.Fmx, B.Fmy, B.lag[lp],
-                                      B.lag[1 - lp], B.avx, B.avy, SUM.mx, SUM.my));
-            lp ^= 1;
-            TIMED(6, launch_fast_vert<R>(P, st, tg, tb, c->vert_smem, dtau, facinv, beta_1, beta_2, Sprev, prt, Sst,
-                                         Acur, B.Fcons, B.Fmz, SUM.mx, SUM.my, B.cA, B.cInvB, B.cCB, B.cP, B.cQ,
-                                         B.avz, SUM.cons, SUM.mz));
+            SubArgs<R> sa = sub_args<R>(g, B, OLD, Sst, SUM, Acur, dtau, facinv, ks & 1);
+            sa.av_init = ks == 0;
+            TIMED(6, launch_substep<R>(P, st, c->sub, ks > 0 ? 2 : (nrk > 0 ? 1 : 0), ks == nsub - 1, sa));
         }
         TIMED(7, launch_post<R>(P, c->tkz, st, slow_dt, OLD, Sst, SUM, Snew, Acur, Anext, nrk < 2 ? 1 : 0, B.mut,
                                 B.tke, B.avx, B.avy, B.avz, Vnew[0], Vnew[1], Vnew[2]));
@@ -659,7 +698,16 @@ int alloc_bulk(erf_b200_ctx* c, Bulk<R>& B) {
     for (int p = 0; p < 2; ++p) { A(&B.aux[p].prim, (nc - 1) * N); A(&B.aux[p].pi, N); A(&B.aux[p].pp, N); }
     A(&B.mut, N);
     A(&B.t11, N); A(&B.t22, N); A(&B.t33, N); A(&B.t12, N); A(&B.t13, NZF); A(&B.t23, NZF);
-    A(&B.cA, NZF); A(&B.cInvB, NZF); A(&B.cCB, NZF); A(&B.cP, NZF); A(&B.cQ, NZF);
+    if (cfg->use_terrain || !c->mixed) {   // (flat: the per-pass make_fast_coeffs only, plain form)
+        A(&B.cA, NZF); A(&B.cInvB, NZF); A(&B.cCB, NZF); A(&B.cP, NZF); A(&B.cQ, NZF);
+    }
+    if (!cfg->use_terrain && (!c->mixed || cfg->substepping_type == ERF_SUBSTEP_IMPLICIT)) {
+        A(&B.sc.fx, N); A(&B.sc.fy, N);
+        A(&B.sc.E, NZF); A(&B.sc.G, NZF); A(&B.sc.I, NZF); A(&B.sc.P, NZF); A(&B.sc.Q, NZF);
+        for (int q = 0; q < 2; ++q) { A(&B.du[q], N); A(&B.dv[q], N); A(&B.dw[q], NZF); }
+        auto D = [&](double** q, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, q, n); };
+        D(&B.dr, N); D(&B.drt, N);
+    }
     if (cfg->les_type == ERF_LES_MLP) {
         A(&B.c12, N); A(&B.c13, N); A(&B.c23, N); A(&B.hx, N); A(&B.hy, N); A(&B.hz, N);
     }
@@ -793,6 +841,7 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     const int nc = cfg->ncomp;
     int rc = ERF_B200_OK;
     auto A = [&](double** p, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, p, n); };
+    c->collect = true;
     for (int s = 0; s < 4; ++s) {
         A(&c->S[s].cons, nc * N); A(&c->S[s].mx, N); A(&c->S[s].my, N); A(&c->S[s].mz, NZF);
     }
@@ -810,14 +859,12 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
         A(&c->znd, (size_t)(cfg->nz + 3) * sk); A(&c->detJ, N); A(&c->zcc, (size_t)(cfg->nz + 1) * sk);
         A(&c->met, (size_t)TER_NMET * NZF);
         if (cfg->terrain_type == ERF_TERRAIN_MOVING) {
-            c->mt.z[0] = c->znd;
             A(&c->mt.z[1], (size_t)(cfg->nz + 3) * sk); A(&c->mt.z[2], (size_t)(cfg->nz + 3) * sk);
             A(&c->mt.met1, (size_t)TER_NMET * NZF); A(&c->mt.detJ1, N); A(&c->mt.zcc1, (size_t)(cfg->nz + 1) * sk);
             A(&c->mt.zt, NZF);
             A(&c->mt.r0o, (size_t)(cfg->nz + 2) * sk); A(&c->mt.p0o, (size_t)(cfg->nz + 2) * sk);
             A(&c->mt.time, 1);
             A(&c->mt.fac, (size_t)cfg->nz + 1);
-            if (rc == ERF_B200_OK) cudaMemsetAsync(c->mt.time, 0, sizeof(double), c->stream);
             if (cfg->substepping_type == ERF_SUBSTEP_IMPLICIT) {
                 A(&c->mt.z[3], (size_t)(cfg->nz + 3) * sk); A(&c->mt.z[4], (size_t)(cfg->nz + 3) * sk);
                 A(&c->mt.detJso, N); A(&c->mt.zpt, NZF); A(&c->mt.trhs, 2 * N); A(&c->mt.om, NZF);
@@ -825,6 +872,8 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
             }
         }
     }
+    if (rc == ERF_B200_OK) rc = commit_allocs(c);
+    c->mt.z[0] = c->znd;
     if (rc == ERF_B200_OK) {
         void* q = nullptr;
         if (cudaMalloc(&q, sizeof(int)) != cudaSuccess) rc = ERF_B200_ENOMEM;
@@ -851,23 +900,22 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     else tiled_setup<double>(c->P, &c->tkz);
     c->tkz.ter_post = !cfg->use_terrain ? 0 : (c->mixed ? ter_post_kz<float>(c->P) : ter_post_kz<double>(c->P));
     c->lag_parity_per_step = substeps_per_step(c->cfg) & 1;
-    // shared-memory tiles of the vertical kernels: TX columns x all levels
+    // shared-memory tiles of the column kernels: TX columns x all levels
     {
         const size_t max_smem = 227 * 1024;
         int nz = cfg->nz;
-        // the widest tile that fits: wide tiles read long contiguous rows
-        // (64 columns: 18 % faster than 32 in the mixed form, where it fits)
-        c->tile_tx = 64;
         const size_t rs = c->mixed ? sizeof(float) : sizeof(double);
+        if ((size_t)(7 * nz + 5) * 4 * rs > max_smem) rc = ERF_B200_ECONFIG;   // the deepest column that is taken
+        // k_fast_coef: wide tiles read long contiguous rows
+        c->tile_tx = 64;
         while (c->tile_tx > 4 && (size_t)(7 * nz + 5) * c->tile_tx * rs > max_smem) c->tile_tx /= 2;
-        c->vert_smem = (size_t)(7 * nz + 5) * c->tile_tx * rs;
         c->coef_smem = (size_t)3 * (nz + 1) * c->tile_tx * rs;
-        if (c->vert_smem > max_smem) rc = ERF_B200_ECONFIG;
-        c->vert_warps = ERFB_VERT_THREADS / c->tile_tx;
         c->coef_warps = c->tile_tx >= 32 ? 8 : 16;
-        if (rc == ERF_B200_OK) {
-            if ((c->mixed ? vert_setup<float>(c->vert_smem, c->coef_smem) : vert_setup<double>(c->vert_smem, c->coef_smem)) != 0)
-                rc = ERF_B200_ECUDA;
+        if (rc == ERF_B200_OK && (c->mixed ? coef_setup<float>(c->coef_smem) : coef_setup<double>(c->coef_smem)) != 0)
+            rc = ERF_B200_ECUDA;
+        if (rc == ERF_B200_OK && !cfg->use_terrain) {
+            c->sub = c->mixed ? sub_shape<float>(c->g) : sub_shape<double>(c->g);
+            if ((c->mixed ? sub_setup<float>(c->g, c->sub) : sub_setup<double>(c->g, c->sub)) != 0) rc = ERF_B200_ECUDA;
         }
         if (rc == ERF_B200_OK && cfg->use_terrain) {
             ter_vert_shape(nz, &c->ter_tx, &c->ter_smem);
@@ -1197,8 +1245,9 @@ int erf_b200_kernels_per_step(const erf_b200_ctx* c, int* launches) {
         int nsub; double a, b;
         stage_schedule(c->cfg, nrk, nsub, a, b);
         int stress = c->P.les == ERF_LES_MLP ? 2 : (c->P.use_diff ? (c->P.most ? 2 : 1) : 0);
-        // slow_cell, slow_mom, post + (fast_coeffs and 2 per substep, or the no-substep update)
-        int fast = no_substepping(c->cfg) ? 1 : 1 + 2 * nsub;
+        // slow_cell, slow_mom, post + (fast_coeffs and the substeps: one kernel each on a flat grid, two
+        // over terrain; or the no-substep update)
+        int fast = no_substepping(c->cfg) ? 1 : 1 + (c->P.ter ? 2 : 1) * nsub;
         n += 3 + fast + stress + ((c->P.moist && c->P.buoy_type == 2) ? 1 : 0);
     }
     *launches = n;
@@ -1413,9 +1462,13 @@ int fast_rhs_pass(erf_b200_ctx* c, bool terrain, int step, int nrk, const erf_b2
     if (step == 0) {
         // make_fast_coeffs at the stage's first substep (ERF_fast_rhs_N.cpp:60-70)
         launch_stage_aux<double>(P, st, Sst.cons, B.aux[0]);
-        dim3 tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1), tcb(c->tile_tx, c->coef_warps, 1);
         double D = dtau * dtau * kBeta2 * kBeta2 * g.dzi;
-        launch_fast_coef<double>(P, st, tg, tcb, c->coef_smem, D, Sst, B.aux[0], B.cA, B.cInvB, B.cCB, B.cP, B.cQ);
+        if (terrain) {
+            dim3 tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1), tcb(c->tile_tx, c->coef_warps, 1);
+            launch_fast_coef<double>(P, st, tg, tcb, c->coef_smem, D, Sst, B.aux[0], B.cA, B.cInvB, B.cCB, B.cP, B.cQ);
+        } else {
+            launch_sub_coef<double>(P, st, c->sub, D, Sst, B.aux[0], B.sc);
+        }
     }
     if (terrain) {
         launch_ter_fast_h<double>(P, st, step, dtau, facinv, Sprev, 0, Sst, B.aux[0], B.Fmx, B.Fmy, B.lag[0],
@@ -1424,12 +1477,12 @@ int fast_rhs_pass(erf_b200_ctx* c, bool terrain, int step, int nrk, const erf_b2
                                      B.aux[0], B.Fcons, B.Fmz, B.ter, B.cA, B.cInvB, B.cCB, B.cP, B.cQ, B.avz,
                                      OUT.cons, OUT.mz);
     } else {
-        launch_fast_h<double>(P, st, step, nrk, dtau, facinv, Sprev, 0, Sst, B.aux[0], B.Fmx, B.Fmy, B.lag[0],
-                              B.lag[1], B.avx, B.avy, OUT.mx, OUT.my);
-        dim3 tb(c->tile_tx, c->vert_warps, 1), tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1);
-        launch_fast_vert<double>(P, st, tg, tb, c->vert_smem, dtau, facinv, kBeta1, kBeta2, Sprev, 0, Sst, B.aux[0],
-                                 B.Fcons, B.Fmz, OUT.mx, OUT.my, B.cA, B.cInvB, B.cCB, B.cP, B.cQ, B.avz, OUT.cons,
-                                 OUT.mz);
+        // from the caller's previous state to a whole new state, with the caller's lagged d(rho theta)
+        SubArgs<double> sa = sub_args<double>(g, B, Sprev, Sst, OUT, B.aux[0], dtau, facinv, 0);
+        sa.grad = !(nrk == 0 && step == 0);
+        sa.lag_in = step == 0 ? nullptr : B.lag[0];
+        sa.lag_out = B.lag[1];
+        launch_substep<double>(P, st, c->sub, 1, true, sa);
     }
     if ((rc = unpack4(c, S_data, 2, OUT.cons, OUT.mx, OUT.my, OUT.mz))) return rc;
     if ((rc = unpack4(c, S_scratch, 0, nullptr, B.avx, B.avy, B.avz))) return rc;
@@ -1652,33 +1705,30 @@ int erf_b200_autotune(erf_b200_ctx* c, int reps, double* best_ms) {
     float best = 0.f;
     int rc = trial(best);
     const int nz = c->cfg.nz;
-    // vertical kernels: columns per block (smaller tiles let two blocks share
-    // an SM, overlapping one block's serial sweep with the other's loads) and
-    // threads per block
-    const size_t rs = c->mixed ? sizeof(float) : sizeof(double);
-    for (int tx : {c->tile_tx, c->tile_tx / 2}) {
-        for (int threads : {256, 512, 1024}) {
-            int vw = threads / tx;
-            if (rc || tx < 4 || vw < 1 || (tx == c->tile_tx && vw == c->vert_warps)) continue;
-            int keep_tx = c->tile_tx, keep_vw = c->vert_warps, keep_cw = c->coef_warps;
-            size_t keep_vs = c->vert_smem, keep_cs = c->coef_smem;
-            c->tile_tx = tx;
-            c->vert_warps = vw;
-            c->vert_smem = (size_t)(7 * nz + 5) * tx * rs;
-            c->coef_smem = (size_t)3 * (nz + 1) * tx * rs;
-            if (c->coef_warps * tx > 1024) c->coef_warps = 1024 / tx;
+    // flat substeps: columns per block (narrower tiles let more blocks share an
+    // SM, overlapping one block's serial sweep with the others' loads) and
+    // threads per block, then the coefficient kernel's threads
+    if (!c->P.ter && !no_substepping(c->cfg)) {
+        auto try_shape = [&](SubShape s) {
+            if (rc || s.tx < 4 || s.rows < 2 || s.coef_rows < 2 ||
+                (s.tx == c->sub.tx && s.rows == c->sub.rows && s.coef_rows == c->sub.coef_rows))
+                return;
+            if ((c->mixed ? sub_setup<float>(c->g, s) : sub_setup<double>(c->g, s)) != 0) return;
+            const SubShape keep = c->sub;
+            c->sub = s;
             float ms;
-            if (trial(ms) == ERF_B200_OK && ms < best) {
-                best = ms;
-            } else {   // slower, or not launchable: keep the previous shape
-                cudaGetLastError();
-                c->tile_tx = keep_tx; c->vert_warps = keep_vw; c->coef_warps = keep_cw;
-                c->vert_smem = keep_vs; c->coef_smem = keep_cs;
-            }
-        }
+            if (trial(ms) == ERF_B200_OK && ms < best) best = ms;
+            else { cudaGetLastError(); c->sub = keep; }   // slower, or not launchable
+        };
+        const SubShape s0 = c->sub;
+        for (int tx : {s0.tx, s0.tx / 2, s0.tx * 2})
+            for (int threads : {256, 512, 1024})
+                if (tx >= 4 && tx <= 32) try_shape({tx, threads / tx, 256 / tx});
+        for (int threads : {128, 512}) try_shape({c->sub.tx, c->sub.rows, threads / c->sub.tx});
     }
+    // the coefficient kernel of the terrain path
     for (int cw : {4, 8, 16}) {
-        if (rc || cw == c->coef_warps || cw * c->tile_tx > 1024) continue;
+        if (rc || !c->P.ter || cw == c->coef_warps || cw * c->tile_tx > 1024) continue;
         int keep = c->coef_warps;
         c->coef_warps = cw;
         float ms;

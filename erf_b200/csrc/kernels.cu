@@ -479,74 +479,6 @@ __device__ __forceinline__ R gatherz_most(const Params& P, const MostView& mv, i
 }
 
 // ---------------------------------------------------------------------------
-// Acoustic substep, horizontal part (ERF_fast_rhs_N.cpp:115-256): lagged
-// d(rho theta) and its forward extrapolation, explicit U'' / V'' update and
-// the average-momentum accumulation.  For substeps after the first, the
-// previous momenta are first passed through the momentum->velocity->momentum
-// round trip of apply_bcs (ERF_TI_fast_rhs_fun.H:183-189).  The increments
-// are perturbations about the stage state, formed in FP64 and carried in R;
-// the new momenta are accumulated in FP64.
-// ---------------------------------------------------------------------------
-template <class R>
-__global__ void k_fast_h(Params P, int step, int nrk, double dtau_d, double facinv, StateBuf Sprev, int prev_rt,
-                         StateBuf Sst, StageAux<R> A, const R* __restrict__ Fmx, const R* __restrict__ Fmy,
-                         const R* __restrict__ lag_in, R* __restrict__ lag_out, R* __restrict__ avx,
-                         R* __restrict__ avy, double* __restrict__ outx, double* __restrict__ outy) {
-    const Geo& g = P.g;
-    int i, j, k;
-    if (!cell_coords(g, i, j, k)) return;
-    const int64_t N = g.ncell;
-    const R dtau = R(dtau_d);
-    int im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
-    int64_t c = cidx(g, i, j, k), cxm = cidx(g, im, j, k), cym = cidx(g, i, jm, k);
-    const R beta_d = R(0.1);
-    auto extrap = [&](int64_t cc) {
-        R drt = R(Sprev.cons[N + cc] - Sst.cons[N + cc]);
-        if (step == 0) return drt;
-        return drt + beta_d * (drt - lag_in[cc]);
-    };
-    R drt_c = R(Sprev.cons[N + c] - Sst.cons[N + c]);
-    lag_out[c] = drt_c;
-    double px = Sprev.mx[c], py = Sprev.my[c];
-    if (prev_rt) {
-        double rs = Sprev.cons[c] + Sprev.cons[cxm];
-        double ut = (px * 2.0) / rs;
-        px = (ut * 0.5) * rs;
-        rs = Sprev.cons[c] + Sprev.cons[cym];
-        double vt = (py * 2.0) / rs;
-        py = (vt * 0.5) * rs;
-    }
-    R ndx, ndy;
-    if (nrk == 0 && step == 0) {
-        ndx = R(px - Sst.mx[c]) + dtau * Fmx[c];
-        ndy = R(py - Sst.my[c]) + dtau * Fmy[c];
-    } else {
-        R ec = extrap(c);
-        R gpx = (ec - extrap(cxm)) * R(g.dxi);
-        gpx *= R(1);
-        R gpy = (ec - extrap(cym)) * R(g.dyi);
-        gpy *= R(1);
-        if (P.moist) {
-            const R* pr = A.prim;
-            R qx = R(0.5) * (pr[4 * N + c] + pr[4 * N + cxm] + pr[5 * N + c] + pr[5 * N + cxm]);
-            R qy = R(0.5) * (pr[4 * N + c] + pr[4 * N + cym] + pr[5 * N + c] + pr[5 * N + cym]);
-            gpx /= (R(1) + qx);
-            gpy /= (R(1) + qy);
-        }
-        R pix = R(0.5) * (A.pi[cxm] + A.pi[c]);
-        R piy = R(0.5) * (A.pi[cym] + A.pi[c]);
-        R fx = R(-Gamma_ * R_d) * pix * gpx;
-        R fy = R(-Gamma_ * R_d) * piy * gpy;
-        ndx = R(px - Sst.mx[c]) + dtau * fx + dtau * Fmx[c];
-        ndy = R(py - Sst.my[c]) + dtau * fy + dtau * Fmy[c];
-    }
-    avx[c] += R(facinv) * ndx;
-    avy[c] += R(facinv) * ndy;
-    outx[c] = Sst.mx[c] + double(ndx);
-    outy[c] = Sst.my[c] + double(ndy);
-}
-
-// ---------------------------------------------------------------------------
 // The stage update without acoustic substepping (no_substep_fun,
 // TimeIntegration/ERF_TI_no_substep_fun.H:6-150, fixed or no terrain):
 // S_sum = S_old + slow_dt * F_slow for rho, rho*theta and the three momenta,
@@ -873,146 +805,6 @@ __global__ void k_fast_coef(Params P, double D_d, StateBuf Sst, StageAux<R> A, R
 }
 
 // ---------------------------------------------------------------------------
-// Acoustic substep, vertical part (erf_fast_rhs_N, ERF_fast_rhs_N.cpp:259-592):
-//   phase 1  horizontal rho / rho*theta fluxes from the new U'', V'' per cell;
-//   phase 2  right-hand side of the implicit w system per face, and
-//            d(rho w) of the previous solution;
-//   phase 3  Thomas forward / back substitution (one warp; FMA only, the
-//            stage's 1/B' and C/B' come from k_fast_coef);
-//   phase 4  vertical fluxes, average z-momentum, rho and rho*theta update.
-// All reads of the previous state happen in phases 1-2, before any write,
-// because the previous and new states may be the same buffers.  The W''
-// system is solved in R; rho, rho*theta and the z-momentum are accumulated
-// in FP64.
-// ---------------------------------------------------------------------------
-template <class R>
-__global__ void __launch_bounds__(1024) k_fast_vert(Params P, double dtau_d, double facinv, double beta_1d,
-                                                    double beta_2d, StateBuf Sprev, int prev_rt, StateBuf Sst,
-                                                    StageAux<R> A, const R* __restrict__ Fcons,
-                                                    const R* __restrict__ Fmz, const double* __restrict__ newx,
-                                                    const double* __restrict__ newy, const R* __restrict__ cA,
-                                                    const R* __restrict__ cInvB, const R* __restrict__ cCB,
-                                                    const R* __restrict__ cP, const R* __restrict__ cQ,
-                                                    R* __restrict__ avz, double* out_cons, double* out_mz) {
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    R* sm = reinterpret_cast<R*>(sm_raw);
-    const Geo& g = P.g;
-    Tile t(g);
-    const int nz = g.nz, TX = t.tx, L = t.lane;
-    R* sT0 = sm;
-    R* sT1 = sT0 + nz * TX;
-    R* sR = sT1 + nz * TX;
-    R* sD = sR + (nz + 1) * TX;
-    R* sA = sD + (nz + 1) * TX;
-    R* sI = sA + (nz + 1) * TX;
-    R* sCB = sI + (nz + 1) * TX;
-
-    const int64_t N = g.ncell;
-    const R dxi = R(g.dxi), dyi = R(g.dyi), dzi = R(g.dzi), halfg = R(P.halfg);
-    const R dtau = R(dtau_d), beta_1 = R(beta_1d), beta_2 = R(beta_2d);
-    const R* th = A.prim;
-    const int i = t.i, j = t.j;
-    int ip = 0, im = 0, jp = 0, jm = 0;
-    if (t.ok) { ip = wrap(i + 1, g.nx); im = wrap(i - 1, g.nx); jp = wrap(j + 1, g.ny); jm = wrap(j - 1, g.ny); }
-    auto prev_mz = [&](int k) {
-        int64_t f = cidx(g, i, j, k);
-        double m = Sprev.mz[f];
-        if (prev_rt) {
-            if (k == 0 || k == nz) return 0.0;
-            double rs = Sprev.cons[f] + Sprev.cons[f - g.sk];
-            double wt = (m * 2.0) / rs;
-            m = (wt * 0.5) * rs;
-        }
-        return m;
-    };
-    auto thz = [&](int k) { return th[cidx(g, i, j, clampk(k, nz))]; };
-    // ---- phase 1
-    if (t.ok) {
-        for (int k = t.w; k < nz; k += t.nw) {
-            int64_t c = cidx(g, i, j, k);
-            R xl = R(newx[c] - Sst.mx[c]) / R(1);
-            R xh = R(newx[cidx(g, ip, j, k)] - Sst.mx[cidx(g, ip, j, k)]) / R(1);
-            R yl = R(newy[c] - Sst.my[c]) / R(1);
-            R yh = R(newy[cidx(g, i, jp, k)] - Sst.my[cidx(g, i, jp, k)]) / R(1);
-            R mfsq = R(1);
-            R tc = th[c];
-            sT0[k * TX + L] = (xh - xl) * dxi * mfsq + (yh - yl) * dyi * mfsq;
-            sT1[k * TX + L] = ((xh * (tc + th[cidx(g, ip, j, k)]) - xl * (tc + th[cidx(g, im, j, k)])) * dxi * mfsq +
-                               (yh * (tc + th[cidx(g, i, jp, k)]) - yl * (tc + th[cidx(g, i, jm, k)])) * dyi * mfsq) * R(0.5);
-        }
-    }
-    __syncthreads();
-    // ---- phase 2
-    if (t.ok) {
-        for (int k = t.w; k <= nz; k += t.nw) {
-            int64_t f = cidx(g, i, j, k);
-            R Ok = R(prev_mz(k) - Sst.mz[f]);
-            sD[k * TX + L] = Ok;
-            sA[k * TX + L] = cA[f];
-            sI[k * TX + L] = cInvB[f];
-            sCB[k * TX + L] = cCB[f];
-            R rhs;
-            if (k == 0 || k == nz) {
-                rhs = Ok + dtau * Fmz[f];
-            } else {
-                int64_t cm = f - g.sk;
-                R Okp1 = R(prev_mz(k + 1) - Sst.mz[f + g.sk]);
-                R Okm1 = R(prev_mz(k - 1) - Sst.mz[cm]);
-                R cPk = cP[f], cQk = cQ[f];
-                R tlo = R(0.5) * (thz(k - 2) + thz(k - 1));
-                R tmid = R(0.5) * (thz(k - 1) + thz(k));
-                R thi = R(0.5) * (thz(k) + thz(k + 1));
-                R drt_k = R(Sprev.cons[N + f] - Sst.cons[N + f]);
-                R drt_km = R(Sprev.cons[N + cm] - Sst.cons[N + cm]);
-                R odk = R(Sprev.cons[f] - Sst.cons[f]);
-                R odkm = R(Sprev.cons[cm] - Sst.cons[cm]);
-                R R0 = cPk * drt_k + cQk * drt_km - halfg * (odk + odkm);
-                R R1 = halfg * (-Fcons[f] - Fcons[cm] + sT0[k * TX + L] + sT0[(k - 1) * TX + L]) +
-                       (cPk * (Fcons[N + f] - sT1[k * TX + L]) + cQk * (Fcons[N + cm] - sT1[(k - 1) * TX + L]));
-                R1 += beta_1 * dzi * ((Okp1 - Okm1) * halfg - (Okp1 * thi - Ok * tmid) * cPk - (Ok * tmid - Okm1 * tlo) * cQk);
-                rhs = Ok + dtau * (Fmz[f] + R0 + dtau * beta_2 * R1);
-            }
-            sR[k * TX + L] = rhs;
-        }
-    }
-    __syncthreads();
-    // ---- phase 3: tridiagonal solve, one warp
-    if (t.w == 0 && t.ok) {
-        R s = sR[L] * sI[L];
-        sR[L] = s;
-        for (int k = 1; k <= nz; ++k) {
-            s = (sR[k * TX + L] - sA[k * TX + L] * s) * sI[k * TX + L];
-            sR[k * TX + L] = s;
-        }
-        for (int k = nz - 1; k >= 0; --k) {
-            s = sR[k * TX + L] - sCB[k * TX + L] * s;
-            sR[k * TX + L] = s;
-        }
-    }
-    __syncthreads();
-    // ---- phase 4
-    if (t.ok) {
-        for (int k = t.w; k < nz; k += t.nw) {
-            int64_t c = cidx(g, i, j, k);
-            R sol = sR[k * TX + L], sol_hi = sR[(k + 1) * TX + L];
-            R zl = beta_2 * sol + beta_1 * sD[k * TX + L];
-            R zh = beta_2 * sol_hi + beta_1 * sD[(k + 1) * TX + L];
-            avz[c] += R(facinv) * zl / (R(1) * R(1));
-            if (k == nz - 1) avz[c + g.sk] += R(facinv) * zh / (R(1) * R(1));
-            R tc = th[c];
-            R t0 = sT0[k * TX + L] + dzi * (zh - zl);
-            R t1 = sT1[k * TX + L] + R(0.5) * dzi * (zh * (tc + thz(k + 1)) - zl * (tc + thz(k - 1)));
-            double pr = Sprev.cons[c], prt = Sprev.cons[N + c];
-            out_cons[c] = pr + double(dtau * (Fcons[c] - t0));
-            out_cons[N + c] = prt + double(dtau * (Fcons[N + c] - t1));
-            double smz = Sst.mz[c];
-            out_mz[c] = smz + double(sol);
-            if (k == nz - 1) out_mz[c + g.sk] = Sst.mz[c + g.sk] + double(sol_hi);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Kessler, one thread per cell: the fall fluxes through the cell's bottom and
 // top faces are evaluated from the pre-update neighbours, so cells are
 // independent (same arithmetic as k_kessler).  A block holds 32 columns x
@@ -1177,10 +969,12 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_CELL) k_slow_cell(Params 
             R frt = tile_div(g, sh, zl, zh);
             zl = zh;
             int64_t c = cidx(g, i, j, k);
-            avx[c] = R(S.mx[c]);
-            avy[c] = R(S.my[c]);
-            avz[c] = R(S.mz[c]);
-            if (k == g.nz - 1) avz[c + g.sk] = R(S.mz[c + g.sk]);
+            if (avx) {   // the per-pass entry wants them; the first substep forms its own
+                avx[c] = R(S.mx[c]);
+                avy[c] = R(S.my[c]);
+                avz[c] = R(S.mz[c]);
+                if (k == g.nz - 1) avz[c + g.sk] = R(S.mz[c + g.sk]);
+            }
             Fcons[c] = R(-1.0 / 1.0 * ((S.mx[cidx(g, ip, j, k)] - S.mx[c]) * g.dxi +
                                        (S.my[cidx(g, i, jp, k)] - S.my[c]) * g.dyi + (S.mz[c + g.sk] - S.mz[c]) * g.dzi));
             if (P.les == ERF_LES_MLP) {
@@ -1732,15 +1526,12 @@ void tiled_setup(const Params& P, TiledKz* t) {
 // size passed at launch still sets each launch's footprint), so that contexts
 // of different sizes never lower it below one another's needs.
 template <class R>
-int vert_setup(size_t vert_smem, size_t coef_smem) {
+int coef_setup(size_t coef_smem) {
     int dev = 0, maxopt = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&maxopt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 1;
-    if (vert_smem > (size_t)maxopt || coef_smem > (size_t)maxopt) return 1;
-    if (cudaFuncSetAttribute(k_fast_vert<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt) != cudaSuccess ||
-        cudaFuncSetAttribute(k_fast_coef<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt) != cudaSuccess)
-        return 1;
-    return 0;
+    if (coef_smem > (size_t)maxopt) return 1;
+    return cudaFuncSetAttribute(k_fast_coef<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt) != cudaSuccess;
 }
 
 template <class R>
@@ -1764,13 +1555,6 @@ void launch_tau(const Params& P, cudaStream_t st, const double* cons, const doub
 template <class R>
 void launch_plane_avg(const Params& P, cudaStream_t st, const double* cons, const R* prim, double* avg) {
     k_plane_avg<R><<<dim3(P.g.nz, PAVG_PARTS), 256, 0, st>>>(P, cons, prim, avg);
-}
-template <class R>
-void launch_fast_h(const Params& P, cudaStream_t st, int step, int nrk, double dtau, double facinv, StateBuf Sprev,
-                   int prev_rt, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in, R* lag_out,
-                   R* avx, R* avy, double* outx, double* outy) {
-    k_fast_h<R><<<cell_grid(P.g), cell_block(), 0, st>>>(P, step, nrk, dtau, facinv, Sprev, prev_rt, Sst, A, Fmx, Fmy,
-                                                         lag_in, lag_out, avx, avy, outx, outy);
 }
 // ABLMost::update_fluxes (BoundaryConditions/ERF_ABLMost.cpp:11-142) on the
 // step's old velocities: plane means of u and v on their faces (the periodic
@@ -1826,15 +1610,6 @@ void launch_fast_coef(const Params& P, cudaStream_t st, dim3 grid, dim3 block, s
     k_fast_coef<R><<<grid, block, smem, st>>>(P, D, Sst, A, cA, cInvB, cCB, cP, cQ);
 }
 template <class R>
-void launch_fast_vert(const Params& P, cudaStream_t st, dim3 grid, dim3 block, size_t smem, double dtau,
-                      double facinv, double beta_1, double beta_2, StateBuf Sprev, int prev_rt, StateBuf Sst,
-                      StageAux<R> A, const R* Fcons, const R* Fmz, const double* newx, const double* newy,
-                      const R* cA, const R* cInvB, const R* cCB, const R* cP, const R* cQ, R* avz, double* out_cons,
-                      double* out_mz) {
-    k_fast_vert<R><<<grid, block, smem, st>>>(P, dtau, facinv, beta_1, beta_2, Sprev, prev_rt, Sst, A, Fcons, Fmz,
-                                              newx, newy, cA, cInvB, cCB, cP, cQ, avz, out_cons, out_mz);
-}
-template <class R>
 void launch_slow_cell(const Params& P, const TiledKz& t, cudaStream_t st, StateBuf S, StageAux<R> A, const R* mut,
                       const R* hx, const R* hy, const R* hz, TkeBuf<R> tke, R* Fcons, R* avx, R* avy, R* avz) {
     slow_cell_kernel<R>(P)<<<tile_grid(P.g, t.cell), dim3(TTX, TTY, 1), 0, st>>>(P, t.cell, S, A, mut, hx, hy, hz,
@@ -1858,7 +1633,7 @@ void launch_post(const Params& P, const TiledKz& t, cudaStream_t st, double slow
 
 #define ERFB_INSTANTIATE(R)                                                                                          \
     template void tiled_setup<R>(const Params&, TiledKz*);                                                           \
-    template int vert_setup<R>(size_t, size_t);                                                                      \
+    template int coef_setup<R>(size_t);                                                                              \
     template void launch_step_begin<R>(const Params&, cudaStream_t, const double*, const double*, const double*,     \
                                        const double*, StateBuf, double*, double*, double*, StageAux<R>, R*,          \
                                        TkeBuf<R>);                                                                   \
@@ -1866,16 +1641,10 @@ void launch_post(const Params& P, const TiledKz& t, cudaStream_t st, double slow
                                 const double*, const R*, R*, R*, R*, R*, R*, R*);                                    \
     template void launch_plane_avg<R>(const Params&, cudaStream_t, const double*, const R*, double*);                \
     template void launch_stage_aux<R>(const Params&, cudaStream_t, const double*, StageAux<R>);                      \
-    template void launch_fast_h<R>(const Params&, cudaStream_t, int, int, double, double, StateBuf, int, StateBuf,   \
-                                   StageAux<R>, const R*, const R*, const R*, R*, R*, R*, double*, double*);         \
     template void launch_no_substep<R>(const Params&, cudaStream_t, double, StateBuf, const R*, const R*, const R*, \
                                        const R*, StateBuf);                                                          \
     template void launch_fast_coef<R>(const Params&, cudaStream_t, dim3, dim3, size_t, double, StateBuf,             \
                                       StageAux<R>, R*, R*, R*, R*, R*);                                              \
-    template void launch_fast_vert<R>(const Params&, cudaStream_t, dim3, dim3, size_t, double, double, double,       \
-                                      double, StateBuf, int, StateBuf, StageAux<R>, const R*, const R*,              \
-                                      const double*, const double*, const R*, const R*, const R*, const R*,          \
-                                      const R*, R*, double*, double*);                                               \
     template void launch_slow_cell<R>(const Params&, const TiledKz&, cudaStream_t, StateBuf, StageAux<R>, const R*,  \
                                       const R*, const R*, const R*, TkeBuf<R>, R*, R*, R*, R*);                      \
     template void launch_slow_mom<R>(const Params&, const TiledKz&, cudaStream_t, StateBuf, StageAux<R>,             \

@@ -113,7 +113,7 @@ constexpr int KESS_KB = 8;
 template <class R>
 void tiled_setup(const Params& P, TiledKz* t);
 template <class R>
-int vert_setup(size_t vert_smem, size_t coef_smem);
+int coef_setup(size_t coef_smem);
 template <class R>
 void launch_step_begin(const Params& P, cudaStream_t st, const double* cons, const double* uo, const double* vo,
                        const double* wo, StateBuf S, double* un, double* vn, double* wn, StageAux<R> A, R* mut,
@@ -130,10 +130,6 @@ constexpr int PAVG_PARTS = 16;
 inline size_t plane_avg_doubles(int nz) { return (size_t)6 * nz + (size_t)5 * nz * PAVG_PARTS + nz; }
 template <class R>
 void launch_plane_avg(const Params& P, cudaStream_t st, const double* cons, const R* prim, double* avg);
-template <class R>
-void launch_fast_h(const Params& P, cudaStream_t st, int step, int nrk, double dtau, double facinv, StateBuf Sprev,
-                   int prev_rt, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in, R* lag_out,
-                   R* avx, R* avy, double* outx, double* outy);
 // MOST plane means and friction velocity of a step from its old velocities
 void launch_most_avg(const Params& P, cudaStream_t st, const double* u, const double* v);
 template <class R>
@@ -142,12 +138,43 @@ void launch_no_substep(const Params& P, cudaStream_t st, double slow_dt, StateBu
 template <class R>
 void launch_fast_coef(const Params& P, cudaStream_t st, dim3 grid, dim3 block, size_t smem, double D, StateBuf Sst,
                       StageAux<R> A, R* cA, R* cInvB, R* cCB, R* cP, R* cQ);
+// Acoustic substeps on a flat grid (substep.cu): the launch shape (columns
+// per block, thread rows of the substep and coefficient kernels), a stage's
+// coefficients and one substep.
+struct SubShape {
+    int tx = 32, rows = 16, coef_rows = 8;
+};
 template <class R>
-void launch_fast_vert(const Params& P, cudaStream_t st, dim3 grid, dim3 block, size_t smem, double dtau,
-                      double facinv, double beta_1, double beta_2, StateBuf Sprev, int prev_rt, StateBuf Sst,
-                      StageAux<R> A, const R* Fcons, const R* Fmz, const double* newx, const double* newy,
-                      const R* cA, const R* cInvB, const R* cCB, const R* cP, const R* cQ, R* avz, double* out_cons,
-                      double* out_mz);
+struct SubCoef {
+    R *fx, *fy;              // pressure-gradient factors on the x / y faces
+    R *E, *G, *I, *P, *Q;    // z faces
+};
+template <class R>
+struct SubArgs {
+    double dtau, facinv, b1, b2;
+    StateBuf old, st, sum;   // step's old state (first substep), stage state, whole new state (last substep)
+    const R* th;             // the stage's theta
+    const R *Fr, *Ft, *Fmx, *Fmy, *Fmz;
+    const R *fx, *fy, *cE, *cG, *cI, *cP, *cQ;
+    const R *ui, *vi, *wi, *ei;   // deviations in: momentum increments, extrapolated d(rho theta)
+    R *uo, *vo, *wo, *eo;         // and out (other arrays: neighbouring blocks read the old ones)
+    double *dr, *drt;             // d(rho), d(rho theta), in place
+    R *avx, *avy, *avz;
+    int av_init;                  // start the averages from the stage momenta
+    int grad;                     // MODE 1: apply the pressure gradient
+    const R* lag_in;              // MODE 1: previous d(rho theta) for the extrapolation (NULL: none)
+    R* lag_out;                   // receives d(rho theta) (NULL: not wanted)
+};
+template <class R>
+SubShape sub_shape(const Geo& g);
+template <class R>
+int sub_setup(const Geo& g, const SubShape& s);
+template <class R>
+void launch_sub_coef(const Params& P, cudaStream_t st, const SubShape& s, double D, StateBuf Sst, StageAux<R> A,
+                     const SubCoef<R>& c);
+// mode 0: no deviations, 1: old - stage, 2: stored; last: write the whole state
+template <class R>
+void launch_substep(const Params& P, cudaStream_t st, const SubShape& s, int mode, bool last, const SubArgs<R>& a);
 template <class R>
 void launch_slow_cell(const Params& P, const TiledKz& t, cudaStream_t st, StateBuf S, StageAux<R> A, const R* mut,
                       const R* hx, const R* hy, const R* hz, TkeBuf<R> tke, R* Fcons, R* avx, R* avy, R* avz);
