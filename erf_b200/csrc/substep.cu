@@ -45,15 +45,27 @@ struct ColTile {
     }
 };
 
-// Level index within an array of the bounds-checked build (cidx's check).
-__device__ __forceinline__ int64_t lev(const Geo& g, int k) {
+// Element e of an array.  The byte offset stays in 32 bits (an array of 4 GB
+// would be 5e8 cells, more than the card holds), so that a thread keeps one
+// offset register per neighbour for all the arrays instead of an address per
+// load: that is what lets it hold its loads in flight together.
+template <class T>
+__device__ __forceinline__ T ld(const T* p, uint32_t e) {
+    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + e * (uint32_t)sizeof(T)));
+}
+template <class T>
+__device__ __forceinline__ T& at(T* p, uint32_t e) {
+    return *reinterpret_cast<T*>(reinterpret_cast<char*>(p) + e * (uint32_t)sizeof(T));
+}
+// Offset of level k (of the bounds-checked build: cidx's check).
+__device__ __forceinline__ uint32_t lev(const Geo& g, int k) {
 #ifdef ERF_B200_BOUNDS
     if ((unsigned)k > (unsigned)g.nz) {
         if (g.oob) atomicOr(g.oob, ST_BOUNDS);
         return 0;
     }
 #endif
-    return g.sk * k;
+    return (uint32_t)g.sk * (uint32_t)k;
 }
 
 // The stage's coefficients.  Per x / y face: the factor of the pressure
@@ -189,81 +201,77 @@ __global__ void __launch_bounds__(1024) k_substep(Params P, SubArgs<R> a) {
     R* sS = reinterpret_cast<R*>(sY + nz * TX);
     R* sE = sS + (nz + 1) * TX;
     R* sG = sE + (nz + 1) * TX;
-    const int64_t N = g.ncell, sk = g.sk;
+    const uint32_t sk = (uint32_t)g.sk, c0 = t.col;
+    const R* th = a.th;
     const R dxi = R(g.dxi), dyi = R(g.dyi), dzi = R(g.dzi);
     const R dtau = R(a.dtau), b1 = R(a.b1), b2 = R(a.b2), c2 = dtau * b2, b1z = b1 * dzi;
-    const R* __restrict__ th = a.th;
-    const int c0 = t.col;
-    // deviations of cell / face index c
-    auto dev_rt = [&](int64_t c) -> double {
+    const double* ort = a.old.cons + g.ncell;
+    const double* srt = a.st.cons + g.ncell;
+    const bool av_init = MODE == 0 || (MODE == 1 && a.av_init), grad = MODE == 2 || (MODE == 1 && a.grad);
+    // deviations of cell / face c
+    auto dev_rt = [&](uint32_t c) -> double {
         if (MODE == 0) return 0.0;
-        if (MODE == 1) return a.old.cons[N + c] - a.st.cons[N + c];
-        return a.drt[c];
+        if (MODE == 1) return ld(ort, c) - ld(srt, c);
+        return at(a.drt, c);
     };
-    auto dev_r = [&](int64_t c) -> double {
+    auto dev_r = [&](uint32_t c) -> double {
         if (MODE == 0) return 0.0;
-        if (MODE == 1) return a.old.cons[c] - a.st.cons[c];
-        return a.dr[c];
+        if (MODE == 1) return ld(a.old.cons, c) - ld(a.st.cons, c);
+        return at(a.dr, c);
     };
-    auto dev_w = [&](int64_t f) -> R {
+    auto dev_m = [&](const double* old, const double* st, const R* dev, uint32_t f) -> R {
         if (MODE == 0) return R(0);
-        if (MODE == 1) return R(a.old.mz[f] - a.st.mz[f]);
-        return __ldg(a.wi + f);
+        if (MODE == 1) return R(ld(old, f) - ld(st, f));
+        return ld(dev, f);
     };
-    auto ext = [&](int64_t c) -> R {   // extrapolated d(rho theta)
-        if (MODE == 0) return R(0);
-        if (MODE == 2) return __ldg(a.ei + c);
+    auto dev_w = [&](uint32_t f) -> R { return dev_m(a.old.mz, a.st.mz, a.wi, f); };
+    auto ext = [&](uint32_t c) -> R {   // extrapolated d(rho theta)
+        if (MODE == 2) return ld(a.ei, c);
         const R d = R(dev_rt(c));
-        return a.lag_in ? d + R(0.1) * (d - a.lag_in[c]) : d;
+        return a.lag_in ? d + R(0.1) * (d - ld(a.lag_in, c)) : d;
     };
     // ---- phase 1
     if (t.ok) {
 #pragma unroll 1
         for (int k = t.w; k < nz; k += t.nw) {
-            const int64_t o = lev(g, k), c = o + c0;
-            auto du = [&](int f, R de) -> R {
-                R p = R(0);
-                if (MODE == 1) p = R(a.old.mx[o + f] - a.st.mx[o + f]);
-                if (MODE == 2) p = __ldg(a.ui + o + f);
-                return MODE == 0 ? dtau * a.Fmx[o + f] : p + dtau * (a.fx[o + f] * de + a.Fmx[o + f]);
-            };
-            auto dv = [&](int f, R de) -> R {
-                R p = R(0);
-                if (MODE == 1) p = R(a.old.my[o + f] - a.st.my[o + f]);
-                if (MODE == 2) p = __ldg(a.vi + o + f);
-                return MODE == 0 ? dtau * a.Fmy[o + f] : p + dtau * (a.fy[o + f] * de + a.Fmy[o + f]);
-            };
-            R exl = R(0), exh = R(0), eyl = R(0), eyh = R(0);
-            if (MODE == 2 || (MODE == 1 && a.grad)) {
+            const uint32_t o = lev(g, k), c = o + c0, xm = o + t.xm, xp = o + t.xp, ym = o + t.ym, yp = o + t.yp;
+            R xl = ld(a.Fmx, c), xh = ld(a.Fmx, xp), yl = ld(a.Fmy, c), yh = ld(a.Fmy, yp);
+            if (grad) {
                 const R ec = ext(c);
-                exl = ec - ext(o + t.xm); exh = ext(o + t.xp) - ec;
-                eyl = ec - ext(o + t.ym); eyh = ext(o + t.yp) - ec;
+                xl += ld(a.fx, c) * (ec - ext(xm));
+                xh += ld(a.fx, xp) * (ext(xp) - ec);
+                yl += ld(a.fy, c) * (ec - ext(ym));
+                yh += ld(a.fy, yp) * (ext(yp) - ec);
             }
-            const R xl = du(c0, exl), xh = du(t.xp, exh), yl = dv(c0, eyl), yh = dv(t.yp, eyh);
-            const R tc = th[c];
+            xl = dev_m(a.old.mx, a.st.mx, a.ui, c) + dtau * xl;
+            xh = dev_m(a.old.mx, a.st.mx, a.ui, xp) + dtau * xh;
+            yl = dev_m(a.old.my, a.st.my, a.vi, c) + dtau * yl;
+            yh = dev_m(a.old.my, a.st.my, a.vi, yp) + dtau * yh;
+            const R tc = ld(th, c);
             const R t0 = (xh - xl) * dxi + (yh - yl) * dyi;
-            const R t1 = ((xh * (tc + th[o + t.xp]) - xl * (tc + th[o + t.xm])) * dxi +
-                          (yh * (tc + th[o + t.yp]) - yl * (tc + th[o + t.ym])) * dyi) * R(0.5);
-            R G0 = a.Fr[c] - t0, G1 = a.Ft[c] - t1;
+            const R t1 = ((xh * (tc + ld(th, xp)) - xl * (tc + ld(th, xm))) * dxi +
+                          (yh * (tc + ld(th, yp)) - yl * (tc + ld(th, ym))) * dyi) * R(0.5);
+            R G0 = ld(a.Fr, c) - t0, G1 = ld(a.Ft, c) - t1;
             if (MODE != 0) {
                 const R wl = dev_w(c), wh = dev_w(c + sk);
-                const R tl = R(0.5) * (tc + th[k > 0 ? c - sk : c]), tu = R(0.5) * (tc + th[k < nz - 1 ? c + sk : c]);
+                const R tl = R(0.5) * (tc + ld(th, k > 0 ? c - sk : c));
+                const R tu = R(0.5) * (tc + ld(th, k < nz - 1 ? c + sk : c));
                 G0 -= b1z * (wh - wl);
                 G1 -= b1z * (wh * tu - wl * tl);
             }
             const double dr = dev_r(c), drt = dev_rt(c);
             sY[k * TX + L] = dr + double(c2 * G0);
             sX[k * TX + L] = drt + double(c2 * G1);
-            if (a.lag_out) a.lag_out[c] = R(drt);
-            const R ax = a.av_init ? R(a.st.mx[c]) : a.avx[c], ay = a.av_init ? R(a.st.my[c]) : a.avy[c];
-            a.avx[c] = ax + R(a.facinv) * xl;
-            a.avy[c] = ay + R(a.facinv) * yl;
+            if (MODE == 1 && a.lag_out) at(a.lag_out, c) = R(drt);
+            const R ax = av_init ? R(ld(a.st.mx, c)) : at(a.avx, c), ay = av_init ? R(ld(a.st.my, c)) : at(a.avy, c);
+            at(a.avx, c) = ax + R(a.facinv) * xl;
+            at(a.avy, c) = ay + R(a.facinv) * yl;
             if (LAST) {
-                a.sum.mx[c] = a.st.mx[c] + double(xl);
-                a.sum.my[c] = a.st.my[c] + double(yl);
+                at(a.sum.mx, c) = ld(a.st.mx, c) + double(xl);
+                at(a.sum.my, c) = ld(a.st.my, c) + double(yl);
             } else {
-                a.uo[c] = xl;
-                a.vo[c] = yl;
+                at(a.uo, c) = xl;
+                at(a.vo, c) = yl;
             }
         }
     }
@@ -273,16 +281,16 @@ __global__ void __launch_bounds__(1024) k_substep(Params P, SubArgs<R> a) {
         const R halfg = R(P.halfg);
 #pragma unroll 2
         for (int k = t.w; k <= nz; k += t.nw) {
-            const int64_t f = lev(g, k) + c0;
+            const uint32_t f = lev(g, k) + c0;
             const int s = k * TX + L;
-            R r = a.Fmz[f];
+            R r = ld(a.Fmz, f);
             if (k > 0 && k < nz) {
                 const R xk = R(sX[s]), xm = R(sX[s - TX]), yk = R(sY[s]), ym = R(sY[s - TX]);
-                r += a.cP[f] * xk + a.cQ[f] * xm - halfg * (yk + ym);
+                r += ld(a.cP, f) * xk + ld(a.cQ, f) * xm - halfg * (yk + ym);
             }
-            sS[s] = (dev_w(f) + dtau * r) * a.cI[f];
-            sE[s] = a.cE[f];
-            sG[s] = a.cG[f];
+            sS[s] = (dev_w(f) + dtau * r) * ld(a.cI, f);
+            sE[s] = ld(a.cE, f);
+            sG[s] = ld(a.cG, f);
         }
     }
     __syncthreads();
@@ -334,30 +342,33 @@ __global__ void __launch_bounds__(1024) k_substep(Params P, SubArgs<R> a) {
         const double ib2 = 1.0 / a.b2;
 #pragma unroll 1
         for (int k = t.w; k < nz; k += t.nw) {
-            const int64_t c = lev(g, k) + c0;
+            const uint32_t c = lev(g, k) + c0;
             const int s = k * TX + L;
             const R sl = sS[s], sh = sS[s + TX];
             const R wl = dev_w(c), wh = dev_w(c + sk);
             const R zl = b2 * sl + b1 * wl;
-            auto avz = [&](int64_t f, R z) { a.avz[f] = (a.av_init ? R(a.st.mz[f]) : a.avz[f]) + R(a.facinv) * z; };
+            auto avz = [&](uint32_t f, R z) {
+                at(a.avz, f) = (av_init ? R(ld(a.st.mz, f)) : at(a.avz, f)) + R(a.facinv) * z;
+            };
             avz(c, zl);
             if (k == nz - 1) avz(c + sk, b2 * sh + b1 * wh);
-            const R tc = th[c];
-            const R tl = R(0.5) * (tc + th[k > 0 ? c - sk : c]), tu = R(0.5) * (tc + th[k < nz - 1 ? c + sk : c]);
+            const R tc = ld(th, c);
+            const R tl = R(0.5) * (tc + ld(th, k > 0 ? c - sk : c));
+            const R tu = R(0.5) * (tc + ld(th, k < nz - 1 ? c + sk : c));
             const double dr = dev_r(c), drt = dev_rt(c);
             const double nr = dr + ((sY[s] - dr) * ib2 - double(c2 * dzi * (sh - sl)));
             const double nrt = drt + ((sX[s] - drt) * ib2 - double(c2 * dzi * (sh * tu - sl * tl)));
             if (LAST) {
-                a.sum.cons[c] = a.st.cons[c] + nr;
-                a.sum.cons[N + c] = a.st.cons[N + c] + nrt;
-                a.sum.mz[c] = a.st.mz[c] + double(sl);
-                if (k == nz - 1) a.sum.mz[c + sk] = a.st.mz[c + sk] + double(sh);
+                at(a.sum.cons, c) = ld(a.st.cons, c) + nr;
+                at(a.sum.cons + g.ncell, c) = ld(srt, c) + nrt;
+                at(a.sum.mz, c) = ld(a.st.mz, c) + double(sl);
+                if (k == nz - 1) at(a.sum.mz, c + sk) = ld(a.st.mz, c + sk) + double(sh);
             } else {
-                a.dr[c] = nr;
-                a.drt[c] = nrt;
-                a.eo[c] = R(nrt) + R(0.1) * (R(nrt) - R(drt));
-                a.wo[c] = sl;
-                if (k == nz - 1) a.wo[c + sk] = sh;
+                at(a.dr, c) = nr;
+                at(a.drt, c) = nrt;
+                at(a.eo, c) = R(nrt) + R(0.1) * (R(nrt) - R(drt));
+                at(a.wo, c) = sl;
+                if (k == nz - 1) at(a.wo, c + sk) = sh;
             }
         }
     }
