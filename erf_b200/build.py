@@ -24,7 +24,7 @@ LIB = os.path.join(HERE, "liberf_b200.so")
 OBJ_BOUNDS = os.path.join(HERE, "_build_bounds")
 LIB_BOUNDS = os.path.join(HERE, "liberf_b200_bounds.so")
 # the two terrain halves take longest, so they start first
-SOURCES = ["terrain.cu", "terrain_f32.cu", "kernels.cu", "substep.cu", "api.cu", "noalloc.cu", "mlp.cu", "closure.cu", "plotfile.cu",
+SOURCES = ["terrain.cu", "terrain_f32.cu", "kernels.cu", "substep.cu", "kessler.cu", "api.cu", "noalloc.cu", "mlp.cu", "closure.cu", "plotfile.cu",
            "checkpoint.cu"]
 # sources a translation unit includes besides the headers
 INCLUDED = {"terrain_f32.cu": ["terrain.cu"]}

@@ -21,8 +21,6 @@ struct NvtxRange {
 };
 
 namespace erfb {
-__global__ void k_kessler(Params P, double* cons, double dtn, double dz);
-__global__ void k_kessler_cells(Params P, const double* cin, double* cout, double dtn, double dz);
 __global__ void k_base_state(int nz, double dz, double g, double rdOcp, const double* th_cc, const double* qv_cc,
                              double th_s, double qv_s, double p_s, double* rho0, double* p0o, double* pi0o,
                              double* th0o);
@@ -349,8 +347,6 @@ void make_params(erf_b200_ctx* c) {
 
 dim3 cell_block() { return dim3(32, 4, 1); }
 dim3 cell_grid(const Geo& g) { return dim3((g.nx + 31) / 32, (g.ny + 3) / 4, g.nz); }
-dim3 col_block() { return dim3(32, 4, 1); }
-dim3 col_grid(const Geo& g) { return dim3((g.nx + 31) / 32, (g.ny + 3) / 4, 1); }
 
 // Substep schedule of MRISplitIntegrator::advance (ERF_MRI.H:255-282).
 // Without substepping every stage takes one update of its whole length.
@@ -411,6 +407,14 @@ static const char* const kPassName[] = {"step_begin", "stress", "slow_cell", "pl
         nvtxRangePop();                       \
     } while (0)
 
+// Kessler at the end of a step: in place on the new state, the rain from the
+// last stage's.
+void kessler_step(erf_b200_ctx* c, StateBuf N0, StateBuf N1) {
+    const Geo& g = c->g;
+    launch_kessler(c->P, c->stream, KessView{N0.cons, g.nx, g.sk, g.ncell}, KessLin{N1.cons + 7 * g.ncell, g.nx, g.sk},
+                   KessLin{N0.cons + 7 * g.ncell, g.nx, g.sk}, c->cfg.dt, c->cfg.dz);
+}
+
 // One full step over static terrain: the same stage / substep schedule with
 // the terrain passes (dry states only).
 template <class R>
@@ -424,9 +428,11 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
     TIMED(0, launch_ter_step_begin<R>(P, st, OLD.cons, Vold[0], Vold[1], Vold[2], OLD, Vnew[0], Vnew[1], Vnew[2],
                                       B.aux[0], B.mut, B.tke));
     // stage outputs alternate between the two scratch states so that the last
-    // one lands in slot 1-p (or in N1 when Kessler moves it to slot 1-p)
+    // one lands in slot 1-p.  The last stage leaves its rain in N1 (whose own
+    // is no longer read: the stage works on its primitives), from where
+    // Kessler moves it on; the other components it updates in place.
     StateBuf outs[3] = {N0, N1, N0};
-    if (P.moist) { outs[0] = N1; outs[1] = N0; outs[2] = N1; }
+    if (P.kessler_rain) outs[2].rain = N1.cons + 7 * g.ncell;
     StateBuf stage[3] = {OLD, outs[0], outs[1]};
     dim3 tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1), tcb(c->tile_tx, c->coef_warps, 1);
     const bool fork = T == nullptr && c->side;
@@ -475,10 +481,7 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
                                     B.ter, B.avx, B.avy, B.avz, Vnew[0], Vnew[1], Vnew[2]));
         a = 1 - a;
     }
-    if (P.moist) {   // Kessler with the sedimentation over detJ
-        dim3 kb(32, 1, KESS_KB), kg((g.nx + 31) / 32, g.ny, (g.nz + KESS_KB - 1) / KESS_KB);
-        TIMED(8, (k_kessler_cells<<<kg, kb, 0, st>>>(P, N1.cons, N0.cons, c->cfg.dt, c->cfg.dz)));
-    }
+    if (P.moist) TIMED(8, kessler_step(c, N0, N1));
 }
 
 // One step over moving terrain without acoustic substepping
@@ -616,9 +619,11 @@ void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
     // the MOST plane means and u* of the step (ERF_Advance.cpp:62-86)
     if (P.most) TIMED(0, launch_most_avg(P, st, Vold[0], Vold[1]));
     // stage outputs alternate between the two scratch states so that the last
-    // one lands in slot 1-p (or in N1 when Kessler moves it to slot 1-p)
+    // one lands in slot 1-p.  The last stage leaves its rain in N1 (whose own
+    // is no longer read: the stage works on its primitives), from where
+    // Kessler moves it on; the other components it updates in place.
     StateBuf outs[3] = {N0, N1, N0};
-    if (P.moist) { outs[0] = N1; outs[1] = N0; outs[2] = N1; }
+    if (P.kessler_rain) outs[2].rain = N1.cons + 7 * g.ncell;
     StateBuf stage[3] = {OLD, outs[0], outs[1]};
     const bool fork = T == nullptr && c->side;   // per-kernel timing keeps one stream
     int a = 0;
@@ -673,10 +678,7 @@ void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
                                 B.tke, B.avx, B.avy, B.avz, Vnew[0], Vnew[1], Vnew[2]));
         a = 1 - a;
     }
-    if (P.moist) {
-        dim3 kb(32, 1, KESS_KB), kg((g.nx + 31) / 32, g.ny, (g.nz + KESS_KB - 1) / KESS_KB);
-        TIMED(8, (k_kessler_cells<<<kg, kb, 0, st>>>(P, N1.cons, N0.cons, c->cfg.dt, c->cfg.dz)));
-    }
+    if (P.moist) TIMED(8, kessler_step(c, N0, N1));
 }
 
 void enqueue_step(erf_b200_ctx* c, int p, LaunchTimer* T = nullptr) {
@@ -1557,11 +1559,7 @@ int erf_b200_kessler_advance(erf_b200_ctx* c, const erf_b200_fab* cons, double d
     if (c->P.ter && !c->ter_set) return ERF_B200_EBADSTATE;   // the sedimentation reads detJ
     const Geo& g = c->g;
     if (!fab_ok(cons, 0, g, c->cfg.ncomp)) return ERF_B200_EINVAL;
-    int rc;
-    if ((rc = pack(c, cons, 0, c->cfg.ncomp, c->S[2].cons))) return rc;
-    k_kessler<<<col_grid(g), col_block(), 0, c->stream>>>(c->P, c->S[2].cons, dt, c->cfg.dz);
-    if ((rc = unpack(c, cons, 0, c->cfg.ncomp, c->S[2].cons))) return rc;
-    return cuda_fail(cudaGetLastError());
+    return cuda_fail(launch_kessler_fab(c->P, c->stream, *cons, c->S[2].cons, dt, c->cfg.dz));
 }
 
 // Attach a trained network to a context created with les_type

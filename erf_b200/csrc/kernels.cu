@@ -502,103 +502,6 @@ __global__ void k_no_substep(Geo g, double slow_dt, StateBuf Sold, const R* __re
 }
 
 // ---------------------------------------------------------------------------
-// Kessler warm-rain microphysics, one thread per column, in place
-// (Microphysics/Kessler/ERF_Kessler.cpp:11-185, ERF_Init_Kessler.cpp:64-99,
-// ERF_Update_Kessler.cpp:14-40).  The rain flux through face k+1 is computed
-// from the pre-update cells k and k+1 before cell k is updated.
-// ---------------------------------------------------------------------------
-__global__ void k_kessler(Params P, double* __restrict__ cons, double dtn, double dz) {
-    const Geo& g = P.g;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    const int64_t N = g.ncell;
-    const int nz = g.nz;
-    const bool rain = P.kessler_rain;
-    const bool has_qp = P.ncomp > 7;
-    const double fac_cond = lcond / P.c_p;
-    auto qp_of = [&](int64_t c) { return has_qp ? cons[7 * N + c] / cons[c] : 0.0; };
-    auto flux = [&](double ra, double qa) {
-        qa = fmax(0.0, qa);
-        double Vt = 36.34 * pow(ra * 0.001 * qa, 0.1346) * pow(ra / 1.16, -0.5);
-        double f = ra * Vt * qa;
-        return (fabs(f) < 1e-14) ? 0.0 : f;
-    };
-    double fz_lo = 0.0;
-    if (rain) {
-        int64_t c0 = cidx(g, i, j, 0);
-        fz_lo = flux(cons[c0], qp_of(c0));
-    }
-    for (int k = 0; k < nz; ++k) {
-        int64_t c = cidx(g, i, j, k);
-        double rho = cons[c];
-        double rt = cons[N + c];
-        double theta = rt / rho;
-        double qv = cons[5 * N + c] / rho;
-        double qc = cons[6 * N + c] / rho;
-        double qp = qp_of(c);
-        double tabs = eos_T(rho, rt, qv);
-        double pres = eos_p(rt, qv) / 100.;
-        if (rain) {
-            double fz_hi;
-            if (k == nz - 1) fz_hi = flux(rho, qp);
-            else {
-                int64_t cu = c + g.sk;
-                fz_hi = flux(0.5 * (rho + cons[cu]), 0.5 * (qp + qp_of(cu)));
-            }
-            qv = fmax(0.0, qv); qc = fmax(0.0, qc); qp = fmax(0.0, qp);
-            double es = esatw(tabs);
-            double qs = Rd_on_Rv * es / fmax(es, pres - es);
-            double dqs = Rd_on_Rv * dtesatw(tabs) / pres;
-            if (qs <= 0.0) qs = 0.0;
-            double d_c2r = 0.0, d_r2v = 0.0, d_v2c = 0.0, d_c2v = 0.0;
-            double fac = 1.0 + (L_v / Cp_d) * dqs;
-            if (qv > qs) d_v2c = fmin(qv, (qv - qs) / (1.0 + fac));
-            if (qv < qs && qc > 0.0) d_c2v = fmin(qc, (qs - qv) / (1.0 + fac));
-            if (qp > 0.0 && qv < qs) {
-                double C = 1.6 + 124.9 * pow(0.001 * rho * qp, 0.2046);
-                d_r2v = 1.0 / (0.001 * rho) * (1.0 - qv / qs) * C * pow(0.001 * rho * qp, 0.525) / (5.4e5 + 2.55e6 / (pres * qs)) * dtn;
-                d_r2v = fmin(qp, d_r2v);
-            }
-            if (qc > 0.0) {
-                double auto_r = (qc > 1.e-3) ? 1.e-3 : 0.0;
-                double accrr = 2.2 * pow(qp, 0.875);
-                d_c2r = dtn * (accrr * qc + auto_r * (qc - 1.e-3));
-                d_c2r = fmin(d_c2r, qc);
-            }
-            // over terrain the fall-flux divergence is per unit computational volume
-            // (dJinv, ERF_Kessler.cpp:82-97)
-            const double dJinv = P.ter ? 1.0 / P.detJ[cidx(g, i, j, k)] : 1.0;
-            double dq_sed = dtn * dJinv * (1.0 / rho) * (fz_hi - fz_lo) / dz;
-            if (fabs(dq_sed) < 1e-14) dq_sed = 0.0;
-            qv += -d_v2c + d_c2v + d_r2v;
-            qc += d_v2c - d_c2v - d_c2r;
-            qp += dq_sed + d_c2r - d_r2v;
-            theta += theta / tabs * fac_cond * (d_v2c - d_c2v - d_r2v);
-            qv = fmax(0.0, qv); qc = fmax(0.0, qc); qp = fmax(0.0, qp);
-            fz_lo = fz_hi;
-        } else {
-            qc = fmax(0.0, qc);
-            double es = esatw(tabs);
-            double qs = Rd_on_Rv * es / fmax(es, pres - es);
-            double dqs = Rd_on_Rv * dtesatw(tabs) / pres;
-            double d_v2c = 0.0, d_c2v = 0.0;
-            double fac = 1.0 + (L_v / Cp_d) * dqs;
-            if (qv > qs) d_v2c = fmin(qv, (qv - qs) / (1.0 + fac));
-            if (qv < qs && qc > 0.0) d_c2v = fmin(qc, (qs - qv) / (1.0 + fac));
-            qv += -d_v2c + d_c2v;
-            qc += d_v2c - d_c2v;
-            theta += theta / tabs * fac_cond * (d_v2c - d_c2v);
-            qv = fmax(0.0, qv); qc = fmax(0.0, qc);
-        }
-        cons[N + c] = rho * theta;
-        cons[5 * N + c] = rho * qv;
-        cons[6 * N + c] = rho * qc;
-        if (has_qp) cons[7 * N + c] = rho * qp;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Hydrostatic base state, one thread: calc_rho_p Newton integration at cell
 // centres (ERF_InputSoundingData.H:176-256, ERF_HSE_utils.H:34-72) and
 // erf_enforce_hse (ERF_init1d.cpp:152-260).  FP64, run once at set-up.
@@ -805,109 +708,6 @@ __global__ void k_fast_coef(Params P, double D_d, StateBuf Sst, StageAux<R> A, R
 }
 
 // ---------------------------------------------------------------------------
-// Kessler, one thread per cell: the fall fluxes through the cell's bottom and
-// top faces are evaluated from the pre-update neighbours, so cells are
-// independent (same arithmetic as k_kessler).  A block holds 32 columns x
-// KESS_KB levels: each thread evaluates the fall flux through its bottom face
-// and takes its top face's from the thread above through shared memory (the
-// block's top level evaluates its own), so each face's flux, with its two
-// pow() calls, is formed once.  The pressure is formed once per cell for
-// both the temperature and the saturation pressure.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32 * KESS_KB) k_kessler_cells(Params P, const double* __restrict__ cin,
-                                                                double* __restrict__ cout, double dtn, double dz) {
-    __shared__ double sfz[KESS_KB][32];
-    const Geo& g = P.g;
-    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y, tz = threadIdx.z;
-    const int k = blockIdx.z * KESS_KB + tz;
-    const bool live = i < g.nx && k < g.nz;
-    const int64_t N = g.ncell;
-    const int nz = g.nz;
-    const bool rain = P.kessler_rain;
-    const bool has_qp = P.ncomp > 7;
-    const double fac_cond = lcond / P.c_p;
-    const int64_t c = live ? cidx(g, i, j, k) : 0;
-    auto qp_of = [&](int64_t cc) { return has_qp ? cin[7 * N + cc] / cin[cc] : 0.0; };
-    auto flux = [&](double ra, double qa) {
-        qa = fmax(0.0, qa);
-        double Vt = 36.34 * pow(ra * 0.001 * qa, 0.1346) * pow(ra / 1.16, -0.5);
-        double f = ra * Vt * qa;
-        return (fabs(f) < 1e-14) ? 0.0 : f;
-    };
-    double rho = 1.0, qp = 0.0, fz_lo = 0.0;
-    if (live) {
-        rho = cin[c];
-        qp = qp_of(c);
-        if (rain) {
-            if (k == 0) fz_lo = flux(rho, qp);
-            else fz_lo = flux(0.5 * (cin[c - g.sk] + rho), 0.5 * (qp_of(c - g.sk) + qp));
-        }
-    }
-    sfz[tz][threadIdx.x] = fz_lo;
-    __syncthreads();
-    if (!live) return;
-    double rt = cin[N + c];
-    double theta = rt / rho;
-    double qv = cin[5 * N + c] / rho;
-    double qc = cin[6 * N + c] / rho;
-    const double p_pa = eos_p(rt, qv);
-    double tabs = p_pa / (R_d * rho * (1.0 + R_v / R_d * qv));   // eos_T(rho, rt, qv) with p formed once
-    double pres = p_pa / 100.;
-    if (rain) {
-        double fz_hi;
-        if (k == nz - 1) fz_hi = flux(rho, qp);
-        else if (tz + 1 < KESS_KB) fz_hi = sfz[tz + 1][threadIdx.x];
-        else fz_hi = flux(0.5 * (rho + cin[c + g.sk]), 0.5 * (qp + qp_of(c + g.sk)));
-        qv = fmax(0.0, qv); qc = fmax(0.0, qc); qp = fmax(0.0, qp);
-        double es = esatw(tabs);
-        double qs = Rd_on_Rv * es / fmax(es, pres - es);
-        double dqs = Rd_on_Rv * dtesatw(tabs) / pres;
-        if (qs <= 0.0) qs = 0.0;
-        double d_c2r = 0.0, d_r2v = 0.0, d_v2c = 0.0, d_c2v = 0.0;
-        double fac = 1.0 + (L_v / Cp_d) * dqs;
-        if (qv > qs) d_v2c = fmin(qv, (qv - qs) / (1.0 + fac));
-        if (qv < qs && qc > 0.0) d_c2v = fmin(qc, (qs - qv) / (1.0 + fac));
-        if (qp > 0.0 && qv < qs) {
-            double C = 1.6 + 124.9 * pow(0.001 * rho * qp, 0.2046);
-            d_r2v = 1.0 / (0.001 * rho) * (1.0 - qv / qs) * C * pow(0.001 * rho * qp, 0.525) / (5.4e5 + 2.55e6 / (pres * qs)) * dtn;
-            d_r2v = fmin(qp, d_r2v);
-        }
-        if (qc > 0.0) {
-            double auto_r = (qc > 1.e-3) ? 1.e-3 : 0.0;
-            double accrr = 2.2 * pow(qp, 0.875);
-            d_c2r = dtn * (accrr * qc + auto_r * (qc - 1.e-3));
-            d_c2r = fmin(d_c2r, qc);
-        }
-        const double dJinv = P.ter ? 1.0 / P.detJ[c] : 1.0;   // ERF_Kessler.cpp:82-97
-        double dq_sed = dtn * dJinv * (1.0 / rho) * (fz_hi - fz_lo) / dz;
-        if (fabs(dq_sed) < 1e-14) dq_sed = 0.0;
-        qv += -d_v2c + d_c2v + d_r2v;
-        qc += d_v2c - d_c2v - d_c2r;
-        qp += dq_sed + d_c2r - d_r2v;
-        theta += theta / tabs * fac_cond * (d_v2c - d_c2v - d_r2v);
-        qv = fmax(0.0, qv); qc = fmax(0.0, qc); qp = fmax(0.0, qp);
-    } else {
-        qc = fmax(0.0, qc);
-        double es = esatw(tabs);
-        double qs = Rd_on_Rv * es / fmax(es, pres - es);
-        double dqs = Rd_on_Rv * dtesatw(tabs) / pres;
-        double d_v2c = 0.0, d_c2v = 0.0;
-        double fac = 1.0 + (L_v / Cp_d) * dqs;
-        if (qv > qs) d_v2c = fmin(qv, (qv - qs) / (1.0 + fac));
-        if (qv < qs && qc > 0.0) d_c2v = fmin(qc, (qs - qv) / (1.0 + fac));
-        qv += -d_v2c + d_c2v;
-        qc += d_v2c - d_c2v;
-        theta += theta / tabs * fac_cond * (d_v2c - d_c2v);
-        qv = fmax(0.0, qv); qc = fmax(0.0, qc);
-    }
-    for (int n = 0; n < P.ncomp; ++n) cout[n * N + c] = cin[n * N + c];
-    cout[N + c] = rho * theta;
-    cout[5 * N + c] = rho * qv;
-    cout[6 * N + c] = rho * qc;
-    if (has_qp) cout[7 * N + c] = rho * qp;
-}
-
-// ---------------------------------------------------------------------------
 // Scalar and momentum transport on x-y tiles marching up in k.  A block owns
 // TTX x TTY columns and `kz` consecutive levels.  At each level every thread
 // evaluates the advective flux through its cell's low x and y faces into
@@ -1096,7 +896,9 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_POST) k_post(Params P, in
                     r -= tke.diss[c];
                 }
                 double v_ = Sold.cons[n * N + c] + slow_dt * double(r);
-                Snew.cons[n * N + c] = (q == 0) ? v_ : fmax(v_, q < nscal ? 0.0 : 2.220446049250313e-16);
+                const double nv = (q == 0) ? v_ : fmax(v_, q < nscal ? 0.0 : 2.220446049250313e-16);
+                if (n == 7 && Snew.rain) Snew.rain[c] = nv;
+                else Snew.cons[n * N + c] = nv;
             }
             Snew.cons[c] = Ssum.cons[c];
             Snew.cons[N + c] = Ssum.cons[N + c];

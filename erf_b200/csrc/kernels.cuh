@@ -60,6 +60,7 @@ struct StateBuf {
     double* mx;   // ncell (periodic x faces)
     double* my;   // ncell
     double* mz;   // nzf
+    double* rain = nullptr;   // where a stage's new rain goes, if not into cons
 };
 
 // Quantities derived from a stage state, stored in the bulk type R.
@@ -108,8 +109,20 @@ int validate_config(const erf_b200_config* c);
 
 // Host launchers of the dycore kernels (kernels.cu), instantiated for
 // R = double (plain form) and R = float (mixed form).
-// Levels per block of k_kessler_cells (blocks of 32 columns x KESS_KB levels)
-constexpr int KESS_KB = 8;
+// Kessler microphysics (kessler.cu): a view of the conserved variables (the
+// pointer is cell (0,0,0)'s; strides in values) and of one array of cells.
+constexpr int KESS_KB = 8;   // levels per block (32 columns x KESS_KB)
+struct KessView {
+    double* p;
+    int64_t js, ks, ns;
+};
+struct KessLin {
+    double* p;
+    int64_t js, ks;
+};
+void launch_kessler(const Params& P, cudaStream_t st, KessView v, KessLin rin, KessLin rout, double dt, double dz);
+cudaError_t launch_kessler_fab(const Params& P, cudaStream_t st, const erf_b200_fab& f, double* stage, double dt,
+                               double dz);
 template <class R>
 void tiled_setup(const Params& P, TiledKz* t);
 template <class R>

@@ -1,10 +1,9 @@
 // noalloc.cu -- Kessler microphysics for callers that cannot allocate device
 // memory.
 //
-// erf_b200_kessler_advance stages the caller's state (an Array4 view with
-// arbitrary ghost widths and strides) in a dense scratch copy owned by the
-// context, runs the column kernel on it and writes the result back.  Creating
-// a context allocates.  Some callers cannot do that: a host code whose device
+// erf_b200_kessler_advance updates the caller's state (an Array4 view with
+// arbitrary ghost widths and strides) in place and stages the rain in scratch
+// owned by the context.  Creating a context allocates.  Some callers cannot do that: a host code whose device
 // memory is entirely reserved up front by its own pool (AMReX's arenas, for
 // example) and which must not see a second allocator next to it.
 // erf_b200_kessler_advance_noalloc does the same work with no context and no
@@ -13,13 +12,6 @@
 #include <mutex>
 
 #include "kernels.cuh"
-
-namespace erfb {
-__global__ void k_kessler(Params P, double* cons, double dtn, double dz);
-__global__ void k_pack(Geo g, erf_b200_fab f, int kind, int ncomp, double* dst);
-__global__ void k_unpack(Geo g, erf_b200_fab f, int kind, int ncomp, const double* src, int tang_lo_zero,
-                         int tang_hi_zero, int wall_w);
-}  // namespace erfb
 
 using namespace erfb;
 
@@ -143,17 +135,9 @@ extern "C" int erf_b200_kessler_advance_noalloc(const erf_b200_config* cfg, cons
     P.kessler_rain = cfg->moisture == ERF_MOIST_KESSLER;
     P.c_p = cfg->c_p;
 
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // every scratch element the column kernel reads is written by the pack
-    // kernel first, so nothing in the shared array has to start at zero
-    dim3 b(32, 4, 1), gp((g.nx + 31) / 32, (g.ny + 3) / 4, g.nz);
-    k_pack<<<gp, b, 0, st>>>(g, *cons, 0, cfg->ncomp, scratch);
-    if (cudaGetLastError() != cudaSuccess) return ERF_B200_ECUDA;
-    dim3 gc((g.nx + 31) / 32, (g.ny + 3) / 4, 1);
-    k_kessler<<<gc, b, 0, st>>>(P, scratch, dt, cfg->dz);
-    if (cudaGetLastError() != cudaSuccess) return ERF_B200_ECUDA;
-    dim3 gu((unsigned)((nxb + 31) / 32), (unsigned)((nyb + 3) / 4), (unsigned)nzb);
-    k_unpack<<<gu, b, 0, st>>>(g, *cons, 0, cfg->ncomp, scratch, g.zlo_noslip, g.zhi_noslip, 0);
-    if (cudaGetLastError() != cudaSuccess) return ERF_B200_ECUDA;
-    return ERF_B200_OK;
+    // every scratch element that is read is written by the same call first, so
+    // nothing in the shared array has to start at zero
+    return launch_kessler_fab(P, static_cast<cudaStream_t>(stream), *cons, scratch, dt, cfg->dz) == cudaSuccess
+               ? ERF_B200_OK
+               : ERF_B200_ECUDA;
 }

@@ -2203,7 +2203,9 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
                 continue;
             }
             double v_ = Sold.cons[n * N + c] + slow_dt * r;
-            Snew.cons[n * N + c] = (q == 0) ? v_ : fmax(v_, species ? 0.0 : 2.220446049250313e-16);
+            const double nv = (q == 0) ? v_ : fmax(v_, species ? 0.0 : 2.220446049250313e-16);
+            if (n == 7 && Snew.rain) Snew.rain[c] = nv;
+            else Snew.cons[n * N + c] = nv;
         }
         Snew.cons[c] = Ssum.cons[c];
         Snew.cons[N + c] = Ssum.cons[N + c];
