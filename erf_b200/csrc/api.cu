@@ -48,6 +48,7 @@ struct Bulk {
     R *hx = nullptr, *hy = nullptr, *hz = nullptr;     // learned closure: rho * heat flux
     TkeBuf<R> tke{nullptr, nullptr, nullptr, nullptr}; // Deardorff closure arrays
     TerBuf<R> ter{};                                    // static terrain scratch
+    MtCoef<R> mc[2]{};                                  // moving terrain: two substeps' coefficients
 };
 
 struct erf_b200_ctx {
@@ -61,6 +62,7 @@ struct erf_b200_ctx {
     // slow_mom (forked and joined with events; captured into the graphs)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_pavg = nullptr, ev_coef = nullptr;
+    cudaEvent_t ev_geo[2] = {}, ev_sub[2] = {};   // moving terrain: a substep's geometry made, a substep done
     int device = 0;
     size_t bytes = 0;
     std::vector<void*> allocs;
@@ -92,14 +94,16 @@ struct erf_b200_ctx {
     // met / detJ / zcc) and at the stage's source (z[1], with met1 / detJ1 /
     // zcc1) and new (z[2]) times; z_t; the step's old base state; the clock
     struct MovingTerrain {
-        double* z[5];                  // + the substep's old and new grids
+        double* z[6];                  // + three substep grids, in rotation
         double *met1, *detJ1, *zcc1;
         double* zt;
         double *r0o, *p0o;
         double* time;
-        double *detJso, *zpt, *trhs, *om, *soln;   // acoustic substeps
+        double* detJso;                           // detJ of the last substep's old grid
+        double *wx, *wy;                          // substeps: h_zeta-weighted horizontal momenta
         double* fac;                              // Sullivan's factor per level
     } mt{};
+    int mt_tx = 0;                                            // moving terrain: columns per block of the substep kernels
     int ter_tx = 0;                                           // k_ter_fast_vert columns per block
     size_t ter_smem = 0;                                      // and its shared memory
     bool ter_set = false;
@@ -517,6 +521,7 @@ void enqueue_step_mt(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
                                       B.aux[0], B.mut, B.tke));
     StateBuf outs[3] = {N0, N1, N0};
     StateBuf stage[3] = {OLD, outs[0], outs[1]};
+    const bool fork = T == nullptr && c->side && !nosub;   // per-kernel timing keeps one stream
     int a = 0;
     for (int nrk = 0; nrk < 3; ++nrk) {
         StateBuf Sst = stage[nrk], Snew = outs[nrk];
@@ -524,6 +529,7 @@ void enqueue_step_mt(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
         int nsub; double dtau, slow_dt;
         stage_schedule(c->cfg, nrk, nsub, dtau, slow_dt);
         const int ts_src = nrk, ts_new = nrk + 1;   // T, T + dt/3, T + dt/2, T + dt
+        if (fork) cudaEventRecord(c->ev_fork, st);   // the stage state is ready
         launch_mt_grid(Po, st, c->mt.time, dt, ts_src, c->mt.z[1]);
         launch_mt_grid(Po, st, c->mt.time, dt, ts_new, c->mt.z[2]);
         launch_ter_metrics(Ps, st, c->mt.detJ1, c->mt.zcc1);
@@ -540,34 +546,45 @@ void enqueue_step_mt(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
                                               c->mt.z[2], SUM));
         } else {
             // fast_rhs_fun, moving terrain (ERF_TI_fast_rhs_fun.H:47-118): per
-            // substep the grids at its old and new times, z_t'', the fast
+            // substep the grids at its old and new times and the fast
             // coefficients on the old grid with the step's old base state;
             // the level keeps the last substep's old grid and its new one
-            // serves the slow-variable update
+            // serves the slow-variable update.  The grids rotate through
+            // three buffers and the coefficients through two, so that the
+            // side stream makes them up to two substeps ahead.
             const double beta_s = 0.1;
             const double D = dtau * dtau * (0.5 * (1.0 + beta_s)) * (0.5 * (1.0 + beta_s)) * c->g.dzi;
-            dim3 tg((c->g.nx + c->tile_tx - 1) / c->tile_tx, c->g.ny, 1), tcb(c->tile_tx, c->coef_warps, 1);
-            Params Pf = Po;
-            Pf.detJ = c->mt.detJso;
-            Pf.r0 = c->mt.r0o;
+            double* const* zb = c->mt.z + 3;
+            cudaStream_t sd = fork ? c->side : st;
+            auto geometry = [&](int ks) {
+                launch_mt_grid_sub(Po, sd, c->mt.time, dtau, ks + 1, zb[(ks + 1) % 3]);
+                TIMED(9, launch_mt_coef<R>(Po, sd, c->mt_tx, D, c->mt.r0o, zb[ks % 3], Sst, Acur, B.mc[ks & 1]));
+                if (fork) cudaEventRecord(c->ev_geo[ks & 1], sd);
+            };
+            if (fork) cudaStreamWaitEvent(sd, c->ev_fork, 0);
+            launch_mt_grid_sub(Po, sd, c->mt.time, dtau, 0, zb[0]);
+            geometry(0);
+            if (nsub > 1) geometry(1);
             int lp = 0;
-            // the substep grids alternate: a substep's new grid is the next one's old grid
-            double *zso = c->mt.z[3], *zsn = c->mt.z[4];
-            launch_mt_grid_sub(Po, st, c->mt.time, dtau, 0, zso);
             for (int ks = 0; ks < nsub; ++ks) {
-                if (ks > 0) std::swap(zso, zsn);
-                launch_mt_grid_sub(Po, st, c->mt.time, dtau, ks + 1, zsn);
-                launch_mt_zpt(Po, st, zso, zsn, dtau, c->mt.zpt);
-                launch_mt_detj(Po, st, zso, c->mt.detJso);
-                TIMED(9, launch_fast_coef<R>(Pf, st, tg, tcb, c->coef_smem, D, Sst, Acur, B.cA, B.cInvB, B.cCB, B.cP,
-                                             B.cQ));
-                TIMED(6, launch_mt_fast<R>(Po, st, ks, c->cfg.no_lagged_delta_rt ? 0 : 1, dtau, beta_s,
+                if (fork) cudaStreamWaitEvent(st, c->ev_geo[ks & 1], 0);
+                TIMED(6, launch_mt_fast<R>(Po, st, c->mt_tx, ks, c->cfg.no_lagged_delta_rt ? 0 : 1, dtau, beta_s,
                                            1.0 / (double)nsub, ks == 0 ? OLD : SUM, Sst, Acur, B.Fcons, B.Fmx, B.Fmy,
-                                           B.Fmz, B.lag[lp], B.lag[1 - lp], B.cA, B.cInvB, B.cCB, B.cP, B.cQ,
-                                           zso, zsn, c->mt.z[1], c->mt.zpt, c->mt.trhs, c->mt.om,
-                                           c->mt.soln, B.avx, B.avy, B.avz, SUM, ks == nsub - 1 ? 1 : 0));
+                                           B.Fmz, B.lag[lp], B.lag[1 - lp], B.mc[ks & 1], zb[ks % 3],
+                                           zb[(ks + 1) % 3], c->mt.z[1], c->mt.wx, c->mt.wy, B.avx, B.avy, B.avz, SUM,
+                                           ks == nsub - 1 ? 1 : 0));
+                if (ks + 2 < nsub) {
+                    if (fork) {
+                        cudaEventRecord(c->ev_sub[ks & 1], st);
+                        cudaStreamWaitEvent(sd, c->ev_sub[ks & 1], 0);
+                    }
+                    geometry(ks + 2);
+                }
                 lp ^= 1;
             }
+            double* zso = zb[(nsub - 1) % 3];
+            double* zsn = zb[nsub % 3];
+            launch_mt_detj(Po, st, zso, c->mt.detJso);
             Pp.znd = zso;
             Pp.detJ = c->mt.detJso;
             Pp.mt_znew = zsn;
@@ -723,6 +740,8 @@ int alloc_bulk(erf_b200_ctx* c, Bulk<R>& B) {
         A(&B.ter.fx[0], N); A(&B.ter.fy[0], N); A(&B.ter.fx[1], N); A(&B.ter.fy[1], N);
         auto D = [&](double** q, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, q, n); };
         D(&B.ter.bnd, 2 * (int64_t)cfg->nx * cfg->ny);
+        if (cfg->terrain_type == ERF_TERRAIN_MOVING && cfg->substepping_type == ERF_SUBSTEP_IMPLICIT)
+            for (MtCoef<R>& m : B.mc) { A(&m.E, NZF); A(&m.G, NZF); A(&m.I, NZF); A(&m.P, NZF); A(&m.Q, NZF); }
     }
     return rc;
 }
@@ -834,7 +853,11 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_pavg, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_coef, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_coef, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_geo[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_geo[1], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_sub[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_sub[1], cudaEventDisableTiming) != cudaSuccess) {
         erf_b200_destroy(c);
         return ERF_B200_ECUDA;
     }
@@ -868,9 +891,8 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
             A(&c->mt.time, 1);
             A(&c->mt.fac, (size_t)cfg->nz + 1);
             if (cfg->substepping_type == ERF_SUBSTEP_IMPLICIT) {
-                A(&c->mt.z[3], (size_t)(cfg->nz + 3) * sk); A(&c->mt.z[4], (size_t)(cfg->nz + 3) * sk);
-                A(&c->mt.detJso, N); A(&c->mt.zpt, NZF); A(&c->mt.trhs, 2 * N); A(&c->mt.om, NZF);
-                A(&c->mt.soln, NZF);
+                for (int q = 3; q < 6; ++q) A(&c->mt.z[q], (size_t)(cfg->nz + 3) * sk);
+                A(&c->mt.detJso, N); A(&c->mt.wx, N); A(&c->mt.wy, N);
             }
         }
     }
@@ -922,6 +944,9 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
         if (rc == ERF_B200_OK && cfg->use_terrain) {
             ter_vert_shape(nz, &c->ter_tx, &c->ter_smem);
             if (c->ter_tx < 1) rc = ERF_B200_ECONFIG;
+            else if (cfg->terrain_type == ERF_TERRAIN_MOVING &&
+                     (c->mixed ? mt_shape<float>(c->g, &c->mt_tx) : mt_shape<double>(c->g, &c->mt_tx)) != 0)
+                rc = ERF_B200_ECUDA;
         }
         if (rc != ERF_B200_OK) { erf_b200_destroy(c); return rc; }
     }
@@ -947,7 +972,7 @@ int erf_b200_destroy(erf_b200_ctx* c) {
     drop_graphs(c);
     for (void* q : c->allocs) cudaFree(q);
     if (c->side) cudaStreamDestroy(c->side);
-    for (cudaEvent_t e : {c->ev_fork, c->ev_pavg, c->ev_coef})
+    for (cudaEvent_t e : {c->ev_fork, c->ev_pavg, c->ev_coef, c->ev_geo[0], c->ev_geo[1], c->ev_sub[0], c->ev_sub[1]})
         if (e) cudaEventDestroy(e);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;

@@ -238,18 +238,25 @@ void launch_mt_advance_time(cudaStream_t st, double* tdev, double dt);
 void launch_diagnostics(const Params& P, cudaStream_t st, const double* cons, const double* w, const double* zgrid,
                         double* part, double* out);
 int diagnostics_scratch_doubles();
-// acoustic substeps over moving terrain: the grid at T + ks dtau, z_t'' of
-// the substep, detJ of a grid, and one substep (last: no boundary fill after
-// it, the slow-variable pass does that)
+// acoustic substeps over moving terrain (moving.cu): the grid at T + ks dtau
+// (terrain.cu), the column launch shape, a substep's coefficients, and one
+// substep (last: the slow-variable pass follows, not another substep)
 void launch_mt_grid_sub(const Params& P, cudaStream_t st, const double* tdev, double dtau, int ks, double* z);
-void launch_mt_zpt(const Params& P, cudaStream_t st, const double* zo, const double* zn, double dtau, double* zpt);
 void launch_mt_detj(const Params& P, cudaStream_t st, const double* z, double* detJ);
 template <class R>
-void launch_mt_fast(const Params& P, cudaStream_t st, int step, int lagged, double dtau, double beta_s, double facinv,
-                    StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fcons, const R* Fmx, const R* Fmy,
-                    const R* Fmz, const R* lag_in, R* lag_out, const R* cA, const R* cInvB, const R* cCB, const R* cP,
-                    const R* cQ, const double* zo, const double* zn, const double* zs, const double* zpt,
-                    double* trhs, double* om, double* soln, R* avx, R* avy, R* avz, StateBuf Ssum, int last);
+struct MtCoef {
+    R *E, *G, *I, *P, *Q;   // on the z faces, as SubCoef's
+};
+template <class R>
+int mt_shape(const Geo& g, int* tx);
+template <class R>
+void launch_mt_coef(const Params& P, cudaStream_t st, int tx, double D, const double* r0, const double* zo, StateBuf Sst,
+                    StageAux<R> A, MtCoef<R> c);
+template <class R>
+void launch_mt_fast(const Params& P, cudaStream_t st, int tx, int step, int lagged, double dtau, double beta_s,
+                    double facinv, StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fcons, const R* Fmx, const R* Fmy,
+                    const R* Fmz, const R* lag_in, R* lag_out, MtCoef<R> c, const double* zo, const double* zn,
+                    const double* zs, double* wx, double* wy, R* avx, R* avy, R* avz, StateBuf Ssum, int last);
 void launch_ter_base_state(const Params& P, cudaStream_t st, const double* zcc, const double* th3, const double* qv3,
                            double th_s, double qv_s, double p_s, double* rho0, double* p0, double* pi0, double* th0);
 template <class R>

@@ -28,6 +28,7 @@
 #include <cfloat>
 
 #include "kernels.cuh"
+#include "moving.cuh"
 #include "tiles.cuh"
 
 // The library compiles this file twice so that the two halves build side by
@@ -174,18 +175,6 @@ ERFB_MT(hxi_EI, MT_HXI_EI)
 ERFB_MT(heta_EI, MT_HETA_EI)
 #undef ERFB_MT
 
-// Face-averaged horizontal components at z-face (i,j,k) of x/y-face arrays
-// given as accessors (extrapolated to the bottom face).
-template <class FU, class FV>
-__device__ __forceinline__ void zface_uv(int i, int j, int k, FU ua, FV va, double& u, double& v) {
-    if (k == 0) {
-        u = 1.5 * (0.5 * (ua(i, j, k) + ua(i + 1, j, k))) - 0.5 * (0.5 * (ua(i, j, k + 1) + ua(i + 1, j, k + 1)));
-        v = 1.5 * (0.5 * (va(i, j, k) + va(i, j + 1, k))) - 0.5 * (0.5 * (va(i, j, k + 1) + va(i, j + 1, k + 1)));
-    } else {
-        u = 0.25 * (ua(i, j, k - 1) + ua(i + 1, j, k - 1) + ua(i, j, k) + ua(i + 1, j, k));
-        v = 0.25 * (va(i, j, k - 1) + va(i, j + 1, k - 1) + va(i, j, k) + va(i, j + 1, k));
-    }
-}
 template <class FU, class FV>
 __device__ __forceinline__ double omega_from_w(const Params& P, int i, int j, int k, double w, FU ua, FV va) {
     double mx = zlo_xi(P, i, j, k), my = zlo_eta(P, i, j, k), u, v;
@@ -315,30 +304,15 @@ void launch_ter_metrics(const Params& P, cudaStream_t st, double* detJ, double* 
 // (the step's old time, the stage's source and new times) from the device
 // copy of the step's old time, so that the step graph replays unchanged.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double mt_time_at(double T, double dt, int tsel) {
-    return tsel == 0 ? T : (tsel == 1 ? T + dt / 3.0 : (tsel == 2 ? T + dt / 2.0 : T + dt));
-}
-// node (i,j,k) of a grid in the znd layout ((nz+3) planes, lateral periodic)
-__device__ __forceinline__ double znode(const double* z, const Geo& g, int i, int j, int k) {
-    return __ldg(z + (int64_t)(k + 1) * g.sk + (int64_t)wrap(j, g.ny) * g.nx + wrap(i, g.nx));
-}
-// make_J of one cell from the nodes (Utils/ERF_TerrainMetrics.cpp:583-640);
-// k = -1 takes level 0 (the grid's ghost level mirrors the first cell)
-__device__ __forceinline__ double mt_detj(const double* z, const Geo& g, int i, int j, int k) {
-    if (k < 0) k = 0;
-    auto Z = [&](int a, int b, int c) { return znode(z, g, a, b, c); };
-    return .25 * g.dzi * (Z(i, j, k + 1) + Z(i + 1, j, k + 1) + Z(i, j + 1, k + 1) + Z(i + 1, j + 1, k + 1)
-                          - Z(i, j, k) - Z(i + 1, j, k) - Z(i, j + 1, k) - Z(i + 1, j + 1, k));
-}
-
 // Problem::init_custom_terrain of the travelling wave
 // (Exec/DevTests/MovingTerrain/ERF_prob.cpp:147-200) and init_terrain_grid
 // with terrain_smoothing = 2 (Utils/ERF_TerrainMetrics.cpp:501-536, 320-333):
 // z(k) = z_k + (1 - z_k / z_top)^3 h over z_k = k dz, z(0) = h,
-// z(-1) = 2 h - z(1), z(nz+1) = 2 z(nz) - z(nz-1).  One thread per column.
+// z(-1) = 2 h - z(1), z(nz+1) = 2 z(nz) - z(nz-1).  One thread per node.
 static __global__ void k_mt_grid(Params P, const double* __restrict__ tdev, double dt, int tsel, double* __restrict__ z) {
     const Geo& g = P.g;
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = (int)blockIdx.z - 1;   // node level -1 .. nz+1
     if (i >= g.nx || j >= g.ny) return;
     // tsel >= 0: a stage point; tsel < 0: substep -1 - tsel of length dt, T + ks dt
     const double t = tsel >= 0 ? mt_time_at(*tdev, dt, tsel) : *tdev + (-1 - tsel) * dt;
@@ -348,23 +322,13 @@ static __global__ void k_mt_grid(Params P, const double* __restrict__ tdev, doub
     // enter z_t through differences over a substep, which magnify any change
     const double hs = __dmul_rn(P.mt_ampl, sin(__dsub_rn(__dmul_rn(P.mt_kp, x), __dmul_rn(P.mt_om, t))));
     const int nz = g.nz;
-    double* col = z + (int64_t)j * g.nx + i;
-    double zk1 = 0.0, zkm1 = 0.0, zk = hs;
-    for (int k = 0; k <= nz; ++k) {
-        const double zl = k * P.mt_dz;
-        double v = __dadd_rn(zl, __dmul_rn(P.mt_fac[k], hs));
-        if (k == 0) v = hs;
-        col[(int64_t)(k + 1) * g.sk] = v;
-        if (k == 1) zk1 = v;
-        if (k == nz - 1) zkm1 = v;
-        if (k == nz) zk = v;
-    }
-    col[0] = 2.0 * hs - zk1;
-    col[(int64_t)(nz + 2) * g.sk] = 2.0 * zk - zkm1;
+    auto node = [&](int kk) { return kk == 0 ? hs : __dadd_rn(kk * P.mt_dz, __dmul_rn(P.mt_fac[kk], hs)); };
+    const double v = k < 0 ? 2.0 * hs - node(1) : (k > nz ? 2.0 * node(nz) - node(nz - 1) : node(k));
+    z[(int64_t)(k + 1) * g.sk + (int64_t)j * g.nx + i] = v;
 }
 #if !ERFB_TER_F32
 void launch_mt_grid(const Params& P, cudaStream_t st, const double* tdev, double dt, int tsel, double* z) {
-    k_mt_grid<<<ter_grid(P.g, 1), ter_block(), 0, st>>>(P, tdev, dt, tsel, z);
+    k_mt_grid<<<ter_grid(P.g, P.g.nz + 3), ter_block(), 0, st>>>(P, tdev, dt, tsel, z);
 }
 #endif
 
@@ -392,46 +356,59 @@ void launch_mt_zt(const Params& P, cudaStream_t st, const double* zo, const doub
 // The base-state update of a moving-terrain stage (ERF_TI_slow_rhs_fun.H:149-210):
 // rho_0 and (rho theta)_0 advanced from the step's old base state by the
 // vertical flux -z_t (face averages of the previous stage's new base state),
-// detJ-weighted old -> source -> new; p_0 from (rho theta)_0.  One thread
-// per column walks up the levels, keeping the level below (already
-// overwritten) in registers; the ghost levels are not updated.
-static __global__ void k_mt_base_state(Params P, const double* __restrict__ r0o, const double* __restrict__ p0o,
+// detJ-weighted old -> source -> new; p_0 from (rho theta)_0; the ghost
+// levels are not updated.  A block owns whole columns, its rows share the
+// levels, and the new values wait in shared memory until every level has
+// read its neighbours' old ones.
+static __global__ void __launch_bounds__(256) k_mt_base_state(Params P, const double* __restrict__ r0o, const double* __restrict__ p0o,
                                 const double* __restrict__ zo, const double* __restrict__ zs,
                                 const double* __restrict__ zn, const double* __restrict__ tdev, double dt,
-                                int tsel_new, double* __restrict__ r0n, double* __restrict__ p0n) {
+                                int tsel_new, double* r0n, double* p0n) {
+    extern __shared__ __align__(16) double sm[];
     const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
+    const int TX = blockDim.x, L = threadIdx.x, col = blockIdx.x * TX + L;
+    const bool ok = col < (int)g.sk;
+    const int j = ok ? col / g.nx : 0, i = ok ? col - j * g.nx : 0;
     const double T = *tdev;
     const double dt_base = mt_time_at(T, dt, tsel_new) - T;
     const double* zt = P.mt_zt;
     auto at = [&](int k) { return (int64_t)(k + 1) * g.sk + (int64_t)j * g.nx + i; };
-    double r_m = r0n[at(-1)], rt_m = eos_rt_given_p(p0n[at(-1)]);
-    double r_c = r0n[at(0)], rt_c = eos_rt_given_p(p0n[at(0)]);
-    for (int k = 0; k < g.nz; ++k) {
-        const double r_p = r0n[at(k + 1)], rt_p = eos_rt_given_p(p0n[at(k + 1)]);
-        const double zl = zt[cidx(g, i, j, k)], zh = zt[cidx(g, i, j, k + 1)];
-        double fr_lo = -zl * 0.5 * (r_c + r_m);
-        double fr_hi = -zh * 0.5 * (r_c + r_p);
-        double frt_lo = fr_lo * 0.5 * (rt_c / r_c + rt_m / r_m);
-        double frt_hi = fr_hi * 0.5 * (rt_c / r_c + rt_p / r_p);
-        const double Js = mt_detj(zs, g, i, j, k), Jo = mt_detj(zo, g, i, j, k), Jn = mt_detj(zn, g, i, j, k);
-        double invdetJ = 1.0 / Js;
-        double src_r = -invdetJ * (fr_hi - fr_lo) * g.dzi;
-        double src_rt = -invdetJ * (frt_hi - frt_lo) * g.dzi;
-        double rho0_new = Jo * r0o[at(k)] + dt_base * Js * src_r;
-        double rt0_new = Jo * eos_rt_given_p(p0o[at(k)]) + dt_base * Js * src_rt;
-        r0n[at(k)] = rho0_new / Jn;
-        rt0_new /= Jn;
-        p0n[at(k)] = eos_p(rt0_new, 0.0);
-        r_m = r_c; rt_m = rt_c; r_c = r_p; rt_c = rt_p;
-    }
+    if (ok)
+        for (int k = threadIdx.y; k < g.nz; k += blockDim.y) {
+            const double r_m = r0n[at(k - 1)], rt_m = eos_rt_given_p(p0n[at(k - 1)]);
+            const double r_c = r0n[at(k)], rt_c = eos_rt_given_p(p0n[at(k)]);
+            const double r_p = r0n[at(k + 1)], rt_p = eos_rt_given_p(p0n[at(k + 1)]);
+            const double zl = zt[cidx(g, i, j, k)], zh = zt[cidx(g, i, j, k + 1)];
+            double fr_lo = -zl * 0.5 * (r_c + r_m);
+            double fr_hi = -zh * 0.5 * (r_c + r_p);
+            double frt_lo = fr_lo * 0.5 * (rt_c / r_c + rt_m / r_m);
+            double frt_hi = fr_hi * 0.5 * (rt_c / r_c + rt_p / r_p);
+            const double Js = mt_detj(zs, g, i, j, k), Jo = mt_detj(zo, g, i, j, k), Jn = mt_detj(zn, g, i, j, k);
+            double invdetJ = 1.0 / Js;
+            double src_r = -invdetJ * (fr_hi - fr_lo) * g.dzi;
+            double src_rt = -invdetJ * (frt_hi - frt_lo) * g.dzi;
+            double rho0_new = Jo * r0o[at(k)] + dt_base * Js * src_r;
+            double rt0_new = Jo * eos_rt_given_p(p0o[at(k)]) + dt_base * Js * src_rt;
+            rt0_new /= Jn;
+            sm[(2 * k) * TX + L] = rho0_new / Jn;
+            sm[(2 * k + 1) * TX + L] = eos_p(rt0_new, 0.0);
+        }
+    __syncthreads();
+    if (ok)
+        for (int k = threadIdx.y; k < g.nz; k += blockDim.y) {
+            r0n[at(k)] = sm[(2 * k) * TX + L];
+            p0n[at(k)] = sm[(2 * k + 1) * TX + L];
+        }
 }
 #if !ERFB_TER_F32
 void launch_mt_base_state(const Params& P, cudaStream_t st, const double* r0o, const double* p0o, const double* zo,
                           const double* zs, const double* zn, const double* tdev, double dt, int tsel_new,
                           double* r0n, double* p0n) {
-    k_mt_base_state<<<ter_grid(P.g, 1), ter_block(), 0, st>>>(P, r0o, p0o, zo, zs, zn, tdev, dt, tsel_new, r0n, p0n);
+    int tx = 8;   // columns per block: 2 nz values each within the 48 KB every kernel may use
+    while (tx > 1 && (size_t)2 * P.g.nz * tx * sizeof(double) > 48 * 1024) tx /= 2;
+    k_mt_base_state<<<(unsigned)((P.g.sk + tx - 1) / tx), dim3(tx, 256 / tx > 64 ? 64 : 256 / tx),
+                      (size_t)2 * P.g.nz * tx * sizeof(double), st>>>(P, r0o, p0o, zo, zs, zn, tdev, dt, tsel_new, r0n,
+                                                                      p0n);
 }
 #endif
 
@@ -439,12 +416,6 @@ void launch_mt_base_state(const Params& P, cudaStream_t st, const double* r0o, c
 // part 1: rho and rho theta detJ-weighted old -> new, the horizontal
 // momenta with h_zeta of their faces (the slow right-hand sides already
 // carry the source geometry's factors).
-__device__ __forceinline__ double mt_hzI(const double* z, const Geo& g, int i, int j, int k) {
-    return 0.5 * g.dzi * (znode(z, g, i, j, k + 1) + znode(z, g, i, j + 1, k + 1) - znode(z, g, i, j, k) - znode(z, g, i, j + 1, k));
-}
-__device__ __forceinline__ double mt_hzJ(const double* z, const Geo& g, int i, int j, int k) {
-    return 0.5 * g.dzi * (znode(z, g, i, j, k + 1) + znode(z, g, i + 1, j, k + 1) - znode(z, g, i, j, k) - znode(z, g, i + 1, j, k));
-}
 template <class R>
 __global__ void k_mt_no_substep_h(Params P, double slow_dt, StateBuf Sold, const R* __restrict__ Fcons,
                                   const R* __restrict__ Fmx, const R* __restrict__ Fmy, const double* __restrict__ zo,
@@ -499,371 +470,11 @@ template void launch_mt_no_substep<float>(const Params&, cudaStream_t, double, S
                                           const float*, const float*, const double*, const double*, StateBuf);
 #endif
 
-// ---------------------------------------------------------------------------
-// Acoustic substeps over moving terrain (erf_fast_rhs_MT,
-// TimeIntegration/ERF_fast_rhs_MT.cpp:48-626).  zo / zn: the grids at the
-// substep's old and new times, zs: the stage's; zpt: the substep's z_t less
-// the stage's.  The new state's horizontal momenta are formed h_zeta-weighted
-// in place, read that way by the flux and Omega'' kernels, then divided by
-// the new grid's h_zeta; one thread per column solves for Omega'' and
-// updates rho w, rho and rho theta.
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ void mt_slopes(const double* z, const Geo& g, int i, int j, int k, double& sx, double& sy) {
-    sx = 0.5 * g.dxi * (znode(z, g, i + 1, j + 1, k) + znode(z, g, i + 1, j, k) - znode(z, g, i, j + 1, k) - znode(z, g, i, j, k));
-    sy = 0.5 * g.dyi * (znode(z, g, i + 1, j + 1, k) + znode(z, g, i, j + 1, k) - znode(z, g, i + 1, j, k) - znode(z, g, i, j, k));
-}
-__device__ __forceinline__ double mt_hxI(const double* z, const Geo& g, int i, int j, int k) {
-    auto Z = [&](int a, int b, int c) { return znode(z, g, a, b, c); };
-    return 0.125 * g.dxi * (Z(i + 1, j, k) + Z(i + 1, j, k + 1) + Z(i + 1, j + 1, k) + Z(i + 1, j + 1, k + 1)
-                            - Z(i - 1, j, k) - Z(i - 1, j, k + 1) - Z(i - 1, j + 1, k) - Z(i - 1, j + 1, k + 1));
-}
-__device__ __forceinline__ double mt_hetaJ(const double* z, const Geo& g, int i, int j, int k) {
-    auto Z = [&](int a, int b, int c) { return znode(z, g, a, b, c); };
-    return 0.125 * g.dyi * (Z(i, j + 1, k) + Z(i, j + 1, k + 1) + Z(i + 1, j + 1, k) + Z(i + 1, j + 1, k + 1)
-                            - Z(i, j - 1, k) - Z(i, j - 1, k + 1) - Z(i + 1, j - 1, k) - Z(i + 1, j - 1, k + 1));
-}
-// OmegaFromW of face (i,j,k) on grid z, horizontal momenta mx / my
-__device__ __forceinline__ double mt_omega(const double* z, const Geo& g, int i, int j, int k, double w,
-                                           const double* mx, const double* my) {
-    auto U = [&](int a, int b, int c) { return mx[cidx(g, wrap(a, g.nx), wrap(b, g.ny), c)]; };
-    auto V = [&](int a, int b, int c) { return my[cidx(g, wrap(a, g.nx), wrap(b, g.ny), c)]; };
-    double sx, sy, u, v;
-    mt_slopes(z, g, i, j, k, sx, sy);
-    zface_uv(i, j, k, U, V, u, v);
-    return w - sx * u - sy * v;
-}
-__device__ __forceinline__ double mt_wfrom(const double* z, const Geo& g, int i, int j, int k, double om,
-                                           const double* mx, const double* my) {
-    auto U = [&](int a, int b, int c) { return mx[cidx(g, wrap(a, g.nx), wrap(b, g.ny), c)]; };
-    auto V = [&](int a, int b, int c) { return my[cidx(g, wrap(a, g.nx), wrap(b, g.ny), c)]; };
-    double sx, sy, u, v;
-    mt_slopes(z, g, i, j, k, sx, sy);
-    zface_uv(i, j, k, U, V, u, v);
-    return om + sx * u + sy * v;
-}
-
-// the substep's z_t less the stage's (ERF_TI_fast_rhs_fun.H:66-90)
-static __global__ void k_mt_zpt(Params P, const double* __restrict__ zo, const double* __restrict__ zn, double inv_dt,
-                         double* __restrict__ zpt) {
-    const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny || k > g.nz) return;
-    auto N = [&](int a, int b) { return znode(zn, g, a, b, k); };
-    auto O = [&](int a, int b) { return znode(zo, g, a, b, k); };
-    const int64_t f = cidx(g, i, j, k);
-    double v = 0.25 * inv_dt * (N(i + 1, j + 1) - O(i + 1, j + 1) + N(i, j + 1) - O(i, j + 1) + N(i + 1, j) - O(i + 1, j) + N(i, j) - O(i, j));
-    zpt[f] = v - P.mt_zt[f];
-}
-// detJ of a grid's cells (make_J)
-static __global__ void k_mt_detj(Params P, const double* __restrict__ z, double* __restrict__ detJ) {
-    const Geo& g = P.g;
-    int i, j, k;
-    if (!cell_ij(g, i, j, k)) return;
-    detJ[cidx(g, i, j, k)] = mt_detj(z, g, i, j, k);
-}
-
-// x / y momenta of the substep, h_zeta-weighted on the old grid
-// (ERF_fast_rhs_MT.cpp:197-273); d(rho theta) extrapolated with or without
-// the lagged correction; the new lag.
-template <class R>
-__global__ void k_mt_fast_h(Params P, int step, int lagged, double dtau, StateBuf Sprev, StateBuf Sst, StageAux<R> A,
-                            const R* __restrict__ Fmx, const R* __restrict__ Fmy, const R* __restrict__ lag_in,
-                            R* __restrict__ lag_out, const double* __restrict__ zo, StateBuf Ssum) {
-    const Geo& g = P.g;
-    int i, j, k;
-    if (!cell_ij(g, i, j, k)) return;
-    const int nz = g.nz;
-    const int64_t N = g.ncell;
-    const int im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
-    const int64_t c = cidx(g, i, j, k), cxm = cidx(g, im, j, k), cym = cidx(g, i, jm, k);
-    const double beta_d = 0.1, dxi = g.dxi, dyi = g.dyi, dzi = g.dzi;
-    auto extrap = [&](int ii, int jj, int kk) {
-        int64_t e = cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), clampk(kk, nz));
-        double d = Sprev.cons[N + e] - Sst.cons[N + e];
-        if (step == 0 || !lagged) return d;
-        return d + beta_d * (d - double(lag_in[e]));
-    };
-    if (step == 0 || lagged) lag_out[c] = R(Sprev.cons[N + c] - Sst.cons[N + c]);
-    double mx, my;
-    {
-        double hxi = mt_hxI(zo, g, i, j, k), hz = mt_hzI(zo, g, i, j, k);
-        double gp_xi = (extrap(i, j, k) - extrap(i - 1, j, k)) * dxi;
-        double gp_zeta = (k == 0) ? 0.5 * dzi * (extrap(i - 1, j, k + 1) + extrap(i, j, k + 1) - extrap(i - 1, j, k) - extrap(i, j, k))
-                                  : 0.25 * dzi * (extrap(i - 1, j, k + 1) + extrap(i, j, k + 1) - extrap(i - 1, j, k - 1) - extrap(i, j, k - 1));
-        double gpx = hz * gp_xi - hxi * gp_zeta;
-        gpx *= 1.0;
-        double pi_c = 0.5 * (double(A.pi[cxm]) + double(A.pi[c]));
-        double f = -Gamma_ * R_d * pi_c * gpx;
-        mx = hz * Sprev.mx[c] + dtau * f + dtau * double(Fmx[c]);
-    }
-    {
-        double het = mt_hetaJ(zo, g, i, j, k), hz = mt_hzJ(zo, g, i, j, k);
-        double gp_eta = (extrap(i, j, k) - extrap(i, j - 1, k)) * dyi;
-        double gp_zeta = (k == 0) ? 0.5 * dzi * (extrap(i, j, k + 1) + extrap(i, j - 1, k + 1) - extrap(i, j, k) - extrap(i, j - 1, k))
-                                  : 0.25 * dzi * (extrap(i, j, k + 1) + extrap(i, j - 1, k + 1) - extrap(i, j, k - 1) - extrap(i, j - 1, k - 1));
-        double gpy = hz * gp_eta - het * gp_zeta;
-        gpy *= 1.0;
-        double pi_c = 0.5 * (double(A.pi[cym]) + double(A.pi[c]));
-        double f = -Gamma_ * R_d * pi_c * gpy;
-        my = hz * Sprev.my[c] + dtau * f + dtau * double(Fmy[c]);
-    }
-    Ssum.mx[c] = mx;
-    Ssum.my[c] = my;
-}
-
-// horizontal fluxes of rho and rho theta (the weighted momenta less the
-// stage's on the stage grid) and Omega'' of the previous substep on the old
-// grid (ERF_fast_rhs_MT.cpp:283-340).  After the first substep the previous
-// and new states are one, so Omega'' reads the weighted momenta, as the
-// reference's aliased arrays do.
-template <class R>
-__global__ void k_mt_fast_flux(Params P, StateBuf Sprev, StateBuf Sst, StageAux<R> A, StateBuf Ssum,
-                               const double* __restrict__ zo, const double* __restrict__ zs,
-                               const double* __restrict__ zpt, double* __restrict__ trhs, double* __restrict__ om) {
-    const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny || k > g.nz) return;
-    const int nz = g.nz;
-    const int64_t N = g.ncell, f = cidx(g, i, j, k);
-    if (k < nz) {
-        const int ip = wrap(i + 1, g.nx), im = wrap(i - 1, g.nx), jp = wrap(j + 1, g.ny), jm = wrap(j - 1, g.ny);
-        const int64_t cxp = cidx(g, ip, j, k), cyp = cidx(g, i, jp, k);
-        double xl = Ssum.mx[f] - Sst.mx[f] * mt_hzI(zs, g, i, j, k), xh = Ssum.mx[cxp] - Sst.mx[cxp] * mt_hzI(zs, g, i + 1, j, k);
-        double yl = Ssum.my[f] - Sst.my[f] * mt_hzJ(zs, g, i, j, k), yh = Ssum.my[cyp] - Sst.my[cyp] * mt_hzJ(zs, g, i, j + 1, k);
-        auto th = [&](int a, int b) { return double(A.prim[cidx(g, a, b, k)]); };
-        const double t0 = th(i, j);
-        trhs[f] = (xh - xl) * g.dxi + (yh - yl) * g.dyi;
-        trhs[N + f] = ((xh * (t0 + th(ip, j)) - xl * (t0 + th(im, j))) * g.dxi +
-                       (yh * (t0 + th(i, jp)) - yl * (t0 + th(i, jm))) * g.dyi) * 0.5;
-    }
-    double o;
-    if (k == 0) o = 0.;
-    else if (k == nz) o = Sprev.mz[f] - Sst.mz[f] - zpt[f];
-    else {
-        double a = mt_omega(zo, g, i, j, k, Sprev.mz[f], Sprev.mx, Sprev.my);
-        double b = mt_omega(zo, g, i, j, k, Sst.mz[f], Sst.mx, Sst.my);
-        o = (a - b) - zpt[f];
-    }
-    om[f] = o;
-}
-
-// the horizontal momenta divided by the new grid's h_zeta; their average
-template <class R>
-__global__ void k_mt_fast_div(Params P, double facinv, StateBuf Sst, const double* __restrict__ zn, StateBuf Ssum,
-                              R* __restrict__ avx, R* __restrict__ avy) {
-    const Geo& g = P.g;
-    int i, j, k;
-    if (!cell_ij(g, i, j, k)) return;
-    const int64_t c = cidx(g, i, j, k);
-    double mx = Ssum.mx[c] / mt_hzI(zn, g, i, j, k);
-    double my = Ssum.my[c] / mt_hzJ(zn, g, i, j, k);
-    Ssum.mx[c] = mx;
-    Ssum.my[c] = my;
-    avx[c] += R(facinv * (mx - Sst.mx[c]));
-    avy[c] += R(facinv * (my - Sst.my[c]));
-}
-
-// The Omega'' column system (ERF_fast_rhs_MT.cpp:375-600) in four kernels:
-// its right-hand side (one thread per z face: the old / new / stage face
-// detJ, the stage's coefficients made on the substep's old grid), the
-// Thomas sweep (one thread per column, the only serial part), rho w from
-// Omega'' with the ground at W from Omega = rho (z_t + z_t'') (one thread
-// per face), then the vertical fluxes, the average contravariant momentum
-// and rho / rho theta detJ-weighted old -> new (one thread per cell).
-// soln: the right-hand side, then the solution, then the new Omega''.
-template <class R>
-__global__ void k_mt_col_rhs(Params P, double dtau, double beta_1, double beta_2, StateBuf Sprev, StateBuf Sst,
-                             StageAux<R> A, const R* __restrict__ Fcons, const R* __restrict__ Fmz,
-                             const R* __restrict__ cP, const R* __restrict__ cQ, const double* __restrict__ zo,
-                             const double* __restrict__ zn, const double* __restrict__ zs,
-                             const double* __restrict__ zpt, const double* __restrict__ om,
-                             const double* __restrict__ trhs, StateBuf Ssum, double* __restrict__ soln) {
-    const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny || k > g.nz) return;
-    const int nz = g.nz;
-    const int64_t N = g.ncell;
-    auto C = [&](int kk) { return cidx(g, i, j, kk); };
-    const int64_t a = C(k);
-    if (k == 0) {
-        const double rho_on_bdy = 0.5 * (Sprev.cons[a] + Sprev.cons[a]);
-        soln[a] = rho_on_bdy * zpt[a];
-        return;
-    }
-    if (k == nz) {
-        soln[a] = 0.0;
-        return;
-    }
-    const double dzi = g.dzi, halfg = fabs(0.5 * -P.gravity);
-    auto th = [&](int kk) { return double(A.prim[C(clampk(kk, nz))]); };
-    auto fJ = [&](const double* z) { return 0.5 * (mt_detj(z, g, i, j, k) + mt_detj(z, g, i, j, k - 1)); };
-    const double Jo = fJ(zo), Jn = fJ(zn), Js = fJ(zs);
-    const double cp = double(cP[a]), cq = double(cQ[a]);
-    const double tlo = 0.5 * (th(k - 2) + th(k - 1)), tmid = 0.5 * (th(k - 1) + th(k)), thi = 0.5 * (th(k) + th(k + 1));
-    const int64_t b = C(k - 1);
-    double R0t = cp * Sprev.cons[N + a] * Jo + cq * Sprev.cons[N + b] * Jo
-                 - cp * Sst.cons[N + a] * Js - cq * Sst.cons[N + b] * Js
-                 - halfg * (Sprev.cons[a] + Sprev.cons[b]) * Jo
-                 + halfg * (Sst.cons[a] + Sst.cons[b]) * Js;
-    double R1t = -halfg * (double(Fcons[a]) + double(Fcons[b])) + (cp * double(Fcons[N + a]) + cq * double(Fcons[N + b]));
-    const double Okp1 = om[C(k + 1)], Ok = om[a], Okm1 = om[b];
-    R1t += (halfg) * (beta_1 * dzi * (Okp1 - Okm1) + trhs[a] + trhs[b]);
-    R1t += -(cp * (beta_1 * dzi * (Okp1 * thi - Ok * tmid) + trhs[N + a]) +
-             cq * (beta_1 * dzi * (Ok * tmid - Okm1 * tlo) + trhs[N + b]));
-    double rhs = Jo * Sprev.mz[a] - Js * Sst.mz[a] + dtau * (double(Fmz[a]) + R0t + dtau * beta_2 * R1t);
-    double un = mt_omega(zn, g, i, j, k, 0., Ssum.mx, Ssum.my);
-    double us = mt_omega(zs, g, i, j, k, 0., Sst.mx, Sst.my);
-    rhs += Jn * un - Js * us;
-    soln[a] = rhs;
-}
-template <class R>
-__global__ void k_mt_col_sweep(Params P, StateBuf Sst, const R* __restrict__ cA, const R* __restrict__ cInvB,
-                               const R* __restrict__ cCB, StateBuf Ssum, double* __restrict__ soln) {
-    const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    const int nz = g.nz;
-    auto C = [&](int kk) { return cidx(g, i, j, kk); };
-    double s = soln[C(0)] * double(cInvB[C(0)]);
-    soln[C(0)] = s;
-    for (int k = 1; k <= nz; ++k) {
-        s = (soln[C(k)] - double(cA[C(k)]) * s) * double(cInvB[C(k)]);
-        soln[C(k)] = s;
-    }
-    Ssum.mz[C(nz)] = Sst.mz[C(nz)] + s;
-    for (int k = nz - 1; k >= 0; --k) {
-        s = soln[C(k)] - double(cCB[C(k)]) * s;
-        soln[C(k)] = s;
-    }
-}
-template <class R>
-__global__ void k_mt_col_w(Params P, StateBuf Sprev, StateBuf Sst, const double* __restrict__ zo,
-                           const double* __restrict__ zn, const double* __restrict__ zs,
-                           const double* __restrict__ zpt, StateBuf Ssum, double* __restrict__ soln) {
-    const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny || k >= g.nz) return;
-    const int64_t a = cidx(g, i, j, k);
-    const double rho_on_face = 0.5 * (Sprev.cons[a] + Sprev.cons[cidx(g, i, j, k > 0 ? k - 1 : 0)]);
-    if (k == 0) {
-        Ssum.mz[a] = mt_wfrom(zn, g, i, j, 0, rho_on_face * (P.mt_zt[a] + zpt[a]), Ssum.mx, Ssum.my);
-        soln[a] = 0.;
-        return;
-    }
-    auto fJ = [&](const double* z) { return 0.5 * (mt_detj(z, g, i, j, k) + mt_detj(z, g, i, j, k - 1)); };
-    double wn = mt_wfrom(zn, g, i, j, k, 0.0, Ssum.mx, Ssum.my);
-    double ws = mt_wfrom(zs, g, i, j, k, 0.0, Sst.mx, Sst.my);
-    double wpp = soln[a] + (wn - ws);
-    double m = fJ(zo) * (Sst.mz[a] + wpp);
-    m /= fJ(zn);
-    Ssum.mz[a] = m;
-    double o1 = mt_omega(zn, g, i, j, k, m, Ssum.mx, Ssum.my);
-    double o2 = mt_omega(zs, g, i, j, k, Sst.mz[a], Sst.mx, Sst.my);
-    double sv = o1 - o2;
-    sv -= rho_on_face * zpt[a];
-    soln[a] = sv;
-}
-template <class R>
-__global__ void k_mt_col_cons(Params P, double dtau, double beta_1, double beta_2, double facinv, StateBuf Sprev,
-                              StageAux<R> A, const R* __restrict__ Fcons, const double* __restrict__ zo,
-                              const double* __restrict__ zn, const double* __restrict__ om,
-                              const double* __restrict__ trhs, const double* __restrict__ soln,
-                              R* __restrict__ avz, StateBuf Ssum) {
-    const Geo& g = P.g;
-    int i, j, k;
-    if (!cell_ij(g, i, j, k)) return;
-    const int nz = g.nz;
-    const int64_t N = g.ncell, a = cidx(g, i, j, k), ah = cidx(g, i, j, k + 1);
-    auto th = [&](int kk) { return double(A.prim[cidx(g, i, j, clampk(kk, nz))]); };
-    double zl = beta_2 * soln[a] + beta_1 * om[a];
-    double zh = beta_2 * soln[ah] + beta_1 * om[ah];
-    avz[a] += R(facinv * zl / (1.0 * 1.0));
-    if (k == nz - 1) avz[ah] += R(facinv * zh / (1.0 * 1.0));
-    const double Jo = mt_detj(zo, g, i, j, k), Jn = mt_detj(zn, g, i, j, k);
-    double frho = -(trhs[a] + (zh - zl) * g.dzi);
-    double tr = Jo * Sprev.cons[a] + dtau * (double(Fcons[a]) + frho);
-    double frt = -(trhs[N + a] + 0.5 * (zh * (th(k) + th(k + 1)) - zl * (th(k) + th(k - 1))) * g.dzi);
-    double tt = Jo * Sprev.cons[N + a] + dtau * (double(Fcons[N + a]) + frt);
-    Ssum.cons[a] = tr / Jn;
-    Ssum.cons[N + a] = tt / Jn;
-}
-
-// the boundary fill after a substep (apply_bcs, fast variables): the
-// momenta through M -> V -> M with the walls' density ghosts; w on the flat
-// lid from Omega = 0, the moving ground untouched but round-tripped
-static __global__ void k_mt_fast_bc(Params P, StateBuf Ssum) {
-    const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny || k > g.nz) return;
-    const int nz = g.nz;
-    const int64_t f = cidx(g, i, j, k);
-    if (k < nz) {
-        double rs = Ssum.cons[f] + Ssum.cons[cidx(g, wrap(i - 1, g.nx), j, k)];
-        double u = (Ssum.mx[f] * 2.0) / rs;
-        Ssum.mx[f] = (u * 0.5) * rs;
-        rs = Ssum.cons[f] + Ssum.cons[cidx(g, i, wrap(j - 1, g.ny), k)];
-        double v = (Ssum.my[f] * 2.0) / rs;
-        Ssum.my[f] = (v * 0.5) * rs;
-    }
-    if (k == nz) {
-        Ssum.mz[f] = 0.0;   // W from Omega = 0 on the flat lid
-    } else {
-        double rs = Ssum.cons[f] + Ssum.cons[k > 0 ? f - g.sk : f];
-        double w = (Ssum.mz[f] * 2.0) / rs;
-        Ssum.mz[f] = (w * 0.5) * rs;
-    }
-}
-
 #if !ERFB_TER_F32
 void launch_mt_grid_sub(const Params& P, cudaStream_t st, const double* tdev, double dtau, int ks, double* z) {
-    k_mt_grid<<<ter_grid(P.g, 1), ter_block(), 0, st>>>(P, tdev, dtau, -1 - ks, z);
+    k_mt_grid<<<ter_grid(P.g, P.g.nz + 3), ter_block(), 0, st>>>(P, tdev, dtau, -1 - ks, z);
 }
 #endif
-#if !ERFB_TER_F32
-void launch_mt_zpt(const Params& P, cudaStream_t st, const double* zo, const double* zn, double dtau, double* zpt) {
-    k_mt_zpt<<<ter_grid(P.g, P.g.nz + 1), ter_block(), 0, st>>>(P, zo, zn, 1. / dtau, zpt);
-}
-#endif
-#if !ERFB_TER_F32
-void launch_mt_detj(const Params& P, cudaStream_t st, const double* z, double* detJ) {
-    k_mt_detj<<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(P, z, detJ);
-}
-#endif
-template <class R>
-void launch_mt_fast(const Params& P, cudaStream_t st, int step, int lagged, double dtau, double beta_s, double facinv,
-                    StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fcons, const R* Fmx, const R* Fmy,
-                    const R* Fmz, const R* lag_in, R* lag_out, const R* cA, const R* cInvB, const R* cCB, const R* cP,
-                    const R* cQ, const double* zo, const double* zn, const double* zs, const double* zpt,
-                    double* trhs, double* om, double* soln, R* avx, R* avy, R* avz, StateBuf Ssum, int last) {
-    const Geo& g = P.g;
-    const double beta_1 = 0.5 * (1.0 - beta_s), beta_2 = 0.5 * (1.0 + beta_s);
-    k_mt_fast_h<R><<<ter_grid(g, g.nz), ter_block(), 0, st>>>(P, step, lagged, dtau, Sprev, Sst, A, Fmx, Fmy, lag_in,
-                                                              lag_out, zo, Ssum);
-    k_mt_fast_flux<R><<<ter_grid(g, g.nz + 1), ter_block(), 0, st>>>(P, Sprev, Sst, A, Ssum, zo, zs, zpt, trhs, om);
-    k_mt_fast_div<R><<<ter_grid(g, g.nz), ter_block(), 0, st>>>(P, facinv, Sst, zn, Ssum, avx, avy);
-    k_mt_col_rhs<R><<<ter_grid(g, g.nz + 1), ter_block(), 0, st>>>(P, dtau, beta_1, beta_2, Sprev, Sst, A, Fcons, Fmz,
-                                                                  cP, cQ, zo, zn, zs, zpt, om, trhs, Ssum, soln);
-    k_mt_col_sweep<R><<<ter_grid(g, 1), ter_block(), 0, st>>>(P, Sst, cA, cInvB, cCB, Ssum, soln);
-    k_mt_col_w<R><<<ter_grid(g, g.nz), ter_block(), 0, st>>>(P, Sprev, Sst, zo, zn, zs, zpt, Ssum, soln);
-    k_mt_col_cons<R><<<ter_grid(g, g.nz), ter_block(), 0, st>>>(P, dtau, beta_1, beta_2, facinv, Sprev, A, Fcons, zo, zn,
-                                                                om, trhs, soln, avz, Ssum);
-    if (!last) k_mt_fast_bc<<<ter_grid(g, g.nz + 1), ter_block(), 0, st>>>(P, Ssum);
-}
-#if !ERFB_TER_F32
-template void launch_mt_fast<double>(const Params&, cudaStream_t, int, int, double, double, double, StateBuf, StateBuf,
-                                     StageAux<double>, const double*, const double*, const double*, const double*,
-                                     const double*, double*, const double*, const double*, const double*,
-                                     const double*, const double*, const double*, const double*, const double*,
-                                     const double*, double*, double*, double*, double*, double*, double*, StateBuf, int);
-#else
-template void launch_mt_fast<float>(const Params&, cudaStream_t, int, int, double, double, double, StateBuf, StateBuf,
-                                    StageAux<float>, const float*, const float*, const float*, const float*,
-                                    const float*, float*, const float*, const float*, const float*, const float*,
-                                    const float*, const double*, const double*, const double*, const double*, double*,
-                                    double*, double*, float*, float*, float*, StateBuf, int);
-#endif
-
 // ---------------------------------------------------------------------------
 // Step diagnostics of a resident state (sum_integrated_quantities /
 // volWgtSumMF, IO/ERF_WriteScalarProfiles.cpp:14-60, 378-420): the
