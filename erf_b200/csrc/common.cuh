@@ -277,5 +277,25 @@ __device__ __forceinline__ int64_t cidx(const Geo& g, int i, int j, int k) {
 #endif
     return (int64_t)i + (int64_t)g.nx * j + g.sk * k;
 }
+// The same in 32 bits, for ld / at below.
+__device__ __forceinline__ uint32_t eidx(const Geo& g, int i, int j, int k) {
+#ifdef ERF_B200_BOUNDS
+    return (uint32_t)cidx(g, i, j, k);
+#else
+    return (uint32_t)i + (uint32_t)g.nx * (uint32_t)j + (uint32_t)g.sk * (uint32_t)k;
+#endif
+}
+// Element e of an array of one component.  The byte offset stays in 32 bits
+// (an array of 4 GB would be 5e8 cells, more than the card holds), so that a
+// thread keeps one offset register per neighbour for all the arrays instead
+// of forming a 64-bit address per load.
+template <class T>
+__device__ __forceinline__ T ld(const T* p, uint32_t e) {
+    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + e * (uint32_t)sizeof(T)));
+}
+template <class T>
+__device__ __forceinline__ T& at(T* p, uint32_t e) {
+    return *reinterpret_cast<T*>(reinterpret_cast<char*>(p) + e * (uint32_t)sizeof(T));
+}
 
 }  // namespace erfb

@@ -6,7 +6,8 @@
 // conditions, so no separate ghost-fill pass is launched between stages and
 // substeps; the reference's momentum<->velocity round trips at every boundary
 // fill (BoundaryConditions/ERF_FillIntermediatePatch.cpp:63-67, 224-236) are
-// applied inline where the filled values are next read.
+// the identity but for rounding (two divisions and an ulp each) and are not
+// applied.
 //
 // The dycore kernels are templates on R, the type of the bulk arrays (derived
 // fields, slow right-hand sides, average momenta, fast coefficients, stresses)
@@ -28,9 +29,9 @@ namespace erfb {
 // the ghost value is 0 (no-slip, ext_dir) or the nearest interior value
 // (slip, foextrap): ERF_BoundaryConditions_xvel.cpp:190-230.
 __device__ __forceinline__ double tang(const double* __restrict__ f, const Geo& g, int i, int j, int k) {
-    if (k < 0) return g.zlo_noslip ? 0.0 : __ldg(f + cidx(g, i, j, 0));
-    if (k >= g.nz) return g.zhi_noslip ? 0.0 : __ldg(f + cidx(g, i, j, g.nz - 1));
-    return __ldg(f + cidx(g, i, j, k));
+    if (k < 0) return g.zlo_noslip ? 0.0 : ld(f, eidx(g, i, j, 0));
+    if (k >= g.nz) return g.zhi_noslip ? 0.0 : ld(f, eidx(g, i, j, g.nz - 1));
+    return ld(f, eidx(g, i, j, k));
 }
 // ---------------------------------------------------------------------------
 // MOST ground (ABLMost::compute_most_bcs with moeng_flux, implicit MOST,
@@ -112,26 +113,26 @@ __device__ __forceinline__ double tang_v(const Params& P, const MostView& m, int
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double strain12(const double* u, const double* v, const Geo& g, int i, int j, int k) {
     int im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
-    return 0.5 * ((__ldg(u + cidx(g, i, j, k)) - __ldg(u + cidx(g, i, jm, k))) * g.dyi +
-                  (__ldg(v + cidx(g, i, j, k)) - __ldg(v + cidx(g, im, j, k))) * g.dxi);
+    return 0.5 * ((ld(u, eidx(g, i, j, k)) - ld(u, eidx(g, i, jm, k))) * g.dyi +
+                  (ld(v, eidx(g, i, j, k)) - ld(v, eidx(g, im, j, k))) * g.dxi);
 }
 // Stage strain at the ground face of a MOST ground: the centred difference
 // with the MOST ghost velocity below
 __device__ __forceinline__ double strain13_most(const Params& P, const MostView& m, const double* w, int i, int j) {
     const Geo& g = P.g;
     int im = wrap(i - 1, g.nx);
-    double wx = (__ldg(w + cidx(g, i, j, 0)) - __ldg(w + cidx(g, im, j, 0))) * g.dxi;
+    double wx = (ld(w, eidx(g, i, j, 0)) - ld(w, eidx(g, im, j, 0))) * g.dxi;
     return 0.5 * ((tang_u(P, m, i, j, 0) - tang_u(P, m, i, j, -1)) * g.dzi + wx);
 }
 __device__ __forceinline__ double strain23_most(const Params& P, const MostView& m, const double* w, int i, int j) {
     const Geo& g = P.g;
     int jm = wrap(j - 1, g.ny);
-    double wy = (__ldg(w + cidx(g, i, j, 0)) - __ldg(w + cidx(g, i, jm, 0))) * g.dyi;
+    double wy = (ld(w, eidx(g, i, j, 0)) - ld(w, eidx(g, i, jm, 0))) * g.dyi;
     return 0.5 * ((tang_v(P, m, i, j, 0) - tang_v(P, m, i, j, -1)) * g.dzi + wy);
 }
 __device__ __forceinline__ double strain13(const double* u, const double* w, const Geo& g, int i, int j, int k) {
     int im = wrap(i - 1, g.nx);
-    double wx = (__ldg(w + cidx(g, i, j, k)) - __ldg(w + cidx(g, im, j, k))) * g.dxi;
+    double wx = (ld(w, eidx(g, i, j, k)) - ld(w, eidx(g, im, j, k))) * g.dxi;
     if (k == 0 && g.zlo_noslip)
         return 0.5 * ((-(8. / 3.) * tang(u, g, i, j, k - 1) + 3. * tang(u, g, i, j, k) - (1. / 3.) * tang(u, g, i, j, k + 1)) * g.dzi + wx);
     if (k == g.nz && g.zhi_noslip)
@@ -140,7 +141,7 @@ __device__ __forceinline__ double strain13(const double* u, const double* w, con
 }
 __device__ __forceinline__ double strain23(const double* v, const double* w, const Geo& g, int i, int j, int k) {
     int jm = wrap(j - 1, g.ny);
-    double wy = (__ldg(w + cidx(g, i, j, k)) - __ldg(w + cidx(g, i, jm, k))) * g.dyi;
+    double wy = (ld(w, eidx(g, i, j, k)) - ld(w, eidx(g, i, jm, k))) * g.dyi;
     if (k == 0 && g.zlo_noslip)
         return 0.5 * ((-(8. / 3.) * tang(v, g, i, j, k - 1) + 3. * tang(v, g, i, j, k) - (1. / 3.) * tang(v, g, i, j, k + 1)) * g.dzi + wy);
     if (k == g.nz && g.zhi_noslip)
@@ -164,11 +165,13 @@ __device__ __forceinline__ void stage_aux_cell(const Params& P, const double* __
     const int64_t N = P.g.ncell;
     double rho = cons[c];
     double rt = cons[N + c];
-    A.prim[c] = R(rt / rho);
-    for (int n = 1; n < P.nprim; ++n) A.prim[n * N + c] = R(cons[(n + 1) * N + c] / rho);
-    A.pi[c] = R(eos_exner(rt, P.rdOcp));
-    double qv = P.moist ? cons[5 * N + c] / rho : 0.0;
-    A.pp[c] = R(eos_p(rt, qv) - (P.ter ? P.p0[c + P.g.sk] : P.p0[k + 1]));
+    const double ir = 1.0 / rho;
+    A.prim[c] = R(rt * ir);
+    for (int n = 1; n < P.nprim; ++n) A.prim[n * N + c] = R(cons[(n + 1) * N + c] * ir);
+    const double x = R_d * rt * ip_0, l = log(x);   // of the Exner function, and of p where the air is dry
+    A.pi[c] = R(exp(Gamma_ * P.rdOcp * l));
+    const double lp = P.moist ? log(x * (1.0 + (R_v / R_d) * (cons[5 * N + c] * ir))) : l;
+    A.pp[c] = R(p_0 * exp(Gamma_ * lp) - (P.ter ? P.p0[c + P.g.sk] : P.p0[k + 1]));
     if (!(rt > 0.0) || !(rho > 0.0)) atomicOr(P.status, ST_BADSTATE);
 }
 
@@ -177,8 +180,7 @@ __device__ __forceinline__ void stage_aux_cell(const Params& P, const double* __
 //   * ComputeStrain_N + ComputeTurbulentViscosityLES (Smagorinsky) from the
 //     old velocities (ERF_advance_dycore.cpp:114-223,
 //     ERF_ComputeTurbulentViscosity.cpp:85-126; EddyViscosity.H:31-83);
-//   * VelocityToMomentum of the old velocities, the MomentumToVelocity /
-//     VelocityToMomentum round trip of apply_bcs(state_old)
+//   * VelocityToMomentum of the old velocities
 //     (ERF_advance_dycore.cpp:260-276);
 //   * cons_to_prim / pi_stage / p' of the old state.
 // ---------------------------------------------------------------------------
@@ -195,20 +197,17 @@ __global__ void k_step_begin(Params P, const double* __restrict__ cons, const do
     double rho = cons[c];
     {
         double rs = rho + cons[cidx(g, im, j, k)];
-        double m0 = (uo[c] * 0.5) * rs, u1 = (m0 * 2.0) / rs;
-        S.mx[c] = (u1 * 0.5) * rs; un[c] = u1;
+        S.mx[c] = (uo[c] * 0.5) * rs; un[c] = uo[c];
     }
     {
         double rs = rho + cons[cidx(g, i, jm, k)];
-        double m0 = (vo[c] * 0.5) * rs, v1 = (m0 * 2.0) / rs;
-        S.my[c] = (v1 * 0.5) * rs; vn[c] = v1;
+        S.my[c] = (vo[c] * 0.5) * rs; vn[c] = vo[c];
     }
     if (k == 0) {
         S.mz[c] = 0.0; wn[c] = 0.0;
     } else {
         double rs = rho + cons[cidx(g, i, j, k - 1)];
-        double m0 = (wo[c] * 0.5) * rs, w1 = (m0 * 2.0) / rs;
-        S.mz[c] = (w1 * 0.5) * rs; wn[c] = w1;
+        S.mz[c] = (wo[c] * 0.5) * rs; wn[c] = wo[c];
     }
     if (k == g.nz - 1) { S.mz[c + g.sk] = 0.0; wn[c + g.sk] = 0.0; }
     // a NaN or infinite velocity in the step's input (the state checks of
@@ -219,8 +218,8 @@ __global__ void k_step_begin(Params P, const double* __restrict__ cons, const do
 
     if (P.les == ERF_LES_SMAGORINSKY || P.les == ERF_LES_MLP || P.les == ERF_LES_DEARDORFF) {
         int ip = wrap(i + 1, g.nx), jp = wrap(j + 1, g.ny);
-        double s11 = (uo[cidx(g, ip, j, k)] - uo[c]) * g.dxi;
-        double s22 = (vo[cidx(g, i, jp, k)] - vo[c]) * g.dyi;
+        double s11 = (ld(uo, eidx(g, ip, j, k)) - uo[c]) * g.dxi;
+        double s22 = (ld(vo, eidx(g, i, jp, k)) - vo[c]) * g.dyi;
         double s33 = (wo[c + g.sk] - wo[c]) * g.dzi;
         double s12 = 0.25 * (strain12(uo, vo, g, i, j, k) + strain12(uo, vo, g, i, jp, k) +
                              strain12(uo, vo, g, ip, j, k) + strain12(uo, vo, g, ip, jp, k));
@@ -291,11 +290,11 @@ __global__ void k_tau(Params P, const double* __restrict__ cons, const double* _
     int i, j, k;
     if (!cell_coords(g, i, j, k)) return;
     int im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny), ip = wrap(i + 1, g.nx), jp = wrap(j + 1, g.ny);
-    int64_t c = cidx(g, i, j, k);
+    const uint32_t c = eidx(g, i, j, k);
     const R OneThird = R(1. / 3.);
-    R s11 = R((u[cidx(g, ip, j, k)] - u[c]) * g.dxi);
-    R s22 = R((v[cidx(g, i, jp, k)] - v[c]) * g.dyi);
-    R s33 = R((w[c + g.sk] - w[c]) * g.dzi);
+    R s11 = R((ld(u, eidx(g, ip, j, k)) - ld(u, c)) * g.dxi);
+    R s22 = R((ld(v, eidx(g, i, jp, k)) - ld(v, c)) * g.dyi);
+    R s33 = R((ld(w, c + (uint32_t)g.sk) - ld(w, c)) * g.dzi);
     R er = s11 + s22 + s33;
     const R mu_eff = R(P.mu_eff);
     R base = P.use_consA ? R(cons[c]) * mu_eff : mu_eff;
@@ -303,15 +302,15 @@ __global__ void k_tau(Params P, const double* __restrict__ cons, const double* _
     t11[c] = -m11 * (s11 - OneThird * er);
     t22[c] = -m11 * (s22 - OneThird * er);
     t33[c] = -m11 * (s33 - OneThird * er);
-    auto mu = [&](int ii, int jj, int kk) { return __ldg(mut + cidx(g, ii, jj, clampk(kk, g.nz))); };
-    auto rho = [&](int ii, int jj, int kk) { return R(__ldg(cons + cidx(g, ii, jj, clampk(kk, g.nz)))); };
+    auto mu = [&](int ii, int jj, int kk) { return ld(mut, eidx(g, ii, jj, clampk(kk, g.nz))); };
+    auto rho = [&](int ii, int jj, int kk) { return R(ld(cons, eidx(g, ii, jj, clampk(kk, g.nz)))); };
     {
         R m = P.use_consA ? R(0.25) * (rho(im, j, k) + rho(i, j, k) + rho(im, jm, k) + rho(i, jm, k)) * mu_eff : mu_eff;
         if (P.use_turb) m = m + R(2) * (R(0.25) * (mu(im, j, k) + mu(i, j, k) + mu(im, jm, k) + mu(i, jm, k)));
         t12[c] = R(strain12(u, v, g, i, j, k)) * -m;
     }
     for (int kk = k; kk <= (k == g.nz - 1 ? g.nz : k); ++kk) {
-        int64_t e = cidx(g, i, j, kk);
+        const uint32_t e = eidx(g, i, j, kk);
         R m = P.use_consA ? R(0.25) * (rho(im, j, kk) + rho(i, j, kk) + rho(im, j, kk - 1) + rho(i, j, kk - 1)) * mu_eff : mu_eff;
         if (P.use_turb) m = m + R(2) * (R(0.25) * (mu(im, j, kk) + mu(i, j, kk) + mu(im, j, kk - 1) + mu(i, j, kk - 1)));
         t13[e] = R(strain13(u, w, g, i, j, kk)) * -m;
@@ -331,8 +330,8 @@ __global__ void k_tau_most_ground(Params P, const double* __restrict__ cons, con
     if (i >= g.nx || j >= g.ny) return;
     const int im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
     const R mu_eff = R(P.mu_eff);
-    auto mu = [&](int ii, int jj, int kk) { return __ldg(mut + cidx(g, ii, jj, clampk(kk, g.nz))); };
-    auto rho = [&](int ii, int jj, int kk) { return R(__ldg(cons + cidx(g, ii, jj, clampk(kk, g.nz)))); };
+    auto mu = [&](int ii, int jj, int kk) { return ld(mut, eidx(g, ii, jj, clampk(kk, g.nz))); };
+    auto rho = [&](int ii, int jj, int kk) { return R(ld(cons, eidx(g, ii, jj, clampk(kk, g.nz)))); };
     const MostView mv{u, v, cons};
     const int64_t e = cidx(g, i, j, 0);
     R m = P.use_consA ? R(0.25) * (rho(im, j, 0) + rho(i, j, 0) + rho(im, j, -1) + rho(i, j, -1)) * mu_eff : mu_eff;
@@ -453,14 +452,25 @@ __global__ void k_plane_avg(Params P, const double* __restrict__ cons, const R* 
 }
 
 // Momentum flux helper: vertical stencil of a face velocity (FP64 state) in R
-// (ERF_AdvectionSrcForMom_N.H:17-274).
+// (ERF_AdvectionSrcForMom_N.H:17-274); away from the walls six loads at
+// constant strides.
 template <int T, class R>
 __device__ __forceinline__ R gatherz_tang(const Geo& g, const double* f, int type, R upw, R frac, int i, int j, int k) {
     R s[6];
     const int w = width_of<T>(type);
-    for (int m = 0; m < 6; ++m) {
-        int off = m - 3;
-        s[m] = (off >= -w && off <= w - 1) ? R(tang(f, g, i, j, k + off)) : R(0);
+    if (k >= w && k + w <= g.nz) {
+        const uint32_t e = eidx(g, i, j, k), sk = (uint32_t)g.sk;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int off = m - 3;
+            s[m] = (off >= -w && off <= w - 1) ? R(ld(f, e + (uint32_t)off * sk)) : R(0);
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int off = m - 3;
+            s[m] = (off >= -w && off <= w - 1) ? R(tang(f, g, i, j, k + off)) : R(0);
+        }
     }
     return interp_of<T, R>(type, s, upw, frac);
 }
@@ -755,7 +765,8 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_CELL) k_slow_cell(Params 
     const int ip = ok ? wrap(i + 1, g.nx) : 0, jp = ok ? wrap(j + 1, g.ny) : 0;
     R zl = R(0), zh = R(0);
     const TileEdge edge = tile_edge(g);
-    load_plane(g, pl, A.prim, k0);
+    const PlaneIdx pidx(g);
+    load_plane(g, pidx, pl, A.prim, k0);
     for (int k = k0; k < k1; ++k) {
         plane_wait();
         __syncthreads();
@@ -764,7 +775,7 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_CELL) k_slow_cell(Params 
                              k, k == k0, zl, zh);
         tile_put_edge<TH>(g, edge, sh, pl, S.mx, S.my, P.dyc_h, R(P.f_dyc_h), k);
         __syncthreads();
-        if (k + 1 < k1) load_plane(g, pl, A.prim, k + 1);   // overlaps the update below
+        if (k + 1 < k1) load_plane(g, pidx, pl, A.prim, k + 1);   // overlaps the update below
         if (ok) {
             R frt = tile_div(g, sh, zl, zh);
             zl = zh;
@@ -806,8 +817,7 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_CELL) k_slow_cell(Params 
 //   * advection (average momenta) and diffusion of the slow scalars
 //     (passive scalar with the dry-scalar scheme; moisture with the moist
 //     scheme), S_new = S_old + slow_dt * RHS (FP64), moisture clipped at 0;
-//   * rho, rho*theta and the momenta copied from the fast solution, with the
-//     momentum/velocity round trips of the two boundary fills;
+//   * rho, rho*theta and the momenta copied from the fast solution;
 //   * the stage velocities, and (unless last) the next stage's primitive
 //     variables, Exner function and p'.
 // ---------------------------------------------------------------------------
@@ -838,13 +848,14 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_POST) k_post(Params P, in
 #pragma unroll
     for (int q = 0; q < NS; ++q) zl[q] = zh[q] = R(0);
     const TileEdge edge = tile_edge(g);
+    const PlaneIdx pidx(g);
     auto comp_of = [&](int q) {
         return q == 0 ? ERF_RHOSCALAR_COMP : (q < nscal ? ERF_RHOQ1_COMP + q - 1 : ERF_RHOKE_COMP);
     };
     auto slow_phi = [&](int q) { return Acur.prim + (int64_t)(comp_of(q) - 1) * N; };
 #pragma unroll
     for (int q = 0; q < NS; ++q)
-        if (q < nslow) load_plane(g, pl[q], slow_phi(q), k0);
+        if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k0);
     for (int k = k0; k < k1; ++k) {
         plane_wait();
         __syncthreads();
@@ -872,7 +883,7 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_POST) k_post(Params P, in
         if (k + 1 < k1) {   // next level's planes arrive during the update below
 #pragma unroll
             for (int q = 0; q < NS; ++q)
-                if (q < nslow) load_plane(g, pl[q], slow_phi(q), k + 1);
+                if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k + 1);
         }
         if (ok) {
             int64_t c = cidx(g, i, j, k);
@@ -906,27 +917,18 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_POST) k_post(Params P, in
             Snew.cons[3 * N + c] = Sst.cons[3 * N + c];
             double rho = Ssum.cons[c];
             {
-                double rs = rho + Ssum.cons[cidx(g, im, j, k)];
-                double m = Ssum.mx[c];
-                double u1 = (m * 2.0) / rs; m = (u1 * 0.5) * rs;
-                double u2 = (m * 2.0) / rs; m = (u2 * 0.5) * rs;
-                Snew.mx[c] = m; un[c] = u2;
+                const double rs = rho + Ssum.cons[cidx(g, im, j, k)], m = Ssum.mx[c];
+                Snew.mx[c] = m; un[c] = (m * 2.0) / rs;
             }
             {
-                double rs = rho + Ssum.cons[cidx(g, i, jm, k)];
-                double m = Ssum.my[c];
-                double v1 = (m * 2.0) / rs; m = (v1 * 0.5) * rs;
-                double v2 = (m * 2.0) / rs; m = (v2 * 0.5) * rs;
-                Snew.my[c] = m; vn[c] = v2;
+                const double rs = rho + Ssum.cons[cidx(g, i, jm, k)], m = Ssum.my[c];
+                Snew.my[c] = m; vn[c] = (m * 2.0) / rs;
             }
             if (k == 0) {
                 Snew.mz[c] = 0.0; wn[c] = 0.0;
             } else {
-                double rs = rho + Ssum.cons[c - g.sk];
-                double m = Ssum.mz[c];
-                double w1 = (m * 2.0) / rs; m = (w1 * 0.5) * rs;
-                double w2 = (m * 2.0) / rs; m = (w2 * 0.5) * rs;
-                Snew.mz[c] = m; wn[c] = w2;
+                const double rs = rho + Ssum.cons[c - g.sk], m = Ssum.mz[c];
+                Snew.mz[c] = m; wn[c] = (m * 2.0) / rs;
             }
             if (k == g.nz - 1) { Snew.mz[c + g.sk] = 0.0; wn[c + g.sk] = 0.0; }
             if (make_next) stage_aux_cell<R>(P, Snew.cons, Anext, c, k);
@@ -967,20 +969,20 @@ template <int HT, class R>
 __device__ __forceinline__ R xmom_flux_x(const Params& P, const double* ru, const Plane<double>& pu, int c0, int ty,
                                          int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(ru[cidx(g, wrap(i - 1, g.nx), j, k)]) + R(ru[cidx(g, i, j, k)]));
+    R a = R(0.5) * (R(ld(ru, eidx(g, wrap(i - 1, g.nx), j, k))) + R(ld(ru, eidx(g, i, j, k))));
     return a * plane_interp_x<HT, R>(pu, ty, c0, P.dyc_h, a, R(P.f_dyc_h));
 }
 template <int HT, class R>
 __device__ __forceinline__ R xmom_flux_y(const Params& P, const double* rv, const Plane<double>& pu, int tx, int r0,
                                          int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(rv[cidx(g, i, j, k)]) + R(rv[cidx(g, wrap(i - 1, g.nx), j, k)]));
+    R a = R(0.5) * (R(ld(rv, eidx(g, i, j, k))) + R(ld(rv, eidx(g, wrap(i - 1, g.nx), j, k))));
     return a * plane_interp_y<HT, R>(pu, r0, tx, P.dyc_h, a, R(P.f_dyc_h));
 }
 template <int VT, class R>
 __device__ __forceinline__ R xmom_flux_z(const Params& P, const double* rw, const MostView& mv, int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(rw[cidx(g, i, j, k)]) + R(rw[cidx(g, wrap(i - 1, g.nx), j, k)]));
+    R a = R(0.5) * (R(ld(rw, eidx(g, i, j, k))) + R(ld(rw, eidx(g, wrap(i - 1, g.nx), j, k))));
     if (P.most && k < 3) return a * gatherz_most<VT, R>(P, mv, 0, P.dyc_v, a, R(P.f_dyc_v), i, j, k);
     return a * gatherz_tang<VT, R>(g, mv.u, P.dyc_v, a, R(P.f_dyc_v), i, j, k);
 }
@@ -988,20 +990,20 @@ template <int HT, class R>
 __device__ __forceinline__ R ymom_flux_x(const Params& P, const double* ru, const Plane<double>& pv, int c0, int ty,
                                          int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(ru[cidx(g, i, j, k)]) + R(ru[cidx(g, i, wrap(j - 1, g.ny), k)]));
+    R a = R(0.5) * (R(ld(ru, eidx(g, i, j, k))) + R(ld(ru, eidx(g, i, wrap(j - 1, g.ny), k))));
     return a * plane_interp_x<HT, R>(pv, ty, c0, P.dyc_h, a, R(P.f_dyc_h));
 }
 template <int HT, class R>
 __device__ __forceinline__ R ymom_flux_y(const Params& P, const double* rv, const Plane<double>& pv, int tx, int r0,
                                          int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(rv[cidx(g, i, j, k)]) + R(rv[cidx(g, i, wrap(j - 1, g.ny), k)]));
+    R a = R(0.5) * (R(ld(rv, eidx(g, i, j, k))) + R(ld(rv, eidx(g, i, wrap(j - 1, g.ny), k))));
     return a * plane_interp_y<HT, R>(pv, r0, tx, P.dyc_h, a, R(P.f_dyc_h));
 }
 template <int VT, class R>
 __device__ __forceinline__ R ymom_flux_z(const Params& P, const double* rw, const MostView& mv, int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(rw[cidx(g, i, j, k)]) + R(rw[cidx(g, i, wrap(j - 1, g.ny), k)]));
+    R a = R(0.5) * (R(ld(rw, eidx(g, i, j, k))) + R(ld(rw, eidx(g, i, wrap(j - 1, g.ny), k))));
     if (P.most && k < 3) return a * gatherz_most<VT, R>(P, mv, 1, P.dyc_v, a, R(P.f_dyc_v), i, j, k);
     return a * gatherz_tang<VT, R>(g, mv.v, P.dyc_v, a, R(P.f_dyc_v), i, j, k);
 }
@@ -1009,14 +1011,14 @@ template <int HT, class R>
 __device__ __forceinline__ R zmom_flux_x(const Params& P, const double* ru, const Plane<double>& pw, int c0, int ty,
                                          int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(ru[cidx(g, i, j, k)]) + R(ru[cidx(g, i, j, k - 1)])) * R(1);
+    R a = R(0.5) * (R(ld(ru, eidx(g, i, j, k))) + R(ld(ru, eidx(g, i, j, k - 1)))) * R(1);
     return a * plane_interp_x<HT, R>(pw, ty, c0, P.dyc_h, a, R(P.f_dyc_h));
 }
 template <int HT, class R>
 __device__ __forceinline__ R zmom_flux_y(const Params& P, const double* rv, const Plane<double>& pw, int tx, int r0,
                                          int i, int j, int k) {
     const Geo& g = P.g;
-    R a = R(0.5) * (R(rv[cidx(g, i, j, k)]) + R(rv[cidx(g, i, j, k - 1)])) * R(1);
+    R a = R(0.5) * (R(ld(rv, eidx(g, i, j, k))) + R(ld(rv, eidx(g, i, j, k - 1)))) * R(1);
     return a * plane_interp_y<HT, R>(pw, r0, tx, P.dyc_h, a, R(P.f_dyc_h));
 }
 // Vertical flux of w between faces kk-1 and kk (the "lo" flux of face kk),
@@ -1028,7 +1030,8 @@ __device__ __forceinline__ R zmom_flux_z(const Params& P, const double* rw, cons
     const Geo& g = P.g;
     const int vt = P.dyc_v, lo_z_face = 0, hi_z_face = g.nz;
     const R vf = R(P.f_dyc_v);
-    auto wz = [&](int q) { return R(__ldg(w + cidx(g, i, j, q))); };
+    const uint32_t e0 = eidx(g, i, j, 0);
+    auto wz = [&](int q) { return R(ld(w, e0 + (uint32_t)g.sk * (uint32_t)q)); };
     auto all = [&](int q, R upw, R frac, int type) {
         R sv[6];
         bool wide = (type == ERF_ADV_UPWIND_5TH || type == ERF_ADV_CENTERED_6TH);
@@ -1049,7 +1052,7 @@ __device__ __forceinline__ R zmom_flux_z(const Params& P, const double* rw, cons
         }
         return interp_of<VT, R>(vt, sv, upw, vf);
     };
-    R a = R(0.5) * (R(rw[cidx(g, i, j, kk)]) + R(rw[cidx(g, i, j, kk - 1)]));
+    R a = R(0.5) * (R(ld(rw, eidx(g, i, j, kk))) + R(ld(rw, eidx(g, i, j, kk - 1))));
     R iv;
     if (kk == hi_z_face || kk == lo_z_face + 1) iv = all(kk, a, R(0), ERF_ADV_CENTERED_2ND);
     else if (kk == lo_z_face + 2 || kk == hi_z_face - 1) {
@@ -1092,6 +1095,7 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
     const int im = ok ? wrap(i - 1, g.nx) : 0, jm = ok ? wrap(j - 1, g.ny) : 0;
     const int ip = ok ? wrap(i + 1, g.nx) : 0, jp = ok ? wrap(j + 1, g.ny) : 0;
     const TileEdge edge = tile_edge(g);
+    const PlaneIdx pidx(g);
     const R dxi = R(g.dxi), dyi = R(g.dyi), dzi = R(g.dzi);
     const MostView mv{u, v, S.cons};   // stage velocities (MOST ghosts below a MOST ground)
     const double* ru = S.mx;
@@ -1102,11 +1106,11 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
     const R* pp = A.pp;
     R zlu = R(0), zhu = R(0), zlv = R(0), zhv = R(0), zlw = R(0), zhw = R(0);
     double t_below = 0.0;   // temperature of the cell below (buoyancy type 2, moist)
-    load_plane(g, pu, u, k0);
-    load_plane(g, pv, v, k0);
-    load_plane(g, pw, w, k0);
+    load_plane(g, pidx, pu, u, k0);
+    load_plane(g, pidx, pv, v, k0);
+    load_plane(g, pidx, pw, w, k0);
     for (int k = k0; k < k1; ++k) {
-        const int64_t c = ok ? cidx(g, i, j, k) : 0;
+        const uint32_t c = ok ? eidx(g, i, j, k) : 0, sk = (uint32_t)g.sk;
         const bool zk = ok && k >= 1;   // z-momentum on interior faces only
         plane_wait();
         __syncthreads();
@@ -1141,9 +1145,9 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
         }
         __syncthreads();
         if (k + 1 < k1) {   // next level's planes arrive during the right-hand sides below
-            load_plane(g, pu, u, k + 1);
-            load_plane(g, pv, v, k + 1);
-            load_plane(g, pw, w, k + 1);
+            load_plane(g, pidx, pu, u, k + 1);
+            load_plane(g, pidx, pv, v, k + 1);
+            load_plane(g, pidx, pw, w, k + 1);
         }
         // ---------------- x-momentum on face i
         if (ok) {
@@ -1151,21 +1155,21 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
                       (sh[0].fy[ty + 1][tx] - sh[0].fy[ty][tx]) * dyi * R(1) + (zhu - zlu) * dzi);
             zlu = zhu;
             if (P.use_diff)
-                rhs -= ((t11[c] - t11[cidx(g, im, j, k)]) * dxi * R(1) + (t12[cidx(g, i, jp, k)] - t12[c]) * dyi * R(1) +
-                        (t13[c + g.sk] - t13[c]) * dzi);
-            R gpx = dxi * (pp[c] - pp[cidx(g, im, j, k)]);
+                rhs -= ((ld(t11, c) - ld(t11, eidx(g, im, j, k))) * dxi * R(1) + (ld(t12, eidx(g, i, jp, k)) - ld(t12, c)) * dyi * R(1) +
+                        (ld(t13, c + sk) - ld(t13, c)) * dzi);
+            R gpx = dxi * (ld(pp, c) - ld(pp, eidx(g, im, j, k)));
             gpx *= R(1);
             R q = R(0);
-            if (P.moist) q = R(0.5) * (prim[4 * N + c] + prim[4 * N + cidx(g, im, j, k)] + prim[5 * N + c] + prim[5 * N + cidx(g, im, j, k)]);
+            if (P.moist) q = R(0.5) * (ld(prim + 4 * N, c) + ld(prim + 4 * N, eidx(g, im, j, k)) + ld(prim + 5 * N, c) + ld(prim + 5 * N, eidx(g, im, j, k)));
             R src = R(0);
             if (P.coriolis) {
-                R rvl = R(0.25) * (R(rv[cidx(g, i, jp, k)]) + R(rv[c]) + R(rv[cidx(g, im, jp, k)]) + R(rv[cidx(g, im, j, k)]));
-                R rwl = R(0.25) * (R(rw[c + g.sk]) + R(rw[c]) + R(rw[cidx(g, i, jm, k + 1)]) + R(rw[cidx(g, i, jm, k)]));
+                R rvl = R(0.25) * (R(ld(rv, eidx(g, i, jp, k))) + R(ld(rv, c)) + R(ld(rv, eidx(g, im, jp, k))) + R(ld(rv, eidx(g, im, j, k))));
+                R rwl = R(0.25) * (R(ld(rw, c + sk)) + R(ld(rw, c)) + R(ld(rw, eidx(g, i, jm, k + 1))) + R(ld(rw, eidx(g, i, jm, k))));
                 src += R(P.cf) * (rvl * R(P.sinphi) - rwl * R(P.cosphi));
             }
-            src += R(0.5) * (R(cd[c]) + R(cd[cidx(g, im, j, k)])) * R(P.geo0);
+            src += R(0.5) * (R(ld(cd, c)) + R(ld(cd, eidx(g, im, j, k)))) * R(P.geo0);
             rhs += (-gpx - R(0)) / (R(1) + q) + src;
-            Fmx[c] = rhs;
+            at(Fmx, c) = rhs;
         }
         // ---------------- y-momentum on face j
         if (ok) {
@@ -1173,51 +1177,51 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
                       (sh[1].fy[ty + 1][tx] - sh[1].fy[ty][tx]) * dyi * R(1) + (zhv - zlv) * dzi);
             zlv = zhv;
             if (P.use_diff)
-                rhs -= ((t12[cidx(g, ip, j, k)] - t12[c]) * dxi * R(1) + (t22[c] - t22[cidx(g, i, jm, k)]) * dyi * R(1) +
-                        (t23[c + g.sk] - t23[c]) * dzi);
-            R gpy = dyi * (pp[c] - pp[cidx(g, i, jm, k)]);
+                rhs -= ((ld(t12, eidx(g, ip, j, k)) - ld(t12, c)) * dxi * R(1) + (ld(t22, c) - ld(t22, eidx(g, i, jm, k))) * dyi * R(1) +
+                        (ld(t23, c + sk) - ld(t23, c)) * dzi);
+            R gpy = dyi * (ld(pp, c) - ld(pp, eidx(g, i, jm, k)));
             gpy *= R(1);
             R q = R(0);
-            if (P.moist) q = R(0.5) * (prim[4 * N + c] + prim[4 * N + cidx(g, i, jm, k)] + prim[5 * N + c] + prim[5 * N + cidx(g, i, jm, k)]);
+            if (P.moist) q = R(0.5) * (ld(prim + 4 * N, c) + ld(prim + 4 * N, eidx(g, i, jm, k)) + ld(prim + 5 * N, c) + ld(prim + 5 * N, eidx(g, i, jm, k)));
             R src = R(0);
             if (P.coriolis) {
-                R rul = R(0.25) * (R(ru[cidx(g, ip, j, k)]) + R(ru[c]) + R(ru[cidx(g, ip, jm, k)]) + R(ru[cidx(g, i, jm, k)]));
+                R rul = R(0.25) * (R(ld(ru, eidx(g, ip, j, k))) + R(ld(ru, c)) + R(ld(ru, eidx(g, ip, jm, k))) + R(ld(ru, eidx(g, i, jm, k))));
                 src += -R(P.cf) * rul * R(P.sinphi);
             }
-            src += R(0.5) * (R(cd[c]) + R(cd[cidx(g, i, jm, k)])) * R(P.geo1);
+            src += R(0.5) * (R(ld(cd, c)) + R(ld(cd, eidx(g, i, jm, k)))) * R(P.geo1);
             rhs += (-gpy - R(0)) / (R(1) + q) + src;
-            Fmy[c] = rhs;
+            at(Fmy, c) = rhs;
         }
         // ---------------- z-momentum on face k
-        if (ok && k == 0) Fmz[c] = R(0);
+        if (ok && k == 0) at(Fmz, c) = R(0);
         if (zk) {
             R rhs = -((sh[2].fx[ty][tx + 1] - sh[2].fx[ty][tx]) * dxi * R(1) +
                       (sh[2].fy[ty + 1][tx] - sh[2].fy[ty][tx]) * dyi * R(1) + (zhw - zlw) * dzi);
             zlw = zhw;
             if (P.use_diff)
-                rhs -= ((t13[cidx(g, ip, j, k)] - t13[c]) * dxi * R(1) + (t23[cidx(g, i, jp, k)] - t23[c]) * dyi * R(1) +
-                        (t33[c] - t33[c - g.sk]) * dzi);
+                rhs -= ((ld(t13, eidx(g, ip, j, k)) - ld(t13, c)) * dxi * R(1) + (ld(t23, eidx(g, i, jp, k)) - ld(t23, c)) * dyi * R(1) +
+                        (ld(t33, c) - ld(t33, c - sk)) * dzi);
             double b;
             double g2 = -P.gravity;
             if (!P.moist) {
                 if (P.buoy_type == 1) {
-                    b = g2 * 0.5 * ((cd[c] - P.r0[k + 1]) + (cd[c - g.sk] - P.r0[k]));
+                    b = g2 * 0.5 * ((ld(cd, c) - P.r0[k + 1]) + (ld(cd, c - sk) - P.r0[k]));
                 } else {
                     auto T0 = [&](int kk) {
                         double rt0 = eos_rt_given_p(P.p0[kk + 1]);
                         return (rt0 / P.r0[kk + 1]) / pow(p_0 / P.p0[kk + 1], P.rdOcp);
                     };
-                    double t0h = T0(k), th_ = eos_T(cd[c], cd[N + c], 0.0);
-                    double t0l = T0(k - 1), tl_ = eos_T(cd[c - g.sk], cd[N + c - g.sk], 0.0);
+                    double t0h = T0(k), th_ = eos_T(ld(cd, c), ld(cd + N, c), 0.0);
+                    double t0l = T0(k - 1), tl_ = eos_T(ld(cd, c - sk), ld(cd + N, c - sk), 0.0);
                     double qp_ = (th_ - t0h) / t0h, qm_ = (tl_ - t0l) / t0l;
                     double r0q = 0.5 * (P.r0[k + 1] * qp_ + P.r0[k] * qm_);
                     b = -r0q * g2;
                 }
             } else if (P.buoy_type == 1) {
                 int nq = P.ncomp - ERF_RHOQ1_COMP;
-                double hi = cd[c] + cd[5 * N + c] + cd[6 * N + c] - P.r0[k + 1];
-                double lo = cd[c - g.sk] + cd[5 * N + c - g.sk] + cd[6 * N + c - g.sk] - P.r0[k];
-                for (int qo = 2; qo < nq; ++qo) { hi += cd[(5 + qo) * N + c]; lo += cd[(5 + qo) * N + c - g.sk]; }
+                double hi = ld(cd, c) + ld(cd + 5 * N, c) + ld(cd + 6 * N, c) - P.r0[k + 1];
+                double lo = ld(cd, c - sk) + ld(cd + 5 * N, c - sk) + ld(cd + 6 * N, c - sk) - P.r0[k];
+                for (int qo = 2; qo < nq; ++qo) { hi += ld(cd + (5 + qo) * N, c); lo += ld(cd + (5 + qo) * N, c - sk); }
                 b = g2 * 0.5 * (hi + lo);
             } else {
                 int nq = P.ncomp - ERF_RHOQ1_COMP;
@@ -1230,13 +1234,13 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
                 double tp1 = pavg[5 * g.nz + k], tm1 = pavg[5 * g.nz + k - 1];
                 // cell temperatures: this level's, and the one below carried
                 // up the block's column (evaluated once per cell)
-                double tp3 = eos_T(cd[c], cd[N + c], cd[5 * N + c] / cd[c]);
-                double tm3 = (k == k0 || k == 1) ? eos_T(cd[c - g.sk], cd[N + c - g.sk], cd[5 * N + c - g.sk] / cd[c - g.sk])
+                double tp3 = eos_T(ld(cd, c), ld(cd + N, c), ld(cd + 5 * N, c) / ld(cd, c));
+                double tm3 = (k == k0 || k == 1) ? eos_T(ld(cd, c - sk), ld(cd + N, c - sk), ld(cd + 5 * N, c - sk) / ld(cd, c - sk))
                                        : t_below;
                 t_below = tp3;
-                double qvp = nq >= 1 ? prim[4 * N + c] : 0.0, qvm = nq >= 1 ? prim[4 * N + c - g.sk] : 0.0;
-                double qcp = nq >= 2 ? prim[5 * N + c] : 0.0, qcm = nq >= 2 ? prim[5 * N + c - g.sk] : 0.0;
-                double qpp = nq >= 3 ? prim[6 * N + c] : 0.0, qpm = nq >= 3 ? prim[6 * N + c - g.sk] : 0.0;
+                double qvp = nq >= 1 ? ld(prim + 4 * N, c) : 0.0, qvm = nq >= 1 ? ld(prim + 4 * N, c - sk) : 0.0;
+                double qcp = nq >= 2 ? ld(prim + 5 * N, c) : 0.0, qcm = nq >= 2 ? ld(prim + 5 * N, c - sk) : 0.0;
+                double qpp = nq >= 3 ? ld(prim + 6 * N, c) : 0.0, qpm = nq >= 3 ? ld(prim + 6 * N, c - sk) : 0.0;
                 double qplus = 0.61 * (qvp - qvd[k]) - (qcp - qcd[k] + qpp - qpd[k]) + (tp3 - tp1) / tp1 * (1.0 + 0.61 * qvd[k] - qcd[k] - qpd[k]);
                 double qminus = 0.61 * (qvm - qvd[k - 1]) - (qcm - qcd[k - 1] + qpm - qpd[k - 1]) + (tm3 - tm1) / tm1 * (1.0 + 0.61 * qvd[k - 1] - qcd[k - 1] - qpd[k - 1]);
                 double qavg = 0.5 * (qplus + qminus);
@@ -1245,17 +1249,17 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
             }
             R zsrc = R(b);
             if (P.coriolis) {
-                R rul = R(0.25) * (R(ru[cidx(g, ip, j, k)]) + R(ru[c]) + R(ru[cidx(g, ip, j, k - 1)]) + R(ru[c - g.sk]));
+                R rul = R(0.25) * (R(ld(ru, eidx(g, ip, j, k))) + R(ld(ru, c)) + R(ld(ru, eidx(g, ip, j, k - 1))) + R(ld(ru, c - sk)));
                 zsrc += R(P.cf) * rul * R(P.cosphi);
             }
-            zsrc += R(0.5) * (R(cd[c]) + R(cd[c - g.sk])) * R(P.geo2);
-            R gpz = dzi * (pp[c] - pp[c - g.sk]) / R(1);
+            zsrc += R(0.5) * (R(ld(cd, c)) + R(ld(cd, c - sk))) * R(P.geo2);
+            R gpz = dzi * (ld(pp, c) - ld(pp, c - sk)) / R(1);
             R q = R(0);
-            if (P.moist) q = R(0.5) * (prim[4 * N + c] + prim[4 * N + c - g.sk] + prim[5 * N + c] + prim[5 * N + c - g.sk]);
+            if (P.moist) q = R(0.5) * (ld(prim + 4 * N, c) + ld(prim + 4 * N, c - sk) + ld(prim + 5 * N, c) + ld(prim + 5 * N, c - sk));
             rhs += (zsrc - gpz - R(0)) / (R(1) + q);
-            Fmz[c] = rhs;
+            at(Fmz, c) = rhs;
         }
-        if (ok && k == g.nz - 1) Fmz[c + g.sk] = R(0);
+        if (ok && k == g.nz - 1) at(Fmz, c + sk) = R(0);
         // the next level's first barrier orders the reuse of sh
     }
 }
@@ -1271,6 +1275,7 @@ dim3 cell_block() { return dim3(32, 4, 1); }
 dim3 cell_grid(const Geo& g) { return dim3((g.nx + 31) / 32, (g.ny + 3) / 4, g.nz); }
 
 constexpr int U5 = ERF_ADV_UPWIND_5TH, W5 = ERF_ADV_WENO_5;
+constexpr int U3 = ERF_ADV_UPWIND_3RD, W3 = ERF_ADV_WENO_3;   // the reference's defaults
 
 template <class R>
 using SlowCellK = void (*)(Params, int, StateBuf, StageAux<R>, const R*, const R*, const R*, const R*, TkeBuf<R>, R*, R*,
@@ -1286,25 +1291,30 @@ template <class R>
 SlowCellK<R> slow_cell_kernel(const Params& P) {
     if (P.dyc_h == U5 && P.dyc_v == U5) return k_slow_cell<R, U5, U5>;
     if (P.dyc_h == W5 && P.dyc_v == W5) return k_slow_cell<R, W5, W5>;
+    if (P.dyc_h == U3 && P.dyc_v == U3) return k_slow_cell<R, U3, U3>;
     return k_slow_cell<R, -1, -1>;
 }
 template <class R>
 SlowMomK<R> slow_mom_kernel(const Params& P) {
     if (P.dyc_h == U5 && P.dyc_v == U5) return k_slow_mom<R, U5, U5>;
+    if (P.dyc_h == U3 && P.dyc_v == U3) return k_slow_mom<R, U3, U3>;
     return k_slow_mom<R, -1, -1>;
 }
 template <class R>
 PostK<R> post_kernel(const Params& P) {
     bool dw = P.dry_h == W5 && P.dry_v == W5, du = P.dry_h == U5 && P.dry_v == U5;
+    const bool d3 = P.dry_h == U3 && P.dry_v == U3, m3 = P.moi_h == W3 && P.moi_v == W3;
     bool mw = P.moi_h == W5 && P.moi_v == W5, mu = P.moi_h == U5 && P.moi_v == U5;
     const int nslow = (P.moist ? 1 + (P.ncomp - ERF_RHOQ1_COMP) : 1) + (P.les == ERF_LES_DEARDORFF ? 1 : 0);
     if (!P.moist) {
         if (dw) return k_post<R, W5, W5, -1, -1, 4>;
         if (du) return k_post<R, U5, U5, -1, -1, 4>;
+        if (d3) return k_post<R, U3, U3, -1, -1, 4>;
     } else if (nslow <= 4) {
         if (dw && mw) return k_post<R, W5, W5, W5, W5, 4>;
         if (du && mu) return k_post<R, U5, U5, U5, U5, 4>;
         if (du && mw) return k_post<R, U5, U5, W5, W5, 4>;
+        if (d3 && m3) return k_post<R, U3, U3, W3, W3, 4>;
     } else {
         if (dw && mw) return k_post<R, W5, W5, W5, W5, 5>;
         if (du && mu) return k_post<R, U5, U5, U5, U5, 5>;

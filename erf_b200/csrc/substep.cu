@@ -45,18 +45,6 @@ struct ColTile {
     }
 };
 
-// Element e of an array.  The byte offset stays in 32 bits (an array of 4 GB
-// would be 5e8 cells, more than the card holds), so that a thread keeps one
-// offset register per neighbour for all the arrays instead of an address per
-// load: that is what lets it hold its loads in flight together.
-template <class T>
-__device__ __forceinline__ T ld(const T* p, uint32_t e) {
-    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + e * (uint32_t)sizeof(T)));
-}
-template <class T>
-__device__ __forceinline__ T& at(T* p, uint32_t e) {
-    return *reinterpret_cast<T*>(reinterpret_cast<char*>(p) + e * (uint32_t)sizeof(T));
-}
 // Offset of level k (of the bounds-checked build: cidx's check).
 __device__ __forceinline__ uint32_t lev(const Geo& g, int k) {
 #ifdef ERF_B200_BOUNDS
@@ -407,9 +395,13 @@ SubShape sub_shape(const Geo& g) {
     s.tx = 32;
     while (s.tx > 8 && 2 * (sub_smem<R>(g.nz, s.tx) + 1024) > (size_t)persm) s.tx /= 2;
     while (s.tx > 2 && sub_smem<R>(g.nz, s.tx) > (size_t)maxopt) s.tx /= 2;
-    // few blocks: all the threads an SM takes; more than one per SM: half each
+    // small planes: narrower tiles while they leave half the SMs without one
+    while (s.tx > 8 && 2 * ((g.sk + s.tx - 1) / s.tx) <= nsm) s.tx /= 2;
+    // few blocks: all the threads an SM takes; more than one per SM: half each;
+    // never more rows than levels
     const int64_t blocks = (g.sk + s.tx - 1) / s.tx;
     s.rows = (blocks <= nsm ? 1024 : 512) / s.tx;
+    while (s.rows > 8 && s.rows / 2 > g.nz) s.rows /= 2;
     s.coef_rows = 256 / s.tx;
     return s;
 }

@@ -63,7 +63,7 @@ __device__ __forceinline__ double Zn(const Params& P, int i, int j, int k) {
 #define ZN(a, b, c) Zn(P, a, b, c)
 __device__ __forceinline__ double detJ_at(const Params& P, int i, int j, int k) {
     const Geo& g = P.g;
-    return __ldg(P.detJ + cidx(g, wrap(i, g.nx), wrap(j, g.ny), clampk(k, g.nz)));
+    return ld(P.detJ, eidx(g, wrap(i, g.nx), wrap(j, g.ny), clampk(k, g.nz)));
 }
 __device__ __forceinline__ double hzeta_cc_fn(const Params& P, int i, int j, int k) {
     return 0.25 * P.g.dzi * (ZN(i + 1, j, k + 1) + ZN(i + 1, j + 1, k + 1) + ZN(i, j, k + 1) + ZN(i, j + 1, k + 1)
@@ -145,7 +145,7 @@ enum { MT_HZETA_I, MT_HXI_I, MT_HZETA_J, MT_HETA_J, MT_HXI_K, MT_HETA_K, MT_HZET
 static_assert(MT_COUNT == TER_NMET, "metric table count");
 __device__ __forceinline__ double mt_at(const Params& P, int q, int i, int j, int k) {
     const Geo& g = P.g;
-    return __ldg(P.met + (int64_t)q * g.nzf + cidx(g, wrap(i, g.nx), wrap(j, g.ny), k));
+    return ld(P.met + (int64_t)q * g.nzf, eidx(g, wrap(i, g.nx), wrap(j, g.ny), k));
 }
 #define ERFB_MT(name, q)                                                           \
     __device__ __forceinline__ double name(const Params& P, int i, int j, int k) { \
@@ -220,20 +220,20 @@ __device__ __forceinline__ double rt_v(const Geo& g, const double* cons, const d
 // indices wrapped here.
 __device__ __forceinline__ double tvel(const double* f, const Geo& g, int i, int j, int k) {
     i = wrap(i, g.nx); j = wrap(j, g.ny);
-    if (k < 0) return g.zlo_noslip ? 0.0 : __ldg(f + cidx(g, i, j, 0));
-    if (k >= g.nz) return g.zhi_noslip ? 0.0 : __ldg(f + cidx(g, i, j, g.nz - 1));
-    return __ldg(f + cidx(g, i, j, k));
+    if (k < 0) return g.zlo_noslip ? 0.0 : ld(f, eidx(g, i, j, 0));
+    if (k >= g.nz) return g.zhi_noslip ? 0.0 : ld(f, eidx(g, i, j, g.nz - 1));
+    return ld(f, eidx(g, i, j, k));
 }
 // w at z-face k in [0, nz], lateral wrap
 __device__ __forceinline__ double wvel(const double* f, const Geo& g, int i, int j, int k) {
     i = wrap(i, g.nx); j = wrap(j, g.ny);
     k = k < 0 ? 0 : (k > g.nz ? g.nz : k);
-    return __ldg(f + cidx(g, i, j, k));
+    return ld(f, eidx(g, i, j, k));
 }
 // cell-centred value with lateral wrap and foextrap in z
 template <class V>
 __device__ __forceinline__ double ccw(const V* f, const Geo& g, int i, int j, int k) {
-    return double(__ldg(f + cidx(g, wrap(i, g.nx), wrap(j, g.ny), clampk(k, g.nz))));
+    return double(ld(f, eidx(g, wrap(i, g.nx), wrap(j, g.ny), clampk(k, g.nz))));
 }
 
 __device__ __forceinline__ bool cell_ij(const Geo& g, int& i, int& j, int& k) {
@@ -912,9 +912,9 @@ __global__ void __launch_bounds__(128, TER_MINB_STRESS) k_ter_stress(Params P, c
     auto mt = [&](int ii, int jj, int kk) { return P.use_turb ? ccw(mut, g, ii, jj, kk) : 0.0; };
     auto S11 = [&](int ii, int jj, int kk) { return ccw(T.s11, g, ii, jj, kk); };
     auto S22 = [&](int ii, int jj, int kk) { return ccw(T.s22, g, ii, jj, kk); };
-    auto E12 = [&](int ii, int jj, int kk) { return double(T.s12[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), clampk(kk, nz))]); };
-    auto E13 = [&](int ii, int jj, int kk) { return double(T.s13[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)]); };
-    auto E23 = [&](int ii, int jj, int kk) { return double(T.s23[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)]); };
+    auto E12 = [&](int ii, int jj, int kk) { return double(ld(T.s12, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), clampk(kk, nz)))); };
+    auto E13 = [&](int ii, int jj, int kk) { return double(ld(T.s13, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
+    auto E23 = [&](int ii, int jj, int kk) { return double(ld(T.s23, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
     {   // tau33
         double mxi = hxi_cc(P, i, j, k), meta = heta_cc(P, i, j, k);
         double t31b = 0.25 * (E13(i, j, k) + E13(i + 1, j, k) + E13(i, j, k + 1) + E13(i + 1, j, k + 1));
@@ -1082,7 +1082,7 @@ __device__ __forceinline__ double omega_mom(const Params& P, StateBuf S, const d
     if (k <= 0) return 0.;
     auto MX = [&](int ii, int jj, int kk) {
         ii = wrap(ii, g.nx); jj = wrap(jj, g.ny);
-        if (kk < g.nz) return S.mx[cidx(g, ii, jj, kk)];
+        if (kk < g.nz) return ld(S.mx, eidx(g, ii, jj, kk));
         // momentum ghost above the lid: V2M of the tangential ghost velocity
         int kt = g.nz - 1;
         double rs = S.cons[cidx(g, ii, jj, kt)] + S.cons[cidx(g, wrap(ii - 1, g.nx), jj, kt)];
@@ -1090,7 +1090,7 @@ __device__ __forceinline__ double omega_mom(const Params& P, StateBuf S, const d
     };
     auto MY = [&](int ii, int jj, int kk) {
         ii = wrap(ii, g.nx); jj = wrap(jj, g.ny);
-        if (kk < g.nz) return S.my[cidx(g, ii, jj, kk)];
+        if (kk < g.nz) return ld(S.my, eidx(g, ii, jj, kk));
         int kt = g.nz - 1;
         double rs = S.cons[cidx(g, ii, jj, kt)] + S.cons[cidx(g, ii, wrap(jj - 1, g.ny), kt)];
         return tvel(v, g, ii, jj, g.nz) * 0.5 * rs;
@@ -1226,9 +1226,9 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
     const int64_t N = g.ncell;
     int64_t c = cidx(g, i, j, k);
     const double dxi = g.dxi, dyi = g.dyi, dzi = g.dzi;
-    auto RU = [&](int ii, int jj, int kk) { return S.mx[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)] * 1.0; };
-    auto RV = [&](int ii, int jj, int kk) { return S.my[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)] * 1.0; };
-    auto Om = [&](int ii, int jj, int kk) { return double(Om_in[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)]); };
+    auto RU = [&](int ii, int jj, int kk) { return ld(S.mx, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)) * 1.0; };
+    auto RV = [&](int ii, int jj, int kk) { return ld(S.my, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)) * 1.0; };
+    auto Om = [&](int ii, int jj, int kk) { return double(ld(Om_in, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
     auto U = [&](int ii, int jj, int kk) { return tvel(u, g, ii, jj, kk); };
     auto V = [&](int ii, int jj, int kk) { return tvel(v, g, ii, jj, kk); };
     auto W = [&](int ii, int jj, int kk) { return wvel(w, g, ii, jj, kk); };
@@ -1265,7 +1265,7 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
         }
         double r = src;
         if (P.use_diff) {
-            auto T11 = [&](int ii) { return double(t11[cidx(g, wrap(ii, g.nx), j, k)]); };
+            auto T11 = [&](int ii) { return double(ld(t11, eidx(g, wrap(ii, g.nx), j, k))); };
             double d = ((T11(i) - T11(i - 1)) * dxi * 1.0 + (double(t12[cidx(g, i, wrap(j + 1, g.ny), k)]) - double(t12[c])) * dyi * 1.0
                         + (double(t13[c + g.sk]) - double(t13[c])) * dzi);
             d /= 0.5 * (Jt(i, j, k) + Jt(i - 1, j, k));
@@ -1317,7 +1317,7 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
         }
         double r = src;
         if (P.use_diff) {
-            auto T22 = [&](int jj) { return double(t22[cidx(g, i, wrap(jj, g.ny), k)]); };
+            auto T22 = [&](int jj) { return double(ld(t22, eidx(g, i, wrap(jj, g.ny), k))); };
             double d = ((double(t12[cidx(g, wrap(i + 1, g.nx), j, k)]) - double(t12[c])) * dxi * 1.0 + (T22(j) - T22(j - 1)) * dyi * 1.0
                         + (double(t23[c + g.sk]) - double(t23[c])) * dzi);
             d /= 0.5 * (Jt(i, j, k) + Jt(i, j - 1, k));
@@ -1596,10 +1596,10 @@ __global__ void __launch_bounds__(1024) k_ter_fast_vert(Params P, double dtau, d
     const int64_t N = g.ncell, sk = g.sk;
     const double dxi = g.dxi, dyi = g.dyi, dzi = g.dzi, halfg = P.halfg;
     auto th = [&](int ii, int jj, int kk) { return ccw(A.prim, g, ii, jj, kk); };
-    auto NDU = [&](int ii, int jj, int kk) { return double(T.ndu[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)]); };
-    auto NDV = [&](int ii, int jj, int kk) { return double(T.ndv[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)]); };
-    auto ODU = [&](int ii, int jj, int kk) { return double(T.odu[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)]); };
-    auto ODV = [&](int ii, int jj, int kk) { return double(T.odv[cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk)]); };
+    auto NDU = [&](int ii, int jj, int kk) { return double(ld(T.ndu, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
+    auto NDV = [&](int ii, int jj, int kk) { return double(ld(T.ndv, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
+    auto ODU = [&](int ii, int jj, int kk) { return double(ld(T.odu, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
+    auto ODV = [&](int ii, int jj, int kk) { return double(ld(T.odv, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
     auto prev_mz = [&](int k) {
         if (prev_rt && (k == 0 || k == nz)) return T.bnd[(k == 0 ? 0 : sk) + (int64_t)j * g.nx + i];
         return prev_mz_ter<R>(P, Sprev, prev_rt, i, j, k);
@@ -1736,13 +1736,14 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
 #pragma unroll
     for (int q = 0; q < NS; ++q) { zl[q] = zh[q] = R(0); dz_lo[q] = 0.0; }
     const TileEdge edge = tile_edge(g);
+    const PlaneIdx pidx(g);
     auto comp_of = [&](int q) {
         return q == 0 ? ERF_RHOSCALAR_COMP : (q < nscal ? ERF_RHOQ1_COMP + q - 1 : ERF_RHOKE_COMP);
     };
     auto slow_phi = [&](int q) { return Acur.prim + (int64_t)(comp_of(q) - 1) * N; };
 #pragma unroll
     for (int q = 0; q < NS; ++q)
-        if (q < nslow) load_plane(g, pl[q], slow_phi(q), k0);
+        if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k0);
     for (int k = k0; k < k1; ++k) {
         plane_wait();
         __syncthreads();
@@ -1771,7 +1772,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
         if (k + 1 < k1) {   // next level's planes arrive during the update below
 #pragma unroll
             for (int q = 0; q < NS; ++q)
-                if (q < nslow) load_plane(g, pl[q], slow_phi(q), k + 1);
+                if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k + 1);
         }
         if (!ok) continue;   // the next level's first barrier orders the reuse of sh
         const int64_t c = cidx(g, i, j, k);

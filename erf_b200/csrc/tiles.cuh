@@ -14,23 +14,34 @@ namespace erfb {
 // Cell-centred scalar with foextrap in z.
 template <class V>
 __device__ __forceinline__ V ccz(const V* __restrict__ f, const Geo& g, int i, int j, int k) {
-    return __ldg(f + cidx(g, i, j, clampk(k, g.nz)));
+    return ld(f, eidx(g, i, j, clampk(k, g.nz)));
 }
 
 // Advective flux of a primitive scalar phi (type R) through the low z face
 // of cell (i,j,k): mom * interp(phi) (Advection/ERF_AdvectionSrcForScalars.H:
 // 7-58).  The advecting momentum M is the FP64 stage momentum (rho, theta)
-// or the R average momentum (slow scalars).
+// or the R average momentum (slow scalars).  Away from the walls the stencil
+// is six loads at constant strides, without a clamp for each.
 template <int T, class R, class M>
 __device__ __forceinline__ R adv_flux_z(const Geo& g, const R* __restrict__ phi, const M* __restrict__ mom, int type,
                                         R frac, int i, int j, int k) {
     R s[6];
     const int w = width_of<T>(type);
-    for (int m = 0; m < 6; ++m) {
-        int off = m - 3;
-        s[m] = (off >= -w && off <= w - 1) ? ccz(phi, g, i, j, k + off) : R(0);
+    const uint32_t e = eidx(g, i, j, k), sk = (uint32_t)g.sk;
+    if (k >= w && k + w <= g.nz) {
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int off = m - 3;
+            s[m] = (off >= -w && off <= w - 1) ? ld(phi, e + (uint32_t)off * sk) : R(0);
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int off = m - 3;
+            s[m] = (off >= -w && off <= w - 1) ? ccz(phi, g, i, j, k + off) : R(0);
+        }
     }
-    R a = R(__ldg(mom + cidx(g, i, j, k)));
+    R a = R(ld(mom, e));
     return a * interp_of<T, R>(type, s, a, frac);
 }
 
@@ -48,24 +59,39 @@ template <class R>
 struct Plane {
     R v[TTY + 2 * PH][TTX + 2 * PH];
 };
+// The plane's elements that a thread copies, as offsets within a level: they
+// are the same on every level and for every field, so the division and the
+// periodic wraps are done once per block.
+struct PlaneIdx {
+    static constexpr int W = TTX + 2 * PH, NE = W * (TTY + 2 * PH), NT = TTX * TTY, M = (NE + NT - 1) / NT;
+    uint32_t o[M];
+    __device__ __forceinline__ PlaneIdx(const Geo& g) {
+        const int t = threadIdx.y * TTX + threadIdx.x;
+        const int i0 = blockIdx.x * TTX - PH, j0 = blockIdx.y * TTY - PH;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int e = min(t + m * NT, NE - 1), b = e / W, a = e - b * W;
+            o[m] = (uint32_t)(wrap_far(i0 + a, g.nx) + g.nx * wrap_far(j0 + b, g.ny));
+        }
+    }
+};
 // Asynchronous copy of the plane (cp.async): the copies land in shared
 // memory while the block works on the previous level; plane_wait() makes
 // this thread's copies complete (a barrier then publishes them).
 template <class R>
-__device__ __forceinline__ void load_plane(const Geo& g, Plane<R>& p, const R* __restrict__ phi, int k) {
+__device__ __forceinline__ void load_plane(const Geo& g, const PlaneIdx& pi, Plane<R>& p, const R* __restrict__ phi,
+                                           int k) {
     const int t = threadIdx.y * TTX + threadIdx.x;
-    const int i0 = blockIdx.x * TTX - PH, j0 = blockIdx.y * TTY - PH;
-    const R* __restrict__ lev = phi + g.sk * k;
-    constexpr int W = TTX + 2 * PH, NE = W * (TTY + 2 * PH);
-    for (int e = t; e < NE; e += TTX * TTY) {
-        const int b = e / W, a = e - b * W;
-        const int gi = wrap_far(i0 + a, g.nx), gj = wrap_far(j0 + b, g.ny);
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(&p.v[b][a]);
-        const R* src = lev + gi + (int64_t)g.nx * gj;
+    const char* lev = reinterpret_cast<const char*>(phi + g.sk * k);
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(&p.v[0][0]) + t * (unsigned)sizeof(R);
+#pragma unroll
+    for (int m = 0; m < PlaneIdx::M; ++m) {
+        if (m == PlaneIdx::M - 1 && t + m * PlaneIdx::NT >= PlaneIdx::NE) break;
+        const char* src = lev + pi.o[m] * (uint32_t)sizeof(R);
         if constexpr (sizeof(R) == 8)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + m * PlaneIdx::NT * 8), "l"(src) : "memory");
         else
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + m * PlaneIdx::NT * 4), "l"(src) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -130,9 +156,9 @@ __device__ __forceinline__ void tile_put(const Geo& g, FluxTile<R>& t, const Pla
                                          const M* __restrict__ az, int th, int tv, R fh, R fv, int i, int j, int k,
                                          bool first, R& zl, R& zh) {
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int64_t c = cidx(g, i, j, k);
-    t.fx[ty][tx] = plane_flux_x<TH>(pl, ty, tx, R(__ldg(ax + c)), th, fh);
-    t.fy[ty][tx] = plane_flux_y<TH>(pl, ty, tx, R(__ldg(ay + c)), th, fh);
+    const uint32_t c = eidx(g, i, j, k);
+    t.fx[ty][tx] = plane_flux_x<TH>(pl, ty, tx, R(ld(ax, c)), th, fh);
+    t.fy[ty][tx] = plane_flux_y<TH>(pl, ty, tx, R(ld(ay, c)), th, fh);
     if (first) zl = adv_flux_z<TV>(g, phi, az, tv, fv, i, j, k);
     zh = adv_flux_z<TV>(g, phi, az, tv, fv, i, j, k + 1);
 }
@@ -143,11 +169,11 @@ __device__ __forceinline__ void tile_put_edge(const Geo& g, const TileEdge& e, F
                                               int k) {
     if (e.row >= 0) {
         const int ih = wrap(e.i0 + e.nvx, g.nx);
-        t.fx[e.row][e.nvx] = plane_flux_x<TH>(pl, e.row, e.nvx, R(__ldg(ax + cidx(g, ih, e.j0 + e.row, k))), th, fh);
+        t.fx[e.row][e.nvx] = plane_flux_x<TH>(pl, e.row, e.nvx, R(ld(ax, eidx(g, ih, e.j0 + e.row, k))), th, fh);
     }
     if (e.col >= 0) {
         const int jh = wrap(e.j0 + e.nvy, g.ny);
-        t.fy[e.nvy][e.col] = plane_flux_y<TH>(pl, e.nvy, e.col, R(__ldg(ay + cidx(g, e.i0 + e.col, jh, k))), th, fh);
+        t.fy[e.nvy][e.col] = plane_flux_y<TH>(pl, e.nvy, e.col, R(ld(ay, eidx(g, e.i0 + e.col, jh, k))), th, fh);
     }
 }
 template <class R>
