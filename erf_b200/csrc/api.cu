@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -36,7 +37,7 @@ template <class R>
 struct Bulk {
     R *Fcons, *Fmx, *Fmy, *Fmz;   // slow right-hand sides
     R *avx, *avy, *avz;           // average momenta of the substeps
-    R* lag[2];                    // lagged d(rho theta) (flat: the extrapolated one), ping-pong
+    R* lag[2];                    // lagged d(rho theta) (flat: the extrapolated one), ping-pong; terrain: per-pass entry
     SubCoef<R> sc{};              // flat substeps: the stage's coefficients,
     R *du[2], *dv[2], *dw[2];     // the momentum increments, ping-pong,
     double *dr, *drt;             // and the deviations of rho and rho theta
@@ -115,7 +116,6 @@ struct erf_b200_ctx {
 
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     cudaGraph_t graph_raw[2] = {nullptr, nullptr};   // kept for ensemble graphs
-    int lag_parity_per_step = 0;
     int cur = -1;             // slot of the resident state (-1: none loaded)
 };
 
@@ -374,13 +374,6 @@ void stage_schedule(const erf_b200_config& f, int nrk, int& nsub, double& dtau, 
     }
 }
 
-int substeps_per_step(const erf_b200_config& f) {
-    if (no_substepping(f)) return 0;   // no acoustic substeps, no lagged d(rho theta)
-    int tot = 0;
-    for (int nrk = 0; nrk < 3; ++nrk) { int n; double a, b; stage_schedule(f, nrk, n, a, b); tot += n; }
-    return tot;
-}
-
 // Optional per-launch event timing (profiling entry point only).
 struct LaunchTimer {
     cudaStream_t st;
@@ -441,7 +434,6 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
     dim3 tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1), tcb(c->tile_tx, c->coef_warps, 1);
     const bool fork = T == nullptr && c->side;
     int a = 0;
-    int lp = (p * c->lag_parity_per_step) & 1;
     const double beta_s = 0.1;
     const double beta_1 = 0.5 * (1.0 - beta_s), beta_2 = 0.5 * (1.0 + beta_s);
     const bool nosub = no_substepping(c->cfg);
@@ -474,9 +466,12 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
         for (int ks = 0; ks < (nosub ? 0 : nsub); ++ks) {
             StateBuf Sprev = (ks == 0) ? OLD : SUM;
             int prt = ks > 0;
-            TIMED(5, launch_ter_fast_h<R>(P, st, ks, dtau, facinv, Sprev, prt, Sst, Acur, B.Fmx, B.Fmy, B.lag[lp],
-                                          B.lag[1 - lp], B.ter, B.avx, B.avy, SUM.mx, SUM.my));
-            lp ^= 1;
+            if (ks > 0) {   // the last substep's new increments are this one's old ones
+                std::swap(B.ter.odu, B.ter.ndu);
+                std::swap(B.ter.odv, B.ter.ndv);
+            }
+            TIMED(5, launch_ter_fast_h<R>(P, st, ks, ks > 0, dtau, facinv, Sprev, Sst, Acur, B.Fmx, B.Fmy, nullptr,
+                                          nullptr, B.ter, B.avx, B.avy, SUM.mx, SUM.my));
             TIMED(6, launch_ter_fast_vert<R>(P, st, c->ter_tx, c->ter_smem, dtau, facinv, beta_1, beta_2, Sprev, prt,
                                              Sst, Acur, B.Fcons, B.Fmz, B.ter, B.cA, B.cInvB, B.cCB, B.cP, B.cQ,
                                              B.avz, SUM.cons, SUM.mz));
@@ -740,6 +735,7 @@ int alloc_bulk(erf_b200_ctx* c, Bulk<R>& B) {
         A(&B.ter.fx[0], N); A(&B.ter.fy[0], N); A(&B.ter.fx[1], N); A(&B.ter.fy[1], N);
         auto D = [&](double** q, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, q, n); };
         D(&B.ter.bnd, 2 * (int64_t)cfg->nx * cfg->ny);
+        D(&B.ter.ec, N);
         if (cfg->terrain_type == ERF_TERRAIN_MOVING && cfg->substepping_type == ERF_SUBSTEP_IMPLICIT)
             for (MtCoef<R>& m : B.mc) { A(&m.E, NZF); A(&m.G, NZF); A(&m.I, NZF); A(&m.P, NZF); A(&m.Q, NZF); }
     }
@@ -923,7 +919,6 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     if (c->mixed) tiled_setup<float>(c->P, &c->tkz);
     else tiled_setup<double>(c->P, &c->tkz);
     c->tkz.ter_post = !cfg->use_terrain ? 0 : (c->mixed ? ter_post_kz<float>(c->P) : ter_post_kz<double>(c->P));
-    c->lag_parity_per_step = substeps_per_step(c->cfg) & 1;
     // shared-memory tiles of the column kernels: TX columns x all levels
     {
         const size_t max_smem = 227 * 1024;
@@ -1498,7 +1493,7 @@ int fast_rhs_pass(erf_b200_ctx* c, bool terrain, int step, int nrk, const erf_b2
         }
     }
     if (terrain) {
-        launch_ter_fast_h<double>(P, st, step, dtau, facinv, Sprev, 0, Sst, B.aux[0], B.Fmx, B.Fmy, B.lag[0],
+        launch_ter_fast_h<double>(P, st, step, false, dtau, facinv, Sprev, Sst, B.aux[0], B.Fmx, B.Fmy, B.lag[0],
                                   B.lag[1], B.ter, B.avx, B.avy, OUT.mx, OUT.my);
         launch_ter_fast_vert<double>(P, st, c->ter_tx, c->ter_smem, dtau, facinv, kBeta1, kBeta2, Sprev, 0, Sst,
                                      B.aux[0], B.Fcons, B.Fmz, B.ter, B.cA, B.cInvB, B.cCB, B.cP, B.cQ, B.avz,

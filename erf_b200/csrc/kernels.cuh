@@ -52,7 +52,7 @@ struct Params {
 };
 
 // Number of static-terrain metric tables (planes of nzf values each).
-constexpr int TER_NMET = 21;
+constexpr int TER_NMET = 24;
 
 // One copy of the prognostic state: cons (ncomp*ncell), face momenta.
 struct StateBuf {
@@ -94,6 +94,7 @@ struct TerBuf {
     R *fx[2], *fy[2];            // raw diffusive face fluxes (two fields)
     double* bnd;                 // substep: the previous momentum on the ground
                                  // and lid faces (two planes)
+    double* ec;                  // substep: extrapolated d(rho theta)
 };
 
 // x-y tile of the transport kernels (slow_cell, slow_mom, post) and the
@@ -276,8 +277,8 @@ void launch_ter_slow_mom(const Params& P, cudaStream_t st, StateBuf S, StageAux<
                          const double* v, const double* w, const R* t11, const R* t22, const R* t33, const R* t12,
                          const R* t13, const R* t23, TerBuf<R> T, const R* Om, R* Fmx, R* Fmy, R* Fmz);
 template <class R>
-void launch_ter_fast_h(const Params& P, cudaStream_t st, int step, double dtau, double facinv, StateBuf Sprev,
-                       int prev_rt, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in,
+void launch_ter_fast_h(const Params& P, cudaStream_t st, int step, bool ec_ready, double dtau, double facinv,
+                       StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in,
                        R* lag_out, TerBuf<R> T, R* avx, R* avy, double* outx, double* outy);
 template <class R>
 void launch_ter_fast_vert(const Params& P, cudaStream_t st, int tx, size_t smem, double dtau, double facinv,

@@ -141,7 +141,7 @@ __device__ __forceinline__ double zlo_eta_fn(const Params& P, int i, int j, int 
 // from four to eight nodes of z_phys_nd; outside [0, nz] the function runs.
 enum { MT_HZETA_I, MT_HXI_I, MT_HZETA_J, MT_HETA_J, MT_HXI_K, MT_HETA_K, MT_HZETA_EK, MT_HZETA_EJ, MT_HZETA_EI,
        MT_ZLO_XI, MT_ZLO_ETA, MT_HZETA_CC, MT_HXI_CC, MT_HETA_CC, MT_HZETA_K, MT_HXI_EK, MT_HETA_EK, MT_HXI_EJ,
-       MT_HETA_EJ, MT_HXI_EI, MT_HETA_EI, MT_COUNT };
+       MT_HETA_EJ, MT_HXI_EI, MT_HETA_EI, MT_RXI_I, MT_RETA_J, MT_IJ, MT_COUNT };
 static_assert(MT_COUNT == TER_NMET, "metric table count");
 __device__ __forceinline__ double mt_at(const Params& P, int q, int i, int j, int k) {
     const Geo& g = P.g;
@@ -174,6 +174,12 @@ ERFB_MT(heta_EJ, MT_HETA_EJ)
 ERFB_MT(hxi_EI, MT_HXI_EI)
 ERFB_MT(heta_EI, MT_HETA_EI)
 #undef ERFB_MT
+// Quotients of them, k in [0, nz): the slopes h_xi / h_zeta and h_eta / h_zeta
+// of the x and y faces and 1 / detJ of the cells (an FP64 division is some
+// twenty instructions, and every pass of every substep needs these).
+__device__ __forceinline__ double slope_I(const Params& P, int i, int j, int k) { return mt_at(P, MT_RXI_I, i, j, k); }
+__device__ __forceinline__ double slope_J(const Params& P, int i, int j, int k) { return mt_at(P, MT_RETA_J, i, j, k); }
+__device__ __forceinline__ double inv_detJ(const Params& P, int i, int j, int k) { return mt_at(P, MT_IJ, i, j, clampk(k, P.g.nz)); }
 
 template <class FU, class FV>
 __device__ __forceinline__ double omega_from_w(const Params& P, int i, int j, int k, double w, FU ua, FV va) {
@@ -290,6 +296,9 @@ static __global__ void k_ter_met_tables(Params P, double* __restrict__ met) {
     m[MT_HETA_EJ * s] = heta_EJ_fn(P, i, j, k);
     m[MT_HXI_EI * s] = hxi_EI_fn(P, i, j, k);
     m[MT_HETA_EI * s] = heta_EI_fn(P, i, j, k);
+    m[MT_RXI_I * s] = hxi_I_fn(P, i, j, k) / hzeta_I_fn(P, i, j, k);
+    m[MT_RETA_J * s] = heta_J_fn(P, i, j, k) / hzeta_J_fn(P, i, j, k);
+    m[MT_IJ * s] = k < P.g.nz ? 1.0 / mt_detj(P.znd, g, i, j, k) : 0.0;
 }
 #if !ERFB_TER_F32
 void launch_ter_metrics(const Params& P, cudaStream_t st, double* detJ, double* zcc) {
@@ -1011,19 +1020,17 @@ struct DiffT {
         const Geo& g = P.g;
         double rA = P.use_consA ? (0.5 * (ccw(rho, g, i, j, k) + ccw(rho, g, i - 1, j, k))) * ae : ae;
         if (P.use_turb) rA += 0.5 * (mu(i, j, k) + mu(i - 1, j, k));
-        double mxi = hxi_I(P, i, j, k), mz = hzeta_I(P, i, j, k);
         double GradCz = 0.25 * g.dzi * (p(i, j, k + 1) + p(i - 1, j, k + 1) - p(i, j, k - 1) - p(i - 1, j, k - 1));
         double GradCx = g.dxi * (p(i, j, k) - p(i - 1, j, k));
-        return -rA * 1.0 * (GradCx - (mxi / mz) * GradCz);
+        return -rA * 1.0 * (GradCx - slope_I(P, i, j, k) * GradCz);
     }
     __device__ __forceinline__ double yraw(int i, int j, int k) const {
         const Geo& g = P.g;
         double rA = P.use_consA ? (0.5 * (ccw(rho, g, i, j, k) + ccw(rho, g, i, j - 1, k))) * ae : ae;
         if (P.use_turb) rA += 0.5 * (mu(i, j, k) + mu(i, j - 1, k));
-        double meta = heta_J(P, i, j, k), mz = hzeta_J(P, i, j, k);
         double GradCz = 0.25 * g.dzi * (p(i, j, k + 1) + p(i, j - 1, k + 1) - p(i, j, k - 1) - p(i, j - 1, k - 1));
         double GradCy = g.dyi * (p(i, j, k) - p(i, j - 1, k));
-        return -rA * 1.0 * (GradCy - (meta / mz) * GradCz);
+        return -rA * 1.0 * (GradCy - slope_J(P, i, j, k) * GradCz);
     }
     __device__ __forceinline__ double xr(int i, int j, int k) const {
         if (fxr) return double(fxr[cidx(P.g, wrap(i, P.g.nx), wrap(j, P.g.ny), k)]);
@@ -1070,7 +1077,7 @@ struct DiffT {
         double fyl = yr(i, j, k) * hzeta_J(P, i, j, k), fyh = yr(i, j + 1, k) * hzeta_J(P, i, j + 1, k);
         double fzl = zflux(i, j, k, raw_lo), fzh = zflux(i, j, k + 1, raw_hi);
         double s = (fxh - fxl) * g.dxi * 1.0 + (fyh - fyl) * g.dyi * 1.0 + (fzh - fzl) * g.dzi;
-        return s / detJ_at(P, i, j, k);
+        return s * inv_detJ(P, i, j, k);
     }
 };
 
@@ -1175,7 +1182,8 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_CELL) k_ter_slow_cell(Param
     avx[c] = R(fxl); avy[c] = R(fyl); avz[c] = R(fzl);
     if (k == nz - 1) avz[c + g.sk] = R(fzh);
     const double Jc = detJ_at(P, i, j, k);
-    double frho = -1.0 / Jc * ((fxh - fxl) * g.dxi + (fyh - fyl) * g.dyi + (fzh - fzl) * g.dzi);
+    const double invdetJ = inv_detJ(P, i, j, k);
+    double frho = -invdetJ * ((fxh - fxl) * g.dxi + (fyh - fyl) * g.dyi + (fzh - fzl) * g.dzi);
     // theta with the dycore scheme, advected by the average momenta
     auto th = [&](int ii, int jj, int kk) { return ccw(A.prim, g, ii, jj, kk); };
     const int ht = P.dyc_h, vt = P.dyc_v;
@@ -1183,7 +1191,6 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_CELL) k_ter_slow_cell(Param
     double tx_l = fxl * interp_dir<HT>(0, i, j, k, th, ht, fxl, hf), tx_h = fxh * interp_dir<HT>(0, i + 1, j, k, th, ht, fxh, hf);
     double ty_l = fyl * interp_dir<HT>(1, i, j, k, th, ht, fyl, hf), ty_h = fyh * interp_dir<HT>(1, i, j + 1, k, th, ht, fyh, hf);
     double tz_l = fzl * interp_dir<VT>(2, i, j, k, th, vt, fzl, vf), tz_h = fzh * interp_dir<VT>(2, i, j, k + 1, th, vt, fzh, vf);
-    double invdetJ = 1. / Jc;
     double frt = -invdetJ * 1.0 * ((tx_h - tx_l) * g.dxi + (ty_h - ty_l) * g.dyi + (tz_h - tz_l) * g.dzi);
     if (P.use_diff) {
         const bool dd = P.les == ERF_LES_DEARDORFF;
@@ -1241,6 +1248,7 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
     const double g2 = -P.gravity;
     // ---------------- x-momentum at face (i,j,k)
     {
+        const double iJ = 1.0 / (0.5 * (Jt(i, j, k) + Jt(i - 1, j, k)));
         double src;
         if (c2) {
             double xh = 0.25 * (RU(i, j, k) * 1.0 + RU(i + 1, j, k) * 1.0) * (U(i + 1, j, k) + U(i, j, k)) * 0.5 * (hzeta_I(P, i, j, k) + hzeta_I(P, i + 1, j, k));
@@ -1250,7 +1258,7 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             double zh = 0.25 * (Om(i, j, k + 1) + Om(i - 1, j, k + 1)) * (U(i, j, k + 1) + U(i, j, k)) * 0.5 * (az + az);
             double zl = 0.25 * (Om(i, j, k) + Om(i - 1, j, k)) * (U(i, j, k - 1) + U(i, j, k)) * 0.5 * (az + az);
             src = (xh - xl) * dxi * 1.0 + (yh - yl) * dyi * 1.0 + (zh - zl) * dzi;
-            src = -src / (0.5 * (Jt(i, j, k) + Jt(i - 1, j, k)));
+            src = -src * iJ;
         } else {
             double a, xh, xl, yh, yl, zh, zl;
             a = 0.5 * (RU(i + 1, j, k) * 1.0 + RU(i, j, k) * 1.0); xh = a * interp_dir<HT>(0, i + 1, j, k, U, ht, a, hf) * 0.5 * (hzeta_I(P, i, j, k) + hzeta_I(P, i + 1, j, k));
@@ -1260,24 +1268,23 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             a = 0.5 * (Om(i, j, k + 1) + Om(i - 1, j, k + 1)) * 0.5 * (az + az); zh = a * interp_dir<VT>(2, i, j, k + 1, U, vt, a, vf);
             a = 0.5 * (Om(i, j, k) + Om(i - 1, j, k)) * 0.5 * (az + az); zl = a * interp_dir<VT>(2, i, j, k, U, vt, a, vf);
             src = (xh - xl) * dxi * 1.0 + (yh - yl) * dyi * 1.0 + (zh - zl) * dzi;
-            src /= 0.5 * (Jt(i, j, k) + Jt(i - 1, j, k));
-            src = -src;
+            src = -src * iJ;
         }
         double r = src;
         if (P.use_diff) {
             auto T11 = [&](int ii) { return double(ld(t11, eidx(g, wrap(ii, g.nx), j, k))); };
             double d = ((T11(i) - T11(i - 1)) * dxi * 1.0 + (double(t12[cidx(g, i, wrap(j + 1, g.ny), k)]) - double(t12[c])) * dyi * 1.0
                         + (double(t13[c + g.sk]) - double(t13[c])) * dzi);
-            d /= 0.5 * (Jt(i, j, k) + Jt(i - 1, j, k));
+            d *= iJ;
             r -= d;
         }
         double gpx = dxi * (pp(i, j, k) - pp(i - 1, j, k));
         {
-            double mxi = hxi_I(P, i, j, k), mz = hzeta_I(P, i, j, k), gz;
+            double gz;
             if (k == 0) gz = 0.5 * dzi * (pp(i - 1, j, k + 1) + pp(i, j, k + 1) - pp(i - 1, j, k) - pp(i, j, k));
             else if (k == nz - 1) gz = 0.5 * dzi * (pp(i - 1, j, k) + pp(i, j, k) - pp(i - 1, j, k - 1) - pp(i, j, k - 1));
             else gz = 0.25 * dzi * (pp(i - 1, j, k + 1) + pp(i, j, k + 1) - pp(i - 1, j, k - 1) - pp(i, j, k - 1));
-            gpx -= (mxi / mz) * gz;
+            gpx -= slope_I(P, i, j, k) * gz;
         }
         gpx *= 1.0;
         double xsrc = 0.0;
@@ -1287,12 +1294,14 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             xsrc += P.cf * (rvl * P.sinphi - rwl * P.cosphi);
         }
         xsrc += 0.5 * (S.cons[c] + S.cons[cidx(g, wrap(i - 1, g.nx), j, k)]) * P.geo0;
-        r += (-gpx - 0.0) / (1.0 + moist_q(P, A.prim, c, cidx(g, wrap(i - 1, g.nx), j, k))) + xsrc;
+        if (P.moist) gpx /= 1.0 + moist_q(P, A.prim, c, cidx(g, wrap(i - 1, g.nx), j, k));
+        r += xsrc - gpx;
         if (P.mt_zt) r *= hzeta_I(P, i, j, k);   // moving terrain (ERF_slow_rhs_pre.cpp:633-636)
         Fmx[c] = R(r);
     }
     // ---------------- y-momentum at face (i,j,k)
     {
+        const double iJ = 1.0 / (0.5 * (Jt(i, j, k) + Jt(i, j - 1, k)));
         double src;
         if (c2) {
             double xh = 0.25 * (RU(i + 1, j, k) * 1.0 + RU(i + 1, j - 1, k) * 1.0) * (V(i + 1, j, k) + V(i, j, k)) * hzeta_EK(P, i + 1, j, k);
@@ -1302,7 +1311,7 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             double zh = 0.25 * (Om(i, j, k + 1) + Om(i, j - 1, k + 1)) * (V(i, j, k + 1) + V(i, j, k)) * 0.5 * (az + az);
             double zl = 0.25 * (Om(i, j, k) + Om(i, j - 1, k)) * (V(i, j, k - 1) + V(i, j, k)) * 0.5 * (az + az);
             src = (xh - xl) * dxi * 1.0 + (yh - yl) * dyi * 1.0 + (zh - zl) * dzi;
-            src = -src / (0.5 * (Jt(i, j, k) + Jt(i, j - 1, k)));
+            src = -src * iJ;
         } else {
             double a, xh, xl, yh, yl, zh, zl;
             a = 0.5 * (RU(i + 1, j, k) * 1.0 + RU(i + 1, j - 1, k) * 1.0); xh = a * interp_dir<HT>(0, i + 1, j, k, V, ht, a, hf) * hzeta_EK(P, i + 1, j, k);
@@ -1312,24 +1321,23 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             a = 0.5 * (Om(i, j, k + 1) + Om(i, j - 1, k + 1)) * 0.5 * (az + az); zh = a * interp_dir<VT>(2, i, j, k + 1, V, vt, a, vf);
             a = 0.5 * (Om(i, j, k) + Om(i, j - 1, k)) * 0.5 * (az + az); zl = a * interp_dir<VT>(2, i, j, k, V, vt, a, vf);
             src = (xh - xl) * dxi * 1.0 + (yh - yl) * dyi * 1.0 + (zh - zl) * dzi;
-            src /= 0.5 * (Jt(i, j, k) + Jt(i, j - 1, k));
-            src = -src;
+            src = -src * iJ;
         }
         double r = src;
         if (P.use_diff) {
             auto T22 = [&](int jj) { return double(ld(t22, eidx(g, i, wrap(jj, g.ny), k))); };
             double d = ((double(t12[cidx(g, wrap(i + 1, g.nx), j, k)]) - double(t12[c])) * dxi * 1.0 + (T22(j) - T22(j - 1)) * dyi * 1.0
                         + (double(t23[c + g.sk]) - double(t23[c])) * dzi);
-            d /= 0.5 * (Jt(i, j, k) + Jt(i, j - 1, k));
+            d *= iJ;
             r -= d;
         }
         double gpy = dyi * (pp(i, j, k) - pp(i, j - 1, k));
         {
-            double meta = heta_J(P, i, j, k), mz = hzeta_J(P, i, j, k), gz;
+            double gz;
             if (k == 0) gz = 0.5 * dzi * (pp(i, j, k + 1) + pp(i, j - 1, k + 1) - pp(i, j, k) - pp(i, j - 1, k));
             else if (k == nz - 1) gz = 0.5 * dzi * (pp(i, j, k) + pp(i, j - 1, k) - pp(i, j, k - 1) - pp(i, j - 1, k - 1));
             else gz = 0.25 * dzi * (pp(i, j, k + 1) + pp(i, j - 1, k + 1) - pp(i, j, k - 1) - pp(i, j - 1, k - 1));
-            gpy -= (meta / mz) * gz;
+            gpy -= slope_J(P, i, j, k) * gz;
         }
         gpy *= 1.0;
         double ysrc = 0.0;
@@ -1338,7 +1346,8 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             ysrc += -P.cf * rul * P.sinphi;
         }
         ysrc += 0.5 * (S.cons[c] + S.cons[cidx(g, i, wrap(j - 1, g.ny), k)]) * P.geo1;
-        r += (-gpy - 0.0) / (1.0 + moist_q(P, A.prim, c, cidx(g, i, wrap(j - 1, g.ny), k))) + ysrc;
+        if (P.moist) gpy /= 1.0 + moist_q(P, A.prim, c, cidx(g, i, wrap(j - 1, g.ny), k));
+        r += ysrc - gpy;
         if (P.mt_zt) r *= hzeta_J(P, i, j, k);   // :681-684
         Fmy[c] = R(r);
     }
@@ -1350,6 +1359,7 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
     }
     {
         const int lo_z_face = 0, hi_z_face = nz;
+        const double iJ = 1.0 / (0.5 * (Jt(i, j, k) + Jt(i, j, k - 1)));
         double src;
         if (c2) {
             double xh = 0.25 * (RU(i + 1, j, k) + RU(i + 1, j, k - 1)) * 1.0 * (W(i + 1, j, k) + W(i, j, k)) * hzeta_EJ(P, i + 1, j, k);
@@ -1360,7 +1370,7 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             double zh = (k == hi_z_face) ? Om(i, j, k) * W(i, j, k) * az
                                          : 0.25 * (Om(i, j, k) + Om(i, j, k + 1)) * (W(i, j, k) + W(i, j, k + 1)) * 0.5 * (az + az);
             src = (xh - xl) * dxi * 1.0 + (yh - yl) * dyi * 1.0 + (zh - zl) * dzi;
-            src = -src / (0.5 * (Jt(i, j, k) + Jt(i, j, k - 1)));
+            src = -src * iJ;
         } else {
             double a, xh, xl, yh, yl, zh, zl;
             a = 0.5 * (RU(i + 1, j, k) + RU(i + 1, j, k - 1)) * 1.0; xh = a * interp_dir<HT>(0, i + 1, j, k, W, ht, a, hf) * hzeta_EJ(P, i + 1, j, k);
@@ -1394,16 +1404,14 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             } else il = interp_dir<VT>(2, i, j, k, W, vt, Ol, vf);
             zl = Ol * il;
             src = (xh - xl) * dxi * 1.0 + (yh - yl) * dyi * 1.0 + (zh - zl) * dzi;
-            double denom = 0.5 * (Jt(i, j, k) + Jt(i, j, k - 1));
-            src /= denom;
-            src = -src;
+            src = -src * iJ;
         }
         double r = src;
         if (P.use_diff) {
             double d = ((double(T.t31[cidx(g, wrap(i + 1, g.nx), j, k)]) - double(T.t31[c])) * dxi * 1.0
                         + (double(T.t32[cidx(g, i, wrap(j + 1, g.ny), k)]) - double(T.t32[c])) * dyi * 1.0
                         + (double(t33[c]) - double(t33[c - g.sk])) * dzi);
-            d /= 0.5 * (Jt(i, j, k) + Jt(i, j, k - 1));
+            d *= iJ;
             r -= d;
         }
         double mz = hzeta_K(P, i, j, k);
@@ -1435,7 +1443,9 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
             zsrc += P.cf * rul * P.cosphi;
         }
         zsrc += 0.5 * (S.cons[c] + S.cons[c - g.sk]) * P.geo2;
-        r += (zsrc - gpz - 0.0) / (1.0 + moist_q(P, A.prim, c, c - g.sk));
+        zsrc -= gpz;
+        if (P.moist) zsrc /= 1.0 + moist_q(P, A.prim, c, c - g.sk);
+        r += zsrc;
         if (P.mt_zt) r *= 0.5 * (Jt(i, j, k) + Jt(i, j, k - 1));   // :741-743
         Fmz[c] = R(r);
         if (k == nz - 1) Fmz[c + g.sk] = R(0);
@@ -1448,67 +1458,62 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
 // terrain-corrected gradient of the extrapolated d(rho theta); the old and
 // new increments are kept for the vertical part.
 // ---------------------------------------------------------------------------
-template <class R>
-__global__ void k_ter_fast_h(Params P, int step, double dtau, double facinv, StateBuf Sprev, int prev_rt,
-                             StateBuf Sst, StageAux<R> A, const R* __restrict__ Fmx, const R* __restrict__ Fmy,
-                             const R* __restrict__ lag_in, R* __restrict__ lag_out, TerBuf<R> T, R* __restrict__ avx,
-                             R* __restrict__ avy, double* __restrict__ outx, double* __restrict__ outy) {
+// After the first substep (of the fused step) the extrapolated d(rho theta)
+// comes from the vertical part, which has both substeps' values in hand, and
+// the old increments are the previous substep's new ones: nine loads in place
+// of twenty-seven.  The M -> V -> M round trip of the fill between substeps
+// is the identity but for rounding and is not applied.
+template <class R, bool FIRST>
+__global__ void k_ter_fast_h(Params P, int step, double dtau, double facinv, StateBuf Sprev, StateBuf Sst, StageAux<R> A,
+                             const R* __restrict__ Fmx, const R* __restrict__ Fmy, const R* __restrict__ lag_in,
+                             R* __restrict__ lag_out, TerBuf<R> T, R* __restrict__ avx, R* __restrict__ avy,
+                             double* __restrict__ outx, double* __restrict__ outy) {
     const Geo& g = P.g;
     int i, j, k;
     if (!cell_ij(g, i, j, k)) return;
-    const int nz = g.nz;
-    const int64_t N = g.ncell;
-    int im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
-    int64_t c = cidx(g, i, j, k), cxm = cidx(g, im, j, k), cym = cidx(g, i, jm, k);
-    const double beta_d = 0.1, dxi = g.dxi, dyi = g.dyi, dzi = g.dzi;
+    const int nz = g.nz, im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
+    const uint32_t c = eidx(g, i, j, k), cxm = eidx(g, im, j, k), cym = eidx(g, i, jm, k);
+    const double beta_d = 0.1, dxi = g.dxi, dyi = g.dyi;
+    const double* prt = Sprev.cons + g.ncell;
+    const double* srt = Sst.cons + g.ncell;
     auto extrap = [&](int ii, int jj, int kk) {
-        int64_t e = cidx(g, wrap(ii, g.nx), wrap(jj, g.ny), clampk(kk, nz));
-        double drt = Sprev.cons[N + e] - Sst.cons[N + e];
-        if (step == 0) return drt;
-        return drt + beta_d * (drt - double(lag_in[e]));
+        const uint32_t e = eidx(g, ii, jj, clampk(kk, nz));
+        if (!FIRST) return ld(T.ec, e);
+        const double drt = ld(prt, e) - ld(srt, e);
+        return step == 0 ? drt : drt + beta_d * (drt - double(ld(lag_in, e)));
     };
-    lag_out[c] = R(Sprev.cons[N + c] - Sst.cons[N + c]);
-    double px = Sprev.mx[c], py = Sprev.my[c];
-    if (prev_rt) {
-        double rs = Sprev.cons[c] + Sprev.cons[cxm];
-        double ut = (px * 2.0) / rs;
-        px = (ut * 0.5) * rs;
-        rs = Sprev.cons[c] + Sprev.cons[cym];
-        double vt = (py * 2.0) / rs;
-        py = (vt * 0.5) * rs;
+    if (FIRST && lag_out) at(lag_out, c) = R(ld(prt, c) - ld(srt, c));
+    double odu, odv;
+    if (FIRST) {
+        odu = ld(Sprev.mx, c) - ld(Sst.mx, c);
+        odv = ld(Sprev.my, c) - ld(Sst.my, c);
+        at(T.odu, c) = R(odu);
+        at(T.odv, c) = R(odv);
+    } else {
+        odu = double(ld(T.odu, c));
+        odv = double(ld(T.odv, c));
     }
-    double odu = px - Sst.mx[c], odv = py - Sst.my[c];
-    double gpx, gpy;
-    {
-        double mxi = hxi_I(P, i, j, k), mz = hzeta_I(P, i, j, k);
-        double gp_xi = (extrap(i, j, k) - extrap(i - 1, j, k)) * dxi;
-        double gp_zeta = (k == 0) ? 0.5 * dzi * (extrap(i - 1, j, k + 1) + extrap(i, j, k + 1) - extrap(i - 1, j, k) - extrap(i, j, k))
-                                  : 0.25 * dzi * (extrap(i - 1, j, k + 1) + extrap(i, j, k + 1) - extrap(i - 1, j, k - 1) - extrap(i, j, k - 1));
-        gpx = gp_xi - (mxi / mz) * gp_zeta;
-        gpx *= 1.0;
-        gpx /= (1.0 + moist_q(P, A.prim, c, cxm));
+    const int km = k == 0 ? 0 : k - 1;   // one-sided in the lowest cell
+    const double fz = (k == 0 ? 0.5 : 0.25) * g.dzi;
+    const double ec = extrap(i, j, k), exm = extrap(im, j, k), eym = extrap(i, jm, k);
+    const double ecz = extrap(i, j, k + 1) - extrap(i, j, km);
+    double gpx = (ec - exm) * dxi - slope_I(P, i, j, k) * (fz * (ecz + extrap(im, j, k + 1) - extrap(im, j, km)));
+    double gpy = (ec - eym) * dyi - slope_J(P, i, j, k) * (fz * (ecz + extrap(i, jm, k + 1) - extrap(i, jm, km)));
+    if (P.moist) {
+        gpx /= 1.0 + moist_q(P, A.prim, c, cxm);
+        gpy /= 1.0 + moist_q(P, A.prim, c, cym);
     }
-    {
-        double meta = heta_J(P, i, j, k), mz = hzeta_J(P, i, j, k);
-        double gp_eta = (extrap(i, j, k) - extrap(i, j - 1, k)) * dyi;
-        double gp_zeta = (k == 0) ? 0.5 * dzi * (extrap(i, j, k + 1) + extrap(i, j - 1, k + 1) - extrap(i, j, k) - extrap(i, j - 1, k))
-                                  : 0.25 * dzi * (extrap(i, j, k + 1) + extrap(i, j - 1, k + 1) - extrap(i, j, k - 1) - extrap(i, j - 1, k - 1));
-        gpy = gp_eta - (meta / mz) * gp_zeta;
-        gpy *= 1.0;
-        gpy /= (1.0 + moist_q(P, A.prim, c, cym));
-    }
-    double pix = 0.5 * (double(A.pi[cxm]) + double(A.pi[c]));
-    double piy = 0.5 * (double(A.pi[cym]) + double(A.pi[c]));
-    double fx = -Gamma_ * R_d * pix * gpx;
-    double fy = -Gamma_ * R_d * piy * gpy;
-    double ndu = odu + dtau * fx + dtau * double(Fmx[c]);
-    double ndv = odv + dtau * fy + dtau * double(Fmy[c]);
-    T.ndu[c] = R(ndu); T.ndv[c] = R(ndv);
-    T.odu[c] = R(odu); T.odv[c] = R(odv);
-    avx[c] += R(facinv * ndu);
-    avy[c] += R(facinv * ndv);
-    outx[c] = Sst.mx[c] + ndu;
-    outy[c] = Sst.my[c] + ndv;
+    const double pc = double(ld(A.pi, c));
+    const double fx = -Gamma_ * R_d * (0.5 * (double(ld(A.pi, cxm)) + pc)) * gpx;
+    const double fy = -Gamma_ * R_d * (0.5 * (double(ld(A.pi, cym)) + pc)) * gpy;
+    const double ndu = odu + dtau * fx + dtau * double(ld(Fmx, c));
+    const double ndv = odv + dtau * fy + dtau * double(ld(Fmy, c));
+    at(T.ndu, c) = R(ndu);
+    at(T.ndv, c) = R(ndv);
+    at(avx, c) += R(facinv * ndu);
+    at(avy, c) += R(facinv * ndv);
+    at(outx, c) = ld(Sst.mx, c) + ndu;
+    at(outy, c) = ld(Sst.my, c) + ndv;
 }
 
 // ---------------------------------------------------------------------------
@@ -1526,8 +1531,7 @@ __device__ __forceinline__ double prev_mz_ter(const Params& P, StateBuf Sprev, i
     const int nz = g.nz;
     int64_t f = cidx(g, i, j, k);
     double m = Sprev.mz[f];
-    if (!prev_rt) return m;
-    if (k == 0 || k == nz) {
+    if (prev_rt && (k == 0 || k == nz)) {
         auto U1 = [&](int ii, int jj, int kk) {
             if (kk >= nz) {
                 if (g.zhi_noslip) return 0.0;
@@ -1547,9 +1551,7 @@ __device__ __forceinline__ double prev_mz_ter(const Params& P, StateBuf Sprev, i
         double wb = w_from_omega(P, i, j, k, 0.0, U1, V1);
         return (wb * 0.5) * (r + r);
     }
-    double rs = Sprev.cons[f] + Sprev.cons[f - g.sk];
-    double wt = (m * 2.0) / rs;
-    return (wt * 0.5) * rs;
+    return m;
 }
 }  // namespace
 
@@ -1689,13 +1691,16 @@ __global__ void __launch_bounds__(1024) k_ter_fast_vert(Params P, double dtau, d
             double zh = beta_2 * sR[(k + 1) * TX + L] + beta_1 * sO[(k + 1) * TX + L];
             avz[c] += R(facinv * zl / (1.0 * 1.0));
             if (k == nz - 1) avz[c + sk] += R(facinv * zh / (1.0 * 1.0));
-            double Jc = detJ_at(P, i, j, k);
+            const double iJ = inv_detJ(P, i, j, k);
             double tc = th(i, j, k);
-            double frho = -(sT0[k * TX + L] + (zh - zl) * dzi) / Jc;
-            double frt = -(sT1[k * TX + L] + 0.5 * (zh * (tc + th(i, j, k + 1)) - zl * (tc + th(i, j, k - 1))) * dzi) / Jc;
+            double frho = -(sT0[k * TX + L] + (zh - zl) * dzi) * iJ;
+            double frt = -(sT1[k * TX + L] + 0.5 * (zh * (tc + th(i, j, k + 1)) - zl * (tc + th(i, j, k - 1))) * dzi) * iJ;
             double pr = Sprev.cons[c], prt = Sprev.cons[N + c];
             out_cons[c] = pr + dtau * (double(Fcons[c]) + frho);
-            out_cons[N + c] = prt + dtau * (double(Fcons[N + c]) + frt);
+            const double nrt = prt + dtau * (double(Fcons[N + c]) + frt);
+            out_cons[N + c] = nrt;
+            // the next substep's extrapolation: d + 0.1 (d - previous d) about the stage
+            T.ec[c] = (nrt - Sst.cons[N + c]) + 0.1 * (nrt - prt);
         }
     }
 }
@@ -1914,12 +1919,14 @@ void launch_ter_slow_mom(const Params& P, cudaStream_t st, StateBuf S, StageAux<
     (u5 ? k_ter_slow_mom<R, TU5, TU5> : k_ter_slow_mom<R, -1, -1>)<<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(
         P, S, A, u, v, w, t11, t22, t33, t12, t13, t23, T, Om, Fmx, Fmy, Fmz);
 }
+// ec_ready: the previous substep left the extrapolated d(rho theta) and its
+// increments (T.odu, T.odv); else both come from Sprev and lag_in.
 template <class R>
-void launch_ter_fast_h(const Params& P, cudaStream_t st, int step, double dtau, double facinv, StateBuf Sprev,
-                       int prev_rt, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in,
+void launch_ter_fast_h(const Params& P, cudaStream_t st, int step, bool ec_ready, double dtau, double facinv,
+                       StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in,
                        R* lag_out, TerBuf<R> T, R* avx, R* avy, double* outx, double* outy) {
-    k_ter_fast_h<R><<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(P, step, dtau, facinv, Sprev, prev_rt, Sst, A, Fmx,
-                                                                   Fmy, lag_in, lag_out, T, avx, avy, outx, outy);
+    (ec_ready ? k_ter_fast_h<R, false> : k_ter_fast_h<R, true>)<<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(
+        P, step, dtau, facinv, Sprev, Sst, A, Fmx, Fmy, lag_in, lag_out, T, avx, avy, outx, outy);
 }
 template <class R>
 void launch_ter_fast_vert(const Params& P, cudaStream_t st, int tx, size_t smem, double dtau, double facinv,
@@ -2005,8 +2012,8 @@ int ter_post_kz(const Params& P) {
     template void launch_ter_slow_mom<R>(const Params&, cudaStream_t, StateBuf, StageAux<R>, const double*,          \
                                          const double*, const double*, const R*, const R*, const R*, const R*,       \
                                          const R*, const R*, TerBuf<R>, const R*, R*, R*, R*);                       \
-    template void launch_ter_fast_h<R>(const Params&, cudaStream_t, int, double, double, StateBuf, int, StateBuf,    \
-                                       StageAux<R>, const R*, const R*, const R*, R*, TerBuf<R>, R*, R*, double*,    \
+    template void launch_ter_fast_h<R>(const Params&, cudaStream_t, int, bool, double, double, StateBuf, StateBuf,    \
+                                       StageAux<R>, const R*, const R*, const R*, R*, TerBuf<R>, R*, R*, double*,      \
                                        double*);                                                                     \
     template void launch_ter_fast_vert<R>(const Params&, cudaStream_t, int, size_t, double, double, double, double, \
                                           StateBuf, int, StateBuf, StageAux<R>, const R*, const R*, TerBuf<R>,       \
