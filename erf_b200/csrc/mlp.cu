@@ -33,26 +33,30 @@ namespace erfb {
 namespace mlp {
 
 // ---------------------------------------------------------------------------
-// Inference: Y = MLP(X) for rows [blockIdx.x*128, +128).  X is [n][13] FP32
-// raw features; the normalisation (mean/std per feature and per output) is
-// applied here.  TMEM: 64 columns, reused by every layer.
+// Inference: Y = MLP(X) for row tiles blockIdx.x, blockIdx.x + gridDim.x, ...
+// X is [n][13] FP32 raw features; the normalisation (mean/std per feature and
+// per output) is applied here.  TMEM: 64 columns, reused by every layer.
+// Bound: the tanh of 192 activations a row (16 a clock per SM) and the
+// latency of four dependent products; five CTAs share an SM (96 registers)
+// and each keeps its 20 KB of weights and its TMEM for all its tiles.  Rows
+// come and go through shared memory, so that a warp's accesses are whole
+// lines (a row is 52 bytes in, 36 out).  524288 rows: 188 us with a CTA per
+// tile that loaded the weights again and touched each line thirteen times.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(ROWS) k_mlp_infer(const float* __restrict__ X, int n, const unsigned char* __restrict__ wpack,
-                                                   const float* __restrict__ bias, const float* __restrict__ norm,
-                                                   float* __restrict__ Y, int* status) {
+__global__ void __launch_bounds__(ROWS, 5) k_mlp_infer(const float* __restrict__ X, int n, const unsigned char* __restrict__ wpack,
+                                                      const float* __restrict__ bias, const float* __restrict__ norm,
+                                                      float* __restrict__ Y, int* status) {
     __shared__ __align__(128) unsigned char sW[T_FWD_END];
     __shared__ __align__(128) unsigned char sX[ROWS * KIN * 2];
     __shared__ __align__(128) unsigned char sH[ROWS * HID * 2];
-    __shared__ float sB[NBIAS];
+    __shared__ float sB[NBIAS], sN[2 * NIN + 2 * NOUT];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tslot;
     const int t = threadIdx.x, warp = t >> 5;
-    const int row = blockIdx.x * ROWS + t;
     for (int q = t; q < T_FWD_END / 16; q += ROWS)
         reinterpret_cast<uint4*>(sW)[q] = reinterpret_cast<const uint4*>(wpack)[q];
     for (int q = t; q < NBIAS; q += ROWS) sB[q] = bias[q];
-    float x[NIN];
-    for (int q = 0; q < NIN; ++q) x[q] = row < n ? (X[(int64_t)row * NIN + q] - norm[q]) / norm[NIN + q] : 0.0f;
+    for (int q = t; q < 2 * NIN + 2 * NOUT; q += ROWS) sN[q] = norm[q];
     if (warp == 0) tmem_alloc(&tslot, 64);
     if (t == 0) bar_init(&bar);
     fence_before();
@@ -60,10 +64,26 @@ __global__ void __launch_bounds__(ROWS) k_mlp_infer(const float* __restrict__ X,
     fence_after();
     const uint32_t tm = tslot;
     uint32_t phase = 0;
-    float y[NOUTP];
-    bool ok = forward_cta(sW, sX, sH, sB, &bar, tm, phase, x, y);
-    if (row < n)
-        for (int q = 0; q < NOUT; ++q) Y[(int64_t)row * NOUT + q] = y[q] * norm[2 * NIN + NOUT + q] + norm[2 * NIN + q];
+    bool ok = true;
+    float* rows = reinterpret_cast<float*>(sH);   // the tile's inputs, then its outputs (no product reads sH then)
+    static_assert(ROWS * NIN * sizeof(float) <= sizeof(sH), "input tile");
+    const int tiles = (n + ROWS - 1) / ROWS;
+    for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
+        const int64_t r0 = (int64_t)b * ROWS;
+        const int m = min(ROWS, n - (int)r0);
+        for (int q = t; q < m * NIN; q += ROWS) rows[q] = X[r0 * NIN + q];
+        __syncthreads();
+        float x[NIN];
+#pragma unroll
+        for (int q = 0; q < NIN; ++q) x[q] = t < m ? (rows[t * NIN + q] - sN[q]) / sN[NIN + q] : 0.0f;
+        float y[NOUTP];
+        ok = forward_cta(sW, sX, sH, sB, &bar, tm, phase, x, y) && ok;   // begins and ends with a barrier
+#pragma unroll
+        for (int q = 0; q < NOUT; ++q) rows[t * NOUT + q] = y[q] * sN[2 * NIN + NOUT + q] + sN[2 * NIN + q];
+        __syncthreads();
+        for (int q = t; q < m * NOUT; q += ROWS) Y[r0 * NOUT + q] = rows[q];
+        __syncthreads();
+    }
     if (!ok && t == 0) atomicOr(status, 1);
     if (warp == 0) tmem_free(tm, 64);
 }
@@ -104,8 +124,10 @@ __global__ void __launch_bounds__(ROWS, 1) k_mlp_train(const float* __restrict__
     float v[HID];
 #pragma unroll
     for (int q = 0; q < HID; ++q) v[q] = 0.0f;
-    if (live)
+    if (live) {
+#pragma unroll
         for (int q = 0; q < NIN; ++q) v[q] = Xn[(int64_t)row * NIN + q];
+    }
     put_row(S.X0, KIN, t, v, KIN);
     put_col(S.X0T, t, v, KIN);
     if (warp == 0) tmem_alloc(&S.tslot, 512);
@@ -130,7 +152,9 @@ __global__ void __launch_bounds__(ROWS, 1) k_mlp_train(const float* __restrict__
         fence_after();
     };
     // ------------------------------------------------------------- forward
-    const int Wf[4] = {T_W1F, T_W2F, T_W3F, T_W4F};
+    // (the layer loops are unrolled so that the rows stay in registers)
+    constexpr int Wf[4] = {T_W1F, T_W2F, T_W3F, T_W4F};
+#pragma unroll
     for (int layer = 0; layer < 4; ++layer) {
         const int N = layer == 3 ? NOUTP : HID, K = layer == 0 ? KIN : HID;
         const unsigned char* A = layer == 0 ? S.X0 : S.H[layer - 1];
@@ -141,7 +165,9 @@ __global__ void __launch_bounds__(ROWS, 1) k_mlp_train(const float* __restrict__
         }
         wait_mma();
         if (layer < 3) {
+#pragma unroll
             for (int c = 0; c < 4; ++c) tmem_ld16(tm + lb + 64 * layer + c * 16, v + c * 16);
+#pragma unroll
             for (int q = 0; q < HID; ++q) v[q] = gelu(v[q] + S.B[layer * HID + q]);
             put_row(S.H[layer], HID, t, v, HID);
             put_col(S.HT[layer], t, v, HID);
@@ -152,6 +178,7 @@ __global__ void __launch_bounds__(ROWS, 1) k_mlp_train(const float* __restrict__
     float e[NOUTP];
     tmem_ld16(tm + lb + 192, e);
     float loss = 0.0f;
+#pragma unroll
     for (int q = 0; q < NOUTP; ++q) {
         float d = 0.0f;
         if (live && q < NOUT) {
@@ -163,28 +190,29 @@ __global__ void __launch_bounds__(ROWS, 1) k_mlp_train(const float* __restrict__
     // ------------------------------------------------------------- backward
     // layer l (3..0): dZ known in `e` (l = 3) or computed from dX; then
     // dW_l = dZ^T H_{l-1} and (l > 0) dX_{l-1} = dZ W_l.
-    const int Wb[4] = {0, T_W2B, T_W3B, T_W4B};
+    constexpr int Wb[4] = {0, T_W2B, T_W3B, T_W4B};
     float* g = gpart + (int64_t)blockIdx.x * NPAR;
-    const int OW[4] = {OW1, OW2, OW3, OW4};
+    constexpr int OW[4] = {OW1, OW2, OW3, OW4}, OB[4] = {OB1, OB2, OB3, OB4};
+#pragma unroll
+    for (int q = 0; q < NOUTP; ++q) v[q] = e[q];
+#pragma unroll
     for (int layer = 3; layer >= 0; --layer) {
         const int nout = layer == 3 ? NOUTP : HID;       // rows of dW (N of this layer)
         const int nin = layer == 0 ? KIN : HID;          // columns of dW (K of this layer)
-        float* dz = (layer == 3) ? e : v;
         // bias gradient: column sums of dZ over the CTA's rows
+#pragma unroll
         for (int q = 0; q < nout; ++q) {
-            float s = dz[q];
+            float s = v[q];
+#pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             if (lane == 0) S.red[warp][q] = s;
         }
-        put_row(S.dZ, nout, t, dz, nout);
-        put_col(S.dZT, t, dz, nout);
+        put_row(S.dZ, nout, t, v, nout);
+        put_col(S.dZT, t, v, nout);
         sync_mma();
-        if (t < nout) {
-            float s = S.red[0][t] + S.red[1][t] + S.red[2][t] + S.red[3][t];
-            g[(layer == 0 ? OB1 : layer == 1 ? OB2 : layer == 2 ? OB3 : OB4) + t] = s;
-        }
+        if (t < nout) g[OB[layer] + t] = S.red[0][t] + S.red[1][t] + S.red[2][t] + S.red[3][t];
         if (t == 0) {
-            const unsigned char* Hb = layer == 0 ? S.X0T : S.HT[layer - 1];
+            const unsigned char* Hb = layer == 0 ? S.X0T : S.HT[layer > 0 ? layer - 1 : 0];
             for (int kk = 0; kk < ROWS / 16; ++kk)
                 mma(tm + 256, sdesc(S.dZT, ROWS, kk), sdesc(Hb, ROWS, kk), idesc(ROWS, nin), kk > 0);
             if (layer > 0)
@@ -195,14 +223,24 @@ __global__ void __launch_bounds__(ROWS, 1) k_mlp_train(const float* __restrict__
         wait_mma();
         // dW rows: thread t < nout holds row t (output feature t)
         float w[HID];
+#pragma unroll
         for (int c = 0; c < nin / 16; ++c) tmem_ld16(tm + lb + 256 + c * 16, w + c * 16);
-        if (t < nout)
-            for (int q = 0; q < nin; ++q) g[OW[layer] + t * nin + q] = w[q];
+        if (t < nout) {
+            float4* gw = reinterpret_cast<float4*>(g + OW[layer] + t * nin);
+#pragma unroll
+            for (int q = 0; q < nin / 4; ++q) gw[q] = make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        }
         if (layer > 0) {
+#pragma unroll
             for (int c = 0; c < 4; ++c) tmem_ld16(tm + lb + 320 + c * 16, w + c * 16);
-            float z[HID];
-            for (int c = 0; c < 4; ++c) tmem_ld16(tm + lb + 64 * (layer - 1) + c * 16, z + c * 16);
-            for (int q = 0; q < HID; ++q) v[q] = live ? w[q] * gelu_grad(z[q] + S.B[(layer - 1) * HID + q]) : 0.0f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float z[16];
+                tmem_ld16(tm + lb + 64 * (layer - 1) + c * 16, z);
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    v[c * 16 + q] = live ? w[c * 16 + q] * gelu_grad(z[q] + S.B[(layer - 1) * HID + c * 16 + q]) : 0.0f;
+            }
         }
         fence_before();
         __syncthreads();
@@ -217,57 +255,72 @@ __global__ void __launch_bounds__(ROWS, 1) k_mlp_train(const float* __restrict__
     if (warp == 0) tmem_free(tm, 512);
 }
 
-// Sum of the per-CTA partials in a fixed order (deterministic).
+// Sum of the per-CTA partials in a fixed order (deterministic): four running
+// sums, so that the loads of four partials are in flight together.
+__device__ __forceinline__ float sum_partials(const float* __restrict__ p, int nblk, int64_t stride) {
+    float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    int b = 0;
+#pragma unroll 4
+    for (; b + 4 <= nblk; b += 4)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] += p[(b + q) * stride];
+    for (; b < nblk; ++b) a[0] += p[b * stride];
+    return (a[0] + a[1]) + (a[2] + a[3]);
+}
 __global__ void k_mlp_reduce(const float* __restrict__ gpart, const float* __restrict__ lpart, int nblk,
                              float* __restrict__ grad, float* __restrict__ loss) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < NPAR) {
-        float s = 0.0f;
-        for (int b = 0; b < nblk; ++b) s += gpart[(int64_t)b * NPAR + p];
-        grad[p] = s;
-    }
-    if (p == 0) {
-        float s = 0.0f;
-        for (int b = 0; b < nblk; ++b) s += lpart[b];
-        *loss = s;
+    if (p < NPAR) grad[p] = sum_partials(gpart + p, nblk, NPAR);
+    if (p == 0) *loss = sum_partials(lpart, nblk, 1);
+}
+
+// One parameter into the BF16 operand tiles (forward and transposed) or the
+// FP32 bias vector.
+__device__ __forceinline__ void pack_param(int p, float x, unsigned char* __restrict__ wpack, float* __restrict__ bias) {
+    auto put = [&](int tile, int r, int k, int K) {
+        *reinterpret_cast<__nv_bfloat16*>(wpack + tile + kmaj(r, k, K)) = __float2bfloat16_rn(x);
+    };
+    if (p < OW2) put(T_W1F, p / KIN, p % KIN, KIN);
+    else if (p < OW4) {
+        const bool second = p < OW3;
+        const int q = p - (second ? OW2 : OW3), r = q / HID, k = q % HID;
+        put(second ? T_W2F : T_W3F, r, k, HID);
+        put(second ? T_W2B : T_W3B, k, r, HID);
+    } else if (p < OB1) {
+        const int q = p - OW4, r = q / HID, k = q % HID;
+        put(T_W4F, r, k, HID);
+        put(T_W4B, k, r, NOUTP);
+    } else {
+        bias[p - OB1] = x;
     }
 }
 
-// Adam (Kingma & Ba 2015) on the FP32 master parameters; padded entries have
-// zero gradient and stay zero.
-__global__ void k_mlp_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v2,
-                           const float* __restrict__ grad, float lr, float b1, float b2, float eps, float c1, float c2) {
+// The end of a training step, one thread per parameter: the gradient from
+// the CTAs' partials, Adam (Kingma & Ba 2015) on the FP32 master parameters
+// (padded entries have zero gradient and stay zero) and the operand tiles
+// (three kernels of a few microseconds each otherwise).
+__global__ void k_mlp_update(const float* __restrict__ gpart, const float* __restrict__ lpart, int nblk,
+                             float* __restrict__ grad, float* __restrict__ loss, float* __restrict__ w,
+                             float* __restrict__ m, float* __restrict__ v2, float lr, float b1, float b2, float eps,
+                             float c1, float c2, unsigned char* __restrict__ wpack, float* __restrict__ bias) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0) *loss = sum_partials(lpart, nblk, 1);
     if (p >= NPAR) return;
-    float gr = grad[p];
+    const float gr = sum_partials(gpart + p, nblk, NPAR);
+    grad[p] = gr;
     float mm = b1 * m[p] + (1.0f - b1) * gr;
     float vv = b2 * v2[p] + (1.0f - b2) * gr * gr;
     m[p] = mm;
     v2[p] = vv;
-    w[p] -= lr * (mm * c1) / (sqrtf(vv * c2) + eps);
+    const float x = w[p] - lr * (mm * c1) / (sqrtf(vv * c2) + eps);
+    w[p] = x;
+    pack_param(p, x, wpack, bias);
 }
 
-// FP32 master parameters -> BF16 operand tiles (forward and transposed) and
-// the FP32 bias vector.
+// All master parameters into the operand tiles and the bias vector.
 __global__ void k_mlp_pack(const float* __restrict__ w, unsigned char* __restrict__ wpack, float* __restrict__ bias) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
-    auto put = [&](int tile, int r, int k, int K, float x) {
-        *reinterpret_cast<__nv_bfloat16*>(wpack + tile + kmaj(r, k, K)) = __float2bfloat16_rn(x);
-    };
-    if (p < HID * KIN) { int r = p / KIN, k = p % KIN; put(T_W1F, r, k, KIN, w[OW1 + p]); }
-    if (p < HID * HID) {
-        int r = p / HID, k = p % HID;
-        put(T_W2F, r, k, HID, w[OW2 + p]);
-        put(T_W3F, r, k, HID, w[OW3 + p]);
-        put(T_W2B, k, r, HID, w[OW2 + p]);
-        put(T_W3B, k, r, HID, w[OW3 + p]);
-    }
-    if (p < NOUTP * HID) {
-        int r = p / HID, k = p % HID;
-        put(T_W4F, r, k, HID, w[OW4 + p]);
-        put(T_W4B, k, r, NOUTP, w[OW4 + p]);
-    }
-    if (p < NBIAS) bias[p] = w[OB1 + p];
+    if (p < NPAR) pack_param(p, w[p], wpack, bias);
 }
 
 }  // namespace mlp
@@ -359,7 +412,7 @@ int erf_b200_mlp_set_params(erf_b200_mlp* M, const float* host_params) {
     cudaMemsetAsync(M->m, 0, NPAR * sizeof(float), M->stream);
     cudaMemsetAsync(M->v, 0, NPAR * sizeof(float), M->stream);
     M->step = 0;
-    k_mlp_pack<<<(HID * HID + 255) / 256, 256, 0, M->stream>>>(M->w, M->wpack, M->bias);
+    k_mlp_pack<<<(NPAR + 127) / 128, 128, 0, M->stream>>>(M->w, M->wpack, M->bias);
     return mlp_fail(cudaStreamSynchronize(M->stream));
 }
 
@@ -428,11 +481,11 @@ int erf_b200_mlp_train(erf_b200_mlp* M, const float* xn, const float* tn, int n,
         k_mlp_train<<<nblk, ROWS, sizeof(TrainSmem), M->stream>>>(xn + off * NIN, tn + off * NOUT, batch,
                                                                   1.0f / (float)(batch * NOUT), M->wpack, M->bias,
                                                                   M->gpart, M->lpart, M->status);
-        k_mlp_reduce<<<(NPAR + 255) / 256, 256, 0, M->stream>>>(M->gpart, M->lpart, nblk, M->grad, M->loss);
         M->step += 1;
         float c1 = 1.0f / (1.0f - powf(b1, (float)M->step)), c2 = 1.0f / (1.0f - powf(b2, (float)M->step));
-        k_mlp_adam<<<(NPAR + 255) / 256, 256, 0, M->stream>>>(M->w, M->m, M->v, M->grad, lr, b1, b2, eps, c1, c2);
-        k_mlp_pack<<<(HID * HID + 255) / 256, 256, 0, M->stream>>>(M->w, M->wpack, M->bias);
+        // 64 threads a block: the 10448 parameters over all SMs
+        k_mlp_update<<<(NPAR + 63) / 64, 64, 0, M->stream>>>(M->gpart, M->lpart, nblk, M->grad, M->loss, M->w, M->m, M->v,
+                                                             lr, b1, b2, eps, c1, c2, M->wpack, M->bias);
         off += batch;
     }
     if ((rc = mlp_fail(cudaGetLastError()))) return rc;
@@ -448,7 +501,11 @@ int erf_b200_mlp_train(erf_b200_mlp* M, const float* xn, const float* tn, int n,
 // Y [n][9] (raw units) = MLP(X [n][13] raw units), device arrays.
 int erf_b200_mlp_infer(erf_b200_mlp* M, const float* x, int n, float* y) {
     if (!M || !x || !y || n <= 0) return ERF_B200_EINVAL;
-    k_mlp_infer<<<(n + ROWS - 1) / ROWS, ROWS, 0, M->stream>>>(x, n, M->wpack, M->bias, M->norm, y, M->status);
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int tiles = (n + ROWS - 1) / ROWS, grid = tiles < 5 * nsm ? tiles : 5 * nsm;
+    k_mlp_infer<<<grid, ROWS, 0, M->stream>>>(x, n, M->wpack, M->bias, M->norm, y, M->status);
     int rc = mlp_fail(cudaGetLastError());
     if (rc) return rc;
     rc = mlp_fail(cudaStreamSynchronize(M->stream));

@@ -109,6 +109,7 @@ __device__ __forceinline__ void put_row(unsigned char* tile, int K, int r, const
 // Column r (as K index) of a K-major tile with ROWS columns: element (f, r)
 // for f < n.
 __device__ __forceinline__ void put_col(unsigned char* tile, int r, const float* v, int n) {
+#pragma unroll
     for (int f = 0; f < n; ++f)
         *reinterpret_cast<__nv_bfloat16*>(tile + kmaj(f, r, ROWS)) = __float2bfloat16_rn(v[f]);
 }
