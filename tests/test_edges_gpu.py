@@ -1,0 +1,167 @@
+"""GPU: the kernels at the sizes where their tiles and dispatches can go
+wrong -- planes that no column tile divides, the smallest box, odd level
+counts (the two eliminations of the W system meet on face nz / 2), columns so
+deep that the tile narrows, level counts that no block of the microphysics
+divides, views with ghost cells, row tiles of the network.
+
+Bars: FP64 against the oracle, relative L2 <= 1e-10 per field (the bar of the
+parity tests: rounding, amplified by a few steps); the FP32-bulk form against
+the oracle <= 1e-4 (its increments carry 24 bits); the network's BF16 products
+<= 1e-2 as in test_mlp_gpu."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+from erf_b200 import cases, config as C, terrain as T
+from helpers import compare_states, rel_l2
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+
+
+def _advance(case, base, state, steps, precision):
+    from erf_b200 import Dycore
+    cfg = case.cfg.copy()
+    cfg.precision = precision
+    dy = Dycore(cfg)
+    dy.set_base_state(base)
+    got = dy.advance_host(*state, steps)
+    assert dy.status() == 0
+    dy.close()
+    return got
+
+
+@pytest.mark.parametrize("size", [(4, 4, 4), (5, 7, 9), (36, 5, 13), (33, 31, 17), (8, 4, 150)])
+@pytest.mark.parametrize("flow,dyc,dry,moist", [("abl", C.UPWIND_5TH, C.UPWIND_5TH, C.WENO_5),
+                                                ("bubble", C.UPWIND_3RD, C.UPWIND_3RD, C.WENO_3)])
+def test_step(size, flow, dyc, dry, moist):
+    nx, ny, nz = size
+    case = cases.abl_dry(nx=nx, ny=ny, nz=nz) if flow == "abl" else cases.moist_bubble(nx=nx, ny=ny, nz=nz)
+    c = case.cfg
+    if nz > 80:
+        c.dz = c.dz * 80 / nz
+        c.dt = 0.5 * c.dt
+    c.dycore_horiz_adv = c.dycore_vert_adv = dyc
+    c.dryscal_horiz_adv = c.dryscal_vert_adv = dry
+    c.moistscal_horiz_adv = c.moistscal_vert_adv = moist
+    case.pert.update({"vel_noise_amp": 0.5})
+    base = oracle.make_base_state(c, case)
+    state = case.build_state(base[0])
+    ref = oracle.advance(c, base, *state, 2)
+    for precision, tol in ((C.PREC_FP64, TOL), (C.PREC_MIXED, 1e-4)):
+        errs = compare_states(_advance(case, base, state, 2, precision), ref)
+        bad = {k: e for k, e in errs.items() if not e <= tol}
+        assert not bad, (precision, errs)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(12, 4, 7), (24, 7, 33)])
+def test_moving_terrain_substeps(nx, ny, nz):
+    case = T.moving_terrain(nx=nx, ny=ny, nz=nz, Lx=5.0 * nx, Ly=5.0 * ny, H=5.0 * nz, ampl=0.05, wavelength=2.5 * nx,
+                            substeps=True, dt=0.02)
+    case.cfg.mri_ratio = 6
+    from erf_b200 import Dycore
+    state = case.build_state()
+    dy = Dycore(case.cfg)
+    dy.set_base_state(case.base)
+    got = dy.advance_host(*state, 3)
+    _, z, r0, p0 = dy.moving_terrain_state()
+    assert dy.status() == 0
+    dy.close()
+    ref = oracle.advance_moving_terrain(case.cfg, 0.0, case.base, *state, 3)
+    errs = {"rho": rel_l2(got[0][0], ref[0][0]), "rhotheta": rel_l2(got[0][1], ref[0][1]), "u": rel_l2(got[1], ref[1]),
+            "w": rel_l2(got[3], ref[3]), "z": rel_l2(z, ref[4]), "r0": rel_l2(r0, ref[5]), "p0": rel_l2(p0, ref[6])}
+    assert all(e <= TOL for e in errs.values()), errs
+
+
+@pytest.mark.parametrize("size,ghost,rain", [((24, 20, 40), 2, True), ((13, 9, 17), 1, True), ((13, 9, 17), 2, False),
+                                             ((33, 4, 8), 0, False)])
+def test_kessler_views(size, ghost, rain):
+    import torch
+    from erf_b200 import Dycore, dycore
+    from test_zz_no_alloc import ghost_fab
+    nx, ny, nz = size
+    case = cases.moist_bubble(nx=nx, ny=ny, nz=nz)
+    cfg = case.cfg
+    if not rain:
+        cfg.moisture, cfg.ncomp, cfg.buoyancy_type = C.MOIST_KESSLER_NORAIN, 7, 1
+    base = oracle.make_base_state(cfg, case)
+    cons = np.ascontiguousarray(case.build_state(base[0])[0][:cfg.ncomp])
+    rng = np.random.default_rng(3)
+    cons[5] *= 1.0 + 0.3 * rng.random(cons[5].shape)
+    cons[6] = cons[0] * 2.0e-3 * rng.random(cons[0].shape)
+    if rain:
+        cons[7] = cons[0] * 1.0e-3 * rng.random(cons[0].shape) * (rng.random(cons[0].shape) > 0.3)
+    ref = oracle.kessler(cfg, cons, cfg.dt)
+    g = ghost
+    x = np.full((cfg.ncomp, nz + 2 * g, ny + 2 * g, nx + 2 * g), -7.0)
+    inner = np.s_[:, g:g + nz, g:g + ny, g:g + nx]
+    x[inner] = cons
+    dy = Dycore(cfg)
+    t = torch.from_numpy(x).cuda()
+    f = ghost_fab(t, g, nx, ny, nz, cfg.ncomp)
+    torch.cuda.synchronize()
+    assert dycore.load_library().erf_b200_kessler_advance(dy.ctx, ctypes.byref(f), cfg.dt) == 0
+    assert dy.status() == 0
+    dy.close()
+    got = t.cpu().numpy()
+    for n in range(cfg.ncomp):
+        assert rel_l2(got[inner][n], ref[n]) <= TOL, n
+    # ghosts: periodic laterally, the nearest level vertically
+    want = np.pad(np.pad(got[inner], ((0, 0), (0, 0), (g, g), (g, g)), mode="wrap"), ((0, 0), (g, g), (0, 0), (0, 0)),
+                  mode="edge")
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 128 * 5 * 148 + 77])
+def test_network_row_tiles(n):
+    """One row, ragged tiles, and more tiles than resident blocks (a block's later tiles)."""
+    import torch
+    from erf_b200.closure import MLP
+    from oracle import mlp as ref
+    p = ref.init_params(4)
+    x = np.random.default_rng(n).standard_normal((n, 13)).astype(np.float32)
+    m = MLP()
+    m.set_params(p)
+    m.set_normalization(np.zeros(13), np.ones(13), np.zeros(9), np.ones(9))
+    y = torch.full((n + 1, 9), -7.0, device="cuda")
+    m.infer(torch.from_numpy(x).cuda(), y, n)
+    m.close()
+    y = y.cpu().numpy()
+    rows = np.unique(np.r_[0:min(n, 300), max(0, n - 300):n])
+    yr = ref.forward(p.astype(np.float64), x[rows].astype(np.float64), bf=True)
+    assert rel_l2(y[rows], yr) <= 1e-2
+    assert np.all(y[n] == -7.0) and np.all(y[:n] != -7.0)
+
+
+def test_training_step_is_adam_on_the_gradient():
+    """One minibatch: the parameters move by Adam's first step on the gradient
+    that erf_b200_mlp_gradient returns (FP32: 1e-6), and the packed tiles
+    follow (the second gradient is that of the moved parameters)."""
+    import torch
+    from erf_b200.closure import MLP
+    from oracle import mlp as ref
+    n, lr = 700, 1e-3
+    rng = np.random.default_rng(2)
+    x = torch.from_numpy(rng.standard_normal((n, 13)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.standard_normal((n, 9)).astype(np.float32)).cuda()
+    p = ref.init_params(6)
+    a, b = MLP(), MLP()
+    for m in (a, b):
+        m.set_params(p)
+        m.set_normalization(np.zeros(13), np.ones(13), np.zeros(9), np.ones(9))
+    loss, g = a.gradient(x, t, n)
+    assert abs(b.train(x, t, n, n, 1, lr) - loss) <= 1e-6 * loss
+    q = b.get_params()
+    g64 = g.astype(np.float64)
+    want = p - lr * g64 / (np.abs(g64) + 1e-8)
+    # eps against the gradient's own rounding where a gradient is near 0
+    ok = (np.abs(g64) > 1e-6) | (g64 == 0.0)
+    assert np.max(np.abs(q - want)[ok]) <= 1e-3 * lr
+    _, g1 = b.gradient(x, t, n)
+    a.set_params(q)
+    _, g2 = a.gradient(x, t, n)
+    a.close()
+    b.close()
+    assert np.array_equal(g1, g2)
