@@ -686,8 +686,9 @@ void enqueue_step_t(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
             sa.av_init = ks == 0;
             TIMED(6, launch_substep<R>(P, st, c->sub, ks > 0 ? 2 : (nrk > 0 ? 1 : 0), ks == nsub - 1, sa));
         }
-        TIMED(7, launch_post<R>(P, c->tkz, st, slow_dt, OLD, Sst, SUM, Snew, Acur, Anext, nrk < 2 ? 1 : 0, B.mut,
-                                B.tke, B.avx, B.avy, B.avz, Vnew[0], Vnew[1], Vnew[2]));
+        // (rho KE without Deardorff and rho QKE pass through: from the old state, at the last stage)
+        TIMED(7, launch_post<R>(P, c->tkz, st, slow_dt, OLD, Sst, SUM, Snew, Acur, Anext, nrk < 2 ? 1 : 0,
+                                nrk < 2 ? nullptr : OLD.cons, B.mut, B.tke, B.avx, B.avy, B.avz, Vnew[0], Vnew[1], Vnew[2]));
         a = 1 - a;
     }
     if (P.moist) TIMED(8, kessler_step(c, N0, N1));
@@ -1568,8 +1569,8 @@ int erf_b200_slow_rhs_post(erf_b200_ctx* c, int nrk, double slow_dt, const erf_b
         launch_ter_post<double>(c->P, c->stream, c->tkz.ter_post, slow_dt, OLD, c->S[2], SUM, NEW, B.aux[0], B.aux[1], 0, B.mut, B.tke,
                                 B.ter, B.avx, B.avy, B.avz, c->vel[1][0], c->vel[1][1], c->vel[1][2]);
     else
-    launch_post<double>(c->P, c->tkz, c->stream, slow_dt, OLD, c->S[2], SUM, NEW, B.aux[0], B.aux[1], 0, B.mut, B.tke,
-                        B.avx, B.avy, B.avz, c->vel[1][0], c->vel[1][1], c->vel[1][2]);
+    launch_post<double>(c->P, c->tkz, c->stream, slow_dt, OLD, c->S[2], SUM, NEW, B.aux[0], B.aux[1], 0, c->S[2].cons,
+                        B.mut, B.tke, B.avx, B.avy, B.avz, c->vel[1][0], c->vel[1][1], c->vel[1][2]);
     if ((rc = unpack4(c, S_new, nc, NEW.cons, NEW.mx, NEW.my, NEW.mz))) return rc;
     return cuda_fail(cudaGetLastError());
 }

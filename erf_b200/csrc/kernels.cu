@@ -156,23 +156,32 @@ __device__ __forceinline__ bool cell_coords(const Geo& g, int& i, int& j, int& k
     return i < g.nx && j < g.ny && k < g.nz;
 }
 
+// Whether any pass reads primitive n: KE with Deardorff only, QKE never (no PBL scheme).
+__device__ __forceinline__ bool prim_read(const Params& P, int n) {
+    return n != ERF_RHOQKE_COMP - 1 && (n != ERF_RHOKE_COMP - 1 || P.les == ERF_LES_DEARDORFF);
+}
+
 // Derived stage quantities of one cell: cons_to_prim + pi_stage
 // (TimeIntegration/ERF_TI_utils.H:4-45) and p' (ERF_slow_rhs_pre.cpp:337-358),
 // evaluated in FP64 from the FP64 state and stored as R.
 template <class R>
+__device__ __forceinline__ void stage_aux_thermo(const Params& P, double rho, double rt, double ir, double qv, StageAux<R> A,
+                                                 int64_t c, int k) {
+    A.prim[c] = R(rt * ir);
+    const double x = R_d * rt * ip_0, l = log(x);   // of the Exner function, and of p where the air is dry
+    A.pi[c] = R(exp(Gamma_ * P.rdOcp * l));
+    const double lp = P.moist ? log(x * (1.0 + (R_v / R_d) * qv)) : l;
+    A.pp[c] = R(p_0 * exp(Gamma_ * lp) - (P.ter ? P.p0[c + P.g.sk] : P.p0[k + 1]));
+    if (!(rt > 0.0) || !(rho > 0.0)) atomicOr(P.status, ST_BADSTATE);
+}
+template <class R>
 __device__ __forceinline__ void stage_aux_cell(const Params& P, const double* __restrict__ cons, StageAux<R> A,
                                                int64_t c, int k) {
     const int64_t N = P.g.ncell;
-    double rho = cons[c];
-    double rt = cons[N + c];
-    const double ir = 1.0 / rho;
-    A.prim[c] = R(rt * ir);
-    for (int n = 1; n < P.nprim; ++n) A.prim[n * N + c] = R(cons[(n + 1) * N + c] * ir);
-    const double x = R_d * rt * ip_0, l = log(x);   // of the Exner function, and of p where the air is dry
-    A.pi[c] = R(exp(Gamma_ * P.rdOcp * l));
-    const double lp = P.moist ? log(x * (1.0 + (R_v / R_d) * (cons[5 * N + c] * ir))) : l;
-    A.pp[c] = R(p_0 * exp(Gamma_ * lp) - (P.ter ? P.p0[c + P.g.sk] : P.p0[k + 1]));
-    if (!(rt > 0.0) || !(rho > 0.0)) atomicOr(P.status, ST_BADSTATE);
+    const double rho = cons[c], ir = 1.0 / rho;
+    for (int n = 1; n < P.nprim; ++n)
+        if (prim_read(P, n)) A.prim[n * N + c] = R(cons[(n + 1) * N + c] * ir);
+    stage_aux_thermo<R>(P, rho, cons[N + c], ir, P.moist ? cons[5 * N + c] * ir : 0.0, A, c, k);
 }
 
 // ---------------------------------------------------------------------------
@@ -389,6 +398,28 @@ __device__ __forceinline__ R scalar_diff(const Params& P, const double* __restri
         if (k == g.nz - 1) fz_out[cidx(g, i, j, k + 1)] = fzh;
     }
     return (fxh - fxl) * dxi * R(1) + (fyh - fyl) * dyi * R(1) + (fzh - fzl) * dzi;
+}
+
+// The same from the cell's and its neighbours' values (p[0] the cell; x low,
+// high; y low, high; z low, high), for a pass that has them staged.
+template <class R>
+__device__ __forceinline__ R scalar_diff_vals(const Params& P, const double* __restrict__ rhoarr, const R (&p)[7],
+                                              const R* __restrict__ mut, double ae_d, double fac_d, int i, int j, int k) {
+    const Geo& g = P.g;
+    const R ae = R(ae_d), fac = R(fac_d);
+    const uint32_t sk = (uint32_t)g.sk, c = eidx(g, i, j, k);
+    const uint32_t e[6] = {eidx(g, wrap(i - 1, g.nx), j, k), eidx(g, wrap(i + 1, g.nx), j, k), eidx(g, i, wrap(j - 1, g.ny), k),
+                           eidx(g, i, wrap(j + 1, g.ny), k), k > 0 ? c - sk : c, k < g.nz - 1 ? c + sk : c};
+    const R rc = P.use_consA ? R(ld(rhoarr, c)) : R(0), mc = P.use_turb ? ld(mut, c) * fac : R(0);
+    R f[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        R r = P.use_consA ? R(0.5) * (rc + R(ld(rhoarr, e[q]))) * ae : ae;
+        if (P.use_turb) r += R(0.5) * (mc + ld(mut, e[q]) * fac);
+        f[q] = -r * (q & 1 ? p[q + 1] - p[0] : p[0] - p[q + 1]);
+    }
+    const R dxi = R(g.dxi), dyi = R(g.dyi), dzi = R(g.dzi);
+    return (f[1] - f[0]) * dxi * dxi + (f[3] - f[2]) * dyi * dyi + (f[5] - f[4]) * dzi * dzi;
 }
 
 // Horizontal plane averages of rho, theta, qv, qc, qp for buoyancy type 2
@@ -822,119 +853,152 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_CELL) k_slow_cell(Params 
 //     variables, Exner function and p'.
 // ---------------------------------------------------------------------------
 // Slow variables, in order: the passive scalar, the moisture species, then
-// (Deardorff) rho*KE.  NS is the kernel's capacity: 4 holds the scalar and
-// three species, 5 adds KE to them.
-template <class R, int DH, int DV, int MH, int MV, int NS>
-__global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_POST) k_post(Params P, int kz, double slow_dt, StateBuf Sold,
-                                                                    StateBuf Sst, StateBuf Ssum, StateBuf Snew,
-                                                                    StageAux<R> Acur, StageAux<R> Anext, int make_next,
-                                                                    const R* __restrict__ mut, TkeBuf<R> tke,
-                                                                    const R* __restrict__ avx,
-                                                                    const R* __restrict__ avy,
-                                                                    const R* __restrict__ avz, double* __restrict__ un,
-                                                                    double* __restrict__ vn, double* __restrict__ wn) {
-    __shared__ FluxTile<R> sh[NS];
-    __shared__ Plane<R> pl[NS];
+// (Deardorff) rho*KE.  A block marches ONE of them up its tile; the rest of
+// the stage's end goes to the scalar's blocks (the copies, momenta and
+// velocities) and to the vapour's (theta, Exner function and p' of the next
+// stage; the scalar's in dry air).  With all variables in one block the
+// vertical stencils were loads, L2 hits mostly, on every level (four of six
+// levels each on the moist bubble, 262 us per stage at 128x128x80); one at a
+// time, the column is a window in registers, fed a level ahead along with the
+// momenta.  The jobs of a tile are neighbours in the grid, so that what they
+// share is read from DRAM once.
+template <class R>
+struct PostArgs {
+    double slow_dt;
+    StateBuf old, st, sum, nw;
+    StageAux<R> cur, next;
+    int make_next;
+    const double* keep;   // the state whose rho KE (no Deardorff) and rho QKE go on
+    const R* mut;
+    TkeBuf<R> tke;
+    const R *avx, *avy, *avz;
+    double *un, *vn, *wn;
+};
+template <class R, int TH, int TV>
+__device__ __forceinline__ void post_march(const Params& P, const PostArgs<R>& a, FluxTile<R>& sh, Plane<R>& pl, int th,
+                                           int tv, R fh, R fv, int q, int nscal, int nslow, int k0, int k1) {
     const Geo& g = P.g;
     const int64_t N = g.ncell;
-    const int i = blockIdx.x * TTX + threadIdx.x, j = blockIdx.y * TTY + threadIdx.y;
+    const uint32_t sk = (uint32_t)g.sk;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int i = blockIdx.x * TTX + tx, j = blockIdx.y * TTY + ty;
     const bool ok = i < g.nx && j < g.ny;
-    const int k0 = blockIdx.z * kz, k1 = min(k0 + kz, g.nz);
     const int im = ok ? wrap(i - 1, g.nx) : 0, jm = ok ? wrap(j - 1, g.ny) : 0;
-    const bool dd = P.les == ERF_LES_DEARDORFF;
-    const int nscal = P.moist ? 1 + (P.ncomp - ERF_RHOQ1_COMP) : 1;
-    const int nslow = nscal + (dd ? 1 : 0);
-    R zl[NS], zh[NS];
-#pragma unroll
-    for (int q = 0; q < NS; ++q) zl[q] = zh[q] = R(0);
+    const bool dd = P.les == ERF_LES_DEARDORFF, ke = q >= nscal;
+    const int n = q == 0 ? ERF_RHOSCALAR_COMP : (ke ? ERF_RHOKE_COMP : ERF_RHOQ1_COMP + q - 1);
+    const bool thermo = P.moist ? n == ERF_RHOQ1_COMP : q == 0;
+    const R* __restrict__ phi = a.cur.prim + (int64_t)(n - 1) * N;
     const TileEdge edge = tile_edge(g);
     const PlaneIdx pidx(g);
-    auto comp_of = [&](int q) {
-        return q == 0 ? ERF_RHOSCALAR_COMP : (q < nscal ? ERF_RHOQ1_COMP + q - 1 : ERF_RHOKE_COMP);
-    };
-    auto slow_phi = [&](int q) { return Acur.prim + (int64_t)(comp_of(q) - 1) * N; };
+    constexpr int W = TV < 0 ? 3 : (TV == ERF_ADV_CENTERED_2ND ? 1 : (TV == ERF_ADV_UPWIND_5TH || TV == ERF_ADV_CENTERED_6TH || TV == ERF_ADV_WENO_5 ? 3 : 2));
+    const uint32_t e0 = ok ? eidx(g, i, j, 0) : 0;
+    auto lvl = [&](int k) { return ld(phi, e0 + sk * (uint32_t)clampk(k, g.nz)); };
+    // win[m]: phi at level f - W + m of the face f whose flux comes next
+    R win[2 * W];
+    auto zflux = [&](R az) {
+        R s[6];
 #pragma unroll
-    for (int q = 0; q < NS; ++q)
-        if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k0);
+        for (int m = 0; m < 6; ++m) s[m] = (m >= 3 - W && m < 3 + W) ? win[m >= 3 - W && m < 3 + W ? m - 3 + W : 0] : R(0);
+        return az * interp_of<TV, R>(tv, s, az, fv);
+    };
+    R zl = R(0), ax = R(0), ay = R(0), az = R(0), top = R(0);
+    load_plane(g, pidx, pl, phi, k0);
+    if (ok) {
+#pragma unroll
+        for (int m = 0; m < 2 * W; ++m) win[m] = lvl(k0 - W + m);
+        const uint32_t c = e0 + sk * (uint32_t)k0;
+        zl = zflux(ld(a.avz, c));
+        ax = ld(a.avx, c); ay = ld(a.avy, c); az = ld(a.avz, c + sk);
+        top = lvl(k0 + W);
+    }
     for (int k = k0; k < k1; ++k) {
+        const uint32_t c = e0 + sk * (uint32_t)k;
+        R zh = R(0), dif = R(0);
         plane_wait();
         __syncthreads();
         if (ok) {
+            sh.fx[ty][tx] = plane_flux_x<TH>(pl, ty, tx, ax, th, fh);
+            sh.fy[ty][tx] = plane_flux_y<TH>(pl, ty, tx, ay, th, fh);
 #pragma unroll
-            for (int q = 0; q < NS; ++q) {
-                if (q >= nslow) break;
-                if (q == 0 || q >= nscal)   // scalar and KE: dry-scalar schemes
-                    tile_put<DH, DV>(g, sh[q], pl[q], slow_phi(q), avx, avy, avz, P.dry_h, P.dry_v, R(P.f_dry_h),
-                                     R(P.f_dry_v), i, j, k, k == k0, zl[q], zh[q]);
-                else
-                    tile_put<MH, MV>(g, sh[q], pl[q], slow_phi(q), avx, avy, avz, P.moi_h, P.moi_v, R(P.f_moi_h),
-                                     R(P.f_moi_v), i, j, k, k == k0, zl[q], zh[q]);
+            for (int m = 0; m < 2 * W - 1; ++m) win[m] = win[m + 1];
+            win[2 * W - 1] = top;
+            zh = zflux(az);
+            if (ke || P.use_diff) {
+                const int y = ty + PH, x = tx + PH;
+                const R pc = pl.v[y][x];
+                const R p[7] = {pc, pl.v[y][x - 1], pl.v[y][x + 1], pl.v[y - 1][x], pl.v[y + 1][x],
+                                W > 1 ? win[W > 1 ? W - 2 : 0] : lvl(k - 1), W > 1 ? win[W] : lvl(k + 1)};
+                dif = scalar_diff_vals<R>(P, a.st.cons, p, a.mut, ke ? 0.0 : P.alphaC_eff, ke ? P.invSigmaK : P.invSc, i, j, k);
             }
         }
-#pragma unroll
-        for (int q = 0; q < NS; ++q) {
-            if (q >= nslow) break;
-            if (q == 0 || q >= nscal)
-                tile_put_edge<DH>(g, edge, sh[q], pl[q], avx, avy, P.dry_h, R(P.f_dry_h), k);
-            else
-                tile_put_edge<MH>(g, edge, sh[q], pl[q], avx, avy, P.moi_h, R(P.f_moi_h), k);
-        }
+        tile_put_edge<TH>(g, edge, sh, pl, a.avx, a.avy, th, fh, k);
         __syncthreads();
-        if (k + 1 < k1) {   // next level's planes arrive during the update below
-#pragma unroll
-            for (int q = 0; q < NS; ++q)
-                if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k + 1);
-        }
+        if (k + 1 < k1) load_plane(g, pidx, pl, phi, k + 1);   // arrives during the update below
         if (ok) {
-            int64_t c = cidx(g, i, j, k);
-#pragma unroll
-            for (int q = 0; q < NS; ++q) {
-                if (q >= nslow) break;
-                const int n = comp_of(q);
-                R r = tile_div(g, sh[q], zl[q], zh[q]);
-                zl[q] = zh[q];
-                if (q < nscal) {
-                    if (P.use_diff)
-                        r -= scalar_diff<R>(P, Sst.cons, Acur.prim + (int64_t)(n - 1) * N, mut, P.alphaC_eff, P.invSc,
-                                            i, j, k);
-                } else {
-                    // KE diffusion (alpha 0, K / sigma_k) and the TKE sources of
-                    // ERF_DiffusionSrcForState_N.cpp:681-707: buoyancy, shear
-                    // production, dissipation
-                    r -= scalar_diff<R>(P, Sst.cons, Acur.prim + (int64_t)(n - 1) * N, mut, 0.0, P.invSigmaK, i, j, k);
-                    r += R(P.g_over_theta0) * tke.hfz[c];
-                    r += R(2.0) * mut[c] * tke.smn[c];
-                    r -= tke.diss[c];
+            if (k + 1 < k1) {   // the next level's operands
+                ax = ld(a.avx, c + sk); ay = ld(a.avy, c + sk); az = ld(a.avz, c + 2 * sk);
+                top = lvl(k + 1 + W);
+            }
+            R r = tile_div(g, sh, zl, zh);
+            zl = zh;
+            r -= dif;
+            if (ke) {
+                // the TKE sources of ERF_DiffusionSrcForState_N.cpp:681-707:
+                // buoyancy, shear production, dissipation
+                r += R(P.g_over_theta0) * a.tke.hfz[c];
+                r += R(2.0) * a.mut[c] * a.tke.smn[c];
+                r -= a.tke.diss[c];
+            }
+            double nv = ld(a.old.cons + n * N, c) + a.slow_dt * double(r);
+            if (q > 0) nv = fmax(nv, ke ? 2.220446049250313e-16 : 0.0);
+            if (n == 7 && a.nw.rain) a.nw.rain[c] = nv;
+            else at(a.nw.cons + n * N, c) = nv;
+            const double rho = ld(a.sum.cons, c);
+            double ir = 0.0;
+            if (a.make_next) {
+                ir = 1.0 / rho;
+                at(a.next.prim + (n - 1) * N, c) = R(nv * ir);
+            }
+            if (thermo && a.make_next)
+                stage_aux_thermo<R>(P, rho, ld(a.sum.cons + N, c), ir, P.moist ? nv * ir : 0.0, a.next, c, k);
+            if (q == 0) {
+                at(a.nw.cons, c) = rho;
+                at(a.nw.cons + N, c) = ld(a.sum.cons + N, c);
+                if (a.keep) {
+                    if (!dd) at(a.nw.cons + 2 * N, c) = ld(a.keep + 2 * N, c);
+                    at(a.nw.cons + 3 * N, c) = ld(a.keep + 3 * N, c);
                 }
-                double v_ = Sold.cons[n * N + c] + slow_dt * double(r);
-                const double nv = (q == 0) ? v_ : fmax(v_, q < nscal ? 0.0 : 2.220446049250313e-16);
-                if (n == 7 && Snew.rain) Snew.rain[c] = nv;
-                else Snew.cons[n * N + c] = nv;
+                {
+                    const double rs = rho + ld(a.sum.cons, eidx(g, im, j, k)), m = ld(a.sum.mx, c);
+                    at(a.nw.mx, c) = m; at(a.un, c) = (m * 2.0) / rs;
+                }
+                {
+                    const double rs = rho + ld(a.sum.cons, eidx(g, i, jm, k)), m = ld(a.sum.my, c);
+                    at(a.nw.my, c) = m; at(a.vn, c) = (m * 2.0) / rs;
+                }
+                if (k == 0) {
+                    at(a.nw.mz, c) = 0.0; at(a.wn, c) = 0.0;
+                } else {
+                    const double rs = rho + ld(a.sum.cons, c - sk), m = ld(a.sum.mz, c);
+                    at(a.nw.mz, c) = m; at(a.wn, c) = (m * 2.0) / rs;
+                }
+                if (k == g.nz - 1) { at(a.nw.mz, c + sk) = 0.0; at(a.wn, c + sk) = 0.0; }
             }
-            Snew.cons[c] = Ssum.cons[c];
-            Snew.cons[N + c] = Ssum.cons[N + c];
-            if (!dd) Snew.cons[2 * N + c] = Sst.cons[2 * N + c];
-            Snew.cons[3 * N + c] = Sst.cons[3 * N + c];
-            double rho = Ssum.cons[c];
-            {
-                const double rs = rho + Ssum.cons[cidx(g, im, j, k)], m = Ssum.mx[c];
-                Snew.mx[c] = m; un[c] = (m * 2.0) / rs;
-            }
-            {
-                const double rs = rho + Ssum.cons[cidx(g, i, jm, k)], m = Ssum.my[c];
-                Snew.my[c] = m; vn[c] = (m * 2.0) / rs;
-            }
-            if (k == 0) {
-                Snew.mz[c] = 0.0; wn[c] = 0.0;
-            } else {
-                const double rs = rho + Ssum.cons[c - g.sk], m = Ssum.mz[c];
-                Snew.mz[c] = m; wn[c] = (m * 2.0) / rs;
-            }
-            if (k == g.nz - 1) { Snew.mz[c + g.sk] = 0.0; wn[c + g.sk] = 0.0; }
-            if (make_next) stage_aux_cell<R>(P, Snew.cons, Anext, c, k);
         }
         // the next level's first barrier orders the reuse of sh
     }
+}
+template <class R, int DH, int DV, int MH, int MV>
+__global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_POST) k_post(Params P, int kz, PostArgs<R> a) {
+    __shared__ FluxTile<R> sh;
+    __shared__ Plane<R> pl;
+    const int nscal = P.moist ? 1 + (P.ncomp - ERF_RHOQ1_COMP) : 1;
+    const int nslow = nscal + (P.les == ERF_LES_DEARDORFF ? 1 : 0);
+    const int q = blockIdx.z % nslow, k0 = blockIdx.z / nslow * kz, k1 = min(k0 + kz, P.g.nz);
+    if (q == 0 || q >= nscal)   // scalar and KE: dry-scalar schemes
+        post_march<R, DH, DV>(P, a, sh, pl, P.dry_h, P.dry_v, R(P.f_dry_h), R(P.f_dry_v), q, nscal, nslow, k0, k1);
+    else
+        post_march<R, MH, MV>(P, a, sh, pl, P.moi_h, P.moi_v, R(P.f_moi_h), R(P.f_moi_v), q, nscal, nslow, k0, k1);
 }
 
 // Momentum fluxes of AdvectionSrcFor{X,Y,Z}Mom_N (ERF_AdvectionSrcForMom_N.H:
@@ -1284,8 +1348,7 @@ template <class R>
 using SlowMomK = void (*)(Params, int, StateBuf, StageAux<R>, const double*, const double*, const double*, const R*,
                           const R*, const R*, const R*, const R*, const R*, const double*, R*, R*, R*);
 template <class R>
-using PostK = void (*)(Params, int, double, StateBuf, StateBuf, StateBuf, StateBuf, StageAux<R>, StageAux<R>, int,
-                       const R*, TkeBuf<R>, const R*, const R*, const R*, double*, double*, double*);
+using PostK = void (*)(Params, int, PostArgs<R>);
 
 template <class R>
 SlowCellK<R> slow_cell_kernel(const Params& P) {
@@ -1300,28 +1363,31 @@ SlowMomK<R> slow_mom_kernel(const Params& P) {
     if (P.dyc_h == U3 && P.dyc_v == U3) return k_slow_mom<R, U3, U3>;
     return k_slow_mom<R, -1, -1>;
 }
+int post_jobs(const Params& P) {
+    return (P.moist ? 1 + (P.ncomp - ERF_RHOQ1_COMP) : 1) + (P.les == ERF_LES_DEARDORFF ? 1 : 0);
+}
 template <class R>
 PostK<R> post_kernel(const Params& P) {
-    bool dw = P.dry_h == W5 && P.dry_v == W5, du = P.dry_h == U5 && P.dry_v == U5;
-    const bool d3 = P.dry_h == U3 && P.dry_v == U3, m3 = P.moi_h == W3 && P.moi_v == W3;
-    bool mw = P.moi_h == W5 && P.moi_v == W5, mu = P.moi_h == U5 && P.moi_v == U5;
-    const int nslow = (P.moist ? 1 + (P.ncomp - ERF_RHOQ1_COMP) : 1) + (P.les == ERF_LES_DEARDORFF ? 1 : 0);
+    const bool dw = P.dry_h == W5 && P.dry_v == W5, du = P.dry_h == U5 && P.dry_v == U5, d3 = P.dry_h == U3 && P.dry_v == U3;
+    const bool mw = P.moi_h == W5 && P.moi_v == W5, mu = P.moi_h == U5 && P.moi_v == U5, m3 = P.moi_h == W3 && P.moi_v == W3;
     if (!P.moist) {
-        if (dw) return k_post<R, W5, W5, -1, -1, 4>;
-        if (du) return k_post<R, U5, U5, -1, -1, 4>;
-        if (d3) return k_post<R, U3, U3, -1, -1, 4>;
-    } else if (nslow <= 4) {
-        if (dw && mw) return k_post<R, W5, W5, W5, W5, 4>;
-        if (du && mu) return k_post<R, U5, U5, U5, U5, 4>;
-        if (du && mw) return k_post<R, U5, U5, W5, W5, 4>;
-        if (d3 && m3) return k_post<R, U3, U3, W3, W3, 4>;
-    } else {
-        if (dw && mw) return k_post<R, W5, W5, W5, W5, 5>;
-        if (du && mu) return k_post<R, U5, U5, U5, U5, 5>;
-        if (du && mw) return k_post<R, U5, U5, W5, W5, 5>;
-        return k_post<R, -1, -1, -1, -1, 5>;
+        if (dw) return k_post<R, W5, W5, W5, W5>;
+        if (du) return k_post<R, U5, U5, W5, W5>;
+        if (d3) return k_post<R, U3, U3, W3, W3>;
+        return k_post<R, -1, -1, -1, -1>;
     }
-    return k_post<R, -1, -1, -1, -1, 4>;
+    if (mw) {
+        if (dw) return k_post<R, W5, W5, W5, W5>;
+        if (du) return k_post<R, U5, U5, W5, W5>;
+        if (d3) return k_post<R, U3, U3, W5, W5>;
+    }
+    if (m3) {
+        if (dw) return k_post<R, W5, W5, W3, W3>;
+        if (du) return k_post<R, U5, U5, W3, W3>;
+        if (d3) return k_post<R, U3, U3, W3, W3>;
+    }
+    if (du && mu) return k_post<R, U5, U5, U5, U5>;
+    return k_post<R, -1, -1, -1, -1>;
 }
 
 }  // namespace
@@ -1330,7 +1396,7 @@ template <class R>
 void tiled_setup(const Params& P, TiledKz* t) {
     t->cell = pick_kz(slow_cell_kernel<R>(P), P.g);
     t->mom = pick_kz(slow_mom_kernel<R>(P), P.g);
-    t->post = pick_kz(post_kernel<R>(P), P.g);
+    t->post = pick_kz(post_kernel<R>(P), P.g, post_jobs(P));
 }
 
 // The dynamic shared-memory opt-in is a property of the kernel for the whole
@@ -1436,11 +1502,11 @@ void launch_slow_mom(const Params& P, const TiledKz& t, cudaStream_t st, StateBu
 }
 template <class R>
 void launch_post(const Params& P, const TiledKz& t, cudaStream_t st, double slow_dt, StateBuf Sold, StateBuf Sst,
-                 StateBuf Ssum, StateBuf Snew, StageAux<R> Acur, StageAux<R> Anext, int make_next, const R* mut,
-                 TkeBuf<R> tke, const R* avx, const R* avy, const R* avz, double* un, double* vn, double* wn) {
-    post_kernel<R>(P)<<<tile_grid(P.g, t.post), dim3(TTX, TTY, 1), 0, st>>>(P, t.post, slow_dt, Sold, Sst, Ssum, Snew,
-                                                                             Acur, Anext, make_next, mut, tke, avx,
-                                                                             avy, avz, un, vn, wn);
+                 StateBuf Ssum, StateBuf Snew, StageAux<R> Acur, StageAux<R> Anext, int make_next, const double* keep,
+                 const R* mut, TkeBuf<R> tke, const R* avx, const R* avy, const R* avz, double* un, double* vn,
+                 double* wn) {
+    const PostArgs<R> a{slow_dt, Sold, Sst, Ssum, Snew, Acur, Anext, make_next, keep, mut, tke, avx, avy, avz, un, vn, wn};
+    post_kernel<R>(P)<<<tile_grid(P.g, t.post, post_jobs(P)), dim3(TTX, TTY, 1), 0, st>>>(P, t.post, a);
 }
 
 #define ERFB_INSTANTIATE(R)                                                                                          \
@@ -1463,8 +1529,8 @@ void launch_post(const Params& P, const TiledKz& t, cudaStream_t st, double slow
                                      const double*, const double*, const double*, const R*, const R*, const R*,      \
                                      const R*, const R*, const R*, const double*, R*, R*, R*);                       \
     template void launch_post<R>(const Params&, const TiledKz&, cudaStream_t, double, StateBuf, StateBuf, StateBuf,  \
-                                 StateBuf, StageAux<R>, StageAux<R>, int, const R*, TkeBuf<R>, const R*, const R*,   \
-                                 const R*, double*, double*, double*);
+                                 StateBuf, StageAux<R>, StageAux<R>, int, const double*, const R*, TkeBuf<R>,        \
+                                 const R*, const R*, const R*, double*, double*, double*);
 
 ERFB_INSTANTIATE(double)
 ERFB_INSTANTIATE(float)

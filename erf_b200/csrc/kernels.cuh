@@ -216,8 +216,9 @@ void launch_slow_mom(const Params& P, const TiledKz& t, cudaStream_t st, StateBu
                      const R* t13, const R* t23, const double* pavg, R* Fmx, R* Fmy, R* Fmz);
 template <class R>
 void launch_post(const Params& P, const TiledKz& t, cudaStream_t st, double slow_dt, StateBuf Sold, StateBuf Sst,
-                 StateBuf Ssum, StateBuf Snew, StageAux<R> Acur, StageAux<R> Anext, int make_next, const R* mut,
-                 TkeBuf<R> tke, const R* avx, const R* avy, const R* avz, double* un, double* vn, double* wn);
+                 StateBuf Ssum, StateBuf Snew, StageAux<R> Acur, StageAux<R> Anext, int make_next, const double* keep,
+                 const R* mut, TkeBuf<R> tke, const R* avx, const R* avy, const R* avz, double* un, double* vn,
+                 double* wn);   // keep: cons of the state whose rho KE (no Deardorff) / rho QKE go on (NULL: not yet)
 
 // Static terrain (terrain.cu): metrics, base state and the _T passes.
 void launch_ter_metrics(const Params& P, cudaStream_t st, double* detJ, double* zcc);

@@ -186,14 +186,15 @@ __device__ __forceinline__ R tile_div(const Geo& g, const FluxTile<R>& t, R zl, 
 // Host side of the tiles.
 // Levels per block: minimise waves x (levels + 1), the cost of a block being
 // its levels plus the extra bottom-face flux evaluation.
+// mult: blocks per tile and level chunk (the jobs that share a tile).
 template <typename K>
-inline int pick_kz(K kern, const Geo& g) {
+inline int pick_kz(K kern, const Geo& g, int mult = 1) {
     int dev = 0, nsm = 148, per = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, TTX * TTY, 0) != cudaSuccess || per < 1) per = 1;
     const long cap = (long)per * nsm;
-    const long nxy = (long)((g.nx + TTX - 1) / TTX) * ((g.ny + TTY - 1) / TTY);
+    const long nxy = (long)((g.nx + TTX - 1) / TTX) * ((g.ny + TTY - 1) / TTY) * mult;
     int best = g.nz;
     double best_cost = 1e30;
     for (int zb = 1; zb <= g.nz; ++zb) {
@@ -206,6 +207,8 @@ inline int pick_kz(K kern, const Geo& g) {
     return best;
 }
 
-inline dim3 tile_grid(const Geo& g, int kz) { return dim3((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + kz - 1) / kz); }
+inline dim3 tile_grid(const Geo& g, int kz, int mult = 1) {
+    return dim3((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + kz - 1) / kz * mult);
+}
 
 }  // namespace erfb
