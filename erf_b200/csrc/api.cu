@@ -790,6 +790,18 @@ int unpack(erf_b200_ctx* c, const erf_b200_fab* f, int kind, int ncomp, const do
     return cuda_fail(cudaGetLastError());
 }
 
+int pack_state(erf_b200_ctx* c, const erf_b200_fab* cons, const erf_b200_fab* u, const erf_b200_fab* v,
+               const erf_b200_fab* w, int slot) {
+    launch_pack_state(c->g, c->stream, StateFabs{{*cons, *u, *v, *w}}, c->cfg.ncomp, c->S[slot].cons, c->vel[slot]);
+    return cuda_fail(cudaGetLastError());
+}
+int unpack_state(erf_b200_ctx* c, const erf_b200_fab* cons, const erf_b200_fab* u, const erf_b200_fab* v,
+                 const erf_b200_fab* w, int slot) {
+    launch_unpack_state(c->g, c->stream, StateFabs{{*cons, *u, *v, *w}}, c->cfg.ncomp, c->S[slot].cons, c->vel[slot],
+                        c->P.ter);
+    return cuda_fail(cudaGetLastError());
+}
+
 }  // namespace
 
 // The configuration checks of erf_b200_create, shared with the entry points
@@ -1145,10 +1157,7 @@ int erf_b200_advance(erf_b200_ctx* c, const erf_b200_fab* cons, const erf_b200_f
     if (!fab_ok(cons, 0, g, c->cfg.ncomp) || !fab_ok(xvel, 1, g, 1) || !fab_ok(yvel, 2, g, 1) || !fab_ok(zvel, 3, g, 1))
         return ERF_B200_EINVAL;
     int rc;
-    if ((rc = pack(c, cons, 0, c->cfg.ncomp, c->S[0].cons))) return rc;
-    if ((rc = pack(c, xvel, 1, 1, c->vel[0][0]))) return rc;
-    if ((rc = pack(c, yvel, 2, 1, c->vel[0][1]))) return rc;
-    if ((rc = pack(c, zvel, 3, 1, c->vel[0][2]))) return rc;
+    if ((rc = pack_state(c, cons, xvel, yvel, zvel, 0))) return rc;
     if (!c->graph[0] || !c->graph[1]) return ERF_B200_EBADSTATE;   // learned closure not attached
     c->cur = -1;
     {
@@ -1160,10 +1169,7 @@ int erf_b200_advance(erf_b200_ctx* c, const erf_b200_fab* cons, const erf_b200_f
     }
     int p = nsteps & 1;
     c->last = p;
-    if ((rc = unpack(c, cons, 0, c->cfg.ncomp, c->S[p].cons))) return rc;
-    if ((rc = unpack(c, xvel, 1, 1, c->vel[p][0]))) return rc;
-    if ((rc = unpack(c, yvel, 2, 1, c->vel[p][1]))) return rc;
-    if ((rc = unpack(c, zvel, 3, 1, c->vel[p][2]))) return rc;
+    if ((rc = unpack_state(c, cons, xvel, yvel, zvel, p))) return rc;
     return cuda_fail(cudaGetLastError());
 }
 
@@ -1234,10 +1240,7 @@ int erf_b200_advance_profiled(erf_b200_ctx* c, const erf_b200_fab* cons, const e
         return ERF_B200_EINVAL;
     for (int q = 0; q < nslots; ++q) { kernel_ms[q] = 0.0; kernel_launches[q] = 0; }
     int rc;
-    if ((rc = pack(c, cons, 0, c->cfg.ncomp, c->S[0].cons))) return rc;
-    if ((rc = pack(c, xvel, 1, 1, c->vel[0][0]))) return rc;
-    if ((rc = pack(c, yvel, 2, 1, c->vel[0][1]))) return rc;
-    if ((rc = pack(c, zvel, 3, 1, c->vel[0][2]))) return rc;
+    if ((rc = pack_state(c, cons, xvel, yvel, zvel, 0))) return rc;
     LaunchTimer T;
     T.st = c->stream;
     for (int s = 0; s < nsteps; ++s) {
@@ -1254,10 +1257,7 @@ int erf_b200_advance_profiled(erf_b200_ctx* c, const erf_b200_fab* cons, const e
     }
     for (cudaEvent_t e : T.ev) cudaEventDestroy(e);
     int p = nsteps & 1;
-    if ((rc = unpack(c, cons, 0, c->cfg.ncomp, c->S[p].cons))) return rc;
-    if ((rc = unpack(c, xvel, 1, 1, c->vel[p][0]))) return rc;
-    if ((rc = unpack(c, yvel, 2, 1, c->vel[p][1]))) return rc;
-    if ((rc = unpack(c, zvel, 3, 1, c->vel[p][2]))) return rc;
+    if ((rc = unpack_state(c, cons, xvel, yvel, zvel, p))) return rc;
     return cuda_fail(cudaGetLastError());
 }
 
@@ -1352,10 +1352,7 @@ int erf_b200_turbulent_viscosity(erf_b200_ctx* c, const erf_b200_fab* xvel, cons
     if (!fab_ok(cons, 0, g, c->cfg.ncomp) || !fab_ok(xvel, 1, g, 1) || !fab_ok(yvel, 2, g, 1) || !fab_ok(zvel, 3, g, 1))
         return ERF_B200_EINVAL;
     int rc;
-    if ((rc = pack(c, cons, 0, c->cfg.ncomp, c->S[0].cons))) return rc;
-    if ((rc = pack(c, xvel, 1, 1, c->vel[0][0])) || (rc = pack(c, yvel, 2, 1, c->vel[0][1])) ||
-        (rc = pack(c, zvel, 3, 1, c->vel[0][2])))
-        return rc;
+    if ((rc = pack_state(c, cons, xvel, yvel, zvel, 0))) return rc;
     // the step prologue forms the eddy viscosity from these velocities (its
     // other outputs go to scratch slots of the context)
     if (c->P.ter) {   // ComputeStrain_T + the terrain filter width
@@ -1658,10 +1655,7 @@ int erf_b200_load_state(erf_b200_ctx* c, const erf_b200_fab* cons, const erf_b20
     if (!fab_ok(cons, 0, g, c->cfg.ncomp) || !fab_ok(xvel, 1, g, 1) || !fab_ok(yvel, 2, g, 1) || !fab_ok(zvel, 3, g, 1))
         return ERF_B200_EINVAL;
     int rc;
-    if ((rc = pack(c, cons, 0, c->cfg.ncomp, c->S[0].cons))) return rc;
-    if ((rc = pack(c, xvel, 1, 1, c->vel[0][0])) || (rc = pack(c, yvel, 2, 1, c->vel[0][1])) ||
-        (rc = pack(c, zvel, 3, 1, c->vel[0][2])))
-        return rc;
+    if ((rc = pack_state(c, cons, xvel, yvel, zvel, 0))) return rc;
     c->cur = 0;
     c->last = 0;
     return cuda_fail(cudaGetLastError());
@@ -1675,10 +1669,7 @@ int erf_b200_store_state(erf_b200_ctx* c, const erf_b200_fab* cons, const erf_b2
     if (!fab_ok(cons, 0, g, c->cfg.ncomp) || !fab_ok(xvel, 1, g, 1) || !fab_ok(yvel, 2, g, 1) || !fab_ok(zvel, 3, g, 1))
         return ERF_B200_EINVAL;
     int p = c->cur, rc;
-    if ((rc = unpack(c, cons, 0, c->cfg.ncomp, c->S[p].cons))) return rc;
-    if ((rc = unpack(c, xvel, 1, 1, c->vel[p][0])) || (rc = unpack(c, yvel, 2, 1, c->vel[p][1])) ||
-        (rc = unpack(c, zvel, 3, 1, c->vel[p][2])))
-        return rc;
+    if ((rc = unpack_state(c, cons, xvel, yvel, zvel, p))) return rc;
     return cuda_fail(cudaGetLastError());
 }
 

@@ -651,6 +651,74 @@ __global__ void k_unpack(Geo g, erf_b200_fab f, int kind, int ncomp, const doubl
 }
 
 
+// The same for a whole state -- the conserved variables and the three face
+// velocities -- in one launch each way: a thread moves all of a cell's values,
+// so that they are in flight together (eight launches a call otherwise, which
+// on a small grid cost as much as its kernels).
+__global__ void __launch_bounds__(256) k_pack_state(Geo g, StateFabs f, int ncomp, double* __restrict__ cons,
+                                                    double* __restrict__ u, double* __restrict__ v,
+                                                    double* __restrict__ w) {
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, k = blockIdx.z;
+    if (i >= g.nx || j >= g.ny) return;
+    auto src = [&](const erf_b200_fab& a) {
+        return a.p + ((i - a.lo[0]) + (j - a.lo[1]) * a.jstride + (k - a.lo[2]) * a.kstride);
+    };
+    const int64_t c = cidx(g, i, j, k);
+    w[c] = *src(f.a[3]);
+    if (k >= g.nz) return;
+    u[c] = *src(f.a[1]);
+    v[c] = *src(f.a[2]);
+    const double* p = src(f.a[0]);
+    for (int n = 0; n < ncomp; ++n) cons[n * g.ncell + c] = p[n * f.a[0].nstride];
+}
+// box: the smallest that holds the four views' boxes
+__global__ void __launch_bounds__(256) k_unpack_state(Geo g, StateFabs f, int lo0, int lo1, int lo2, int ncomp,
+                                                      const double* __restrict__ cons, const double* __restrict__ u,
+                                                      const double* __restrict__ v, const double* __restrict__ w,
+                                                      int wall_w) {
+    const int i = lo0 + (int)(blockIdx.x * 32 + threadIdx.x), j = lo1 + (int)(blockIdx.y * 8 + threadIdx.y);
+    const int k = lo2 + (int)blockIdx.z;
+    const int ii = (unsigned)i < (unsigned)g.nx ? i : ((i % g.nx) + g.nx) % g.nx;
+    const int jj = (unsigned)j < (unsigned)g.ny ? j : ((j % g.ny) + g.ny) % g.ny;
+    auto in = [&](const erf_b200_fab& a) {
+        return i >= a.lo[0] && i <= a.hi[0] && j >= a.lo[1] && j <= a.hi[1] && k >= a.lo[2] && k <= a.hi[2];
+    };
+    auto dst = [&](const erf_b200_fab& a) {
+        return a.p + ((i - a.lo[0]) + (j - a.lo[1]) * a.jstride + (k - a.lo[2]) * a.kstride);
+    };
+    const int64_t c = cidx(g, ii, jj, clampk(k, g.nz));
+    // tangential velocity beyond a no-slip wall: 0
+    const bool zero = (k < 0 && g.zlo_noslip) || (k >= g.nz && g.zhi_noslip);
+    if (in(f.a[1])) *dst(f.a[1]) = zero ? 0.0 : u[c];
+    if (in(f.a[2])) *dst(f.a[2]) = zero ? 0.0 : v[c];
+    if (in(f.a[3]))
+        // beyond the walls 0; on the walls 0 without terrain, the stored value
+        // (w from Omega = 0) with terrain
+        *dst(f.a[3]) = (k < 0 || k > g.nz || (!wall_w && (k == 0 || k == g.nz))) ? 0.0 : w[cidx(g, ii, jj, k)];
+    if (in(f.a[0])) {
+        double* p = dst(f.a[0]);
+        for (int n = 0; n < ncomp; ++n) p[n * f.a[0].nstride] = cons[n * g.ncell + c];
+    }
+}
+void launch_pack_state(const Geo& g, cudaStream_t st, const StateFabs& f, int ncomp, double* cons, double* const* vel) {
+    k_pack_state<<<dim3((g.nx + 31) / 32, (g.ny + 7) / 8, g.nz + 1), dim3(32, 8), 0, st>>>(g, f, ncomp, cons, vel[0],
+                                                                                            vel[1], vel[2]);
+}
+void launch_unpack_state(const Geo& g, cudaStream_t st, const StateFabs& f, int ncomp, const double* cons,
+                         double* const* vel, int wall_w) {
+    int lo[3], hi[3];
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = f.a[0].lo[d];
+        hi[d] = f.a[0].hi[d];
+        for (int q = 1; q < 4; ++q) {
+            lo[d] = f.a[q].lo[d] < lo[d] ? f.a[q].lo[d] : lo[d];
+            hi[d] = f.a[q].hi[d] > hi[d] ? f.a[q].hi[d] : hi[d];
+        }
+    }
+    k_unpack_state<<<dim3((hi[0] - lo[0] + 32) / 32, (hi[1] - lo[1] + 8) / 8, hi[2] - lo[2] + 1), dim3(32, 8), 0, st>>>(
+        g, f, lo[0], lo[1], lo[2], ncomp, cons, vel[0], vel[1], vel[2], wall_w);
+}
+
 // ---------------------------------------------------------------------------
 // Tile layout shared by the two vertical kernels below: a block owns TX
 // adjacent columns (i = blockIdx.x*TX + threadIdx.x, j = blockIdx.y) and

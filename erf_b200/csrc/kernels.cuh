@@ -144,6 +144,13 @@ constexpr int PAVG_PARTS = 16;
 inline size_t plane_avg_doubles(int nz) { return (size_t)6 * nz + (size_t)5 * nz * PAVG_PARTS + nz; }
 template <class R>
 void launch_plane_avg(const Params& P, cudaStream_t st, const double* cons, const R* prim, double* avg);
+// A caller's state {cons, u, v, w} into the internal arrays and back
+struct StateFabs {
+    erf_b200_fab a[4];
+};
+void launch_pack_state(const Geo& g, cudaStream_t st, const StateFabs& f, int ncomp, double* cons, double* const* vel);
+void launch_unpack_state(const Geo& g, cudaStream_t st, const StateFabs& f, int ncomp, const double* cons,
+                         double* const* vel, int wall_w);
 // MOST plane means and friction velocity of a step from its old velocities
 void launch_most_avg(const Params& P, cudaStream_t st, const double* u, const double* v);
 template <class R>
