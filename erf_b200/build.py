@@ -24,11 +24,11 @@ LIB = os.path.join(HERE, "liberf_b200.so")
 OBJ_BOUNDS = os.path.join(HERE, "_build_bounds")
 LIB_BOUNDS = os.path.join(HERE, "liberf_b200_bounds.so")
 # the two terrain halves take longest, so they start first
-SOURCES = ["terrain.cu", "terrain_f32.cu", "kernels.cu", "substep.cu", "kessler.cu", "moving.cu", "api.cu", "noalloc.cu", "mlp.cu", "closure.cu", "plotfile.cu",
+SOURCES = ["terrain.cu", "terrain_f32.cu", "kernels.cu", "substep.cu", "kessler.cu", "moving.cu", "ter_fast.cu", "api.cu", "noalloc.cu", "mlp.cu", "closure.cu", "plotfile.cu",
            "checkpoint.cu"]
 # sources a translation unit includes besides the headers
 INCLUDED = {"terrain_f32.cu": ["terrain.cu"]}
-HEADERS = ["common.cuh", "kernels.cuh", "tiles.cuh", "moving.cuh", "tcgen05.cuh", "mlp.cuh", "amrex_io.h"]
+HEADERS = ["common.cuh", "kernels.cuh", "tiles.cuh", "moving.cuh", "terrain.cuh", "tcgen05.cuh", "mlp.cuh", "amrex_io.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",

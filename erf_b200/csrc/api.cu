@@ -106,7 +106,6 @@ struct erf_b200_ctx {
     } mt{};
     int mt_tx = 0;                                            // moving terrain: columns per block of the substep kernels
     int ter_tx = 0;                                           // k_ter_fast_vert columns per block
-    size_t ter_smem = 0;                                      // and its shared memory
     bool ter_set = false;
     int last = -1;               // state slot of the latest state (erf_b200_diagnostics)
     double* diag = nullptr;      // its scratch (partials, result)
@@ -431,7 +430,6 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
     StateBuf outs[3] = {N0, N1, N0};
     if (P.kessler_rain) outs[2].rain = N1.cons + 7 * g.ncell;
     StateBuf stage[3] = {OLD, outs[0], outs[1]};
-    dim3 tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1), tcb(c->tile_tx, c->coef_warps, 1);
     const bool fork = T == nullptr && c->side;
     int a = 0;
     const double beta_s = 0.1;
@@ -447,7 +445,7 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
         if (fork && !nosub) {
             cudaEventRecord(c->ev_fork, st);
             cudaStreamWaitEvent(c->side, c->ev_fork, 0);
-            launch_fast_coef<R>(P, c->side, tg, tcb, c->coef_smem, D, Sst, Acur, B.cA, B.cInvB, B.cCB, B.cP, B.cQ);
+            launch_ter_coef<R>(P, c->side, c->ter_tx, D, Sst, Acur, B.mc[0]);
             cudaEventRecord(c->ev_coef, c->side);
         }
         if (P.use_diff)
@@ -460,7 +458,7 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
         if (nosub)
             TIMED(10, launch_no_substep<R>(P, st, slow_dt, OLD, B.Fcons, B.Fmx, B.Fmy, B.Fmz, SUM));
         else if (!fork)
-            TIMED(9, launch_fast_coef<R>(P, st, tg, tcb, c->coef_smem, D, Sst, Acur, B.cA, B.cInvB, B.cCB, B.cP, B.cQ));
+            TIMED(9, launch_ter_coef<R>(P, st, c->ter_tx, D, Sst, Acur, B.mc[0]));
         else
             cudaStreamWaitEvent(st, c->ev_coef, 0);
         for (int ks = 0; ks < (nosub ? 0 : nsub); ++ks) {
@@ -472,9 +470,8 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
             }
             TIMED(5, launch_ter_fast_h<R>(P, st, ks, ks > 0, dtau, facinv, Sprev, Sst, Acur, B.Fmx, B.Fmy, nullptr,
                                           nullptr, B.ter, B.avx, B.avy, SUM.mx, SUM.my));
-            TIMED(6, launch_ter_fast_vert<R>(P, st, c->ter_tx, c->ter_smem, dtau, facinv, beta_1, beta_2, Sprev, prt,
-                                             Sst, Acur, B.Fcons, B.Fmz, B.ter, B.cA, B.cInvB, B.cCB, B.cP, B.cQ,
-                                             B.avz, SUM.cons, SUM.mz));
+            TIMED(6, launch_ter_fast_vert<R>(P, st, c->ter_tx, dtau, facinv, beta_1, beta_2, Sprev, prt, Sst, Acur,
+                                             B.Fcons, B.Fmz, B.ter, B.mc[0], B.avz, SUM.cons, SUM.mz));
         }
         TIMED(7, launch_ter_post<R>(P, st, c->tkz.ter_post, slow_dt, OLD, Sst, SUM, Snew, Acur, Anext, nrk < 2 ? 1 : 0, B.mut, B.tke,
                                     B.ter, B.avx, B.avy, B.avz, Vnew[0], Vnew[1], Vnew[2]));
@@ -713,7 +710,7 @@ int alloc_bulk(erf_b200_ctx* c, Bulk<R>& B) {
     for (int p = 0; p < 2; ++p) { A(&B.aux[p].prim, (nc - 1) * N); A(&B.aux[p].pi, N); A(&B.aux[p].pp, N); }
     A(&B.mut, N);
     A(&B.t11, N); A(&B.t22, N); A(&B.t33, N); A(&B.t12, N); A(&B.t13, NZF); A(&B.t23, NZF);
-    if (cfg->use_terrain || !c->mixed) {   // (flat: the per-pass make_fast_coeffs only, plain form)
+    if (!c->mixed) {   // the per-pass make_fast_coeffs
         A(&B.cA, NZF); A(&B.cInvB, NZF); A(&B.cCB, NZF); A(&B.cP, NZF); A(&B.cQ, NZF);
     }
     if (!cfg->use_terrain && (!c->mixed || cfg->substepping_type == ERF_SUBSTEP_IMPLICIT)) {
@@ -737,8 +734,10 @@ int alloc_bulk(erf_b200_ctx* c, Bulk<R>& B) {
         auto D = [&](double** q, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, q, n); };
         D(&B.ter.bnd, 2 * (int64_t)cfg->nx * cfg->ny);
         D(&B.ter.ec, N);
-        if (cfg->terrain_type == ERF_TERRAIN_MOVING && cfg->substepping_type == ERF_SUBSTEP_IMPLICIT)
-            for (MtCoef<R>& m : B.mc) { A(&m.E, NZF); A(&m.G, NZF); A(&m.I, NZF); A(&m.P, NZF); A(&m.Q, NZF); }
+        for (MtCoef<R>& m : B.mc) {   // static terrain: one stage's; moving: two substeps'
+            if (&m != B.mc && (cfg->terrain_type != ERF_TERRAIN_MOVING || cfg->substepping_type != ERF_SUBSTEP_IMPLICIT)) break;
+            A(&m.E, NZF); A(&m.G, NZF); A(&m.I, NZF); A(&m.P, NZF); A(&m.Q, NZF);
+        }
     }
     return rc;
 }
@@ -950,8 +949,9 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
             if ((c->mixed ? sub_setup<float>(c->g, c->sub) : sub_setup<double>(c->g, c->sub)) != 0) rc = ERF_B200_ECUDA;
         }
         if (rc == ERF_B200_OK && cfg->use_terrain) {
-            ter_vert_shape(nz, &c->ter_tx, &c->ter_smem);
+            const int bad = c->mixed ? ter_vert_shape<float>(nz, &c->ter_tx) : ter_vert_shape<double>(nz, &c->ter_tx);
             if (c->ter_tx < 1) rc = ERF_B200_ECONFIG;
+            else if (bad) rc = ERF_B200_ECUDA;
             else if (cfg->terrain_type == ERF_TERRAIN_MOVING &&
                      (c->mixed ? mt_shape<float>(c->g, &c->mt_tx) : mt_shape<double>(c->g, &c->mt_tx)) != 0)
                 rc = ERF_B200_ECUDA;
@@ -1484,8 +1484,7 @@ int fast_rhs_pass(erf_b200_ctx* c, bool terrain, int step, int nrk, const erf_b2
         launch_stage_aux<double>(P, st, Sst.cons, B.aux[0]);
         double D = dtau * dtau * kBeta2 * kBeta2 * g.dzi;
         if (terrain) {
-            dim3 tg((g.nx + c->tile_tx - 1) / c->tile_tx, g.ny, 1), tcb(c->tile_tx, c->coef_warps, 1);
-            launch_fast_coef<double>(P, st, tg, tcb, c->coef_smem, D, Sst, B.aux[0], B.cA, B.cInvB, B.cCB, B.cP, B.cQ);
+            launch_ter_coef<double>(P, st, c->ter_tx, D, Sst, B.aux[0], B.mc[0]);
         } else {
             launch_sub_coef<double>(P, st, c->sub, D, Sst, B.aux[0], B.sc);
         }
@@ -1493,9 +1492,8 @@ int fast_rhs_pass(erf_b200_ctx* c, bool terrain, int step, int nrk, const erf_b2
     if (terrain) {
         launch_ter_fast_h<double>(P, st, step, false, dtau, facinv, Sprev, Sst, B.aux[0], B.Fmx, B.Fmy, B.lag[0],
                                   B.lag[1], B.ter, B.avx, B.avy, OUT.mx, OUT.my);
-        launch_ter_fast_vert<double>(P, st, c->ter_tx, c->ter_smem, dtau, facinv, kBeta1, kBeta2, Sprev, 0, Sst,
-                                     B.aux[0], B.Fcons, B.Fmz, B.ter, B.cA, B.cInvB, B.cCB, B.cP, B.cQ, B.avz,
-                                     OUT.cons, OUT.mz);
+        launch_ter_fast_vert<double>(P, st, c->ter_tx, dtau, facinv, kBeta1, kBeta2, Sprev, 0, Sst, B.aux[0], B.Fcons,
+                                     B.Fmz, B.ter, B.mc[0], B.avz, OUT.cons, OUT.mz);
     } else {
         // from the caller's previous state to a whole new state, with the caller's lagged d(rho theta)
         SubArgs<double> sa = sub_args<double>(g, B, Sprev, Sst, OUT, B.aux[0], dtau, facinv, 0);
@@ -1735,15 +1733,6 @@ int erf_b200_autotune(erf_b200_ctx* c, int reps, double* best_ms) {
             for (int threads : {256, 512, 1024})
                 if (tx >= 4 && tx <= 32) try_shape({tx, threads / tx, 256 / tx});
         for (int threads : {128, 512}) try_shape({c->sub.tx, c->sub.rows, threads / c->sub.tx});
-    }
-    // the coefficient kernel of the terrain path
-    for (int cw : {4, 8, 16}) {
-        if (rc || !c->P.ter || cw == c->coef_warps || cw * c->tile_tx > 1024) continue;
-        int keep = c->coef_warps;
-        c->coef_warps = cw;
-        float ms;
-        if (trial(ms) == ERF_B200_OK && ms < best) best = ms;
-        else { cudaGetLastError(); c->coef_warps = keep; }
     }
     int* kz[3] = {&c->tkz.cell, &c->tkz.mom, &c->tkz.post};
     for (int q = 0; q < 3 && !rc; ++q) {

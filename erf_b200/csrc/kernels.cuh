@@ -288,12 +288,16 @@ template <class R>
 void launch_ter_fast_h(const Params& P, cudaStream_t st, int step, bool ec_ready, double dtau, double facinv,
                        StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in,
                        R* lag_out, TerBuf<R> T, R* avx, R* avy, double* outx, double* outy);
+// (ter_fast.cu) a stage's coefficients and the column part of a substep;
+// tx: columns per block (ter_vert_shape)
 template <class R>
-void launch_ter_fast_vert(const Params& P, cudaStream_t st, int tx, size_t smem, double dtau, double facinv,
-                          double beta_1, double beta_2, StateBuf Sprev, int prev_rt, StateBuf Sst, StageAux<R> A,
-                          const R* Fcons, const R* Fmz, TerBuf<R> T, const R* cA, const R* cInvB, const R* cCB,
-                          const R* cP, const R* cQ, R* avz, double* out_cons, double* out_mz);
-void ter_vert_shape(int nz, int* tx, size_t* smem);
+void launch_ter_coef(const Params& P, cudaStream_t st, int tx, double D, StateBuf Sst, StageAux<R> A, MtCoef<R> c);
+template <class R>
+void launch_ter_fast_vert(const Params& P, cudaStream_t st, int tx, double dtau, double facinv, double beta_1,
+                          double beta_2, StateBuf Sprev, int prev_rt, StateBuf Sst, StageAux<R> A, const R* Fcons,
+                          const R* Fmz, TerBuf<R> T, MtCoef<R> c, R* avz, double* out_cons, double* out_mz);
+template <class R>
+int ter_vert_shape(int nz, int* tx);
 template <class R>
 void launch_ter_post(const Params& P, cudaStream_t st, int kz, double slow_dt, StateBuf Sold, StateBuf Sst,
                      StateBuf Ssum, StateBuf Snew, StageAux<R> Acur, StageAux<R> Anext, int make_next, const R* mut,

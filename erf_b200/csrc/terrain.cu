@@ -20,15 +20,12 @@
 //   k_ter_slow_cell   rho / rho*theta slow RHS with face areas and detJ
 //   k_ter_slow_mom    AdvectionSrcForMom_T, DiffusionSrcForMom_T, terrain
 //                     pressure gradient, sources
-//   k_ter_fast_h,     erf_fast_rhs_T (TimeIntegration/ERF_fast_rhs_T.cpp)
-//   k_ter_fv_bnd,
-//   k_ter_fast_vert
+//   (ter_fast.cu)     erf_fast_rhs_T (TimeIntegration/ERF_fast_rhs_T.cpp)
 //   k_ter_post        erf_slow_rhs_post with terrain and the stage's
 //                     boundary round trips
 #include <cfloat>
 
-#include "kernels.cuh"
-#include "moving.cuh"
+#include "terrain.cuh"
 #include "tiles.cuh"
 
 // The library compiles this file twice so that the two halves build side by
@@ -52,204 +49,6 @@ namespace {
 #define TER_MINB_SLOW_MOM 8
 #define TER_MINB_STRESS 8
 constexpr int TU5 = ERF_ADV_UPWIND_5TH, TW5 = ERF_ADV_WENO_5;   // compile-time scheme codes
-
-// ---------------------------------------------------------------------------
-// Metric terms (Utils/ERF_TerrainMetrics.H:33-395), same operand order.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double Zn(const Params& P, int i, int j, int k) {
-    const Geo& g = P.g;
-    return __ldg(P.znd + (int64_t)(k + 1) * g.sk + (int64_t)wrap(j, g.ny) * g.nx + wrap(i, g.nx));
-}
-#define ZN(a, b, c) Zn(P, a, b, c)
-__device__ __forceinline__ double detJ_at(const Params& P, int i, int j, int k) {
-    const Geo& g = P.g;
-    return ld(P.detJ, eidx(g, wrap(i, g.nx), wrap(j, g.ny), clampk(k, g.nz)));
-}
-__device__ __forceinline__ double hzeta_cc_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dzi * (ZN(i + 1, j, k + 1) + ZN(i + 1, j + 1, k + 1) + ZN(i, j, k + 1) + ZN(i, j + 1, k + 1)
-                             - ZN(i + 1, j, k) - ZN(i + 1, j + 1, k) - ZN(i, j, k) - ZN(i, j + 1, k));
-}
-__device__ __forceinline__ double hxi_cc_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dxi * (ZN(i + 1, j, k) + ZN(i + 1, j + 1, k) + ZN(i + 1, j, k + 1) + ZN(i + 1, j + 1, k + 1)
-                             - ZN(i, j, k) - ZN(i, j + 1, k) - ZN(i, j, k + 1) - ZN(i, j + 1, k + 1));
-}
-__device__ __forceinline__ double heta_cc_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dyi * (ZN(i, j + 1, k) + ZN(i + 1, j + 1, k) + ZN(i, j + 1, k + 1) + ZN(i + 1, j + 1, k + 1)
-                             - ZN(i, j, k) - ZN(i + 1, j, k) - ZN(i, j, k + 1) - ZN(i + 1, j, k + 1));
-}
-// x faces (also ax) and y faces (also ay)
-__device__ __forceinline__ double hzeta_I_fn(const Params& P, int i, int j, int k) {
-    return 0.5 * P.g.dzi * (ZN(i, j, k + 1) + ZN(i, j + 1, k + 1) - ZN(i, j, k) - ZN(i, j + 1, k));
-}
-__device__ __forceinline__ double hxi_I_fn(const Params& P, int i, int j, int k) {
-    return 0.125 * P.g.dxi * (ZN(i + 1, j, k) + ZN(i + 1, j, k + 1) + ZN(i + 1, j + 1, k) + ZN(i + 1, j + 1, k + 1)
-                              - ZN(i - 1, j, k) - ZN(i - 1, j, k + 1) - ZN(i - 1, j + 1, k) - ZN(i - 1, j + 1, k + 1));
-}
-__device__ __forceinline__ double hzeta_J_fn(const Params& P, int i, int j, int k) {
-    return 0.5 * P.g.dzi * (ZN(i, j, k + 1) + ZN(i + 1, j, k + 1) - ZN(i, j, k) - ZN(i + 1, j, k));
-}
-__device__ __forceinline__ double heta_J_fn(const Params& P, int i, int j, int k) {
-    return 0.125 * P.g.dyi * (ZN(i, j + 1, k) + ZN(i, j + 1, k + 1) + ZN(i + 1, j + 1, k) + ZN(i + 1, j + 1, k + 1)
-                              - ZN(i, j - 1, k) - ZN(i, j - 1, k + 1) - ZN(i + 1, j - 1, k) - ZN(i + 1, j - 1, k + 1));
-}
-// z faces
-__device__ __forceinline__ double hzeta_K_fn(const Params& P, int i, int j, int k) {
-    return 0.125 * P.g.dzi * (ZN(i, j, k + 1) + ZN(i + 1, j, k + 1) + ZN(i, j + 1, k + 1) + ZN(i + 1, j + 1, k + 1)
-                              - ZN(i, j, k - 1) - ZN(i + 1, j, k - 1) - ZN(i, j + 1, k - 1) - ZN(i + 1, j + 1, k - 1));
-}
-__device__ __forceinline__ double hxi_K_fn(const Params& P, int i, int j, int k) {
-    return 0.5 * P.g.dxi * (ZN(i + 1, j, k) + ZN(i + 1, j + 1, k) - ZN(i, j, k) - ZN(i, j + 1, k));
-}
-__device__ __forceinline__ double heta_K_fn(const Params& P, int i, int j, int k) {
-    return 0.5 * P.g.dyi * (ZN(i, j + 1, k) + ZN(i + 1, j + 1, k) - ZN(i, j, k) - ZN(i + 1, j, k));
-}
-// xy edges (EdgeCenterK), xz edges (EdgeCenterJ), yz edges (EdgeCenterI)
-__device__ __forceinline__ double hzeta_EK_fn(const Params& P, int i, int j, int k) { return P.g.dzi * (ZN(i, j, k + 1) - ZN(i, j, k)); }
-__device__ __forceinline__ double hxi_EK_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dxi * (ZN(i + 1, j, k) + ZN(i + 1, j, k + 1) - ZN(i - 1, j, k) - ZN(i - 1, j, k + 1));
-}
-__device__ __forceinline__ double heta_EK_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dyi * (ZN(i, j + 1, k) + ZN(i, j + 1, k + 1) - ZN(i, j - 1, k) - ZN(i, j - 1, k + 1));
-}
-__device__ __forceinline__ double hzeta_EJ_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dzi * (ZN(i, j, k + 1) + ZN(i, j + 1, k + 1) - ZN(i, j, k - 1) - ZN(i, j + 1, k - 1));
-}
-__device__ __forceinline__ double hxi_EJ_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dxi * (ZN(i + 1, j + 1, k) + ZN(i + 1, j, k) - ZN(i - 1, j + 1, k) - ZN(i - 1, j, k));
-}
-__device__ __forceinline__ double heta_EJ_fn(const Params& P, int i, int j, int k) { return P.g.dyi * (ZN(i, j + 1, k) - ZN(i, j, k)); }
-__device__ __forceinline__ double hzeta_EI_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dzi * (ZN(i, j, k + 1) + ZN(i + 1, j, k + 1) - ZN(i, j, k - 1) - ZN(i + 1, j, k - 1));
-}
-__device__ __forceinline__ double hxi_EI_fn(const Params& P, int i, int j, int k) { return P.g.dxi * (ZN(i + 1, j, k) - ZN(i, j, k)); }
-__device__ __forceinline__ double heta_EI_fn(const Params& P, int i, int j, int k) {
-    return 0.25 * P.g.dyi * (ZN(i + 1, j + 1, k) + ZN(i, j + 1, k) - ZN(i + 1, j - 1, k) - ZN(i, j - 1, k));
-}
-// slopes of a z-face (OmegaFromW / WFromOmega, ERF_TerrainMetrics.H:455-520)
-__device__ __forceinline__ double zlo_xi_fn(const Params& P, int i, int j, int k) {
-    return 0.5 * P.g.dxi * (ZN(i + 1, j + 1, k) + ZN(i + 1, j, k) - ZN(i, j + 1, k) - ZN(i, j, k));
-}
-__device__ __forceinline__ double zlo_eta_fn(const Params& P, int i, int j, int k) {
-    return 0.5 * P.g.dyi * (ZN(i + 1, j + 1, k) + ZN(i, j + 1, k) - ZN(i + 1, j, k) - ZN(i, j, k));
-}
-#undef ZN
-
-// Static-terrain metric tables: the metric terms the passes read,
-// evaluated once per cell / face / edge by the functions above (so bit-identical to
-// evaluating them in place) and stored as TER_NMET planes of (nz+1) x ny x
-// nx values, k in [0, nz].  A pass reads one value instead of re-deriving it
-// from four to eight nodes of z_phys_nd; outside [0, nz] the function runs.
-enum { MT_HZETA_I, MT_HXI_I, MT_HZETA_J, MT_HETA_J, MT_HXI_K, MT_HETA_K, MT_HZETA_EK, MT_HZETA_EJ, MT_HZETA_EI,
-       MT_ZLO_XI, MT_ZLO_ETA, MT_HZETA_CC, MT_HXI_CC, MT_HETA_CC, MT_HZETA_K, MT_HXI_EK, MT_HETA_EK, MT_HXI_EJ,
-       MT_HETA_EJ, MT_HXI_EI, MT_HETA_EI, MT_RXI_I, MT_RETA_J, MT_IJ, MT_COUNT };
-static_assert(MT_COUNT == TER_NMET, "metric table count");
-__device__ __forceinline__ double mt_at(const Params& P, int q, int i, int j, int k) {
-    const Geo& g = P.g;
-    return ld(P.met + (int64_t)q * g.nzf, eidx(g, wrap(i, g.nx), wrap(j, g.ny), k));
-}
-#define ERFB_MT(name, q)                                                           \
-    __device__ __forceinline__ double name(const Params& P, int i, int j, int k) { \
-        if (k >= 0 && k <= P.g.nz) return mt_at(P, q, i, j, k);                   \
-        return name##_fn(P, i, j, k);                                              \
-    }
-ERFB_MT(hzeta_I, MT_HZETA_I)
-ERFB_MT(hxi_I, MT_HXI_I)
-ERFB_MT(hzeta_J, MT_HZETA_J)
-ERFB_MT(heta_J, MT_HETA_J)
-ERFB_MT(hxi_K, MT_HXI_K)
-ERFB_MT(heta_K, MT_HETA_K)
-ERFB_MT(hzeta_EK, MT_HZETA_EK)
-ERFB_MT(hzeta_EJ, MT_HZETA_EJ)
-ERFB_MT(hzeta_EI, MT_HZETA_EI)
-ERFB_MT(zlo_xi, MT_ZLO_XI)
-ERFB_MT(zlo_eta, MT_ZLO_ETA)
-ERFB_MT(hzeta_cc, MT_HZETA_CC)
-ERFB_MT(hxi_cc, MT_HXI_CC)
-ERFB_MT(heta_cc, MT_HETA_CC)
-ERFB_MT(hzeta_K, MT_HZETA_K)
-ERFB_MT(hxi_EK, MT_HXI_EK)
-ERFB_MT(heta_EK, MT_HETA_EK)
-ERFB_MT(hxi_EJ, MT_HXI_EJ)
-ERFB_MT(heta_EJ, MT_HETA_EJ)
-ERFB_MT(hxi_EI, MT_HXI_EI)
-ERFB_MT(heta_EI, MT_HETA_EI)
-#undef ERFB_MT
-// Quotients of them, k in [0, nz): the slopes h_xi / h_zeta and h_eta / h_zeta
-// of the x and y faces and 1 / detJ of the cells (an FP64 division is some
-// twenty instructions, and every pass of every substep needs these).
-__device__ __forceinline__ double slope_I(const Params& P, int i, int j, int k) { return mt_at(P, MT_RXI_I, i, j, k); }
-__device__ __forceinline__ double slope_J(const Params& P, int i, int j, int k) { return mt_at(P, MT_RETA_J, i, j, k); }
-__device__ __forceinline__ double inv_detJ(const Params& P, int i, int j, int k) { return mt_at(P, MT_IJ, i, j, clampk(k, P.g.nz)); }
-
-template <class FU, class FV>
-__device__ __forceinline__ double omega_from_w(const Params& P, int i, int j, int k, double w, FU ua, FV va) {
-    double mx = zlo_xi(P, i, j, k), my = zlo_eta(P, i, j, k), u, v;
-    zface_uv(i, j, k, ua, va, u, v);
-    return w - mx * u - my * v;
-}
-template <class FU, class FV>
-__device__ __forceinline__ double w_from_omega(const Params& P, int i, int j, int k, double om, FU ua, FV va) {
-    double mx = zlo_xi(P, i, j, k), my = zlo_eta(P, i, j, k), u, v;
-    zface_uv(i, j, k, ua, va, u, v);
-    return om + mx * u + my * v;
-}
-
-// qv + qc averaged over two cells (the moist pressure-gradient factor
-// 1 + q of ERF_slow_rhs_pre.cpp:594-744 and ERF_fast_rhs_T.cpp:230-300);
-// 0 for a dry state.
-template <class R>
-__device__ __forceinline__ double moist_q(const Params& P, const R* prim, int64_t a, int64_t b) {
-    if (!P.moist) return 0.0;
-    const int64_t N = P.g.ncell;
-    return 0.5 * (double(prim[4 * N + a]) + double(prim[4 * N + b]) + double(prim[5 * N + a]) + double(prim[5 * N + b]));
-}
-
-// Base state at (i,j,k), k in [-1, nz].
-__device__ __forceinline__ double bs(const double* f, const Geo& g, int i, int j, int k) {
-    return __ldg(f + (int64_t)(k + 1) * g.sk + (int64_t)j * g.nx + i);
-}
-
-// Horizontal momentum after the M -> V -> M round trip of a boundary fill
-// (face (i,j,k) wrapped laterally, k in [0, nz)) and the velocity it gives.
-__device__ __forceinline__ double rt_u(const Geo& g, const double* cons, const double* mx, int i, int j, int k) {
-    i = wrap(i, g.nx); j = wrap(j, g.ny);
-    double rs = cons[cidx(g, i, j, k)] + cons[cidx(g, wrap(i - 1, g.nx), j, k)];
-    return (mx[cidx(g, i, j, k)] * 2.0) / rs;
-}
-__device__ __forceinline__ double rt_v(const Geo& g, const double* cons, const double* my, int i, int j, int k) {
-    i = wrap(i, g.nx); j = wrap(j, g.ny);
-    double rs = cons[cidx(g, i, j, k)] + cons[cidx(g, i, wrap(j - 1, g.ny), k)];
-    return (my[cidx(g, i, j, k)] * 2.0) / rs;
-}
-
-// Tangential velocity with its wall ghost (ext_dir 0 or foextrap), lateral
-// indices wrapped here.
-__device__ __forceinline__ double tvel(const double* f, const Geo& g, int i, int j, int k) {
-    i = wrap(i, g.nx); j = wrap(j, g.ny);
-    if (k < 0) return g.zlo_noslip ? 0.0 : ld(f, eidx(g, i, j, 0));
-    if (k >= g.nz) return g.zhi_noslip ? 0.0 : ld(f, eidx(g, i, j, g.nz - 1));
-    return ld(f, eidx(g, i, j, k));
-}
-// w at z-face k in [0, nz], lateral wrap
-__device__ __forceinline__ double wvel(const double* f, const Geo& g, int i, int j, int k) {
-    i = wrap(i, g.nx); j = wrap(j, g.ny);
-    k = k < 0 ? 0 : (k > g.nz ? g.nz : k);
-    return ld(f, eidx(g, i, j, k));
-}
-// cell-centred value with lateral wrap and foextrap in z
-template <class V>
-__device__ __forceinline__ double ccw(const V* f, const Geo& g, int i, int j, int k) {
-    return double(ld(f, eidx(g, wrap(i, g.nx), wrap(j, g.ny), clampk(k, g.nz))));
-}
-
-__device__ __forceinline__ bool cell_ij(const Geo& g, int& i, int& j, int& k) {
-    i = blockIdx.x * blockDim.x + threadIdx.x;
-    j = blockIdx.y * blockDim.y + threadIdx.y;
-    k = blockIdx.z;
-    return i < g.nx && j < g.ny && k < g.nz;
-}
-dim3 ter_block() { return dim3(32, 4, 1); }
-dim3 ter_grid(const Geo& g, int nk) { return dim3((g.nx + 31) / 32, (g.ny + 3) / 4, nk); }
 
 }  // namespace
 
@@ -1453,259 +1252,6 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
 }
 
 // ---------------------------------------------------------------------------
-// Acoustic substep with terrain, horizontal part (ERF_fast_rhs_T.cpp:130-320):
-// lagged d(rho theta) and its extrapolation, U'' / V'' with the
-// terrain-corrected gradient of the extrapolated d(rho theta); the old and
-// new increments are kept for the vertical part.
-// ---------------------------------------------------------------------------
-// After the first substep (of the fused step) the extrapolated d(rho theta)
-// comes from the vertical part, which has both substeps' values in hand, and
-// the old increments are the previous substep's new ones: nine loads in place
-// of twenty-seven.  The M -> V -> M round trip of the fill between substeps
-// is the identity but for rounding and is not applied.
-template <class R, bool FIRST>
-__global__ void k_ter_fast_h(Params P, int step, double dtau, double facinv, StateBuf Sprev, StateBuf Sst, StageAux<R> A,
-                             const R* __restrict__ Fmx, const R* __restrict__ Fmy, const R* __restrict__ lag_in,
-                             R* __restrict__ lag_out, TerBuf<R> T, R* __restrict__ avx, R* __restrict__ avy,
-                             double* __restrict__ outx, double* __restrict__ outy) {
-    const Geo& g = P.g;
-    int i, j, k;
-    if (!cell_ij(g, i, j, k)) return;
-    const int nz = g.nz, im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
-    const uint32_t c = eidx(g, i, j, k), cxm = eidx(g, im, j, k), cym = eidx(g, i, jm, k);
-    const double beta_d = 0.1, dxi = g.dxi, dyi = g.dyi;
-    const double* prt = Sprev.cons + g.ncell;
-    const double* srt = Sst.cons + g.ncell;
-    auto extrap = [&](int ii, int jj, int kk) {
-        const uint32_t e = eidx(g, ii, jj, clampk(kk, nz));
-        if (!FIRST) return ld(T.ec, e);
-        const double drt = ld(prt, e) - ld(srt, e);
-        return step == 0 ? drt : drt + beta_d * (drt - double(ld(lag_in, e)));
-    };
-    if (FIRST && lag_out) at(lag_out, c) = R(ld(prt, c) - ld(srt, c));
-    double odu, odv;
-    if (FIRST) {
-        odu = ld(Sprev.mx, c) - ld(Sst.mx, c);
-        odv = ld(Sprev.my, c) - ld(Sst.my, c);
-        at(T.odu, c) = R(odu);
-        at(T.odv, c) = R(odv);
-    } else {
-        odu = double(ld(T.odu, c));
-        odv = double(ld(T.odv, c));
-    }
-    const int km = k == 0 ? 0 : k - 1;   // one-sided in the lowest cell
-    const double fz = (k == 0 ? 0.5 : 0.25) * g.dzi;
-    const double ec = extrap(i, j, k), exm = extrap(im, j, k), eym = extrap(i, jm, k);
-    const double ecz = extrap(i, j, k + 1) - extrap(i, j, km);
-    double gpx = (ec - exm) * dxi - slope_I(P, i, j, k) * (fz * (ecz + extrap(im, j, k + 1) - extrap(im, j, km)));
-    double gpy = (ec - eym) * dyi - slope_J(P, i, j, k) * (fz * (ecz + extrap(i, jm, k + 1) - extrap(i, jm, km)));
-    if (P.moist) {
-        gpx /= 1.0 + moist_q(P, A.prim, c, cxm);
-        gpy /= 1.0 + moist_q(P, A.prim, c, cym);
-    }
-    const double pc = double(ld(A.pi, c));
-    const double fx = -Gamma_ * R_d * (0.5 * (double(ld(A.pi, cxm)) + pc)) * gpx;
-    const double fy = -Gamma_ * R_d * (0.5 * (double(ld(A.pi, cym)) + pc)) * gpy;
-    const double ndu = odu + dtau * fx + dtau * double(ld(Fmx, c));
-    const double ndv = odv + dtau * fy + dtau * double(ld(Fmy, c));
-    at(T.ndu, c) = R(ndu);
-    at(T.ndv, c) = R(ndv);
-    at(avx, c) += R(facinv * ndu);
-    at(avy, c) += R(facinv * ndv);
-    at(outx, c) = ld(Sst.mx, c) + ndu;
-    at(outy, c) = ld(Sst.my, c) + ndv;
-}
-
-// ---------------------------------------------------------------------------
-// Acoustic substep with terrain, vertical part (ERF_fast_rhs_T.cpp:320-680):
-// horizontal rho / rho*theta fluxes through the sloping faces, Omega of the
-// previous increments, the detJ-weighted right-hand side of the Omega''
-// system, the Thomas sweep on the stage's coefficients, then w'' from
-// Omega'', the vertical fluxes, the average contravariant momentum, rho and
-// rho*theta (k_ter_fast_vert below).
-// ---------------------------------------------------------------------------
-namespace {
-template <class R>
-__device__ __forceinline__ double prev_mz_ter(const Params& P, StateBuf Sprev, int prev_rt, int i, int j, int k) {
-    const Geo& g = P.g;
-    const int nz = g.nz;
-    int64_t f = cidx(g, i, j, k);
-    double m = Sprev.mz[f];
-    if (prev_rt && (k == 0 || k == nz)) {
-        auto U1 = [&](int ii, int jj, int kk) {
-            if (kk >= nz) {
-                if (g.zhi_noslip) return 0.0;
-                kk = nz - 1;
-            }
-            return rt_u(g, Sprev.cons, Sprev.mx, ii, jj, kk);
-        };
-        auto V1 = [&](int ii, int jj, int kk) {
-            if (kk >= nz) {
-                if (g.zhi_noslip) return 0.0;
-                kk = nz - 1;
-            }
-            return rt_v(g, Sprev.cons, Sprev.my, ii, jj, kk);
-        };
-        int kc = (k == 0) ? 0 : nz - 1;
-        double r = Sprev.cons[cidx(g, i, j, kc)];
-        double wb = w_from_omega(P, i, j, k, 0.0, U1, V1);
-        return (wb * 0.5) * (r + r);
-    }
-    return m;
-}
-}  // namespace
-
-// The same vertical part as one pass per column tile (the layout of
-// k_fast_vert: TX columns of a row j, the block's warps spread over the
-// levels, the column arrays in shared memory), so that the horizontal
-// fluxes, Omega of the old increments, the right-hand side and the solution
-// never leave the SM; one warp runs the Thomas sweep.  The momentum of the
-// previous substep on the ground and lid faces (w from Omega = 0 of its
-// round-tripped u, v) reads neighbouring columns of a state the update
-// overwrites in place, so k_ter_fv_bnd forms it first.
-template <class R>
-__global__ void k_ter_fv_bnd(Params P, StateBuf Sprev, TerBuf<R> T) {
-    const Geo& g = P.g;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    const int64_t col = (int64_t)j * g.nx + i;
-    T.bnd[col] = prev_mz_ter<R>(P, Sprev, 1, i, j, 0);
-    T.bnd[g.sk + col] = prev_mz_ter<R>(P, Sprev, 1, i, j, g.nz);
-}
-
-template <class R>
-__global__ void __launch_bounds__(1024) k_ter_fast_vert(Params P, double dtau, double facinv, double beta_1,
-                                                        double beta_2, StateBuf Sprev, int prev_rt, StateBuf Sst,
-                                                        StageAux<R> A, const R* __restrict__ Fcons,
-                                                        const R* __restrict__ Fmz, TerBuf<R> T,
-                                                        const R* __restrict__ cA, const R* __restrict__ cInvB,
-                                                        const R* __restrict__ cCB, const R* __restrict__ cP,
-                                                        const R* __restrict__ cQ, R* __restrict__ avz,
-                                                        double* out_cons, double* out_mz) {
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    double* sm = reinterpret_cast<double*>(sm_raw);
-    const Geo& g = P.g;
-    const int nz = g.nz, TX = blockDim.x, L = threadIdx.x, w0 = threadIdx.y, nw = blockDim.y;
-    const int i = blockIdx.x * TX + L, j = blockIdx.y;
-    const bool ok = i < g.nx;
-    double* sT0 = sm;                   // horizontal rho flux divergence (cells)
-    double* sT1 = sT0 + nz * TX;        // horizontal rho*theta flux divergence (cells)
-    double* sO = sT1 + nz * TX;         // Omega of the old increments (faces)
-    double* sR = sO + (nz + 1) * TX;    // right-hand side, then the solution (faces)
-    double* sA = sR + (nz + 1) * TX;
-    double* sI = sA + (nz + 1) * TX;
-    double* sCB = sI + (nz + 1) * TX;
-    const int64_t N = g.ncell, sk = g.sk;
-    const double dxi = g.dxi, dyi = g.dyi, dzi = g.dzi, halfg = P.halfg;
-    auto th = [&](int ii, int jj, int kk) { return ccw(A.prim, g, ii, jj, kk); };
-    auto NDU = [&](int ii, int jj, int kk) { return double(ld(T.ndu, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
-    auto NDV = [&](int ii, int jj, int kk) { return double(ld(T.ndv, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
-    auto ODU = [&](int ii, int jj, int kk) { return double(ld(T.odu, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
-    auto ODV = [&](int ii, int jj, int kk) { return double(ld(T.odv, eidx(g, wrap(ii, g.nx), wrap(jj, g.ny), kk))); };
-    auto prev_mz = [&](int k) {
-        if (prev_rt && (k == 0 || k == nz)) return T.bnd[(k == 0 ? 0 : sk) + (int64_t)j * g.nx + i];
-        return prev_mz_ter<R>(P, Sprev, prev_rt, i, j, k);
-    };
-    // ---- phase 1: horizontal fluxes (cells), Omega'' of the old increments and the coefficients (faces)
-    if (ok) {
-        for (int k = w0; k <= nz; k += nw) {
-            const int64_t f = cidx(g, i, j, k);
-            if (k < nz) {
-                double hxh = hzeta_I(P, i + 1, j, k), hxl = hzeta_I(P, i, j, k);
-                double hyh = hzeta_J(P, i, j + 1, k), hyl = hzeta_J(P, i, j, k);
-                double xl = NDU(i, j, k) * hxl / 1.0, xh = NDU(i + 1, j, k) * hxh / 1.0;
-                double yl = NDV(i, j, k) * hyl / 1.0, yh = NDV(i, j + 1, k) * hyh / 1.0;
-                double mfsq = 1.0;
-                double tc = th(i, j, k);
-                sT0[k * TX + L] = (xh - xl) * dxi * mfsq + (yh - yl) * dyi * mfsq;
-                sT1[k * TX + L] = ((xh * (tc + th(i + 1, j, k)) - xl * (tc + th(i - 1, j, k))) * dxi * mfsq +
-                                   (yh * (tc + th(i, j + 1, k)) - yl * (tc + th(i, j - 1, k))) * dyi * mfsq) * 0.5;
-            }
-            double odw = prev_mz(k) - Sst.mz[f];
-            double om;
-            if (k == 0) om = 0.;
-            else if (k == nz) om = odw;
-            else om = omega_from_w(P, i, j, k, odw, ODU, ODV);
-            sO[k * TX + L] = om;
-            sA[k * TX + L] = double(cA[f]);
-            sI[k * TX + L] = double(cInvB[f]);
-            sCB[k * TX + L] = double(cCB[f]);
-        }
-    }
-    __syncthreads();
-    // ---- phase 2: the detJ-weighted right-hand side of the Omega'' system (faces)
-    if (ok) {
-        for (int k = w0; k <= nz; k += nw) {
-            const int64_t f = cidx(g, i, j, k);
-            if (k == 0 || k == nz) {
-                sR[k * TX + L] = dtau * double(Fmz[f]);
-                continue;
-            }
-            int64_t cm = f - sk;
-            double Jk = detJ_at(P, i, j, k), Jkm = detJ_at(P, i, j, k - 1);
-            double dJk = 0.5 * (Jk + Jkm);
-            double cPk = double(cP[f]), cQk = double(cQ[f]);
-            double tlo = 0.5 * (th(i, j, k - 2) + th(i, j, k - 1));
-            double tmid = 0.5 * (th(i, j, k - 1) + th(i, j, k));
-            double thi = 0.5 * (th(i, j, k) + th(i, j, k + 1));
-            double odr_k = Sprev.cons[f] - Sst.cons[f], odr_km = Sprev.cons[cm] - Sst.cons[cm];
-            double odrt_k = Sprev.cons[N + f] - Sst.cons[N + f], odrt_km = Sprev.cons[N + cm] - Sst.cons[N + cm];
-            double R0t = (-halfg * odr_k + cPk * odrt_k) * Jk + (-halfg * odr_km + cQk * odrt_km) * Jkm;
-            double R1t = -halfg * (double(Fcons[f]) * Jk + double(Fcons[cm]) * Jkm)
-                         + (cPk * double(Fcons[N + f]) * Jk + cQk * double(Fcons[N + cm]) * Jkm);
-            double Okp1 = sO[(k + 1) * TX + L], Ok = sO[k * TX + L], Okm1 = sO[(k - 1) * TX + L];
-            R1t += (halfg) * (beta_1 * dzi * (Okp1 - Okm1) + sT0[k * TX + L] + sT0[(k - 1) * TX + L]);
-            R1t += -(cPk * (beta_1 * dzi * (Okp1 * thi - Ok * tmid) + sT1[k * TX + L]) +
-                     cQk * (beta_1 * dzi * (Ok * tmid - Okm1 * tlo) + sT1[(k - 1) * TX + L]));
-            double odw = prev_mz(k) - Sst.mz[f];
-            double rhs = dJk * odw + dtau * (dJk * double(Fmz[f]) + R0t + dtau * beta_2 * R1t);
-            rhs += dJk * omega_from_w(P, i, j, k, 0., NDU, NDV);
-            sR[k * TX + L] = rhs;
-        }
-    }
-    __syncthreads();
-    // ---- phase 3: forward elimination / back substitution, one warp
-    if (w0 == 0 && ok) {
-        double s = sR[L] * sI[L];
-        sR[L] = s;
-        for (int k = 1; k <= nz; ++k) {
-            s = (sR[k * TX + L] - sA[k * TX + L] * s) * sI[k * TX + L];
-            sR[k * TX + L] = s;
-        }
-        for (int k = nz - 1; k >= 0; --k) {
-            s = sR[k * TX + L] - sCB[k * TX + L] * s;
-            sR[k * TX + L] = s;
-        }
-    }
-    __syncthreads();
-    // ---- phase 4: w'' from Omega'', vertical fluxes, average Omega, rho and rho*theta
-    if (ok) {
-        for (int k = w0; k <= nz; k += nw) {
-            const int64_t f = cidx(g, i, j, k);
-            double m = Sst.mz[f];
-            if (k >= 1 && k <= nz - 1) m += w_from_omega(P, i, j, k, sR[k * TX + L], NDU, NDV);
-            out_mz[f] = m;
-            if (k == nz) continue;
-            const int64_t c = f;
-            double zl = beta_2 * sR[k * TX + L] + beta_1 * sO[k * TX + L];
-            double zh = beta_2 * sR[(k + 1) * TX + L] + beta_1 * sO[(k + 1) * TX + L];
-            avz[c] += R(facinv * zl / (1.0 * 1.0));
-            if (k == nz - 1) avz[c + sk] += R(facinv * zh / (1.0 * 1.0));
-            const double iJ = inv_detJ(P, i, j, k);
-            double tc = th(i, j, k);
-            double frho = -(sT0[k * TX + L] + (zh - zl) * dzi) * iJ;
-            double frt = -(sT1[k * TX + L] + 0.5 * (zh * (tc + th(i, j, k + 1)) - zl * (tc + th(i, j, k - 1))) * dzi) * iJ;
-            double pr = Sprev.cons[c], prt = Sprev.cons[N + c];
-            out_cons[c] = pr + dtau * (double(Fcons[c]) + frho);
-            const double nrt = prt + dtau * (double(Fcons[N + c]) + frt);
-            out_cons[N + c] = nrt;
-            // the next substep's extrapolation: d + 0.1 (d - previous d) about the stage
-            T.ec[c] = (nrt - Sst.cons[N + c]) + 0.1 * (nrt - prt);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Slow RHS of the slow variables with terrain and the stage update
 // (ERF_slow_rhs_post.cpp:169-530): passive scalar and (Deardorff) rho*KE
 // advected with the average momenta (over detJ), DiffusionSrcForState_T with
@@ -1919,48 +1465,6 @@ void launch_ter_slow_mom(const Params& P, cudaStream_t st, StateBuf S, StageAux<
     (u5 ? k_ter_slow_mom<R, TU5, TU5> : k_ter_slow_mom<R, -1, -1>)<<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(
         P, S, A, u, v, w, t11, t22, t33, t12, t13, t23, T, Om, Fmx, Fmy, Fmz);
 }
-// ec_ready: the previous substep left the extrapolated d(rho theta) and its
-// increments (T.odu, T.odv); else both come from Sprev and lag_in.
-template <class R>
-void launch_ter_fast_h(const Params& P, cudaStream_t st, int step, bool ec_ready, double dtau, double facinv,
-                       StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fmx, const R* Fmy, const R* lag_in,
-                       R* lag_out, TerBuf<R> T, R* avx, R* avy, double* outx, double* outy) {
-    (ec_ready ? k_ter_fast_h<R, false> : k_ter_fast_h<R, true>)<<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(
-        P, step, dtau, facinv, Sprev, Sst, A, Fmx, Fmy, lag_in, lag_out, T, avx, avy, outx, outy);
-}
-template <class R>
-void launch_ter_fast_vert(const Params& P, cudaStream_t st, int tx, size_t smem, double dtau, double facinv,
-                          double beta_1, double beta_2, StateBuf Sprev, int prev_rt, StateBuf Sst, StageAux<R> A,
-                          const R* Fcons, const R* Fmz, TerBuf<R> T, const R* cA, const R* cInvB, const R* cCB,
-                          const R* cP, const R* cQ, R* avz, double* out_cons, double* out_mz) {
-    if (prev_rt)
-        k_ter_fv_bnd<R><<<dim3((P.g.nx + 31) / 32, (P.g.ny + 3) / 4, 1), ter_block(), 0, st>>>(P, Sprev, T);
-    dim3 grid((P.g.nx + tx - 1) / tx, P.g.ny, 1), block(tx, 1024 / tx, 1);
-    k_ter_fast_vert<R><<<grid, block, smem, st>>>(P, dtau, facinv, beta_1, beta_2, Sprev, prev_rt, Sst, A, Fcons, Fmz,
-                                                  T, cA, cInvB, cCB, cP, cQ, avz, out_cons, out_mz);
-}
-// Columns per block of k_ter_fast_vert (the widest power of two up to 32 whose
-// FP64 column arrays fit) and its shared memory; 0 columns if none fits.
-template <class R>
-void ter_vert_attr(size_t smem) {
-    cudaFuncSetAttribute(k_ter_fast_vert<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-#if !ERFB_TER_F32
-extern template void ter_vert_attr<float>(size_t);
-void ter_vert_shape(int nz, int* tx, size_t* smem) {
-    int dev = 0, maxopt = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&maxopt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    int t = 32;
-    while (t >= 1 && (size_t)(7 * nz + 5) * t * sizeof(double) > (size_t)maxopt) t /= 2;
-    *tx = t;
-    *smem = t >= 1 ? (size_t)(7 * nz + 5) * t * sizeof(double) : 0;
-    if (t >= 1) {
-        ter_vert_attr<double>(*smem);
-        ter_vert_attr<float>(*smem);
-    }
-}
-#endif
 namespace {
 // The tiled post pass per scheme: dry scalars (and KE) and moisture
 // species compile-time Upwind5 / WENO5 where the configuration has them,
@@ -2012,17 +1516,10 @@ int ter_post_kz(const Params& P) {
     template void launch_ter_slow_mom<R>(const Params&, cudaStream_t, StateBuf, StageAux<R>, const double*,          \
                                          const double*, const double*, const R*, const R*, const R*, const R*,       \
                                          const R*, const R*, TerBuf<R>, const R*, R*, R*, R*);                       \
-    template void launch_ter_fast_h<R>(const Params&, cudaStream_t, int, bool, double, double, StateBuf, StateBuf,    \
-                                       StageAux<R>, const R*, const R*, const R*, R*, TerBuf<R>, R*, R*, double*,      \
-                                       double*);                                                                     \
-    template void launch_ter_fast_vert<R>(const Params&, cudaStream_t, int, size_t, double, double, double, double, \
-                                          StateBuf, int, StateBuf, StageAux<R>, const R*, const R*, TerBuf<R>,       \
-                                          const R*, const R*, const R*, const R*, const R*, R*, double*, double*);   \
     template void launch_ter_post<R>(const Params&, cudaStream_t, int, double, StateBuf, StateBuf, StateBuf,         \
                                      StateBuf, StageAux<R>, StageAux<R>, int, const R*, TkeBuf<R>, TerBuf<R>,        \
                                      const R*, const R*, const R*, double*, double*, double*);                       \
-    template int ter_post_kz<R>(const Params&);                                                                      \
-    template void ter_vert_attr<R>(size_t);
+    template int ter_post_kz<R>(const Params&);
 
 #if !ERFB_TER_F32
 ERFB_TER_INSTANTIATE(double)

@@ -56,6 +56,30 @@ def test_step(size, flow, dyc, dry, moist):
         assert not bad, (precision, errs)
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(4, 4, 4), (13, 9, 33), (9, 5, 150)])
+def test_terrain_substeps(nx, ny, nz):
+    from erf_b200 import Dycore
+    case = T.abl_terrain(nx=nx, ny=ny, nz=nz, dx=25.0, dz0=320.0 / nz, stretch=1.01, h0=30.0, r0=100.0,
+                         amp=5.0)
+    case.cfg.dt *= min(1.0, 16.0 / nz)
+    for precision in (C.PREC_FP64, C.PREC_MIXED):
+        cfg = case.cfg.copy()
+        cfg.precision = precision
+        dy = Dycore(cfg)
+        dy.set_terrain(case.z_nd)
+        base = dy.make_base_state_terrain(case)
+        dy.set_base_state(base)
+        state = case.build_state(base[0])
+        got = dy.advance_host(*state, 2)
+        assert dy.status() == 0
+        dy.close()
+        errs = compare_states(got, oracle.advance_terrain(case.cfg, case.z_nd, base, *state, 2))
+        if precision == C.PREC_FP64:
+            assert all(e <= TOL for e in errs.values()), errs
+        else:   # the bars of test_terrain_mixed_form_error
+            assert errs["rho"] < 1e-6 and errs["u"] < 1e-3 and errs["w"] < 1e-2, errs
+
+
 @pytest.mark.parametrize("nx,ny,nz", [(12, 4, 7), (24, 7, 33)])
 def test_moving_terrain_substeps(nx, ny, nz):
     case = T.moving_terrain(nx=nx, ny=ny, nz=nz, Lx=5.0 * nx, Ly=5.0 * ny, H=5.0 * nz, ampl=0.05, wavelength=2.5 * nx,
