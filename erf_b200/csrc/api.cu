@@ -451,7 +451,7 @@ void enqueue_step_ter(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
         if (P.use_diff)
             TIMED(1, launch_ter_tau<R>(P, st, nrk, Sst.cons, Vnew[0], Vnew[1], Vnew[2], B.mut, B.ter, B.tke, B.t11,
                                        B.t22, B.t33, B.t12, B.t13, B.t23));
-        TIMED(2, launch_ter_slow_cell<R>(P, st, Sst, Acur, Vnew[0], Vnew[1], B.mut, B.tke, B.ter, B.Fcons, B.avx,
+        TIMED(2, launch_ter_slow_cell<R>(P, st, c->tkz.ter_cell, Sst, Acur, Vnew[0], Vnew[1], B.mut, B.tke, B.ter, B.Fcons, B.avx,
                                          B.avy, B.avz));
         TIMED(4, launch_ter_slow_mom<R>(P, st, Sst, Acur, Vnew[0], Vnew[1], Vnew[2], B.t11, B.t22, B.t33, B.t12, B.t13,
                                         B.t23, B.ter, B.avz, B.Fmx, B.Fmy, B.Fmz));
@@ -526,7 +526,7 @@ void enqueue_step_mt(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
         launch_mt_grid(Po, st, c->mt.time, dt, ts_new, c->mt.z[2]);
         launch_ter_metrics(Ps, st, c->mt.detJ1, c->mt.zcc1);
         launch_mt_zt(Po, st, c->mt.z[0], c->mt.z[2], c->mt.time, dt, ts_new, c->mt.zt);
-        TIMED(2, launch_ter_slow_cell<R>(Ps, st, Sst, Acur, Vnew[0], Vnew[1], B.mut, B.tke, B.ter, B.Fcons, B.avx,
+        TIMED(2, launch_ter_slow_cell<R>(Ps, st, c->tkz.ter_cell, Sst, Acur, Vnew[0], Vnew[1], B.mut, B.tke, B.ter, B.Fcons, B.avx,
                                          B.avy, B.avz));
         TIMED(4, launch_ter_slow_mom<R>(Ps, st, Sst, Acur, Vnew[0], Vnew[1], Vnew[2], B.t11, B.t22, B.t33, B.t12,
                                         B.t13, B.t23, B.ter, B.avz, B.Fmx, B.Fmy, B.Fmz));
@@ -930,6 +930,7 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     }
     if (c->mixed) tiled_setup<float>(c->P, &c->tkz);
     else tiled_setup<double>(c->P, &c->tkz);
+    c->tkz.ter_cell = !cfg->use_terrain ? 0 : (c->mixed ? ter_cell_kz<float>(c->P) : ter_cell_kz<double>(c->P));
     c->tkz.ter_post = !cfg->use_terrain ? 0 : (c->mixed ? ter_post_kz<float>(c->P) : ter_post_kz<double>(c->P));
     // shared-memory tiles of the column kernels: TX columns x all levels
     {
@@ -1407,7 +1408,7 @@ int erf_b200_slow_rhs_pre(erf_b200_ctx* c, int nrk, double slow_dt, const erf_b2
         if (P.use_diff)
             launch_ter_tau<double>(P, st, nrk, Sst.cons, V[0], V[1], V[2], B.mut, B.ter, B.tke, B.t11, B.t22, B.t33,
                                    B.t12, B.t13, B.t23);
-        launch_ter_slow_cell<double>(P, st, Sst, B.aux[0], V[0], V[1], B.mut, B.tke, B.ter, B.Fcons, B.avx, B.avy,
+        launch_ter_slow_cell<double>(P, st, c->tkz.ter_cell, Sst, B.aux[0], V[0], V[1], B.mut, B.tke, B.ter, B.Fcons, B.avx, B.avy,
                                      B.avz);
         launch_ter_slow_mom<double>(P, st, Sst, B.aux[0], V[0], V[1], V[2], B.t11, B.t22, B.t33, B.t12, B.t13, B.t23,
                                     B.ter, B.avz, B.Fmx, B.Fmy, B.Fmz);

@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_CELL) k_slow_cell(Params 
 // velocities) and to the vapour's (theta, Exner function and p' of the next
 // stage; the scalar's in dry air).  With all variables in one block the
 // vertical stencils were loads, L2 hits mostly, on every level (four of six
-// levels each on the moist bubble, 262 us per stage at 128x128x80); one at a
+// levels each on the moist bubble, 262 us per stage at 128x128x80, 200 now); one at a
 // time, the column is a window in registers, fed a level ahead along with the
 // momenta.  The jobs of a tile are neighbours in the grid, so that what they
 // share is read from DRAM once.

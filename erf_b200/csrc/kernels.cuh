@@ -102,7 +102,7 @@ struct TerBuf {
 constexpr int TTX = 32, TTY = 8;
 struct TiledKz {
     int cell, mom, post;
-    int ter_post;   // the terrain post pass (terrain contexts)
+    int ter_cell, ter_post;   // the tiled terrain passes (terrain contexts)
 };
 
 // erf_b200_create's configuration checks (api.cu): ERF_B200_OK or an error code.
@@ -277,7 +277,9 @@ void launch_ter_tau(const Params& P, cudaStream_t st, int nrk, const double* con
                     const double* w, const R* mut, TerBuf<R> T, TkeBuf<R> tke, R* t11, R* t22, R* t33, R* t12, R* t13,
                     R* t23);
 template <class R>
-void launch_ter_slow_cell(const Params& P, cudaStream_t st, StateBuf S, StageAux<R> A, const double* u,
+int ter_cell_kz(const Params& P);
+template <class R>
+void launch_ter_slow_cell(const Params& P, cudaStream_t st, int kz, StateBuf S, StageAux<R> A, const double* u,
                           const double* v, const R* mut, TkeBuf<R> tke, TerBuf<R> T, R* Fcons, R* avx, R* avy,
                           R* avz);
 template <class R>

