@@ -832,11 +832,11 @@ struct DiffT {
         return -rA * 1.0 * (GradCy - slope_J(P, i, j, k) * GradCz);
     }
     __device__ __forceinline__ double xr(int i, int j, int k) const {
-        if (fxr) return double(fxr[cidx(P.g, wrap(i, P.g.nx), wrap(j, P.g.ny), k)]);
+        if (fxr) return double(ld(fxr, eidx(P.g, wrap(i, P.g.nx), wrap(j, P.g.ny), k)));
         return xraw(i, j, k);
     }
     __device__ __forceinline__ double yr(int i, int j, int k) const {
-        if (fyr) return double(fyr[cidx(P.g, wrap(i, P.g.nx), wrap(j, P.g.ny), k)]);
+        if (fyr) return double(ld(fyr, eidx(P.g, wrap(i, P.g.nx), wrap(j, P.g.ny), k)));
         return yraw(i, j, k);
     }
     // z-face flux (k in [0, nz]); raw receives the flux before the cross terms
@@ -964,7 +964,7 @@ __global__ void k_ter_rawflux(Params P, const double* __restrict__ rho, const R*
 // eight momenta and velocities each) from both sides.  x and y faces go
 // through shared memory, z faces are carried up the column, theta's x / y
 // stencils read the staged plane.  All in FP64 (the tiles too), as before.
-// 256x256x96, FP64: 908 us with one thread per cell, 577 now.
+// 256x256x96, FP64: 908 us with one thread per cell, 580 now.
 // ---------------------------------------------------------------------------
 template <class R, int HT, int VT>
 __global__ void __launch_bounds__(TTX * TTY, TER_MINB_SLOW_CELL) k_ter_slow_cell(
@@ -1365,9 +1365,9 @@ __global__ void __launch_bounds__(128, TER_MINB_SLOW_MOM) k_ter_slow_mom(Params 
 // (ERF_slow_rhs_post.cpp:169-530): passive scalar and (Deardorff) rho*KE
 // advected with the average momenta (over detJ), DiffusionSrcForState_T with
 // the TKE sources, S_new = S_old + dt RHS (KE clipped at DBL_EPSILON); rho,
-// rho*theta and the momenta from the fast solution through the two boundary
-// round trips, w on the ground and the lid from Omega = 0 of the new u, v;
-// the next stage's primitives.
+// rho*theta and the momenta from the fast solution, w on the ground and the lid from Omega = 0 of the new u, v;
+// the next stage's primitives.  Bound by instruction issue; 256x256x96, FP64:
+// 1128 us with the round trips' divisions, 1045 without.
 // ---------------------------------------------------------------------------
 template <class R, int DH, int DV, int MH, int MV, int NS, bool MT = false>
 __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P, int kz, double slow_dt, StateBuf Sold,
@@ -1384,6 +1384,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
     const Geo& g = P.g;
     const int nz = g.nz;
     const int64_t N = g.ncell;
+    const uint32_t sk = (uint32_t)g.sk;
     const int i = blockIdx.x * TTX + threadIdx.x, j = blockIdx.y * TTY + threadIdx.y;
     const bool ok = i < g.nx && j < g.ny;
     const int k0 = blockIdx.z * kz, k1 = min(k0 + kz, g.nz);
@@ -1435,8 +1436,8 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
                 if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k + 1);
         }
         if (!ok) continue;   // the next level's first barrier orders the reuse of sh
-        const int64_t c = cidx(g, i, j, k);
-        const double invdetJ = 1. / detJ_at(P, i, j, k);
+        const uint32_t c = eidx(g, i, j, k);
+        const double invdetJ = MT ? 1. / detJ_at(P, i, j, k) : inv_detJ(P, i, j, k);   // (moving: the tables are another grid's)
 #pragma unroll
         for (int q = 0; q < NS; ++q) {
             if (q >= nslow) break;
@@ -1458,12 +1459,12 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
                 double fzh = D.zflux(i, j, k + 1, raw);
                 dz_lo[q] = fzh;
                 double sd = (fxh - fxl) * g.dxi * 1.0 + (fyh - fyl) * g.dyi * 1.0 + (fzh - fzl) * g.dzi;
-                r -= sd / detJ_at(P, i, j, k);
+                r -= sd * invdetJ;
             }
             if (ke) {
-                r += P.g_over_theta0 * double(tke.hfz[c]);
-                r += 2.0 * double(mut[c]) * double(tke.smn[c]);
-                r -= double(tke.diss[c]);
+                r += P.g_over_theta0 * double(ld(tke.hfz, c));
+                r += 2.0 * double(ld(mut, c)) * double(ld(tke.smn, c));
+                r -= double(ld(tke.diss, c));
             }
             if (MT) {
                 // moving terrain (ERF_slow_rhs_post.cpp:467-478): detJ-weighted
@@ -1479,60 +1480,48 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
             if (n == 7 && Snew.rain) Snew.rain[c] = nv;
             else Snew.cons[n * N + c] = nv;
         }
-        Snew.cons[c] = Ssum.cons[c];
-        Snew.cons[N + c] = Ssum.cons[N + c];
-        if (!dd) Snew.cons[2 * N + c] = Sst.cons[2 * N + c];
-        Snew.cons[3 * N + c] = Sst.cons[3 * N + c];
-        double rho = Ssum.cons[c];
-        // horizontal momenta through the two round trips; velocity u2
-        auto u2f = [&](int ii, int jj, int kk) {
+        const double rho = ld(Ssum.cons, c);
+        at(Snew.cons, c) = rho;
+        at(Snew.cons + N, c) = ld(Ssum.cons + N, c);
+        if (!dd) at(Snew.cons + 2 * N, c) = ld(Sst.cons + 2 * N, c);
+        at(Snew.cons + 3 * N, c) = ld(Sst.cons + 3 * N, c);
+        // velocities of the new momenta (the M -> V -> M round trips of the
+        // fills are the identity but for rounding and are not applied)
+        auto uf = [&](int ii, int jj, int kk) {
             if (kk < 0 || kk >= nz) {
                 if ((kk < 0 && g.zlo_noslip) || (kk >= nz && g.zhi_noslip)) return 0.0;
                 kk = kk < 0 ? 0 : nz - 1;
             }
             ii = wrap(ii, g.nx); jj = wrap(jj, g.ny);
-            int64_t e = cidx(g, ii, jj, kk);
-            double rs = Ssum.cons[e] + Ssum.cons[cidx(g, wrap(ii - 1, g.nx), jj, kk)];
-            double m = Ssum.mx[e];
-            double u1 = (m * 2.0) / rs; m = (u1 * 0.5) * rs;
-            return (m * 2.0) / rs;
+            const uint32_t e = eidx(g, ii, jj, kk);
+            return 2.0 * ld(Ssum.mx, e) / (ld(Ssum.cons, e) + ld(Ssum.cons, eidx(g, wrap(ii - 1, g.nx), jj, kk)));
         };
-        auto v2f = [&](int ii, int jj, int kk) {
+        auto vf = [&](int ii, int jj, int kk) {
             if (kk < 0 || kk >= nz) {
                 if ((kk < 0 && g.zlo_noslip) || (kk >= nz && g.zhi_noslip)) return 0.0;
                 kk = kk < 0 ? 0 : nz - 1;
             }
             ii = wrap(ii, g.nx); jj = wrap(jj, g.ny);
-            int64_t e = cidx(g, ii, jj, kk);
-            double rs = Ssum.cons[e] + Ssum.cons[cidx(g, ii, wrap(jj - 1, g.ny), kk)];
-            double m = Ssum.my[e];
-            double v1 = (m * 2.0) / rs; m = (v1 * 0.5) * rs;
-            return (m * 2.0) / rs;
+            const uint32_t e = eidx(g, ii, jj, kk);
+            return 2.0 * ld(Ssum.my, e) / (ld(Ssum.cons, e) + ld(Ssum.cons, eidx(g, ii, wrap(jj - 1, g.ny), kk)));
         };
-        {
-            double rs = rho + Ssum.cons[cidx(g, wrap(i - 1, g.nx), j, k)];
-            double u2 = u2f(i, j, k);
-            Snew.mx[c] = (u2 * 0.5) * rs; un[c] = u2;
-        }
-        {
-            double rs = rho + Ssum.cons[cidx(g, i, wrap(j - 1, g.ny), k)];
-            double v2 = v2f(i, j, k);
-            Snew.my[c] = (v2 * 0.5) * rs; vn[c] = v2;
-        }
+        at(Snew.mx, c) = ld(Ssum.mx, c);
+        at(un, c) = uf(i, j, k);
+        at(Snew.my, c) = ld(Ssum.my, c);
+        at(vn, c) = vf(i, j, k);
         if (k == 0 && !MT) {
-            double wb = w_from_omega(P, i, j, 0, 0.0, u2f, v2f);
-            Snew.mz[c] = (wb * 0.5) * (rho + rho); wn[c] = wb;
-        } else {
-            // (on a moving ground the w of the update, through the two round trips)
-            double rs = rho + (k == 0 ? rho : Ssum.cons[c - g.sk]);
-            double m = Ssum.mz[c];
-            double w1 = (m * 2.0) / rs; m = (w1 * 0.5) * rs;
-            double w2 = (m * 2.0) / rs; m = (w2 * 0.5) * rs;
-            Snew.mz[c] = m; wn[c] = w2;
+            const double wb = w_from_omega(P, i, j, 0, 0.0, uf, vf);
+            at(Snew.mz, c) = wb * rho;
+            at(wn, c) = wb;
+        } else {   // (on a moving ground the w of the update)
+            const double m = ld(Ssum.mz, c);
+            at(Snew.mz, c) = m;
+            at(wn, c) = 2.0 * m / (rho + (k == 0 ? rho : ld(Ssum.cons, c - sk)));
         }
         if (k == nz - 1) {
-            double wt = w_from_omega(P, i, j, nz, 0.0, u2f, v2f);
-            Snew.mz[c + g.sk] = (wt * 0.5) * (rho + rho); wn[c + g.sk] = wt;
+            const double wt = w_from_omega(P, i, j, nz, 0.0, uf, vf);
+            at(Snew.mz, c + sk) = wt * rho;
+            at(wn, c + sk) = wt;
         }
         if (make_next) stage_aux_ter<R>(P, Snew.cons, Anext, c, k);
     }
