@@ -64,25 +64,25 @@ def algorithmic_values_per_cell(cfg):
         "step_begin": (cfg.ncomp + 3 + 3 + 3, (cfg.ncomp - 1) + 2 + les),
         # reads u,v,w, rho | mu_t; writes 6 stresses
         "stress": (4, d + 6),
-        # reads 3 momenta, (rho) | theta, (mu_t); writes rhs rho, rho-theta, 3 avg momenta
-        "slow_cell": (3 + d, 1 + d + 2 + 3),
+        # reads 3 momenta, (rho) | theta, (mu_t); writes rhs rho, rho-theta
+        "slow_cell": (3 + d, 1 + d + 2),
         # reads rho | theta, (qv, qc, qp)
         "plane_avg": (1, 4 if moist else 1),
         # reads 3 momenta, 3 velocities, rho | p', (qv, qc), (6 stresses); writes 3 rhs
         "slow_mom": (7, 1 + m2 + 6 * d + 3),
-        # reads prev 2 mom, rho-theta, rho; stage 2 mom, rho-theta; writes new 2 mom |
-        # reads 2 rhs, lag, pi, (qv, qc), avg 2; writes avg 2, lag
+        # (terrain only; the flat substep is one kernel)
         "fast_horizontal": (9, 9 + m2),
-        # reads prev rho, rho-theta, w-mom; stage rho, rho-theta, 3 mom; new 2 mom; writes rho,
-        # rho-theta, w-mom | theta, 5 coefficients, rhs rho, rho-theta, w; avg w read+write
-        "fast_column": (13, 11),
+        # reads and writes the deviations of rho, rho-theta | reads 3 momentum increments, the
+        # extrapolated rho-theta, theta, 2 + 5 coefficients, 5 rhs; writes the 4 increments; 3 avg
+        # momenta read + write
+        "fast_column": (4, 27),
         # reads old scalars (1+nq), sum rho, rho-theta, 3 mom; writes ncomp, 3 mom, 3 vel |
         # reads scalar prims (1+nq), 3 avg mom; writes next prim (ncomp-1), pi, p'
         "slow_post": ((1 + nq) + 5 + cfg.ncomp + 6, (1 + nq) + 3 + (cfg.ncomp - 1) + 2),
-        # reads rho, rho-theta, 3 moisture; writes all ncomp (into the other buffer)
-        "kessler": ((5 + cfg.ncomp) if moist else 0, 0),
-        # reads stage rho-theta | theta, pi, (qv, qc); writes A, 1/B', C/B', P, Q
-        "fast_coeffs": (1, 1 + 1 + m2 + 5),
+        # reads rho, rho-theta, the species; writes rho-theta and the species
+        "kessler": (2 * (2 + nq) - 1 if moist else 0, 0),
+        # reads stage rho-theta | theta, pi, (qv, qc); writes 2 face factors and 5 z-face coefficients
+        "fast_coeffs": (1, 1 + 1 + m2 + 7),
     }
 
 
