@@ -101,14 +101,17 @@ __global__ void __launch_bounds__(512) k_ter_coef(Params P, double D, StateBuf S
 // ---------------------------------------------------------------------------
 // After the first substep (of the fused step) the extrapolated d(rho theta)
 // comes from the vertical part, which has both substeps' values in hand, and
-// the old increments are the previous substep's new ones: nine loads in place
-// of twenty-seven.  The M -> V -> M round trip of the fill between substeps
-// is the identity but for rounding and is not applied.
+// in the FP64 form the old increments are the previous substep's new ones:
+// nine loads in place of twenty-seven.  In the mixed form the stored
+// increments have 24 bits (the vertical part reads those), so that the old
+// ones are formed from the FP64 momenta again and the state accumulates in
+// FP64.  The M -> V -> M round trip of the fill between substeps is the
+// identity but for rounding and is not applied.
 template <class R, bool FIRST>
 __global__ void k_ter_fast_h(Params P, int step, double dtau, double facinv, StateBuf Sprev, StateBuf Sst, StageAux<R> A,
                              const R* __restrict__ Fmx, const R* __restrict__ Fmy, const R* __restrict__ lag_in,
                              R* __restrict__ lag_out, TerBuf<R> T, R* __restrict__ avx, R* __restrict__ avy,
-                             double* __restrict__ outx, double* __restrict__ outy) {
+                             double* outx, double* outy) {
     const Geo& g = P.g;
     int i, j, k;
     if (!cell_ij(g, i, j, k)) return;
@@ -125,11 +128,13 @@ __global__ void k_ter_fast_h(Params P, int step, double dtau, double facinv, Sta
     };
     if (FIRST && lag_out) at(lag_out, c) = R(ld(prt, c) - ld(srt, c));
     double odu, odv;
-    if (FIRST) {
-        odu = ld(Sprev.mx, c) - ld(Sst.mx, c);
-        odv = ld(Sprev.my, c) - ld(Sst.my, c);
-        at(T.odu, c) = R(odu);
-        at(T.odv, c) = R(odv);
+    if (FIRST || sizeof(R) < sizeof(double)) {   // (after the first substep Sprev is the array written below)
+        odu = at(Sprev.mx, c) - ld(Sst.mx, c);
+        odv = at(Sprev.my, c) - ld(Sst.my, c);
+        if (FIRST) {
+            at(T.odu, c) = R(odu);
+            at(T.odv, c) = R(odv);
+        }
     } else {
         odu = double(ld(T.odu, c));
         odv = double(ld(T.odv, c));

@@ -80,6 +80,34 @@ def test_terrain_substeps(nx, ny, nz):
             assert errs["rho"] < 1e-6 and errs["u"] < 1e-3 and errs["w"] < 1e-2, errs
 
 
+def test_terrain_momentum_accumulates_in_fp64():
+    """Uniform flow over flat ground, no gravity, a constant force: nothing but
+    the force acts, so a step adds dt F to the momenta whatever the number of
+    substeps.  The mixed form stores F in FP32 but accumulates the state in
+    FP64: each of the ~150 substeps rounds to 2^-53 of a momentum of the size
+    of dt F (bar 1e-13 of the velocity), where 24 bits would leave 1e-9."""
+    from erf_b200 import Dycore
+    nx, ny, nz = 8, 6, 8
+    cfg = T.abl_terrain(nx=nx, ny=ny, nz=nz, les="smagorinsky").cfg
+    cfg.les_type, cfg.zlo_bc, cfg.gravity, cfg.use_coriolis = C.LES_NONE, C.BC_SLIP_WALL, 0.0, 0
+    cfg.precision, cfg.mri_ratio, cfg.dt = C.PREC_MIXED, 100, 1.5
+    cfg.abl_geo_forcing[:] = [0.7, -0.3, 0.0]
+    rho, theta, u0, v0 = 1.1, 300.0, 1.0, -0.5
+    pi = (C.R_D * rho * theta / 1.0e5) ** (T.GAMMA * C.R_D / cfg.c_p)
+    p = 1.0e5 * (C.R_D * rho * theta / 1.0e5) ** T.GAMMA
+    dy = Dycore(cfg)
+    dy.set_terrain(T.btf_nodes(T.zlevels(nz, cfg.dz), np.zeros((ny + 1, nx + 1))))
+    dy.set_base_state([np.full((nz + 2) * ny * nx, b) for b in (rho, p, pi, theta)])
+    cons = np.zeros((5, nz, ny, nx))
+    cons[0], cons[1] = rho, rho * theta
+    got = dy.advance_host(cons, np.full((nz, ny, nx + 1), u0), np.full((nz, ny + 1, nx), v0), np.zeros((nz + 1, ny, nx)), 1)
+    assert dy.status() == 0
+    dy.close()
+    for vel, start, a in ((got[1], u0, 0.7), (got[2], v0, -0.3)):
+        want = start + cfg.dt * float(np.float32(rho * a)) / rho
+        assert np.max(np.abs(vel - want)) <= 1e-13 * abs(want), np.max(np.abs(vel - want))
+
+
 @pytest.mark.parametrize("nx,ny,nz", [(12, 4, 7), (24, 7, 33)])
 def test_moving_terrain_substeps(nx, ny, nz):
     case = T.moving_terrain(nx=nx, ny=ny, nz=nz, Lx=5.0 * nx, Ly=5.0 * ny, H=5.0 * nz, ampl=0.05, wavelength=2.5 * nx,
