@@ -277,14 +277,36 @@ __device__ __forceinline__ int64_t cidx(const Geo& g, int i, int j, int k) {
 #endif
     return (int64_t)i + (int64_t)g.nx * j + g.sk * k;
 }
-// The same in 32 bits, for ld / at below.
-__device__ __forceinline__ uint32_t eidx(const Geo& g, int i, int j, int k) {
+// The same in 32 bits, for ld / at below.  In the bounds-checked build the
+// offset carries the arrays' bound (nz+1 levels), so that an offset added to
+// it later (a neighbour level) is checked too, where it is used.
 #ifdef ERF_B200_BOUNDS
-    return (uint32_t)cidx(g, i, j, k);
+struct Elem {
+    uint32_t e, n;
+    int* oob;
+    __host__ __device__ operator uint32_t() const {
+        if (e < n) return e;
+#ifdef __CUDA_ARCH__
+        if (oob) atomicOr(oob, ST_BOUNDS);
 #else
-    return (uint32_t)i + (uint32_t)g.nx * (uint32_t)j + (uint32_t)g.sk * (uint32_t)k;
+        if (oob) *oob |= ST_BOUNDS;
 #endif
+        return 0;
+    }
+    template <class I>
+    __host__ __device__ Elem operator+(I d) const { return {e + (uint32_t)d, n, oob}; }
+    template <class I>
+    __host__ __device__ Elem operator-(I d) const { return {e - (uint32_t)d, n, oob}; }
+};
+__device__ __forceinline__ Elem eidx(const Geo& g, int i, int j, int k) {
+    return {(uint32_t)cidx(g, i, j, k), (uint32_t)g.nzf, g.oob};
 }
+#else
+using Elem = uint32_t;
+__device__ __forceinline__ Elem eidx(const Geo& g, int i, int j, int k) {
+    return (uint32_t)i + (uint32_t)g.nx * (uint32_t)j + (uint32_t)g.sk * (uint32_t)k;
+}
+#endif
 // Element e of an array of one component.  The byte offset stays in 32 bits
 // (an array of 4 GB would be 5e8 cells, more than the card holds), so that a
 // thread keeps one offset register per neighbour for all the arrays instead

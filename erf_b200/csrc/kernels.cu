@@ -299,7 +299,7 @@ __global__ void k_tau(Params P, const double* __restrict__ cons, const double* _
     int i, j, k;
     if (!cell_coords(g, i, j, k)) return;
     int im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny), ip = wrap(i + 1, g.nx), jp = wrap(j + 1, g.ny);
-    const uint32_t c = eidx(g, i, j, k);
+    const Elem c = eidx(g, i, j, k);
     const R OneThird = R(1. / 3.);
     R s11 = R((ld(u, eidx(g, ip, j, k)) - ld(u, c)) * g.dxi);
     R s22 = R((ld(v, eidx(g, i, jp, k)) - ld(v, c)) * g.dyi);
@@ -319,7 +319,7 @@ __global__ void k_tau(Params P, const double* __restrict__ cons, const double* _
         t12[c] = R(strain12(u, v, g, i, j, k)) * -m;
     }
     for (int kk = k; kk <= (k == g.nz - 1 ? g.nz : k); ++kk) {
-        const uint32_t e = eidx(g, i, j, kk);
+        const Elem e = eidx(g, i, j, kk);
         R m = P.use_consA ? R(0.25) * (rho(im, j, kk) + rho(i, j, kk) + rho(im, j, kk - 1) + rho(i, j, kk - 1)) * mu_eff : mu_eff;
         if (P.use_turb) m = m + R(2) * (R(0.25) * (mu(im, j, kk) + mu(i, j, kk) + mu(im, j, kk - 1) + mu(i, j, kk - 1)));
         t13[e] = R(strain13(u, w, g, i, j, kk)) * -m;
@@ -407,8 +407,9 @@ __device__ __forceinline__ R scalar_diff_vals(const Params& P, const double* __r
                                               const R* __restrict__ mut, double ae_d, double fac_d, int i, int j, int k) {
     const Geo& g = P.g;
     const R ae = R(ae_d), fac = R(fac_d);
-    const uint32_t sk = (uint32_t)g.sk, c = eidx(g, i, j, k);
-    const uint32_t e[6] = {eidx(g, wrap(i - 1, g.nx), j, k), eidx(g, wrap(i + 1, g.nx), j, k), eidx(g, i, wrap(j - 1, g.ny), k),
+    const uint32_t sk = (uint32_t)g.sk;
+    const Elem c = eidx(g, i, j, k);
+    const Elem e[6] = {eidx(g, wrap(i - 1, g.nx), j, k), eidx(g, wrap(i + 1, g.nx), j, k), eidx(g, i, wrap(j - 1, g.ny), k),
                            eidx(g, i, wrap(j + 1, g.ny), k), k > 0 ? c - sk : c, k < g.nz - 1 ? c + sk : c};
     const R rc = P.use_consA ? R(ld(rhoarr, c)) : R(0), mc = P.use_turb ? ld(mut, c) * fac : R(0);
     R f[6];
@@ -490,7 +491,8 @@ __device__ __forceinline__ R gatherz_tang(const Geo& g, const double* f, int typ
     R s[6];
     const int w = width_of<T>(type);
     if (k >= w && k + w <= g.nz) {
-        const uint32_t e = eidx(g, i, j, k), sk = (uint32_t)g.sk;
+        const Elem e = eidx(g, i, j, k);
+        const uint32_t sk = (uint32_t)g.sk;
 #pragma unroll
         for (int m = 0; m < 6; ++m) {
             const int off = m - 3;
@@ -959,7 +961,7 @@ __device__ __forceinline__ void post_march(const Params& P, const PostArgs<R>& a
     const TileEdge edge = tile_edge(g);
     const PlaneIdx pidx(g);
     constexpr int W = TV < 0 ? 3 : (TV == ERF_ADV_CENTERED_2ND ? 1 : (TV == ERF_ADV_UPWIND_5TH || TV == ERF_ADV_CENTERED_6TH || TV == ERF_ADV_WENO_5 ? 3 : 2));
-    const uint32_t e0 = ok ? eidx(g, i, j, 0) : 0;
+    const Elem e0 = ok ? eidx(g, i, j, 0) : eidx(g, 0, 0, 0);
     auto lvl = [&](int k) { return ld(phi, e0 + sk * (uint32_t)clampk(k, g.nz)); };
     // win[m]: phi at level f - W + m of the face f whose flux comes next
     R win[2 * W];
@@ -974,13 +976,13 @@ __device__ __forceinline__ void post_march(const Params& P, const PostArgs<R>& a
     if (ok) {
 #pragma unroll
         for (int m = 0; m < 2 * W; ++m) win[m] = lvl(k0 - W + m);
-        const uint32_t c = e0 + sk * (uint32_t)k0;
+        const Elem c = e0 + sk * (uint32_t)k0;
         zl = zflux(ld(a.avz, c));
         ax = ld(a.avx, c); ay = ld(a.avy, c); az = ld(a.avz, c + sk);
         top = lvl(k0 + W);
     }
     for (int k = k0; k < k1; ++k) {
-        const uint32_t c = e0 + sk * (uint32_t)k;
+        const Elem c = e0 + sk * (uint32_t)k;
         R zh = R(0), dif = R(0);
         plane_wait();
         __syncthreads();
@@ -1162,7 +1164,7 @@ __device__ __forceinline__ R zmom_flux_z(const Params& P, const double* rw, cons
     const Geo& g = P.g;
     const int vt = P.dyc_v, lo_z_face = 0, hi_z_face = g.nz;
     const R vf = R(P.f_dyc_v);
-    const uint32_t e0 = eidx(g, i, j, 0);
+    const Elem e0 = eidx(g, i, j, 0);
     auto wz = [&](int q) { return R(ld(w, e0 + (uint32_t)g.sk * (uint32_t)q)); };
     auto all = [&](int q, R upw, R frac, int type) {
         R sv[6];
@@ -1242,7 +1244,8 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_MOM) k_slow_mom(Params P,
     load_plane(g, pidx, pv, v, k0);
     load_plane(g, pidx, pw, w, k0);
     for (int k = k0; k < k1; ++k) {
-        const uint32_t c = ok ? eidx(g, i, j, k) : 0, sk = (uint32_t)g.sk;
+        const Elem c = ok ? eidx(g, i, j, k) : eidx(g, 0, 0, 0);
+        const uint32_t sk = (uint32_t)g.sk;
         const bool zk = ok && k >= 1;   // z-momentum on interior faces only
         plane_wait();
         __syncthreads();

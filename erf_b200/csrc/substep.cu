@@ -45,16 +45,8 @@ struct ColTile {
     }
 };
 
-// Offset of level k (of the bounds-checked build: cidx's check).
-__device__ __forceinline__ uint32_t lev(const Geo& g, int k) {
-#ifdef ERF_B200_BOUNDS
-    if ((unsigned)k > (unsigned)g.nz) {
-        if (g.oob) atomicOr(g.oob, ST_BOUNDS);
-        return 0;
-    }
-#endif
-    return (uint32_t)g.sk * (uint32_t)k;
-}
+// Offset of level k.
+__device__ __forceinline__ Elem lev(const Geo& g, int k) { return eidx(g, 0, 0, k); }
 
 // The stage's coefficients.  Per x / y face: the factor of the pressure
 // gradient of the extrapolated d(rho theta).  Per z face: P and Q, and the
@@ -79,23 +71,23 @@ __global__ void k_sub_coef(Params P, double D_d, StateBuf Sst, StageAux<R> A, R*
     const R* __restrict__ th = A.prim;
     if (t.ok) {
         for (int k = t.w; k < nz; k += t.nw) {
-            const int64_t o = lev(g, k);
+            const Elem o = lev(g, k);
             const R pc = A.pi[o + t.col];
             R gx = R(-Gamma_ * R_d) * (R(0.5) * (A.pi[o + t.xm] + pc)) * R(g.dxi);
             R gy = R(-Gamma_ * R_d) * (R(0.5) * (A.pi[o + t.ym] + pc)) * R(g.dyi);
             R q = R(0), qm = R(0);
             if (P.moist) {
-                const R* qv = th + 4 * N + o;
-                const R* qc = th + 5 * N + o;
-                q = qv[t.col] + qc[t.col];
-                gx /= R(1) + R(0.5) * (q + qv[t.xm] + qc[t.xm]);
-                gy /= R(1) + R(0.5) * (q + qv[t.ym] + qc[t.ym]);
-                if (k > 0) qm = (qv - sk)[t.col] + (qc - sk)[t.col];
+                const R* qv = th + 4 * N;
+                const R* qc = th + 5 * N;
+                q = qv[o + t.col] + qc[o + t.col];
+                gx /= R(1) + R(0.5) * (q + qv[o + t.xm] + qc[o + t.xm]);
+                gy /= R(1) + R(0.5) * (q + qv[o + t.ym] + qc[o + t.ym]);
+                if (k > 0) qm = qv[o + t.col - sk] + qc[o + t.col - sk];
             }
             fx[o + t.col] = gx;
             fy[o + t.col] = gy;
             if (k == 0) continue;
-            const int64_t c = o + t.col, cm = c - sk;
+            const Elem c = o + t.col, cm = c - sk;
             const R pi_c = R(0.5) * (A.pi[cm] + pc);
             R P_ = R(-Gamma_ * R_d * g.dzi + P.halfg * R_d * P.r0[k + 1] / (P.c_v * P.pi0[k + 1] * Sst.cons[N + c]));
             R Q_ = R(Gamma_ * R_d * g.dzi + P.halfg * R_d * P.r0[k] / (P.c_v * P.pi0[k] * Sst.cons[N + cm]));
@@ -118,7 +110,7 @@ __global__ void k_sub_coef(Params P, double D_d, StateBuf Sst, StageAux<R> A, R*
         if (t.w == 0)
             for (int k : {0, nz}) {
                 sA[k * TX + L] = R(0); sB[k * TX + L] = R(1); sC[k * TX + L] = R(0);
-                const int64_t f = lev(g, k) + t.col;
+                const Elem f = lev(g, k) + t.col;
                 cP[f] = R(0); cQ[f] = R(0);
             }
     }
@@ -154,7 +146,7 @@ __global__ void k_sub_coef(Params P, double D_d, StateBuf Sst, StageAux<R> A, R*
                 e = (k < m ? sA[s] : sC[s]) * inv;
                 gm = k < m ? sC[s] : sA[s];
             }
-            const int64_t f = lev(g, k) + t.col;
+            const Elem f = lev(g, k) + t.col;
             cI[f] = inv;
             cE[f] = e;
             cG[f] = gm;
@@ -197,23 +189,23 @@ __global__ void __launch_bounds__(1024) k_substep(Params P, SubArgs<R> a) {
     const double* srt = a.st.cons + g.ncell;
     const bool av_init = MODE == 0 || (MODE == 1 && a.av_init), grad = MODE == 2 || (MODE == 1 && a.grad);
     // deviations of cell / face c
-    auto dev_rt = [&](uint32_t c) -> double {
+    auto dev_rt = [&](Elem c) -> double {
         if (MODE == 0) return 0.0;
         if (MODE == 1) return ld(ort, c) - ld(srt, c);
         return at(a.drt, c);
     };
-    auto dev_r = [&](uint32_t c) -> double {
+    auto dev_r = [&](Elem c) -> double {
         if (MODE == 0) return 0.0;
         if (MODE == 1) return ld(a.old.cons, c) - ld(a.st.cons, c);
         return at(a.dr, c);
     };
-    auto dev_m = [&](const double* old, const double* st, const R* dev, uint32_t f) -> R {
+    auto dev_m = [&](const double* old, const double* st, const R* dev, Elem f) -> R {
         if (MODE == 0) return R(0);
         if (MODE == 1) return R(ld(old, f) - ld(st, f));
         return ld(dev, f);
     };
-    auto dev_w = [&](uint32_t f) -> R { return dev_m(a.old.mz, a.st.mz, a.wi, f); };
-    auto ext = [&](uint32_t c) -> R {   // extrapolated d(rho theta)
+    auto dev_w = [&](Elem f) -> R { return dev_m(a.old.mz, a.st.mz, a.wi, f); };
+    auto ext = [&](Elem c) -> R {   // extrapolated d(rho theta)
         if (MODE == 2) return ld(a.ei, c);
         const R d = R(dev_rt(c));
         return a.lag_in ? d + R(0.1) * (d - ld(a.lag_in, c)) : d;
@@ -222,7 +214,7 @@ __global__ void __launch_bounds__(1024) k_substep(Params P, SubArgs<R> a) {
     if (t.ok) {
 #pragma unroll 1
         for (int k = t.w; k < nz; k += t.nw) {
-            const uint32_t o = lev(g, k), c = o + c0, xm = o + t.xm, xp = o + t.xp, ym = o + t.ym, yp = o + t.yp;
+            const Elem o = lev(g, k), c = o + c0, xm = o + t.xm, xp = o + t.xp, ym = o + t.ym, yp = o + t.yp;
             R xl = ld(a.Fmx, c), xh = ld(a.Fmx, xp), yl = ld(a.Fmy, c), yh = ld(a.Fmy, yp);
             if (grad) {
                 const R ec = ext(c);
@@ -269,7 +261,7 @@ __global__ void __launch_bounds__(1024) k_substep(Params P, SubArgs<R> a) {
         const R halfg = R(P.halfg);
 #pragma unroll 2
         for (int k = t.w; k <= nz; k += t.nw) {
-            const uint32_t f = lev(g, k) + c0;
+            const Elem f = lev(g, k) + c0;
             const int s = k * TX + L;
             R r = ld(a.Fmz, f);
             if (k > 0 && k < nz) {
@@ -330,12 +322,12 @@ __global__ void __launch_bounds__(1024) k_substep(Params P, SubArgs<R> a) {
         const double ib2 = 1.0 / a.b2;
 #pragma unroll 1
         for (int k = t.w; k < nz; k += t.nw) {
-            const uint32_t c = lev(g, k) + c0;
+            const Elem c = lev(g, k) + c0;
             const int s = k * TX + L;
             const R sl = sS[s], sh = sS[s + TX];
             const R wl = dev_w(c), wh = dev_w(c + sk);
             const R zl = b2 * sl + b1 * wl;
-            auto avz = [&](uint32_t f, R z) {
+            auto avz = [&](Elem f, R z) {
                 at(a.avz, f) = (av_init ? R(ld(a.st.mz, f)) : at(a.avz, f)) + R(a.facinv) * z;
             };
             avz(c, zl);

@@ -28,10 +28,10 @@ __global__ void __launch_bounds__(512) k_ter_coef(Params P, double D, StateBuf S
     auto th = [&](int kk) { return ccw(A.prim, g, i, j, kk); };
     if (ok) {
         for (int k = w; k <= nz; k += nw) {
-            const uint32_t f = eidx(g, i, j, k);
+            const Elem f = eidx(g, i, j, k);
             double a = 0.0, b = 1.0, cc = 0.0, p = 0.0, q = 0.0;
             if (k > 0 && k < nz) {
-                const uint32_t fm = f - sk;
+                const Elem fm = f - sk;
                 const double dJ = 0.5 * (detJ_at(P, i, j, k) + detJ_at(P, i, j, k - 1)), iJ = 1. / dJ;
                 const double pi_c = 0.5 * (double(ld(A.pi, fm)) + double(ld(A.pi, f)));
                 p = (-Gamma_ * R_d * dzi * iJ + halfg * R_d * ld(P.r0, f + sk) / (P.c_v * ld(P.pi0, f + sk) * ld(srt, f))) * pi_c;
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(512) k_ter_coef(Params P, double D, StateBuf S
     if (ok) {
         for (int k = w; k <= nz; k += nw) {
             const int s = k * TX + L;
-            const uint32_t f = eidx(g, i, j, k);
+            const Elem f = eidx(g, i, j, k);
             double inv = sB[s], e, gm;
             if (k == m) {
                 const double bet = sB[s] - sA[s] * sC[s - TX] - sC[s] * sA[s + TX];
@@ -116,12 +116,12 @@ __global__ void k_ter_fast_h(Params P, int step, double dtau, double facinv, Sta
     int i, j, k;
     if (!cell_ij(g, i, j, k)) return;
     const int nz = g.nz, im = wrap(i - 1, g.nx), jm = wrap(j - 1, g.ny);
-    const uint32_t c = eidx(g, i, j, k), cxm = eidx(g, im, j, k), cym = eidx(g, i, jm, k);
+    const Elem c = eidx(g, i, j, k), cxm = eidx(g, im, j, k), cym = eidx(g, i, jm, k);
     const double beta_d = 0.1, dxi = g.dxi, dyi = g.dyi;
     const double* prt = Sprev.cons + g.ncell;
     const double* srt = Sst.cons + g.ncell;
     auto extrap = [&](int ii, int jj, int kk) {
-        const uint32_t e = eidx(g, ii, jj, clampk(kk, nz));
+        const Elem e = eidx(g, ii, jj, clampk(kk, nz));
         if (!FIRST) return ld(T.ec, e);
         const double drt = ld(prt, e) - ld(srt, e);
         return step == 0 ? drt : drt + beta_d * (drt - double(ld(lag_in, e)));
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(1024) k_ter_fast_vert(Params P, double dtau, d
     const double* srt = Sst.cons + g.ncell;
     const R* Ft = Fcons + g.ncell;
     auto th = [&](int ii, int jj, int kk) { return ccw(A.prim, g, ii, jj, kk); };
-    auto prev_mz = [&](int k, uint32_t f) {
+    auto prev_mz = [&](int k, Elem f) {
         if (prev_rt && (k == 0 || k == nz)) return T.bnd[(k == 0 ? 0 : g.sk) + (int64_t)j * g.nx + i];
         return Sprev.mz[f];
     };
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(1024) k_ter_fast_vert(Params P, double dtau, d
     // Omega'' and the coefficients (faces)
     if (ok) {
         for (int k = w0; k <= nz; k += nw) {
-            const uint32_t f = eidx(g, i, j, k), fx = eidx(g, ip, j, k), fy = eidx(g, i, jp, k);
+            const Elem f = eidx(g, i, j, k), fx = eidx(g, ip, j, k), fy = eidx(g, i, jp, k);
             const int s = k * TX + L;
             double du = 0.0, dup = 0.0, dv = 0.0, dvp = 0.0;
             if (k < nz) {
@@ -292,11 +292,11 @@ __global__ void __launch_bounds__(1024) k_ter_fast_vert(Params P, double dtau, d
     // ---- phase 2: the detJ-weighted right-hand side of the Omega'' system (faces)
     if (ok) {
         for (int k = w0; k <= nz; k += nw) {
-            const uint32_t f = eidx(g, i, j, k);
+            const Elem f = eidx(g, i, j, k);
             const int s = k * TX + L;
             double rhs = dtau * double(ld(Fmz, f));
             if (k > 0 && k < nz) {
-                const uint32_t cm = f - sk;
+                const Elem cm = f - sk;
                 const double Jk = detJ_at(P, i, j, k), Jkm = detJ_at(P, i, j, k - 1), dJk = 0.5 * (Jk + Jkm);
                 const double cPk = double(ld(cf.P, f)), cQk = double(ld(cf.Q, f));
                 const double t_2 = th(i, j, k - 2), t_1 = th(i, j, k - 1), t0 = th(i, j, k), t1 = th(i, j, k + 1);
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(1024) k_ter_fast_vert(Params P, double dtau, d
     // ---- phase 4: w'' from Omega'', vertical fluxes, average Omega, rho and rho*theta
     if (ok) {
         for (int k = w0; k <= nz; k += nw) {
-            const uint32_t c = eidx(g, i, j, k);
+            const Elem c = eidx(g, i, j, k);
             const int s = k * TX + L;
             double mz = ld(Sst.mz, c);
             if (k >= 1 && k <= nz - 1) mz += sR[s] + sN[s];

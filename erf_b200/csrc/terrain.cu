@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_SLOW_CELL) k_ter_slow_cell
     const PlaneIdx pidx(g);
     const DiffT<R> D{P, S.cons, A.prim, mut, dd ? tke.kthv : nullptr, P.alphaT_eff, P.invPr, T.fx[0], T.fy[0]};
     auto xface = [&](int r, int c, int ii, int jj, int k) {
-        const uint32_t e = eidx(g, ii, jj, k);
+        const Elem e = eidx(g, ii, jj, k);
         const double h = hzeta_I(P, ii, jj, k), m = h * ld(S.mx, e);
         const int w = width_of<HT>(ht);
         double s[6];
@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_SLOW_CELL) k_ter_slow_cell
         if (diff) sd.fx[r][c] = double(ld(T.fx[0], e)) * h;
     };
     auto yface = [&](int r, int c, int ii, int jj, int k) {
-        const uint32_t e = eidx(g, ii, jj, k);
+        const Elem e = eidx(g, ii, jj, k);
         const double h = hzeta_J(P, ii, jj, k), m = h * ld(S.my, e);
         const int w = width_of<HT>(ht);
         double s[6];
@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_SLOW_CELL) k_ter_slow_cell
         const double fl = fh, tl = th, dl = dh, rl = rh;
         zflux(k + 1, fh, th, dh, rh);
         if (k < k0) continue;
-        const uint32_t c = eidx(g, i, j, k);
+        const Elem c = eidx(g, i, j, k);
         at(avx, c) = R(sm.fx[ty][tx]);
         at(avy, c) = R(sm.fy[ty][tx]);
         at(avz, c) = R(fl);
@@ -1436,7 +1436,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
                 if (q < nslow) load_plane(g, pidx, pl[q], slow_phi(q), k + 1);
         }
         if (!ok) continue;   // the next level's first barrier orders the reuse of sh
-        const uint32_t c = eidx(g, i, j, k);
+        const Elem c = eidx(g, i, j, k);
         const double invdetJ = MT ? 1. / detJ_at(P, i, j, k) : inv_detJ(P, i, j, k);   // (moving: the tables are another grid's)
 #pragma unroll
         for (int q = 0; q < NS; ++q) {
@@ -1493,7 +1493,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
                 kk = kk < 0 ? 0 : nz - 1;
             }
             ii = wrap(ii, g.nx); jj = wrap(jj, g.ny);
-            const uint32_t e = eidx(g, ii, jj, kk);
+            const Elem e = eidx(g, ii, jj, kk);
             return 2.0 * ld(Ssum.mx, e) / (ld(Ssum.cons, e) + ld(Ssum.cons, eidx(g, wrap(ii - 1, g.nx), jj, kk)));
         };
         auto vf = [&](int ii, int jj, int kk) {
@@ -1502,7 +1502,7 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_POST) k_ter_post(Params P,
                 kk = kk < 0 ? 0 : nz - 1;
             }
             ii = wrap(ii, g.nx); jj = wrap(jj, g.ny);
-            const uint32_t e = eidx(g, ii, jj, kk);
+            const Elem e = eidx(g, ii, jj, kk);
             return 2.0 * ld(Ssum.my, e) / (ld(Ssum.cons, e) + ld(Ssum.cons, eidx(g, ii, wrap(jj - 1, g.ny), kk)));
         };
         at(Snew.mx, c) = ld(Ssum.mx, c);

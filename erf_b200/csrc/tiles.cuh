@@ -27,7 +27,8 @@ __device__ __forceinline__ R adv_flux_z(const Geo& g, const R* __restrict__ phi,
                                         R frac, int i, int j, int k) {
     R s[6];
     const int w = width_of<T>(type);
-    const uint32_t e = eidx(g, i, j, k), sk = (uint32_t)g.sk;
+    const Elem e = eidx(g, i, j, k);
+    const uint32_t sk = (uint32_t)g.sk;
     if (k >= w && k + w <= g.nz) {
 #pragma unroll
         for (int m = 0; m < 6; ++m) {
@@ -156,7 +157,7 @@ __device__ __forceinline__ void tile_put(const Geo& g, FluxTile<R>& t, const Pla
                                          const M* __restrict__ az, int th, int tv, R fh, R fv, int i, int j, int k,
                                          bool first, R& zl, R& zh) {
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const uint32_t c = eidx(g, i, j, k);
+    const Elem c = eidx(g, i, j, k);
     t.fx[ty][tx] = plane_flux_x<TH>(pl, ty, tx, R(ld(ax, c)), th, fh);
     t.fy[ty][tx] = plane_flux_y<TH>(pl, ty, tx, R(ld(ay, c)), th, fh);
     if (first) zl = adv_flux_z<TV>(g, phi, az, tv, fv, i, j, k);
