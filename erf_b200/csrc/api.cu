@@ -2,6 +2,7 @@
 // step sequence (MRISplitIntegrator::advance, TimeIntegration/ERF_MRI.H:187-369)
 // and its CUDA-graph replay.
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -848,6 +849,9 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     *out = nullptr;
     int v = validate(cfg);
     if (v != ERF_B200_OK) return v;
+    // the kernels' byte offsets within an array have 32 bits (ld / at, common.cuh)
+    const int64_t planes = cfg->nz + (cfg->use_terrain ? 2 : 1);   // the base state's over terrain
+    if (planes > (int64_t)UINT32_MAX / (int64_t)sizeof(double) / ((int64_t)cfg->nx * cfg->ny)) return ERF_B200_ENOMEM;
     erf_b200_ctx* c = new (std::nothrow) erf_b200_ctx();
     if (!c) return ERF_B200_ENOMEM;
     c->cfg = *cfg;

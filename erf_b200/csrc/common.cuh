@@ -308,7 +308,7 @@ __device__ __forceinline__ Elem eidx(const Geo& g, int i, int j, int k) {
 }
 #endif
 // Element e of an array of one component.  The byte offset stays in 32 bits
-// (an array of 4 GB would be 5e8 cells, more than the card holds), so that a
+// (an array of 4 GB would be 5e8 cells; erf_b200_create refuses them), so that a
 // thread keeps one offset register per neighbour for all the arrays instead
 // of forming a 64-bit address per load.
 template <class T>

@@ -216,7 +216,9 @@ typedef struct erf_b200_ctx erf_b200_ctx;
 int erf_b200_config_defaults(erf_b200_config* cfg);
 
 /* Create a context on the current CUDA device; all scratch is allocated here
- * and never inside a step.  `stream` is a cudaStream_t (NULL = legacy default). */
+ * and never inside a step.  `stream` is a cudaStream_t (NULL = legacy default).
+ * A grid that does not fit the device, or one component of which takes 4 GB or
+ * more (5e8 cells), gives ERF_B200_ENOMEM. */
 int erf_b200_create(erf_b200_ctx** ctx, const erf_b200_config* cfg, void* stream);
 int erf_b200_destroy(erf_b200_ctx* ctx);
 int erf_b200_set_stream(erf_b200_ctx* ctx, void* stream);

@@ -121,6 +121,20 @@ def test_create_rejects_unsupported_most_config(lib, change):
     assert lib.erf_b200_create(ctypes.byref(ctx), ctypes.byref(c), None) == 8  # ERF_B200_ECONFIG
 
 
+@pytest.mark.parametrize("nx,ny,nz,ter", [(4096, 4096, 31, 0), (4096, 4096, 30, 1), (65536, 65536, 4, 0),
+                                          (2 ** 31 - 1, 2 ** 31 - 1, 4, 0)])
+def test_create_refuses_arrays_of_4_gb(lib, nx, ny, nz, ter):
+    """One component of 2^32 bytes or more (z faces; over terrain the base
+    state's planes) is past the kernels' 32-bit offsets: refused as out of
+    memory before any CUDA call, on a card of any size."""
+    c = C.defaults()
+    c.nx, c.ny, c.nz, c.use_terrain = nx, ny, nz, ter
+    c.dycore_horiz_adv = c.dycore_vert_adv = C.UPWIND_5TH
+    ctx = ctypes.c_void_p()
+    lib.erf_b200_create.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_void_p, ctypes.c_void_p]
+    assert lib.erf_b200_create(ctypes.byref(ctx), ctypes.byref(c), None) == 3 and not ctx  # ERF_B200_ENOMEM
+
+
 @pytest.mark.parametrize("moist", [False, True])
 def test_create_accepts_most_config(lib, moist):
     """The supported MOST ground passes validation, dry or with Kessler
