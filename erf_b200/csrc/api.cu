@@ -957,7 +957,7 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
             const int bad = c->mixed ? ter_vert_shape<float>(nz, &c->ter_tx) : ter_vert_shape<double>(nz, &c->ter_tx);
             if (c->ter_tx < 1) rc = ERF_B200_ECONFIG;
             else if (bad) rc = ERF_B200_ECUDA;
-            else if (cfg->terrain_type == ERF_TERRAIN_MOVING &&
+            else if (cfg->terrain_type == ERF_TERRAIN_MOVING && !no_substepping(*cfg) &&
                      (c->mixed ? mt_shape<float>(c->g, &c->mt_tx) : mt_shape<double>(c->g, &c->mt_tx)) != 0)
                 rc = ERF_B200_ECUDA;
         }

@@ -351,7 +351,8 @@ constexpr int MT_COL_ARRAYS = 9, MT_COEF_ARRAYS = 3;
 
 // Columns per block: 16 (a row of 16 FP64 values is a line) where two blocks
 // share an SM, fewer where the plane would leave SMs without a block: the
-// levels of a tile are worked in parallel, so a narrow tile is as quick.
+// levels of a tile are worked in parallel, so a narrow tile is as quick.  A
+// single column holds every depth that erf_b200_create takes.
 template <class R>
 int mt_shape(const Geo& g, int* tx) {
     int dev = 0, nsm = 148, maxopt = 0, persm = 0;
@@ -362,6 +363,7 @@ int mt_shape(const Geo& g, int* tx) {
     int t = 16;
     while (t > 2 && 2 * (mt_smem(g.nz, t, MT_COL_ARRAYS) + 1024) > (size_t)persm) t /= 2;
     while (t > 2 && (g.sk + t - 1) / t < nsm) t /= 2;
+    while (t > 1 && mt_smem(g.nz, t, MT_COL_ARRAYS) > (size_t)maxopt) t /= 2;
     *tx = t;
     if (mt_smem(g.nz, t, MT_COL_ARRAYS) > (size_t)maxopt) return 1;
     return cudaFuncSetAttribute(k_mt_coef<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt) != cudaSuccess ||

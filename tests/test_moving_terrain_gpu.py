@@ -221,3 +221,22 @@ def test_moving_terrain_plotfile_matches_gold_header(tmp_path):
         worst[nm] = e
     print("plotfile vs gold header:", worst)
     assert all(e <= 2e-10 for e in worst.values()), worst
+
+
+@pytest.mark.parametrize("substeps", [True, False])
+def test_deep_mixed_columns(substeps):
+    """The mixed form takes columns of up to 2074 levels, with substeps and
+    without: two columns of 1800 levels are past what a block can share.
+    FP32 increments against the FP64 oracle: <= 1e-6 per field (24 bits), w
+    against its own size <= 1e-4."""
+    nz = 1800
+    case = T.moving_terrain(nx=8, ny=4, nz=nz, Lx=40.0, Ly=20.0, H=0.5 * nz, ampl=0.05, wavelength=20.0,
+                            substeps=substeps, dt=0.001, steps=2)
+    case.cfg.mri_ratio = 4
+    got, _, _, _, _, status = _gpu(case, case.steps, precision=C.PREC_MIXED)
+    assert status == 0
+    ref = oracle.advance_moving_terrain(case.cfg, 0.0, case.base, *case.build_state(), case.steps)
+    errs = _errors(got, ref[:4])
+    print("deep columns, mixed:", errs)
+    w = errs.pop("w")
+    assert all(e <= 1e-6 for e in errs.values()) and w <= 1e-4, (errs, w)
