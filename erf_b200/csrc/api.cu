@@ -1,6 +1,7 @@
 // api.cu -- host side of the C-ABI: context, device buffers, the multirate RK3
 // step sequence (MRISplitIntegrator::advance, TimeIntegration/ERF_MRI.H:187-369)
 // and its CUDA-graph replay.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -45,7 +46,8 @@ struct Bulk {
     StageAux<R> aux[2];           // stage primitives, Exner, p'
     R* mut;                       // eddy viscosity
     R *t11, *t22, *t33, *t12, *t13, *t23;
-    R *cA, *cInvB, *cCB, *cP, *cQ;  // fast coefficients of the current stage
+    R* tau;                       // t11 ... t23, and what shares their block (bind_bulk)
+    R *cA, *cInvB, *cCB, *cP, *cQ;  // the per-pass make_fast_coeffs
     R *c12 = nullptr, *c13 = nullptr, *c23 = nullptr;  // learned closure: cell-centred off-diagonal stresses
     R *hx = nullptr, *hy = nullptr, *hz = nullptr;     // learned closure: rho * heat flux
     TkeBuf<R> tke{nullptr, nullptr, nullptr, nullptr}; // Deardorff closure arrays
@@ -697,28 +699,35 @@ void enqueue_step(erf_b200_ctx* c, int p, LaunchTimer* T = nullptr) {
     else enqueue_step_t<double>(c, c->bd, p, T);
 }
 
+// The stresses (dead once the momenta's right-hand side has read them), the
+// increments of the flat substeps that follow, and the per-pass
+// make_fast_coeffs' five arrays (exported by the same call) take turns in one
+// block.  Neither step keeps a primitive for rho QKE on a flat grid
+// (prim_read), so those two slots hold the pressure-gradient factors.
+int64_t padded64(int64_t n) { return (n + 63) / 64 * 64; }
 template <class R>
 int alloc_bulk(erf_b200_ctx* c, Bulk<R>& B) {
     const erf_b200_config* cfg = &c->cfg;
     const int64_t N = (int64_t)cfg->nx * cfg->ny * cfg->nz;
     const int64_t NZF = (int64_t)cfg->nx * cfg->ny * (cfg->nz + 1);
     const int nc = cfg->ncomp;
+    const bool ter = cfg->use_terrain, moving = ter && cfg->terrain_type == ERF_TERRAIN_MOVING;
+    const bool diff = cfg->les_type != ERF_LES_NONE || cfg->molec_diff_type != ERF_MOLEC_NONE;
+    // the per-pass substeps (plain form, not over a moving grid) need a substep's arrays whatever the step takes
+    const bool sub = cfg->substepping_type == ERF_SUBSTEP_IMPLICIT || (!c->mixed && !moving);
     int rc = ERF_B200_OK;
     auto A = [&](R** p, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, p, n); };
+    auto D = [&](double** p, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, p, n); };
     A(&B.Fcons, 2 * N); A(&B.Fmx, N); A(&B.Fmy, N); A(&B.Fmz, NZF);
     A(&B.avx, N); A(&B.avy, N); A(&B.avz, NZF);
     A(&B.lag[0], N); A(&B.lag[1], N);
     for (int p = 0; p < 2; ++p) { A(&B.aux[p].prim, (nc - 1) * N); A(&B.aux[p].pi, N); A(&B.aux[p].pp, N); }
     A(&B.mut, N);
-    A(&B.t11, N); A(&B.t22, N); A(&B.t33, N); A(&B.t12, N); A(&B.t13, NZF); A(&B.t23, NZF);
-    if (!c->mixed) {   // the per-pass make_fast_coeffs
-        A(&B.cA, NZF); A(&B.cInvB, NZF); A(&B.cCB, NZF); A(&B.cP, NZF); A(&B.cQ, NZF);
-    }
-    if (!cfg->use_terrain && (!c->mixed || cfg->substepping_type == ERF_SUBSTEP_IMPLICIT)) {
-        A(&B.sc.fx, N); A(&B.sc.fy, N);
+    int64_t tau = 4 * padded64(N) + 2 * padded64(NZF);
+    if (!c->mixed) tau = std::max(tau, 5 * padded64(NZF));
+    A(&B.tau, tau);
+    if (!ter && sub) {
         A(&B.sc.E, NZF); A(&B.sc.G, NZF); A(&B.sc.I, NZF); A(&B.sc.P, NZF); A(&B.sc.Q, NZF);
-        for (int q = 0; q < 2; ++q) { A(&B.du[q], N); A(&B.dv[q], N); A(&B.dw[q], NZF); }
-        auto D = [&](double** q, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, q, n); };
         D(&B.dr, N); D(&B.drt, N);
     }
     if (cfg->les_type == ERF_LES_MLP) {
@@ -727,20 +736,35 @@ int alloc_bulk(erf_b200_ctx* c, Bulk<R>& B) {
     if (cfg->les_type == ERF_LES_DEARDORFF) {
         A(&B.tke.kthv, N); A(&B.tke.diss, N); A(&B.tke.smn, N); A(&B.tke.hfz, NZF);
     }
-    if (cfg->use_terrain) {
+    if (ter && diff) {
         A(&B.ter.s11, N); A(&B.ter.s22, N); A(&B.ter.s33, N); A(&B.ter.s12, N); A(&B.ter.s13, NZF);
         A(&B.ter.s23, NZF); A(&B.ter.t31, NZF); A(&B.ter.t32, NZF);
-        A(&B.ter.ndu, N); A(&B.ter.ndv, N); A(&B.ter.odu, N); A(&B.ter.odv, N);
         A(&B.ter.fx[0], N); A(&B.ter.fy[0], N); A(&B.ter.fx[1], N); A(&B.ter.fy[1], N);
-        auto D = [&](double** q, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, q, n); };
+    }
+    if (ter && !moving && sub) {
+        A(&B.ter.ndu, N); A(&B.ter.ndv, N); A(&B.ter.odu, N); A(&B.ter.odv, N);
         D(&B.ter.bnd, 2 * (int64_t)cfg->nx * cfg->ny);
         D(&B.ter.ec, N);
-        for (MtCoef<R>& m : B.mc) {   // static terrain: one stage's; moving: two substeps'
-            if (&m != B.mc && (cfg->terrain_type != ERF_TERRAIN_MOVING || cfg->substepping_type != ERF_SUBSTEP_IMPLICIT)) break;
-            A(&m.E, NZF); A(&m.G, NZF); A(&m.I, NZF); A(&m.P, NZF); A(&m.Q, NZF);
-        }
+    }
+    for (int q = 0; ter && sub && q < (moving ? 2 : 1); ++q) {   // static terrain: one stage's; moving: two substeps'
+        MtCoef<R>& m = B.mc[q];
+        A(&m.E, NZF); A(&m.G, NZF); A(&m.I, NZF); A(&m.P, NZF); A(&m.Q, NZF);
     }
     return rc;
+}
+// The pointers into shared blocks, once the blocks are there.
+template <class R>
+void bind_bulk(erf_b200_ctx* c, Bulk<R>& B) {
+    const Geo& g = c->g;
+    const int64_t n = padded64(g.ncell), f = padded64(g.nzf);
+    R* cell[4] = {B.tau, B.tau + n, B.tau + 2 * n, B.tau + 3 * n};
+    R* face[2] = {B.tau + 4 * n, B.tau + 4 * n + f};
+    B.t11 = cell[0]; B.t22 = cell[1]; B.t33 = cell[2]; B.t12 = cell[3];
+    B.t13 = face[0]; B.t23 = face[1];
+    for (int q = 0; q < 2; ++q) { B.du[q] = cell[q]; B.dv[q] = cell[2 + q]; B.dw[q] = face[q]; }
+    B.cA = B.tau; B.cInvB = B.tau + f; B.cCB = B.tau + 2 * f; B.cP = B.tau + 3 * f; B.cQ = B.tau + 4 * f;
+    B.sc.fx = B.aux[0].prim + (ERF_RHOQKE_COMP - 1) * g.ncell;
+    B.sc.fy = B.aux[1].prim + (ERF_RHOQKE_COMP - 1) * g.ncell;
 }
 
 int build_graphs(erf_b200_ctx* c) {
@@ -879,8 +903,8 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     int rc = ERF_B200_OK;
     auto A = [&](double** p, size_t n) { if (rc == ERF_B200_OK) rc = dalloc(c, p, n); };
     c->collect = true;
-    for (int s = 0; s < 4; ++s) {
-        A(&c->S[s].cons, nc * N); A(&c->S[s].mx, N); A(&c->S[s].my, N); A(&c->S[s].mz, NZF);
+    for (int s = 0; s < 4; ++s) {   // (the fast sum has rho and rho theta only)
+        A(&c->S[s].cons, (s == 3 ? 2 : nc) * N); A(&c->S[s].mx, N); A(&c->S[s].my, N); A(&c->S[s].mz, NZF);
     }
     for (int p = 0; p < 2; ++p) { A(&c->vel[p][0], N); A(&c->vel[p][1], N); A(&c->vel[p][2], NZF); }
     A(&c->pavg, plane_avg_doubles(cfg->nz));
@@ -917,6 +941,8 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
     }
     if (rc != ERF_B200_OK) { erf_b200_destroy(c); return rc; }
     make_params(c);
+    if (c->mixed) bind_bulk(c, c->bf);
+    else bind_bulk(c, c->bd);
     // a moving grid is generated by the step itself
     if (cfg->use_terrain && cfg->terrain_type == ERF_TERRAIN_MOVING) {
         c->ter_set = true;
@@ -1562,7 +1588,7 @@ int erf_b200_slow_rhs_post(erf_b200_ctx* c, int nrk, double slow_dt, const erf_b
     StateBuf OLD = c->S[0], NEW = c->S[1], SUM = c->S[3];
     int rc;
     if ((rc = pack4(c, S_old, nc, OLD.cons, OLD.mx, OLD.my, OLD.mz))) return rc;
-    if ((rc = pack4(c, S_data, nc, SUM.cons, SUM.mx, SUM.my, SUM.mz))) return rc;
+    if ((rc = pack4(c, S_data, 2, SUM.cons, SUM.mx, SUM.my, SUM.mz))) return rc;
     if ((rc = pack4(c, S_scratch, 0, nullptr, B.avx, B.avy, B.avz))) return rc;
     // stage state and primitives: those of the preceding slow_rhs_pre
     if (c->P.ter)

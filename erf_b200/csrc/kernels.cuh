@@ -52,7 +52,7 @@ struct Params {
 };
 
 // Number of static-terrain metric tables (planes of nzf values each).
-constexpr int TER_NMET = 24;
+constexpr int TER_NMET = 22;
 
 // One copy of the prognostic state: cons (ncomp*ncell), face momenta.
 struct StateBuf {

@@ -75,9 +75,7 @@ static __global__ void k_ter_met_tables(Params P, double* __restrict__ met) {
     double* m = met + cidx(g, i, j, k);
     const int64_t s = g.nzf;
     m[MT_HZETA_I * s] = hzeta_I_fn(P, i, j, k);
-    m[MT_HXI_I * s] = hxi_I_fn(P, i, j, k);
     m[MT_HZETA_J * s] = hzeta_J_fn(P, i, j, k);
-    m[MT_HETA_J * s] = heta_J_fn(P, i, j, k);
     m[MT_HXI_K * s] = hxi_K_fn(P, i, j, k);
     m[MT_HETA_K * s] = heta_K_fn(P, i, j, k);
     m[MT_HZETA_EK * s] = hzeta_EK_fn(P, i, j, k);

@@ -94,7 +94,7 @@ __device__ __forceinline__ double zlo_eta_fn(const Params& P, int i, int j, int 
 // evaluating them in place) and stored as TER_NMET planes of (nz+1) x ny x
 // nx values, k in [0, nz].  A pass reads one value instead of re-deriving it
 // from four to eight nodes of z_phys_nd; outside [0, nz] the function runs.
-enum { MT_HZETA_I, MT_HXI_I, MT_HZETA_J, MT_HETA_J, MT_HXI_K, MT_HETA_K, MT_HZETA_EK, MT_HZETA_EJ, MT_HZETA_EI,
+enum { MT_HZETA_I, MT_HZETA_J, MT_HXI_K, MT_HETA_K, MT_HZETA_EK, MT_HZETA_EJ, MT_HZETA_EI,
        MT_ZLO_XI, MT_ZLO_ETA, MT_HZETA_CC, MT_HXI_CC, MT_HETA_CC, MT_HZETA_K, MT_HXI_EK, MT_HETA_EK, MT_HXI_EJ,
        MT_HETA_EJ, MT_HXI_EI, MT_HETA_EI, MT_RXI_I, MT_RETA_J, MT_IJ, MT_COUNT };
 static_assert(MT_COUNT == TER_NMET, "metric table count");
@@ -108,9 +108,7 @@ __device__ __forceinline__ double mt_at(const Params& P, int q, int i, int j, in
         return name##_fn(P, i, j, k);                                              \
     }
 ERFB_MT(hzeta_I, MT_HZETA_I)
-ERFB_MT(hxi_I, MT_HXI_I)
 ERFB_MT(hzeta_J, MT_HZETA_J)
-ERFB_MT(heta_J, MT_HETA_J)
 ERFB_MT(hxi_K, MT_HXI_K)
 ERFB_MT(heta_K, MT_HETA_K)
 ERFB_MT(hzeta_EK, MT_HZETA_EK)

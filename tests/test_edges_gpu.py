@@ -127,6 +127,37 @@ def test_moving_terrain_substeps(nx, ny, nz):
     assert all(e <= TOL for e in errs.values()), errs
 
 
+def _held(which):
+    """(case, bytes that a context may hold).  Flat grids: the state three
+    times and its fast sum, two sets of velocities and the stage's arrays, as
+    cells and z faces of FP64 and of the bulk type; terrain: the same with
+    the metric tables, as measured when the substeps were separate horizontal
+    and vertical kernels."""
+    n, f = 24 * 20 * 32, 24 * 20 * 33
+    if which == "dry":
+        return cases.abl_dry(nx=24, ny=20, nz=32), 8 * (57 * n + 15 * f)
+    if which == "moist":
+        return cases.moist_bubble(nx=24, ny=20, nz=32), 8 * (75 * n + 15 * f)
+    if which == "mixed":
+        case = cases.abl_dry(nx=24, ny=20, nz=32)
+        case.cfg.precision = C.PREC_MIXED
+        return case, 8 * (32 * n + 6 * f) + 4 * (25 * n + 9 * f)
+    if which == "terrain":
+        return T.abl_terrain(nx=64, ny=64, nz=64, dt=0.25, h0=30.0, r0=200.0, amp=2.0), 253505056
+    return T.moving_terrain(substeps=True), 31041904
+
+
+@pytest.mark.parametrize("which", ["dry", "moist", "mixed", "terrain", "moving"])
+def test_memory_of_a_context(which):
+    """The largest grid that fits the card is set by what a context holds."""
+    from erf_b200 import Dycore
+    case, most = _held(which)
+    dy = Dycore(case.cfg)
+    held = dy.scratch_bytes()
+    dy.close()
+    assert held <= most, (held, most)
+
+
 @pytest.mark.parametrize("size,ghost,rain", [((24, 20, 40), 2, True), ((13, 9, 17), 1, True), ((13, 9, 17), 2, False),
                                              ((33, 4, 8), 0, False)])
 def test_kessler_views(size, ghost, rain):
