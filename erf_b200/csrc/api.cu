@@ -954,7 +954,10 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
             const double zl = k * cfg->dz;
             fac[k] = std::pow(1. - zl / ztop, 3.0);
         }
-        if (cudaMemcpy(c->mt.fac, fac.data(), fac.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+        // (on the context's stream, after the zeroing of its memory)
+        if (cudaMemcpyAsync(c->mt.fac, fac.data(), fac.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(c->stream) != cudaSuccess)
             rc = ERF_B200_ECUDA;
         if (rc != ERF_B200_OK) { erf_b200_destroy(c); return rc; }
     }
@@ -1032,7 +1035,7 @@ int erf_b200_get_status(erf_b200_ctx* c) {
     CK(cudaStreamSynchronize(c->stream));
     int h = 0;
     CK(cudaMemcpy(&h, c->status, sizeof(int), cudaMemcpyDeviceToHost));
-    CK(cudaMemset(c->status, 0, sizeof(int)));
+    CK(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     if (h & ST_BOUNDS) return ERF_B200_EBOUNDS;
     if (h & ST_TIMEOUT) return ERF_B200_ETIMEOUT;
     if (h & ST_NAN) return ERF_B200_ENAN;
@@ -1627,7 +1630,7 @@ int erf_b200_closure_fallbacks(erf_b200_ctx* c, unsigned long long* count) {
     CK(cudaStreamSynchronize(c->stream));
     unsigned int h = 0;
     CK(cudaMemcpy(&h, c->fallback, sizeof(h), cudaMemcpyDeviceToHost));
-    CK(cudaMemset(c->fallback, 0, sizeof(h)));
+    CK(cudaMemsetAsync(c->fallback, 0, sizeof(h), c->stream));
     *count = h;
     return ERF_B200_OK;
 }

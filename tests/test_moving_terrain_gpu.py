@@ -240,3 +240,22 @@ def test_deep_mixed_columns(substeps):
     print("deep columns, mixed:", errs)
     w = errs.pop("w")
     assert all(e <= 1e-6 for e in errs.values()) and w <= 1e-4, (errs, w)
+
+
+def test_create_on_a_busy_stream():
+    """A context's arrays are zeroed on its stream, so what erf_b200_create
+    writes into them has to follow on that stream: with work queued there, a
+    copy on another stream came first and the grid's factors were zeroed."""
+    import torch
+    from erf_b200 import Dycore
+    case = T.moving_terrain(nx=12, ny=4, nz=8, Lx=60.0, Ly=20.0, H=40.0, wavelength=30.0, substeps=True, steps=1)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(200_000_000)   # about 0.1 s
+        dy = Dycore(case.cfg, stream=s.cuda_stream)
+        dy.set_base_state(case.base)
+        dy.advance_host(*case.build_state(), 1)
+        _, z, _, _ = dy.moving_terrain_state()
+        dy.close()
+    ref = oracle.advance_moving_terrain(case.cfg, 0.0, case.base, *case.build_state(), 1)
+    assert rel_l2(z, ref[4]) <= 1e-14
