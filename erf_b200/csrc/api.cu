@@ -103,7 +103,7 @@ struct erf_b200_ctx {
         double* zt;
         double *r0o, *p0o;
         double* time;
-        double* detJso;                           // detJ of the last substep's old grid
+        double* dJ[3];                            // and their detJ
         double *wx, *wy;                          // substeps: h_zeta-weighted horizontal momenta
         double* fac;                              // Sullivan's factor per level
     } mt{};
@@ -550,24 +550,27 @@ void enqueue_step_mt(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
             const double beta_s = 0.1;
             const double D = dtau * dtau * (0.5 * (1.0 + beta_s)) * (0.5 * (1.0 + beta_s)) * c->g.dzi;
             double* const* zb = c->mt.z + 3;
+            double* const* dJ = c->mt.dJ;
             cudaStream_t sd = fork ? c->side : st;
             auto geometry = [&](int ks) {
                 launch_mt_grid_sub(Po, sd, c->mt.time, dtau, ks + 1, zb[(ks + 1) % 3]);
-                TIMED(9, launch_mt_coef<R>(Po, sd, c->mt_tx, D, c->mt.r0o, zb[ks % 3], Sst, Acur, B.mc[ks & 1]));
+                launch_mt_detj(Po, sd, zb[(ks + 1) % 3], dJ[(ks + 1) % 3]);
+                TIMED(9, launch_mt_coef<R>(Po, sd, c->mt_tx, D, c->mt.r0o, dJ[ks % 3], Sst, Acur, B.mc[ks & 1]));
                 if (fork) cudaEventRecord(c->ev_geo[ks & 1], sd);
             };
             if (fork) cudaStreamWaitEvent(sd, c->ev_fork, 0);
             launch_mt_grid_sub(Po, sd, c->mt.time, dtau, 0, zb[0]);
+            launch_mt_detj(Po, sd, zb[0], dJ[0]);
             geometry(0);
             if (nsub > 1) geometry(1);
             int lp = 0;
             for (int ks = 0; ks < nsub; ++ks) {
                 if (fork) cudaStreamWaitEvent(st, c->ev_geo[ks & 1], 0);
-                TIMED(6, launch_mt_fast<R>(Po, st, c->mt_tx, ks, c->cfg.no_lagged_delta_rt ? 0 : 1, dtau, beta_s,
+                TIMED(6, launch_mt_fast<R>(Ps, st, c->mt_tx, ks, c->cfg.no_lagged_delta_rt ? 0 : 1, dtau, beta_s,
                                            1.0 / (double)nsub, ks == 0 ? OLD : SUM, Sst, Acur, B.Fcons, B.Fmx, B.Fmy,
                                            B.Fmz, B.lag[lp], B.lag[1 - lp], B.mc[ks & 1], zb[ks % 3],
-                                           zb[(ks + 1) % 3], c->mt.z[1], c->mt.wx, c->mt.wy, B.avx, B.avy, B.avz, SUM,
-                                           ks == nsub - 1 ? 1 : 0));
+                                           zb[(ks + 1) % 3], dJ[ks % 3], dJ[(ks + 1) % 3], c->mt.wx, c->mt.wy, B.avx,
+                                           B.avy, B.avz, SUM, ks == nsub - 1 ? 1 : 0));
                 if (ks + 2 < nsub) {
                     if (fork) {
                         cudaEventRecord(c->ev_sub[ks & 1], st);
@@ -577,12 +580,9 @@ void enqueue_step_mt(erf_b200_ctx* c, Bulk<R>& B, int p, LaunchTimer* T) {
                 }
                 lp ^= 1;
             }
-            double* zso = zb[(nsub - 1) % 3];
-            double* zsn = zb[nsub % 3];
-            launch_mt_detj(Po, st, zso, c->mt.detJso);
-            Pp.znd = zso;
-            Pp.detJ = c->mt.detJso;
-            Pp.mt_znew = zsn;
+            Pp.znd = zb[(nsub - 1) % 3];
+            Pp.detJ = dJ[(nsub - 1) % 3];
+            Pp.mt_znew = zb[nsub % 3];
         }
         TIMED(7, launch_ter_post<R>(Pp, st, c->tkz.ter_post, slow_dt, OLD, Sst, SUM, Snew, Acur, Anext,
                                     nrk < 2 ? 1 : 0, B.mut, B.tke, B.ter, B.avx, B.avy, B.avz, Vnew[0], Vnew[1],
@@ -928,7 +928,8 @@ int erf_b200_create(erf_b200_ctx** out, const erf_b200_config* cfg, void* stream
             A(&c->mt.fac, (size_t)cfg->nz + 1);
             if (cfg->substepping_type == ERF_SUBSTEP_IMPLICIT) {
                 for (int q = 3; q < 6; ++q) A(&c->mt.z[q], (size_t)(cfg->nz + 3) * sk);
-                A(&c->mt.detJso, N); A(&c->mt.wx, N); A(&c->mt.wy, N);
+                for (double*& q : c->mt.dJ) A(&q, N);
+                A(&c->mt.wx, N); A(&c->mt.wy, N);
             }
         }
     }

@@ -259,13 +259,14 @@ struct MtCoef {
 template <class R>
 int mt_shape(const Geo& g, int* tx);
 template <class R>
-void launch_mt_coef(const Params& P, cudaStream_t st, int tx, double D, const double* r0, const double* zo, StateBuf Sst,
+void launch_mt_coef(const Params& P, cudaStream_t st, int tx, double D, const double* r0, const double* dJo, StateBuf Sst,
                     StageAux<R> A, MtCoef<R> c);
 template <class R>
 void launch_mt_fast(const Params& P, cudaStream_t st, int tx, int step, int lagged, double dtau, double beta_s,
                     double facinv, StateBuf Sprev, StateBuf Sst, StageAux<R> A, const R* Fcons, const R* Fmx, const R* Fmy,
                     const R* Fmz, const R* lag_in, R* lag_out, MtCoef<R> c, const double* zo, const double* zn,
-                    const double* zs, double* wx, double* wy, R* avx, R* avy, R* avz, StateBuf Ssum, int last);
+                    const double* dJo, const double* dJn, double* wx, double* wy, R* avx, R* avy, R* avz, StateBuf Ssum,
+                    int last);   // P: the stage grid's; zo, dJo / zn, dJn: nodes and detJ at the substep's old / new time
 void launch_ter_base_state(const Params& P, cudaStream_t st, const double* zcc, const double* th3, const double* qv3,
                            double th_s, double qv_s, double p_s, double* rho0, double* p0, double* pi0, double* th0);
 template <class R>
