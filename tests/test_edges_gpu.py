@@ -6,7 +6,8 @@ divides, views with ghost cells, row tiles of the network.
 
 Bars: FP64 against the oracle, relative L2 <= 1e-10 per field (the bar of the
 parity tests: rounding, amplified by a few steps); the FP32-bulk form against
-the oracle <= 1e-4 (its increments carry 24 bits); the network's BF16 products
+the oracle <= 1e-4 on flat grids (its increments carry 24 bits), over terrain
+the bars stated there; the network's BF16 products
 <= 1e-2 as in test_mlp_gpu."""
 import ctypes
 
@@ -19,6 +20,10 @@ from helpers import compare_states, rel_l2
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-10
+# the mixed form over terrain, two steps: ten times the largest error measured on these planes (w, smallest of
+# the winds, 1.4e-6; v 2.1e-7; u 2.3e-8)
+MIXED_TERRAIN = {"rho": 2.4e-8, "rhotheta": 7.4e-9, "rhoKE": 5.2e-7, "theta": 2.2e-8, "u": 2.3e-7, "v": 2.2e-6,
+                 "w": 1.4e-5}
 
 
 def _advance(case, base, state, steps, precision):
@@ -33,11 +38,18 @@ def _advance(case, base, state, steps, precision):
     return got
 
 
-@pytest.mark.parametrize("size", [(4, 4, 4), (5, 7, 9), (36, 5, 13), (33, 31, 17), (8, 4, 150)])
+def _marches(nx, ny, nz):
+    """Whether the tiled passes take several levels per block: more 32 x 8 tiles x levels than a wave of
+    256-thread blocks (8 fit an SM at most, 148 SMs)."""
+    return -(-nx // 32) * -(-ny // 8) * nz > 8 * 148
+
+
+@pytest.mark.parametrize("size", [(4, 4, 4), (5, 7, 9), (36, 5, 13), (33, 31, 17), (8, 4, 150), (101, 75, 41)])
 @pytest.mark.parametrize("flow,dyc,dry,moist", [("abl", C.UPWIND_5TH, C.UPWIND_5TH, C.WENO_5),
                                                 ("bubble", C.UPWIND_3RD, C.UPWIND_3RD, C.WENO_3)])
 def test_step(size, flow, dyc, dry, moist):
     nx, ny, nz = size
+    assert _marches(nx, ny, nz) == (nx > 100)
     case = cases.abl_dry(nx=nx, ny=ny, nz=nz) if flow == "abl" else cases.moist_bubble(nx=nx, ny=ny, nz=nz)
     c = case.cfg
     if nz > 80:
@@ -56,28 +68,35 @@ def test_step(size, flow, dyc, dry, moist):
         assert not bad, (precision, errs)
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(4, 4, 4), (13, 9, 33), (9, 5, 150)])
-def test_terrain_substeps(nx, ny, nz):
+@pytest.mark.parametrize("nx,ny,nz,dyc", [(4, 4, 4, C.UPWIND_5TH), (13, 9, 33, C.UPWIND_5TH), (9, 5, 150, C.UPWIND_5TH),
+                                           (101, 75, 41, C.UPWIND_5TH), (101, 75, 41, C.UPWIND_3RD)])
+def test_terrain_substeps(nx, ny, nz, dyc):
     from erf_b200 import Dycore
+    assert _marches(nx, ny, nz) == (nx > 100)   # the larger planes run the tiled passes on ragged tiles
     case = T.abl_terrain(nx=nx, ny=ny, nz=nz, dx=25.0, dz0=320.0 / nz, stretch=1.01, h0=30.0, r0=100.0,
                          amp=5.0)
     case.cfg.dt *= min(1.0, 16.0 / nz)
+    case.cfg.dycore_horiz_adv = case.cfg.dycore_vert_adv = dyc
+    ref = None
     for precision in (C.PREC_FP64, C.PREC_MIXED):
         cfg = case.cfg.copy()
         cfg.precision = precision
         dy = Dycore(cfg)
         dy.set_terrain(case.z_nd)
-        base = dy.make_base_state_terrain(case)
+        if ref is None:
+            base = dy.make_base_state_terrain(case)
+            cons, u, v, w = case.build_state(base[0])
+            v = v + 2.0 * np.sin(2.0 * np.pi * np.arange(ny + 1) / ny)[None, :, None]
+            v[:, ny] = v[:, 0]
+            ref = oracle.advance_terrain(case.cfg, case.z_nd, base, cons, u, v, w, 2)
         dy.set_base_state(base)
-        state = case.build_state(base[0])
-        got = dy.advance_host(*state, 2)
+        got = dy.advance_host(cons, u, v, w, 2)
         assert dy.status() == 0
         dy.close()
-        errs = compare_states(got, oracle.advance_terrain(case.cfg, case.z_nd, base, *state, 2))
-        if precision == C.PREC_FP64:
-            assert all(e <= TOL for e in errs.values()), errs
-        else:   # the bars of test_terrain_mixed_form_error
-            assert errs["rho"] < 1e-6 and errs["u"] < 1e-3 and errs["w"] < 1e-2, errs
+        errs = compare_states(got, ref)
+        print("terrain", (nx, ny, nz), dyc, precision, errs)
+        bars = {k: TOL for k in errs} if precision == C.PREC_FP64 else MIXED_TERRAIN
+        assert all(e <= bars[k] for k, e in errs.items()), errs
 
 
 def test_terrain_momentum_accumulates_in_fp64():
@@ -108,11 +127,12 @@ def test_terrain_momentum_accumulates_in_fp64():
         assert np.max(np.abs(vel - want)) <= 1e-13 * abs(want), np.max(np.abs(vel - want))
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(12, 4, 7), (24, 7, 33), (37, 23, 9), (67, 29, 12), (61, 41, 20)])
+@pytest.mark.parametrize("nx,ny,nz", [(12, 4, 7), (24, 7, 33), (37, 23, 9), (67, 29, 12), (61, 41, 20), (101, 75, 32)])
 @pytest.mark.parametrize("precision", [C.PREC_FP64, C.PREC_MIXED])
 def test_moving_terrain_substeps(nx, ny, nz, precision):
     """Column tiles of 2 (the first two planes), 4, 8 and 16 columns, the last
-    tile ragged; a wind that varies in y, and a scalar.  FP64 <= 1e-10; mixed
+    tile ragged, and a plane whose slow passes march ragged x-y tiles; a wind
+    that varies in y, and a scalar.  FP64 <= 1e-10; mixed
     (FP32 tendencies and averages) <= 1e-6, w, the smallest wind, <= 1e-5."""
     case = T.moving_terrain(nx=nx, ny=ny, nz=nz, Lx=5.0 * nx, Ly=5.0 * ny, H=5.0 * nz, ampl=0.05, wavelength=2.5 * nx,
                             substeps=True, dt=0.02)
