@@ -1723,8 +1723,8 @@ int erf_b200_advance_resident(erf_b200_ctx* c, int nsteps) {
 // the resident state.  Every trial recomputes the step from the resident slot
 // (a step reads only that slot's state and velocities and writes the other
 // slots), so the resident state is left unchanged.  Coordinate search over
-// the vertical solver's threads per block, the coefficient kernel's warps and
-// the levels per block of the three tiled transport kernels.
+// the flat substeps' columns and threads per block, their coefficient kernel's
+// threads and the levels per block of the three tiled transport kernels.
 int erf_b200_autotune(erf_b200_ctx* c, int reps, double* best_ms) {
     if (!c || reps < 1) return ERF_B200_EINVAL;
     if (c->cur < 0 || (c->P.les == ERF_LES_MLP && !c->net)) return ERF_B200_EBADSTATE;

@@ -7,7 +7,7 @@
 // substeps; the reference's momentum<->velocity round trips at every boundary
 // fill (BoundaryConditions/ERF_FillIntermediatePatch.cpp:63-67, 224-236) are
 // the identity but for rounding (two divisions and an ulp each) and are not
-// applied.
+// applied (but by k_ter_step_begin, terrain.cu).
 //
 // The dycore kernels are templates on R, the type of the bulk arrays (derived
 // fields, slow right-hand sides, average momenta, fast coefficients, stresses)
@@ -526,8 +526,8 @@ __device__ __forceinline__ R gatherz_most(const Params& P, const MostView& mv, i
 // TimeIntegration/ERF_TI_no_substep_fun.H:6-150, fixed or no terrain):
 // S_sum = S_old + slow_dt * F_slow for rho, rho*theta and the three momenta,
 // accumulated in FP64 from the slow right-hand side (type R).  The boundary
-// fill that follows in the reference (apply_bcs of S_sum) is the first of the
-// two momentum round trips the slow-post kernels apply on read.
+// fill that follows in the reference (apply_bcs of S_sum) changes no valid
+// value but for rounding.
 // ---------------------------------------------------------------------------
 template <class R>
 __global__ void k_no_substep(Geo g, double slow_dt, StateBuf Sold, const R* __restrict__ Fcons,
@@ -722,7 +722,7 @@ void launch_unpack_state(const Geo& g, cudaStream_t st, const StateFabs& f, int 
 }
 
 // ---------------------------------------------------------------------------
-// Tile layout shared by the two vertical kernels below: a block owns TX
+// Tile layout of k_fast_coef below: a block owns TX
 // adjacent columns (i = blockIdx.x*TX + threadIdx.x, j = blockIdx.y) and
 // blockDim.y warps split the levels; per-column data live in shared memory as
 // [level][column] so a warp touches consecutive banks.
@@ -946,7 +946,7 @@ struct PostArgs {
 };
 template <class R, int TH, int TV>
 __device__ __forceinline__ void post_march(const Params& P, const PostArgs<R>& a, FluxTile<R>& sh, Plane<R>& pl, int th,
-                                           int tv, R fh, R fv, int q, int nscal, int nslow, int k0, int k1) {
+                                           int tv, R fh, R fv, int q, int nscal, int k0, int k1) {
     const Geo& g = P.g;
     const int64_t N = g.ncell;
     const uint32_t sk = (uint32_t)g.sk;
@@ -1066,9 +1066,9 @@ __global__ void __launch_bounds__(TTX * TTY, ERFB_MINB_POST) k_post(Params P, in
     const int nslow = nscal + (P.les == ERF_LES_DEARDORFF ? 1 : 0);
     const int q = blockIdx.z % nslow, k0 = blockIdx.z / nslow * kz, k1 = min(k0 + kz, P.g.nz);
     if (q == 0 || q >= nscal)   // scalar and KE: dry-scalar schemes
-        post_march<R, DH, DV>(P, a, sh, pl, P.dry_h, P.dry_v, R(P.f_dry_h), R(P.f_dry_v), q, nscal, nslow, k0, k1);
+        post_march<R, DH, DV>(P, a, sh, pl, P.dry_h, P.dry_v, R(P.f_dry_h), R(P.f_dry_v), q, nscal, k0, k1);
     else
-        post_march<R, MH, MV>(P, a, sh, pl, P.moi_h, P.moi_v, R(P.f_moi_h), R(P.f_moi_v), q, nscal, nslow, k0, k1);
+        post_march<R, MH, MV>(P, a, sh, pl, P.moi_h, P.moi_v, R(P.f_moi_h), R(P.f_moi_v), q, nscal, k0, k1);
 }
 
 // Momentum fluxes of AdvectionSrcFor{X,Y,Z}Mom_N (ERF_AdvectionSrcForMom_N.H:
@@ -1424,7 +1424,6 @@ using PostK = void (*)(Params, int, PostArgs<R>);
 template <class R>
 SlowCellK<R> slow_cell_kernel(const Params& P) {
     if (P.dyc_h == U5 && P.dyc_v == U5) return k_slow_cell<R, U5, U5>;
-    if (P.dyc_h == W5 && P.dyc_v == W5) return k_slow_cell<R, W5, W5>;
     if (P.dyc_h == U3 && P.dyc_v == U3) return k_slow_cell<R, U3, U3>;
     return k_slow_cell<R, -1, -1>;
 }

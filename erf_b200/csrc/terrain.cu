@@ -21,8 +21,8 @@
 //   k_ter_slow_mom    AdvectionSrcForMom_T, DiffusionSrcForMom_T, terrain
 //                     pressure gradient, sources
 //   (ter_fast.cu)     erf_fast_rhs_T (TimeIntegration/ERF_fast_rhs_T.cpp)
-//   k_ter_post        erf_slow_rhs_post with terrain and the stage's
-//                     boundary round trips
+//   k_ter_post        erf_slow_rhs_post with terrain, the stage's velocities
+//                     and w on the ground and the lid
 #include <cfloat>
 
 #include "terrain.cuh"
@@ -553,8 +553,8 @@ __device__ __forceinline__ void stage_aux_ter(const Params& P, const double* __r
 
 // ---------------------------------------------------------------------------
 // Step prologue with terrain.  The old velocities give the momenta through
-// the V -> M -> V -> M round trip of apply_bcs(state_old) (as without
-// terrain); w on the ground and on the lid is WFromOmega(Omega = 0) of the
+// the V -> M -> V -> M round trip of apply_bcs(state_old) (the one pass that
+// applies it; it is the identity but for rounding); w on the ground and on the lid is WFromOmega(Omega = 0) of the
 // round-tripped u, v (ERF_BoundaryConditions_zvel.cpp:200-262).  The eddy
 // viscosity uses the input velocities with w from the same condition, the
 // terrain strain and a local filter width (dz / h_zeta;
@@ -1063,9 +1063,14 @@ __global__ void __launch_bounds__(TTX * TTY, TER_MINB_SLOW_CELL) k_ter_slow_cell
 }
 
 // The same with one thread per cell, for planes so small that a tile's chunk
-// is one level: there nothing is carried, the chip is not filled, and the
-// tiles' barriers only lengthen the call (moving terrain 40x8x79: 12 against
-// 25 us).
+// is one level (pick_kz: every level of every tile in one wave): there nothing
+// is carried, the chip is not filled, and the tiles' barriers only lengthen the
+// call.  From two levels on the tiles win.  us, one thread per cell / tiles,
+// FP64, static terrain: 24x16x24 15.8 / 17.1 (one level), 40x24x80 26.7 / 25.2,
+// 60x30x60 29.4 / 27.6 (two levels), 64x64x64 48.7 / 39.7, 101x75x41 65.5 / 49.6,
+// 128x128x48 117 / 87, 200x100x96 312 / 223, 256x256x96 869 / 578; moving
+// terrain: 40x8x79 11.3 / 13.1 (one level), 100x30x33 17.5 / 18.3 (two levels),
+// 96x48x79 40 / 34, 512x128x79 489 / 333.
 template <class R, int HT, int VT>
 __global__ void __launch_bounds__(128, 4) k_ter_slow_cell_small(Params P, StateBuf S, StageAux<R> A, const double* __restrict__ u,
                                 const double* __restrict__ v, const R* __restrict__ mut, TkeBuf<R> tke, TerBuf<R> T,
