@@ -128,7 +128,7 @@ def test_create_refuses_arrays_of_4_gb(lib, nx, ny, nz, ter):
     state's planes) is past the kernels' 32-bit offsets: refused as out of
     memory before any CUDA call, on a card of any size."""
     c = C.defaults()
-    c.nx, c.ny, c.nz, c.use_terrain = nx, ny, nz, ter
+    c.nx, c.ny, c.nz, c.use_terrain, c.molec_diff_type = nx, ny, nz, ter, C.MOLEC_NONE
     c.dycore_horiz_adv = c.dycore_vert_adv = C.UPWIND_5TH
     ctx = ctypes.c_void_p()
     lib.erf_b200_create.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_void_p, ctypes.c_void_p]
