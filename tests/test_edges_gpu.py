@@ -104,7 +104,8 @@ def test_terrain_momentum_accumulates_in_fp64():
     the force acts, so a step adds dt F to the momenta whatever the number of
     substeps.  The mixed form stores F in FP32 but accumulates the state in
     FP64: each of the ~150 substeps rounds to 2^-53 of a momentum of the size
-    of dt F (bar 1e-13 of the velocity), where 24 bits would leave 1e-9."""
+    of dt F (bar 1e-13 of the velocity); increments carried in 24 bits left
+    1.7e-7."""
     from erf_b200 import Dycore
     nx, ny, nz = 8, 6, 8
     cfg = T.abl_terrain(nx=nx, ny=ny, nz=nz, les="smagorinsky").cfg

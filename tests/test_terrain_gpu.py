@@ -78,13 +78,15 @@ def test_terrain_parity_slip_ground_upwind3():
 
 
 def test_terrain_mixed_form_error():
-    """FP32 bulk over terrain stays close to the FP64 oracle (10 steps)."""
+    """FP32 bulk over terrain stays close to the FP64 oracle (10 steps): ten
+    times the errors measured (rho 4.5e-9, u 3.9e-8, v 4.9e-7, w 2.6e-7)."""
     case = _hill()
     base, init, got, st = _gpu_run(case, 10, precision=C.PREC_MIXED)
     assert st == 0
     ref = oracle.advance_terrain(case.cfg, case.z_nd, base, *init, 10)
     errs = compare_states(got, ref)
-    assert errs["rho"] < 1e-6 and errs["u"] < 1e-3 and errs["w"] < 1e-2, errs
+    bars = {"rho": 5e-8, "rhotheta": 1.5e-8, "rhoKE": 4e-7, "theta": 5e-8, "u": 4e-7, "v": 5e-6, "w": 3e-6}
+    assert all(e <= bars[k] for k, e in errs.items()), errs
 
 
 def test_flat_terrain_matches_flat_grid():
