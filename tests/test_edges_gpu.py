@@ -135,6 +135,7 @@ def test_moving_terrain_substeps(nx, ny, nz, precision):
     tile ragged, and a plane whose slow passes march ragged x-y tiles; a wind
     that varies in y, and a scalar.  FP64 <= 1e-10; mixed
     (FP32 tendencies and averages) <= 1e-6, w, the smallest wind, <= 1e-5."""
+    assert _marches(nx, ny, nz) == (nx > 100)
     case = T.moving_terrain(nx=nx, ny=ny, nz=nz, Lx=5.0 * nx, Ly=5.0 * ny, H=5.0 * nz, ampl=0.05, wavelength=2.5 * nx,
                             substeps=True, dt=0.02)
     case.cfg.mri_ratio = 6
